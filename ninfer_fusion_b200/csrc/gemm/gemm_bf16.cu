@@ -1350,29 +1350,14 @@ int gemm_pick_splits(int T, int N, int K, int epi, int sm_count) {
 
 namespace {
 
-// 65 to 256 tokens and few tiles of weight rows: a tile that holds all tokens leaves most SMs idle (N = 2048: 16 CTAs walk
-// the whole contraction, 28 us at K = 4096, T = 128 for 17 MB of weights).  Narrower token tiles, and the contraction cut
-// inside clusters where SMs are left, put them to work; the weights are then read once from HBM and again from L2.  Takes
-// the cheapest of the one-wave plans by the times of a k-block, of the exchange inside a cluster and of the epilogue.
-void narrow_plan(int T, int w_tiles, int num_kb, int epi, int* tn_out, int* splits_out) {
-  const int sms = device_sm_count();
-  const auto kb_ns = [](int tn) { return 211. + 0.55 * tn; };
-  const int wide = T <= 128 ? 128 : persist_tile_tokens(T, w_tiles, num_kb, sms);
-  const long long wide_tiles = static_cast<long long>(w_tiles) * ((T + wide - 1) / wide);
-  double best = static_cast<double>((wide_tiles + sms - 1) / sms) * num_kb * kb_ns(wide) + 60. * wide;
-  for (int tn = 64; tn >= 32; tn /= 2) {
-    const int tiles = w_tiles * ((T + tn - 1) / tn);
-    if (tiles > sms) continue;
-    int cap = gemm_max_cluster(tn);
-    if (epi != kEpiSwiglu && deep_enabled()) cap = tn == 64 ? 6 : 8;
-    for (int s = 1; s <= cap && tiles * s <= sms; ++s) {
-      const int per = (num_kb + s - 1) / s;
-      if (s > 1 && (per < 8 || (num_kb + per - 1) / per != s)) continue;
-      if (s > 1 && max_active_clusters(tn, epi, use_deep(tn, static_cast<long long>(tiles) * s), s) < tiles) continue;
-      const double ns = per * kb_ns(tn) + (s > 1 ? 1500. + 10. * (s - 1) * tn : 0.) + 60. * tn;
-      if (ns < 0.95 * best) { best = ns; *tn_out = tn; *splits_out = s; }
-    }
-  }
+// Tokens per tile for 65 to 256 tokens.  With few tiles of weight rows a tile that holds all tokens leaves most SMs idle
+// (N = 2048: 16 CTAs walk the whole contraction), so the narrower of 32 and 64 whose tiles all run at once is taken: a k-block
+// of a narrower tile takes less time (persist_kblock_ns), its epilogue too, and the weights are read once from HBM and again
+// from L2.  The contraction is not cut: a row's sums keep one order whatever the number of rows beside it.
+int narrow_tile(int T, int w_tiles, int tn) {
+  for (int n = 32; n <= 64; n *= 2)
+    if (static_cast<long long>(w_tiles) * ((T + n - 1) / n) <= device_sm_count()) return n;
+  return tn;
 }
 
 }  // namespace
@@ -1403,7 +1388,7 @@ const char* gemm_bf16(const GemmArgs& a) {
   int splits = a.splits < 1 ? 1 : a.splits;
   if (splits > kp.num_kb) splits = kp.num_kb;
   if (splits != (a.splits < 1 ? 1 : a.splits)) return "gemm_bf16: split count leaves an empty split";
-  if (splits == 1 && plain && tn >= 128 && kp.T <= 256 && !g_trace_enabled) narrow_plan(kp.T, w_tiles, kp.num_kb, a.epi, &tn, &splits);
+  if (splits == 1 && plain && tn >= 128 && kp.T <= 256) tn = narrow_tile(kp.T, w_tiles, tn);
   kp.kb_per_split = (kp.num_kb + splits - 1) / splits;
   if ((kp.num_kb + kp.kb_per_split - 1) / kp.kb_per_split != splits) return "gemm_bf16: split count leaves an empty split";
   kp.cluster = 1;

@@ -181,8 +181,8 @@ def test_gemm_persistent_prefill_kernel(ops, status, T):
 @pytest.mark.parametrize("T", [65, 128, 129, 160, 256, 257, 300, 1873])
 @pytest.mark.parametrize("N,K", [(264, 2048), (2048, 520), (2048, 4096), (5120, 128)])
 def test_gemm_token_tiles(ops, status, T, N, K):
-    """Sizes whose token tile depends on the other sizes (few or many weight tiles, last rounds): narrow tiles with and
-    without in-cluster split-K, persistent tiles of 64 to 256 tokens, each epilogue, ragged last tiles."""
+    """Sizes whose token tile depends on the other sizes (few or many weight tiles, last rounds): narrow tiles,
+    persistent tiles of 64 to 256 tokens, each epilogue, ragged last tiles."""
     x, w = _mk(T, N, K, seed=4)
     ref = x.float() @ w.float().t()
     out = torch.full((T + 1, N), float("nan"), device="cuda", dtype=torch.bfloat16)
@@ -202,6 +202,23 @@ def test_gemm_token_tiles(ops, status, T, N, K):
         assert (act[:T].float() - want).abs().max() <= want.abs().max() * 2.0 ** -7
         assert act[T].isnan().all()
     status.check("token tiles")
+
+
+@pytest.mark.parametrize("T", [65, 100, 128, 129, 160, 256])
+@pytest.mark.parametrize("N,K", [(264, 2048), (2048, 520), (2048, 4096), (5120, 1024)])
+def test_gemm_rows_keep_their_bits(ops, status, T, N, K):
+    """Without a split that the caller asked for, a row's sums run over the contraction in one order: the row has the same bits
+    whatever the number of rows beside it, and with it the token tile."""
+    x, w = _mk(400, N, K, seed=6)
+    resid = torch.randn(400, N, device="cuda").to(torch.bfloat16)
+
+    def run(rows, epi):
+        out = resid[:rows].clone() if epi == EPI_RESIDUAL else torch.empty((rows, N // (2 if epi == EPI_SWIGLU else 1)), device="cuda", dtype=torch.bfloat16)
+        ops.gemm_bf16(x[:rows], w, out, epi, out if epi == EPI_RESIDUAL else None, None, None, 1, status.tensor, False)
+        return out
+    for epi in (EPI_STORE, EPI_RESIDUAL, EPI_SWIGLU):
+        assert torch.equal(run(T, epi), run(400, epi)[:T]), epi
+    status.check("rows")
 
 
 @pytest.mark.parametrize("T", [1, 16, 17, 33, 64])
