@@ -16,9 +16,10 @@
 //   12      issues the products: S of tile i + 1 goes in front of P V of tile i, so that the softmax of one tile runs beside
 //           the products of its neighbours
 // The row scales of fp8 pages never touch the operands: the K scale multiplies a key's column of S, the V scale its
-// probability.  A row's exponentials are taken against a frame that only moves when the maximum has outgrown it by
-// kFrameSlack (then O is rescaled in TMEM): nearly always once, at the first tile.  K / V of the chunk itself were appended
-// by attn_prep before this kernel runs, so the key loop covers [first visible key, last visible key] with a limit per row.
+// probability.  A row's exponentials are taken against its largest score so far, so that no probability exceeds one (times an
+// fp8 V scale: at most 65504, fp16's largest); O is rescaled in TMEM by the warps that have a row whose maximum has grown.  K /
+// V of the chunk itself were appended by attn_prep before this kernel runs, so the key loop covers [first visible key, last
+// visible key] with a limit per row.
 //
 // TMEM is full (two S buffers of 64 columns, Q 128, O 256).  Q lies there and not in shared memory because the gathers need
 // the room: with Q and 128-key K and V tiles in shared memory (192 KB) 28 KB of L1 were left, which bound the loads in flight
@@ -54,9 +55,6 @@ constexpr int kStagePitch = 2 * D + 16;      // bytes per row of the output tile
 constexpr uint32_t kColQ = 128, kColO = 256; // TMEM: S / P of even tiles at 0, of odd tiles at 64, then Q and O
 constexpr uint32_t kIdescS = umma_idesc(128, kKeys, 0, 0);
 constexpr uint32_t kIdescPV = umma_idesc(128, D, 0, 0) | (1u << 16);   // B (= V) is MN-major
-// log2 units a score may exceed its row's frame: p <= 16.  Tiles with a V scale above kBigScale take no slack, so that
-// p x scale stays within fp16 whatever the scale.
-constexpr float kFrameSlack = 4.f, kBigScale = 1024.f;
 enum : int { kStatusPrefillWait = 6 };
 
 struct Bars {
@@ -117,18 +115,6 @@ __device__ __forceinline__ float ex2(float x) {
   return y;
 }
 __device__ __forceinline__ void group_bar(int id) { asm volatile("bar.sync %0, 128;" ::"r"(id) : "memory"); }
-// barrier of the softmax threads that also ORs a predicate over them
-__device__ __forceinline__ bool softmax_any(bool v) {
-  uint32_t r;
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\t"
-      "setp.ne.u32 q, %1, 0;\n\t"
-      "bar.red.or.pred p, 1, 128, q;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}\n"
-      : "=r"(r) : "r"(static_cast<uint32_t>(v)) : "memory");
-  return r != 0;
-}
-
 // 16 bytes of a bf16 row: rows at any even element address are accepted, 16-byte accesses are used where all of them are aligned
 __device__ __forceinline__ uint4 load_row16(const __nv_bfloat16* src, bool wide) {
   if (wide) return *reinterpret_cast<const uint4*>(src);
@@ -406,17 +392,18 @@ __global__ void __launch_bounds__(kThreads, 1) paged_attn_prefill_kernel(const P
       fetch_scale(0);
       fetch_page(1);
     }
-    float frame = -CUDART_INF_F, l = 0.f;
+    float top = -CUDART_INF_F;   // the row's largest score so far
+    // The row sum in four parts, by pairs of keys: a row's parts are summed in key order whatever the block it is in.
+    float l4[4] = {0.f, 0.f, 0.f, 0.f};
     for (int i = 0; i < n_tiles; ++i) {
       const int b = i & 1, kb = k_first + i * kKeys;
-      float slack = kFrameSlack;
       const float* ks = scale_s[b][0];
       const float* vs = scale_s[b][1];
       if constexpr (kScaled) {
         const float value = FORMAT == kKvFp8Row ? __half2float(__ushort_as_half(static_cast<unsigned short>(scale_raw))) : __uint_as_float(scale_raw);
         const float scale = scale_live ? value : 0.f;
         scale_s[b][sv][skey] = scale;
-        if (softmax_any(sv == 1 && scale > kBigScale)) slack = 0.f;
+        group_bar(1);
         fetch_scale(i + 1);
         fetch_page(i + 2);
       }
@@ -451,11 +438,10 @@ __global__ void __launch_bounds__(kThreads, 1) paged_attn_prefill_kernel(const P
 #pragma unroll
       for (int j = 4; j < kKeys; ++j) m4[j & 3] = fmaxf(m4[j & 3], __uint_as_float(v[j]));
       const float mx = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3]));
-      const bool move = mx > frame + slack;
+      const bool move = mx > top;
+      const float corr = move ? ex2(top - mx) : 1.f;   // (a row's first keys: exp2(-inf) = 0)
       if (__any_sync(0xffffffffu, move)) {
-        const float corr = move ? ex2(frame - mx) : 1.f;   // (a row's first frame: exp2(-inf) = 0)
-        if (move) frame = mx;
-        l *= corr;
+        if (move) top = mx;
         if (i > 0) {
           mbar_wait(smem_u32(&bars.v_empty[b ^ 1]), ((i - 1) >> 1) & 1, abortp, p.status, kStatusPrefillWait);
           __syncwarp();
@@ -471,8 +457,7 @@ __global__ void __launch_bounds__(kThreads, 1) paged_attn_prefill_kernel(const P
           }
         }
       }
-      const float at = frame == -CUDART_INF_F ? 0.f : frame;   // (a row that has seen no key yet)
-      float l4[4] = {0.f, 0.f, 0.f, 0.f};
+      const float at = top == -CUDART_INF_F ? 0.f : top;   // (a row that has seen no key yet)
       uint32_t pk[kKeys / 4];
 #pragma unroll
       for (int j = 0; j < kKeys; j += 4) {
@@ -480,7 +465,8 @@ __global__ void __launch_bounds__(kThreads, 1) paged_attn_prefill_kernel(const P
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
           e[q] = ex2(__uint_as_float(v[j + q]) - at);
-          l4[q] += e[q];
+          float& part = l4[((j + q) >> 1) & 3];
+          part = j + q < 8 && (q & 1) == 0 ? fmaf(part, corr, e[q]) : part + e[q];   // (a part's first key of the tile)
         }
         if constexpr (kScaled) {
           const float4 v4 = *reinterpret_cast<const float4*>(vs + j);
@@ -492,7 +478,6 @@ __global__ void __launch_bounds__(kThreads, 1) paged_attn_prefill_kernel(const P
         if (j == kKeys / 2 - 4) tmem_st_x16(s_addr, pk);
         if (j == kKeys - 4) tmem_st_x16(s_addr + 16, pk);
       }
-      l += (l4[0] + l4[1]) + (l4[2] + l4[3]);
       tmem_st_wait();
       tc_fence_before();
       __syncwarp();
@@ -503,6 +488,7 @@ __global__ void __launch_bounds__(kThreads, 1) paged_attn_prefill_kernel(const P
       mbar_wait(smem_u32(&bars.o_done), 0, abortp, p.status, kStatusPrefillWait);
       tc_fence_after();
     }
+    const float l = (l4[0] + l4[1]) + (l4[2] + l4[3]);
     const float inv = l > 0.f ? 1.f / l : 0.f;
 #pragma unroll 1
     for (int c = 0; c < D; c += 32) {

@@ -432,6 +432,28 @@ def test_prefill_attention_tile_edges(ops, status, name, fmt, group, hq, hkv, n,
     status.check("prefill attention")
 
 
+def test_prefill_attention_largest_key_weighs_one(ops, status):
+    """The 64 keys of the first tile score 0, one key of the second 2.03125 (in powers of two): that key's probability against
+    the row's largest score is one, exactly, so outputs are its value times an fp32 factor.  Against the first tile's frame it
+    would be 2^2.03125, which fp16 holds 4e-4 too small: every fourth output would round the other way."""
+    H, D, P, n = 8, 256, 64, 128
+    table = torch.arange(2).int().view(1, 2).cuda()
+    k, v, _, _ = _planes(2, H, P, D, R.KV_BF16, 256)
+    k.view(torch.bfloat16)[1, :, 0, 0] = 2.03125
+    val = torch.randn(H, D, generator=torch.Generator().manual_seed(2)).to(torch.bfloat16)
+    v.view(torch.bfloat16)[1, :, 0] = val.cuda()
+    q = torch.zeros((1, H, D), dtype=torch.bfloat16, device="cuda")
+    q[:, :, 0] = 1.0
+    out = torch.empty((1, H * D), dtype=torch.bfloat16, device="cuda")
+    one = torch.ones(1, dtype=torch.int32, device="cuda")
+    ops.paged_attention_prefill(q, H, H, D, 0 * one, n * one, 0 * one, one, table, k, v, None, None, P, R.KV_BF16, 256,
+                                1 / 1.4426950408889634, None, out, False, 0, None, status.tensor)
+    want = (val.double() / (1 + 127 * 2.0 ** -2.03125)).to(torch.bfloat16).view(1, -1)
+    # a handful of fp32 roundings (1e-6 of a value) moves an output across a bf16 tie in one of some 4000 cases
+    assert (out.cpu() != want).sum() <= 4
+    status.check("largest key")
+
+
 def test_stochastic_draft_verification_preserves_the_target_distribution(ops):
     """Deterministic drafts verified by speculative sampling: accept w.p. p(draft), else draw from p without the
     draft.  Over many seeds the emitted token must follow p itself and the acceptance rate must be p(draft)."""
