@@ -154,28 +154,34 @@ __global__ void __launch_bounds__(128, 3) gdn_chunk_prepare_kernel(const ChunkPa
   cp_async_wait<0>();
   __syncthreads();
 
-  // ---- row norms (two threads per row, every other 16 bytes), inclusive scan of the log decays (warp 0) ----
-  {
-    const int r = tid >> 1;
-    float sk = 0.f, sq = 0.f;
+  // ---- row norms (16 rows per warp, four at a time), inclusive scan of the log decays (warp 0) ----
+#pragma unroll 1
+  for (int r0 = warp * 16; r0 < warp * 16 + 16; r0 += 4) {
+    float sk[4], sq[4];
 #pragma unroll
-    for (int i = 0; i < kD / 16; ++i) {
-      const int c = (2 * i + (tid & 1)) * 8;
-      const uint4 kw = *reinterpret_cast<const uint4*>(&sm.k[r][c]), qw = *reinterpret_cast<const uint4*>(&sm.q[r][c]);
+    for (int m = 0; m < 4; ++m) {
+      const uint2 kw = *reinterpret_cast<const uint2*>(&sm.k[r0 + m][lane * 4]), qw = *reinterpret_cast<const uint2*>(&sm.q[r0 + m][lane * 4]);
       const __nv_bfloat162* k2 = reinterpret_cast<const __nv_bfloat162*>(&kw);
       const __nv_bfloat162* q2 = reinterpret_cast<const __nv_bfloat162*>(&qw);
+      sk[m] = sq[m] = 0.f;
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
+      for (int e = 0; e < 2; ++e) {
         const float2 kf = __bfloat1622float2(k2[e]), qf = __bfloat1622float2(q2[e]);
-        sk += kf.x * kf.x + kf.y * kf.y;
-        sq += qf.x * qf.x + qf.y * qf.y;
+        sk[m] = fmaf(kf.y, kf.y, fmaf(kf.x, kf.x, sk[m]));
+        sq[m] = fmaf(qf.y, qf.y, fmaf(qf.x, qf.x, sq[m]));
       }
     }
-    sk += __shfl_xor_sync(0xffffffffu, sk, 1);
-    sq += __shfl_xor_sync(0xffffffffu, sq, 1);
-    if ((tid & 1) == 0) {
-      sm.rk[r] = rsqrtf(sk + 1e-6f);
-      sm.rq[r] = rsqrtf(sq + 1e-6f);
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+      sk[m] = warp_sum(sk[m]);
+      sq[m] = warp_sum(sq[m]);
+    }
+    if (lane == 0) {
+#pragma unroll
+      for (int m = 0; m < 4; ++m) {
+        sm.rk[r0 + m] = rsqrtf(sk[m] + 1e-6f);
+        sm.rq[r0 + m] = rsqrtf(sq[m] + 1e-6f);
+      }
     }
   }
   if (warp == 0) {
@@ -241,23 +247,31 @@ __global__ void __launch_bounds__(128, 3) gdn_chunk_prepare_kernel(const ChunkPa
   }
   __syncthreads();
 
-  // ---- X = (I + A)^-1 by halves: X = [X1 0; X21 X2] with X21 = -X2 A21 X1.  Warps 0 and 1 invert the diagonal halves
-  //      (lane c owns column c, forward substitution in registers, the result over A's half); the other two scale the
-  //      right-hand sides meanwhile ----
+  // ---- X = (I + A)^-1 by forward substitution, each entry's terms in the order of its row (four running sums, by column mod
+  //      4).  Columns 0..31: warp 0 takes rows 0..31; then all warps take the terms of rows 32..63 with those; then warp 0 the
+  //      rest of rows 32..63.  Columns 32..63 start at row 32 and are warp 1's meanwhile.  Lane c owns a column; the other two
+  //      warps scale the right-hand sides ----
   constexpr int kH = kC / 2;
-  if (warp < 2) {
-    const int o = warp * kH;
-    float x[kH];
+  auto substitute = [&](int o, const float4* start, float* x) {   // rows o .. o + 31 and as many columns of A
 #pragma unroll
     for (int i = 0; i < kH; ++i) {
       float acc[4] = {i == lane ? 1.f : 0.f, 0.f, 0.f, 0.f};
+      if (start != nullptr) {
+        const float4 s = start[i * kH + lane];
+        acc[0] = s.x; acc[1] = s.y; acc[2] = s.z; acc[3] = s.w;
+      }
 #pragma unroll
       for (int j = 0; j < i; ++j) acc[j & 3] -= sm.a[o + i][o + j] * x[j];
       x[i] = (acc[0] + acc[1]) + (acc[2] + acc[3]);
     }
-    __syncwarp();
+  };
+  float x[kH];   // warps 0 and 1: rows of this lane's column in the diagonal half
+  if (warp < 2) {
+    substitute(warp * kH, nullptr, x);
+    if (warp == 0) {   // (above the diagonal half: read below by all warps)
 #pragma unroll
-    for (int i = 0; i < kH; ++i) sm.a[o + i][o + lane] = x[i];
+      for (int i = 0; i < kH; ++i) sm.a[i][kH + lane] = x[i];
+    }
   } else {
     for (int i = tid - kC; i < kC * (kD / 2); i += blockDim.x - kC) {
       const int r = i / (kD / 2), c2 = (i % (kD / 2)) * 2;
@@ -269,48 +283,52 @@ __global__ void __launch_bounds__(128, 3) gdn_chunk_prepare_kernel(const ChunkPa
     }
   }
   __syncthreads();
+  float4* const sums = reinterpret_cast<float4*>(sm.k);   // [32 rows][32 columns] of four running sums, over the raw k rows
+  static_assert(sizeof(float4) * kH * kH <= sizeof(sm.k), "the running sums lie over the k rows");
   {
-    // rows 8 warp .. + 7 and column `lane` of the 32 x 32 products A21 X1 (kept above the diagonal) and X2 (A21 X1)
-    const int m0 = warp * 8;
-    float t[8], x21[8];
-    auto product = [&](int ra, int ca, int rb, int cb, float* out) {
+    const int m0 = warp * 8;   // rows 32 + m0 .. + 7 and column `lane`
+    float acc[8][4];
 #pragma unroll
-      for (int m = 0; m < 8; ++m) out[m] = 0.f;
+    for (int m = 0; m < 8; ++m)
 #pragma unroll
-      for (int k = 0; k < kH; k += 4) {
-        float bcol[4];
+      for (int e = 0; e < 4; ++e) acc[m][e] = 0.f;
 #pragma unroll
-        for (int e = 0; e < 4; ++e) bcol[e] = sm.a[rb + k + e][cb + lane];
+    for (int j = 0; j < kH; j += 4) {
+      float xc[4];
 #pragma unroll
-        for (int m = 0; m < 8; ++m) {
-          const float4 r = *reinterpret_cast<const float4*>(&sm.a[ra + m0 + m][ca + k]);
-          out[m] += (r.x * bcol[0] + r.y * bcol[1]) + (r.z * bcol[2] + r.w * bcol[3]);
-        }
+      for (int e = 0; e < 4; ++e) xc[e] = sm.a[j + e][kH + lane];
+#pragma unroll
+      for (int m = 0; m < 8; ++m) {
+        const float4 r = *reinterpret_cast<const float4*>(&sm.a[kH + m0 + m][j]);
+        acc[m][0] -= r.x * xc[0];
+        acc[m][1] -= r.y * xc[1];
+        acc[m][2] -= r.z * xc[2];
+        acc[m][3] -= r.w * xc[3];
       }
-    };
-    product(kH, 0, 0, 0, t);
-#pragma unroll
-    for (int m = 0; m < 8; ++m) sm.a[m0 + m][kH + lane] = t[m];
-    __syncthreads();
-    product(kH, kH, 0, kH, x21);
-    float x1[8], x2[8];
-#pragma unroll
-    for (int m = 0; m < 8; ++m) {
-      x1[m] = sm.a[m0 + m][lane];
-      x2[m] = sm.a[kH + m0 + m][kH + lane];
     }
-    __syncthreads();
-    auto put = [&](int i, int c, float x) {
-      const __nv_bfloat16 hi = __float2bfloat16(x);
+#pragma unroll
+    for (int m = 0; m < 8; ++m) sums[(m0 + m) * kH + lane] = make_float4(acc[m][0], acc[m][1], acc[m][2], acc[m][3]);
+  }
+  __syncthreads();
+  float x21[kH];
+  if (warp == 0) substitute(kH, sums, x21);
+  __syncthreads();   // (the bf16 pair lies over A)
+  {
+    auto put = [&](int i, int c, float v) {
+      const __nv_bfloat16 hi = __float2bfloat16(v);
       sm.xh[i][c] = hi;
-      sm.xl[i][c] = __float2bfloat16(x - __bfloat162float(hi));
+      sm.xl[i][c] = __float2bfloat16(v - __bfloat162float(hi));
     };
     // (the products below never read above the diagonal half)
+    if (warp == 0) {
 #pragma unroll
-    for (int m = 0; m < 8; ++m) {
-      put(m0 + m, lane, x1[m]);
-      put(kH + m0 + m, kH + lane, x2[m]);
-      put(kH + m0 + m, lane, -x21[m]);
+      for (int i = 0; i < kH; ++i) {
+        put(i, lane, x[i]);
+        put(kH + i, lane, x21[i]);
+      }
+    } else if (warp == 1) {
+#pragma unroll
+      for (int i = 0; i < kH; ++i) put(kH + i, kH + lane, x[i]);
     }
   }
   __syncthreads();

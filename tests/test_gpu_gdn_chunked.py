@@ -1,4 +1,6 @@
 """Chunked (WY) tensor-core gated delta rule against the fp32 token-by-token oracle and the recurrent kernel."""
+import hashlib
+
 import pytest
 import torch
 
@@ -73,3 +75,28 @@ def test_gdn_chunked_matches_oracle(ops, lens, heads):
     assert worst_s < 1e-2, worst_s
     for s_ in [s for s in range(n_slots) if s not in slots]:
         assert torch.equal(ssm_c[s_].cpu(), ssm[s_])
+
+
+@pytest.mark.parametrize("heads,lens,digest", [
+    ((16, 32), [300, 40], "4057cf1b77dfa7bb"), ((16, 48), [256], "b9c98feedeeefb66"), ((2, 6), [129, 64, 1], "4dfad92842017fbe")])
+def test_gdn_chunked_keeps_its_bits(ops, heads, lens, digest):
+    """A last bit of a state that moves is another expert in a router further on, so the order of every sum is part of the
+    kernel's contract: norms, inverse and products of fixed inputs give the bits that they gave when this was recorded."""
+    (hk, hv), d = heads, 128
+    qk, vd = hk * d, hv * d
+    C, T, B = 2 * qk + vd, sum(lens), len(lens)
+    ld = (C + vd + 2 * hv + 7) // 8 * 8
+    g = torch.Generator().manual_seed(3)
+
+    def mk(shape, top):   # (integers: the same on every CPU)
+        return torch.randint(-32768, 32769, shape, generator=g).float() * (top * 2.0 ** -15)
+    proj, conv = mk((T, ld), 1.5).bfloat16().cuda(), mk((T, C), 1.5).bfloat16().cuda()
+    A_log, dt_bias, nw = mk((hv,), 2.0).cuda(), mk((hv,), 2.0).cuda() - 1.0, 1 + mk((d,), 0.2).bfloat16().cuda()
+    ssm = mk((4, hv, d, d), 0.2).cuda()
+    cu = torch.tensor([0] + list(torch.tensor(lens).cumsum(0)), dtype=torch.int32).cuda()
+    ws = torch.empty(int(ops.gdn_chunked_workspace_bytes(T, B, hv)), dtype=torch.uint8, device="cuda")
+    out = torch.empty((T, vd), dtype=torch.bfloat16, device="cuda")
+    ops.gdn_recurrent(conv, 0, qk, 2 * qk, proj, C, C + vd, C + vd + hv, hk, hv, A_log, dt_bias, nw, 1e-6, cu,
+                      torch.tensor([3, 0, 2][:B]).int().cuda(), ssm, True, out, False, None, None, ws)
+    bits = out.cpu().view(torch.uint8).numpy().tobytes() + ssm.cpu().numpy().tobytes()
+    assert hashlib.sha256(bits).hexdigest()[:16] == digest
