@@ -227,7 +227,10 @@ __global__ void __launch_bounds__(kThreads, 1) paged_attn_prefill_kernel(const P
       bool ok = n_tiles > 0 && mbar_wait(smem_u32(&bars.p_full[1]), 0, abortp, p.status, kStatusPrefillWait) && scores(0);
       for (int i = 0; i < n_tiles && ok; ++i) {
         const int b = i & 1;
-        // (the buffer of S(i + 1) held P(i - 1): its product was issued before and products retire in order)
+        // The buffer of S(i + 1) holds P(i - 1) until that tile's product has read it: products with unlike accumulators and
+        // shapes may pass one another.
+        if (i > 0 && i + 1 < n_tiles &&
+            !mbar_wait(smem_u32(&bars.v_empty[b ^ 1]), ((i - 1) >> 1) & 1, abortp, p.status, kStatusPrefillWait)) break;
         if (i + 1 < n_tiles && !scores(i + 1)) break;
         if (!mbar_wait(smem_u32(&bars.v_full[b]), (i >> 1) & 1, abortp, p.status, kStatusPrefillWait)) break;
         if (!mbar_wait(smem_u32(&bars.p_full[b]), ((i >> 1) + b) & 1, abortp, p.status, kStatusPrefillWait)) break;

@@ -391,7 +391,7 @@ def test_prefill_attention(ops, name, fmt, group, hq, hkv):
 
 @pytest.mark.parametrize("name,fmt,group", FORMATS)
 @pytest.mark.parametrize("hq,hkv,n,T", [(2, 2, 1, 1), (24, 4, 63, 63), (24, 4, 64, 3), (24, 4, 65, 65), (128, 1, 129, 3),
-                                        (16, 2, 191, 40), (6, 1, 200, 200)])
+                                        (16, 2, 191, 40), (6, 1, 200, 200), (24, 4, 1100, 30)])
 def test_prefill_attention_tile_edges(ops, status, name, fmt, group, hq, hkv, n, T):
     """The last T of n positions at the edges of the 64-key tiles, groups from one head to all 128 rows: keys that grow along
     the sequence (a row's frame moves in most tiles), values so large that fp8 rows have scales above 1024, a gate whose rows
