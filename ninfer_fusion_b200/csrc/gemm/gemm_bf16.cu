@@ -1333,7 +1333,7 @@ int gemm_pick_splits(int T, int N, int K, int epi, int sm_count) {
   if (s > 8) s = 8;
   if (tn == 64 && s > 6) s = 6;
   if (tn == 64 && epi == kEpiRsAg && s > 5) s = 5;   // its row staging tile shares the pipeline stages
-  if (!deep_enabled() && s > gemm_max_cluster(tn)) s = gemm_max_cluster(tn);
+  if ((!deep_enabled() || epi == kEpiSwiglu) && s > gemm_max_cluster(tn)) s = gemm_max_cluster(tn);
   // the largest split whose clusters are all resident at once (one wave), that leaves every split at least eight
   // k-blocks and no split empty
   for (; s > 1; --s) {

@@ -221,6 +221,22 @@ def test_gemm_rows_keep_their_bits(ops, status, T, N, K):
     status.check("rows")
 
 
+@pytest.mark.parametrize("T", [1, 16, 17, 32, 33, 48, 64])
+@pytest.mark.parametrize("N,K", [(1024, 2048), (512, 4096)])
+def test_gemm_takes_the_split_that_is_picked(ops, status, T, N, K):
+    """Few weight tiles and a long contraction, the shared expert of a sparse decoder: the split picked for an epilogue is one
+    that the kernel takes."""
+    x, w = _mk(T, N, K, seed=7)
+    ref = x.float() @ w.float().t()
+    for epi in (EPI_STORE, EPI_SWIGLU):
+        out = torch.empty((T, N // (2 if epi == EPI_SWIGLU else 1)), device="cuda", dtype=torch.bfloat16)
+        ops.gemm_bf16(x, w, out, epi, None, None, None, int(ops.gemm_pick_splits(T, N, K, epi)), status.tensor, False)
+        want = torch.nn.functional.silu(ref[:, : N // 2]) * ref[:, N // 2:] if epi == EPI_SWIGLU else ref
+        # one rounding to bf16 (2^-9) and fp32 sums of K products in another order
+        assert (out.float() - want).abs().max() <= want.abs().max() * 2.0 ** -7
+    status.check("picked split")
+
+
 @pytest.mark.parametrize("T", [1, 16, 17, 33, 64])
 @pytest.mark.parametrize("inter,K", [(64 * 149, 64), (9792, 1096)])
 def test_gemm_swiglu_streams_weight_tiles(ops, status, T, inter, K):
