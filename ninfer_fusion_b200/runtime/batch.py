@@ -53,6 +53,7 @@ class StepBuffers:
         self.dev = torch.zeros(off, dtype=torch.int32, device=self.device)
         self._np = self.host.numpy()
         self._sent = torch.cuda.Event() if pin else None   # the last upload out of `host`
+        self._decode_views: dict = {}   # sequences of a one-token step -> its views of both buffers (at most max_seqs entries)
 
     def _hview(self, name: str, n: int):
         off, cap = self.offsets[name]
@@ -79,36 +80,48 @@ class StepBuffers:
 
     def build_decode(self, table_rows: Sequence[int], state_slots: Sequence[int], start_pos: Sequence[int], tokens: Sequence[int],
                      rope_delta: Sequence[int]) -> StepBatch:
-        """One token per sequence, logits for all of them: what `build` makes of B one-token chunks, without a loop over them."""
+        """One token per sequence, logits for all of them: what `build` makes of B one-token chunks, without a loop over them;
+        the views of a batch size are made once."""
         B = len(tokens)
         if B > self.max_tokens or B > self.max_seqs:
             raise ValueError(f"step ({B} tokens, {B} seqs) exceeds buffers ({self.max_tokens}, {self.max_seqs})")
+        kept = self._decode_views.get(B)
+        if kept is None:
+            count = np.arange(B + 1, dtype=np.int32)
+            host = {name: self._hview(name, n) for name, n in (
+                ("ids", B), ("table_row", B), ("cache_pos", B), ("rope_pos", B * self.pos_axes), ("kv_len", B), ("state_slot", B))}
+            fixed = [(self._hview(name, len(values)), values) for name, values in (
+                ("token_seq", count[:B]), ("cu_seqlens", count), ("logit_rows", count[:B]), ("qblk_start", count[:B]),
+                ("qblk_count", np.ones(B, dtype=np.int32)))]
+            kept = self._decode_views[B] = (host, fixed, self._device_views(B, B, B, B))
+        host, fixed, dev = kept
         self._begin()
         pos = np.asarray(start_pos, dtype=np.int32)
+        host["ids"][:] = tokens
+        host["table_row"][:] = table_rows
+        host["state_slot"][:] = state_slots
+        host["cache_pos"][:] = pos
+        np.add(pos, 1, out=host["kv_len"])
         rope = pos.copy()
         d = np.asarray(rope_delta, dtype=np.int32)[:B]
         rope[: len(d)] += d
-        count = np.arange(B + 1, dtype=np.int32)
-        for name, values in (("ids", tokens), ("token_seq", count[:B]), ("table_row", table_rows), ("cache_pos", pos),
-                             ("rope_pos", np.repeat(rope, self.pos_axes)), ("kv_len", pos + 1), ("cu_seqlens", count),
-                             ("state_slot", state_slots), ("logit_rows", count[:B]), ("qblk_start", count[:B]),
-                             ("qblk_count", np.ones(B, dtype=np.int32))):
-            self._hview(name, len(values))[:] = values
+        host["rope_pos"][:] = rope if self.pos_axes == 1 else np.repeat(rope, self.pos_axes)
+        for view, values in fixed:   # (`build` writes them for other steps)
+            view[:] = values
         self._upload()
-        rows, ends = [int(r) for r in table_rows], (pos + 1).tolist()
-        return self._views(B, B, B, B, max(ends, default=1), True, 1, [(r, 1, e) for r, e in zip(rows, ends)])
+        seq_host = [(int(r), 1, e) for r, e in zip(table_rows, host["kv_len"].tolist())]
+        return StepBatch(**dev, max_kv_len=max((e for _, _, e in seq_host), default=1), n_tokens=B, n_seqs=B, one_token_per_seq=True,
+                         max_seq_tokens=1, seq_host=seq_host, plans={})
 
-    def _views(self, T: int, B: int, n_logit: int, nb: int, max_kv: int, one_token: bool, longest: int, seq_host: list) -> StepBatch:
+    def _device_views(self, T: int, B: int, n_logit: int, nb: int) -> dict:
         rp = self._dview("rope_pos", T * self.pos_axes)
         if self.pos_axes == 3:
             rp = rp.view(T, 3)
-        return StepBatch(ids=self._dview("ids", T), token_seq=self._dview("token_seq", T),
-                         table_row=self._dview("table_row", T), cache_pos=self._dview("cache_pos", T), rope_pos=rp,
-                         kv_len=self._dview("kv_len", T), cu_seqlens=self._dview("cu_seqlens", B + 1),
-                         state_slot=self._dview("state_slot", B), logit_rows=self._dview("logit_rows", n_logit),
-                         max_kv_len=max_kv, n_tokens=T, n_seqs=B, one_token_per_seq=one_token, max_seq_tokens=longest,
-                         qblk_start=self._dview("qblk_start", nb), qblk_count=self._dview("qblk_count", nb),
-                         seq_host=seq_host, plans={})
+        return dict(ids=self._dview("ids", T), token_seq=self._dview("token_seq", T), table_row=self._dview("table_row", T),
+                    cache_pos=self._dview("cache_pos", T), rope_pos=rp, kv_len=self._dview("kv_len", T),
+                    cu_seqlens=self._dview("cu_seqlens", B + 1), state_slot=self._dview("state_slot", B),
+                    logit_rows=self._dview("logit_rows", n_logit), qblk_start=self._dview("qblk_start", nb),
+                    qblk_count=self._dview("qblk_count", nb))
 
     def build(self, chunks: List[SeqChunk], upload: bool = True, rope_delta: Sequence[int] | None = None) -> StepBatch:
         T = sum(len(c.tokens) for c in chunks)
@@ -167,6 +180,7 @@ class StepBuffers:
         self._hview("qblk_count", nb)[:] = blk_c
         if upload:
             self._upload()
-        return self._views(T, B, n_logit, nb, max_kv, all(len(c.tokens) == 1 for c in chunks),
-                           max((len(c.tokens) for c in chunks), default=1),
-                           [(c.table_row, len(c.tokens), c.start_pos + len(c.tokens)) for c in chunks])
+        return StepBatch(**self._device_views(T, B, n_logit, nb), max_kv_len=max_kv, n_tokens=T, n_seqs=B,
+                         one_token_per_seq=all(len(c.tokens) == 1 for c in chunks),
+                         max_seq_tokens=max((len(c.tokens) for c in chunks), default=1),
+                         seq_host=[(c.table_row, len(c.tokens), c.start_pos + len(c.tokens)) for c in chunks], plans={})
