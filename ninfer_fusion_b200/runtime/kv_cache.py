@@ -666,12 +666,13 @@ class RecurrentStatePool:
         if len(self._free) < n:
             raise MemoryError("recurrent state slots exhausted")
         slots = [self._free.pop() for _ in range(n)]
-        if n:
+        arrays = self.tensors()
+        if n and arrays:   # (a decoder without recurrent layers has no arrays)
             lo = min(slots)
             if max(slots) - lo + 1 == n:   # neighbours: one view per array, all arrays in a few launches
-                torch._foreach_zero_([t[lo:lo + n] for t in self.tensors()])
+                torch._foreach_zero_([t[lo:lo + n] for t in arrays])
             else:
-                torch._foreach_zero_([t[s] for t in self.tensors() for s in slots])
+                torch._foreach_zero_([t[s] for t in arrays for s in slots])
         return slots
 
     def release(self, slot: int) -> None:

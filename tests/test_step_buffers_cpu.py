@@ -25,9 +25,10 @@ def test_build_decode_is_build_of_one_token_chunks(B, deltas, mrope):
         bufs[1].build_decode([0] * 9, [0] * 9, [0] * 9, [0] * 9, [])
 
 
+@pytest.mark.parametrize("shapes", [[[((3, 4), torch.bfloat16), ((2, 5), torch.float32)], [((7,), torch.float32)]], []])
 @pytest.mark.parametrize("taken,n", [([], 6), ([1, 3], 2), ([0, 2], 4), ([], 0)])
-def test_alloc_many_is_alloc_n_times(taken, n):
-    shapes = [[((3, 4), torch.bfloat16), ((2, 5), torch.float32)], [((7,), torch.float32)]]
+def test_alloc_many_is_alloc_n_times(taken, n, shapes):
+    """(`shapes` empty: a decoder without recurrent layers)"""
     pools = [RecurrentStatePool(shapes, 6, "cpu") for _ in range(2)]
     for pool in pools:
         held = [pool.alloc() for _ in range(6)]
