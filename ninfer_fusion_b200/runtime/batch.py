@@ -73,10 +73,11 @@ class StepBuffers:
         if self._sent is not None:
             self._sent.synchronize()
 
-    def _upload(self) -> None:
+    def upload(self) -> None:
+        """Copies `host` to the device on the current stream; every upload goes through here, so that `_begin` knows of it."""
         self.dev.copy_(self.host, non_blocking=True)
         if self._sent is not None:
-            self._sent.record()
+            self._sent.record(torch.cuda.current_stream(self.device))
 
     def build_decode(self, table_rows: Sequence[int], state_slots: Sequence[int], start_pos: Sequence[int], tokens: Sequence[int],
                      rope_delta: Sequence[int]) -> StepBatch:
@@ -108,7 +109,7 @@ class StepBuffers:
         host["rope_pos"][:] = rope if self.pos_axes == 1 else np.repeat(rope, self.pos_axes)
         for view, values in fixed:   # (`build` writes them for other steps)
             view[:] = values
-        self._upload()
+        self.upload()
         seq_host = [(int(r), 1, e) for r, e in zip(table_rows, host["kv_len"].tolist())]
         return StepBatch(**dev, max_kv_len=max((e for _, _, e in seq_host), default=1), n_tokens=B, n_seqs=B, one_token_per_seq=True,
                          max_seq_tokens=1, seq_host=seq_host, plans={})
@@ -179,7 +180,7 @@ class StepBuffers:
         self._hview("qblk_start", nb)[:] = blk_s
         self._hview("qblk_count", nb)[:] = blk_c
         if upload:
-            self._upload()
+            self.upload()
         return StepBatch(**self._device_views(T, B, n_logit, nb), max_kv_len=max_kv, n_tokens=T, n_seqs=B,
                          one_token_per_seq=all(len(c.tokens) == 1 for c in chunks),
                          max_seq_tokens=max((len(c.tokens) for c in chunks), default=1),

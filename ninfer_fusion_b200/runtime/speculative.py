@@ -561,12 +561,12 @@ class SpeculativeGenerator(Generator):
         with torch.cuda.stream(stream):
             for _ in range(2):   # warm-up outside capture; a round moves the recurrent state and the draft inputs
                 self._snapshot_states()
-                self.bufs_draft.dev.copy_(self.bufs_draft.host, non_blocking=True)
+                self.bufs_draft.upload()
                 self._round_body(B, bd, bv)
                 restore()
         torch.cuda.current_stream().wait_stream(stream)
         torch.cuda.synchronize(self.device)
-        self.bufs_draft.dev.copy_(self.bufs_draft.host, non_blocking=True)
+        self.bufs_draft.upload()
         graph = torch.cuda.CUDAGraph()
         self._snapshot_states()
         with torch.cuda.graph(graph):

@@ -25,6 +25,27 @@ def test_build_decode_is_build_of_one_token_chunks(B, deltas, mrope):
         bufs[1].build_decode([0] * 9, [0] * 9, [0] * 9, [0] * 9, [])
 
 
+def test_every_upload_is_waited_for_before_the_buffer_is_written(monkeypatch):
+    """An upload by itself (a speculative round that is captured) counts like the one of `build`: the buffer is not written
+    before the event behind it."""
+    log = []
+
+    class Event:
+        def record(self, stream=None):
+            log.append("sent")
+
+        def synchronize(self):
+            log.append("wait")
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda device=None: None)
+    bufs = StepBuffers(8, 8, "cpu")
+    bufs._sent = Event()
+    bufs.upload()
+    bufs.build([SeqChunk(0, 0, 5, [3, 4], True)])
+    bufs.upload()
+    bufs.build_decode([0], [0], [7], [1], [0])
+    assert log == ["sent", "wait", "sent", "sent", "wait", "sent"]
+
+
 @pytest.mark.parametrize("shapes", [[[((3, 4), torch.bfloat16), ((2, 5), torch.float32)], [((7,), torch.float32)]], []])
 @pytest.mark.parametrize("taken,n", [([], 6), ([1, 3], 2), ([0, 2], 4), ([], 0)])
 def test_alloc_many_is_alloc_n_times(taken, n, shapes):
