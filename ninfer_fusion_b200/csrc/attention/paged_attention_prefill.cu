@@ -305,34 +305,43 @@ __global__ void __launch_bounds__(kThreads, 1) paged_attn_prefill_kernel(const P
       if constexpr (kSets == 2)
         if (i + 1 < n_tiles) step(i + 1, raw[1], live[1]);
     }
-    // ---- gate beside the last products, then the normalised rows from the stage ----
-    constexpr int kOut = kRows * (D / 8) / (2 * kGroup);   // 16-byte pieces per thread
-    uint4 gate[kOut];
+    // ---- the normalised rows from the stage, times the gate: four 16-byte pieces of a thread at a time, the first four gates
+    //      loaded beside the last products.  (All sixteen in a row are code that every launch fetches anew: a prompt of 37 tokens,
+    //      one key tile, took 59 us a layer so, 39 in a loop.) ----
+    constexpr int kOut = kRows * (D / 8) / (2 * kGroup), kBatch = 4;   // 16-byte pieces per thread, and at a time
+    uint4 gate[kBatch];
     const int otid = threadIdx.x - kGroup;
+    auto load_gates = [&](int j0) {
 #pragma unroll
-    for (int j = 0; j < kOut; ++j) {
-      const int i = j * 2 * kGroup + otid, r = i >> 5, c = i & 31;
-      gate[j] = make_uint4(0, 0, 0, 0);
-      if (p.gate != nullptr && r < n_rows)
-        gate[j] = load_row16(p.gate + static_cast<long long>(t0 + r / G) * p.ld_gate + (kvh * G + r % G) * D + c * 8, wide);
-    }
-    asm volatile("bar.sync 4, 384;" ::: "memory");
-#pragma unroll
-    for (int j = 0; j < kOut; ++j) {
-      const int i = j * 2 * kGroup + otid, r = i >> 5, c = i & 31;
-      if (r >= n_rows) continue;
-      uint4 o = *reinterpret_cast<const uint4*>(stage + r * kStagePitch + c * 16);
-      if (p.gate != nullptr) {
-        const __nv_bfloat162* g2 = reinterpret_cast<const __nv_bfloat162*>(&gate[j]);
-        uint32_t* ow = reinterpret_cast<uint32_t*>(&o);
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const __nv_bfloat162 v = *reinterpret_cast<const __nv_bfloat162*>(&ow[e]);
-          ow[e] = pack_bf16x2(__bfloat162float(v.x) / (1.f + __expf(-__bfloat162float(g2[e].x))),
-                              __bfloat162float(v.y) / (1.f + __expf(-__bfloat162float(g2[e].y))));
-        }
+      for (int j = 0; j < kBatch; ++j) {
+        const int i = (j0 + j) * 2 * kGroup + otid, r = i >> 5, c = i & 31;
+        gate[j] = make_uint4(0, 0, 0, 0);
+        if (p.gate != nullptr && r < n_rows)
+          gate[j] = load_row16(p.gate + static_cast<long long>(t0 + r / G) * p.ld_gate + (kvh * G + r % G) * D + c * 8, wide);
       }
-      store_row16(p.out + (static_cast<long long>(t0 + r / G) * p.n_q_heads + kvh * G + r % G) * D + c * 8, o, wide);
+    };
+    load_gates(0);
+    asm volatile("bar.sync 4, 384;" ::: "memory");
+#pragma unroll 1
+    for (int j0 = 0; j0 < kOut && (j0 * 2 * kGroup >> 5) < n_rows; j0 += kBatch) {
+#pragma unroll
+      for (int j = 0; j < kBatch; ++j) {
+        const int i = (j0 + j) * 2 * kGroup + otid, r = i >> 5, c = i & 31;
+        if (r >= n_rows) continue;
+        uint4 o = *reinterpret_cast<const uint4*>(stage + r * kStagePitch + c * 16);
+        if (p.gate != nullptr) {
+          const __nv_bfloat162* g2 = reinterpret_cast<const __nv_bfloat162*>(&gate[j]);
+          uint32_t* ow = reinterpret_cast<uint32_t*>(&o);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const __nv_bfloat162 v = *reinterpret_cast<const __nv_bfloat162*>(&ow[e]);
+            ow[e] = pack_bf16x2(__bfloat162float(v.x) / (1.f + __expf(-__bfloat162float(g2[e].x))),
+                                __bfloat162float(v.y) / (1.f + __expf(-__bfloat162float(g2[e].y))));
+          }
+        }
+        store_row16(p.out + (static_cast<long long>(t0 + r / G) * p.n_q_heads + kvh * G + r % G) * D + c * 8, o, wide);
+      }
+      if (j0 + kBatch < kOut) load_gates(j0 + kBatch);
     }
   } else {
     // =========================== softmax: thread = row = TMEM lane ===========================
@@ -450,13 +459,14 @@ __global__ void __launch_bounds__(kThreads, 1) paged_attn_prefill_kernel(const P
           __syncwarp();
           tc_fence_after();
 #pragma unroll 1
-          for (int c = 0; c < D; c += 16) {
-            uint32_t o[16];
-            tmem_ld_x16(tmem + lane_sel + kColO + c, o);
-            tmem_ld_wait_x16(o);
+          for (int c = 0; c < D; c += 32) {
+            uint32_t o[32];
+            tmem_ld_x32(tmem + lane_sel + kColO + c, o);
+            tmem_ld_wait_x32(o);
 #pragma unroll
-            for (int j = 0; j < 16; ++j) o[j] = __float_as_uint(__uint_as_float(o[j]) * corr);
+            for (int j = 0; j < 32; ++j) o[j] = __float_as_uint(__uint_as_float(o[j]) * corr);
             tmem_st_x16(tmem + lane_sel + kColO + c, o);
+            tmem_st_x16(tmem + lane_sel + kColO + c + 16, o + 16);
           }
         }
       }
