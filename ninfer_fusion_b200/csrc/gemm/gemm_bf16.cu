@@ -1492,10 +1492,14 @@ const char* gemm_bf16(const GemmArgs& a) {
     const char* e = getenv("NFB_GEMM_PERSISTENT");
     return !(e != nullptr && e[0] == '0');
   }();
-  // Up to 64 tokens, SwiGLU with more weight tiles than SMs: the same kernel streams the weights in whole rounds of one tile
-  // per SM.  (34816 x 5120 is 544 tiles: 1.84 rounds at two CTAs per SM, 3.68 here; one token's round of eight layers
-  // 1623 -> 1600 us, 37 tokens 2192 -> 2147.  The plain store gained nothing, the language-model head lost 1 %.)
-  const bool stream = tn <= 64 && a.epi == kEpiSwiglu && w_tiles > device_sm_count();
+  // Up to 64 tokens, SwiGLU with more weight tiles than SMs and at least three quarters of them busy in the last round: the
+  // same kernel streams the weights in whole rounds of one tile per SM, where two CTAs per SM run them in one.  34816 x 5120,
+  // 272 tiles, 1.84 rounds: 37 tokens 75.8 -> 67.6 us, one token 70.1 -> 69.6; 24576 x 4096, 192 tiles, whose second round would
+  // leave 104 SMs idle: one token 47.1 us with two CTAs per SM, 50.1 in rounds.  (The plain store gained nothing, the
+  // language-model head lost 1 %.)
+  const int last_round = w_tiles % device_sm_count();
+  const bool stream = tn <= 64 && a.epi == kEpiSwiglu && w_tiles > device_sm_count() &&
+                      (last_round == 0 || 4 * last_round >= 3 * device_sm_count());
   const bool persistent = (tn == 256 || stream) && splits == 1 && persistent_enabled && !g_trace_enabled && plain;
   const int box_tokens = persistent && !stream ? persist_tile_tokens(kp.T, w_tiles, kp.num_kb, device_sm_count()) : tn;
   kp.tn = box_tokens;
