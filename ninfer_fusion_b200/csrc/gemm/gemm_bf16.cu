@@ -751,8 +751,9 @@ __global__ void __launch_bounds__(128) gemm_ws_kernel(const __grid_constant__ CU
 int device_sm_count();
 
 // ------------------------------------------------------------------------------------------------------------
-// Persistent kernel for more than 128 tokens: one CTA per SM walks output tiles of 128 weight rows x `tn` tokens, with
-// the roles split over ten warps so that the epilogue of tile i overlaps the main loop of tile i + 1:
+// Persistent kernel for more than 128 tokens, and for SwiGLU of up to 64 whose weight tiles fill whole rounds: one CTA per SM
+// walks output tiles of 128 weight rows x `tn` tokens, with the roles split over ten warps so that the epilogue of tile i
+// overlaps the main loop of tile i + 1:
 //   warp 0  TMA producer (as many stages of 16 KB weights + tn x 128 B tokens as fit, one running counter over tiles)
 //   warp 1  MMA issuer; the fp32 accumulator alternates between TMEM columns [0, 256) and [256, 512)
 //   warps 2..9  epilogue: warp w drains TMEM lanes 32 (w % 4) .., every second chunk of 16 tokens; tcgen05.ld -> bias /
@@ -760,12 +761,13 @@ int device_sm_count();
 // Two warps per lane group, because with short contractions (K = 2048: 13 us per 128 x 256 tile) one warp per group took
 // longer to drain a tile than the tensor core to fill the next.  Tiles are numbered token-tile fastest, so the CTAs
 // running at one time share a few weight tiles and all token tiles through L2.  The main loop is bound by the tensor
-// rate at 256 tokens and by the operands' latency from L2 below (five stages or more from 224 tokens down).
+// rate at 256 tokens and by the operands' latency from L2 below (five stages or more from 224 tokens down, with SwiGLU's
+// exchange from 192).
 // T = 2048, us, before (256 tokens always, four epilogue warps) -> now: 5120 x 6144 residual 131 -> 94, 5120 x 17408
 // residual 332 -> 251, 34816 x 5120 SwiGLU 514 -> 461, 14336 x 5120 219 -> 204, 12352 x 2048 125 -> 84; and with fewer tiles
-// than SMs (one-tile-per-CTA kernel before) 2048 x 4096 55 -> 40, 264 x 2048 33 -> 17; T = 160: 5120 x 17408 111 -> 72.
+// than SMs (one-tile-per-CTA kernel before) 2048 x 4096 55 -> 40, 264 x 2048 33 -> 17.
 constexpr int kPersistMaxTN = 256;
-constexpr int kPersistMinTN = 64;
+constexpr int kPersistMinTN = 64;   // narrowest that persist_tile_tokens weighs (SwiGLU of up to 64 tokens: 16, 32 or 64)
 constexpr int kPersistMaxStages = 12;
 constexpr int kPersistEpiWarps = 8;
 constexpr int kPersistThreads = 64 + 32 * kPersistEpiWarps;
@@ -773,8 +775,12 @@ constexpr int kPersistSmemBytes = 226 * 1024;
 constexpr int kPersistExchangeBytes = 4 * 2 * 2 * 8 * 32 * 4;   // SwiGLU: per warp pair two buffers x two directions x 8 x 32
 constexpr int persist_ring_bytes(int epi) { return kPersistSmemBytes - 1024 - (epi == kEpiSwiglu ? kPersistExchangeBytes : 0); }
 // Time of one k-block of 64 by tokens per tile, all SMs busy: a line through what widths of 64 to 224 took (246 to 334 ns);
-// at 240 and 256 only four stages fit, which costs another 30 ns (measured 368 and 387).
-constexpr double persist_kblock_ns(int tn) { return 211. + 0.55 * tn + (tn > 224 ? 30. : 0.); }
+// where only four stages fit, from 240 tokens or, beside SwiGLU's exchange, from 208, another 30 ns (240 and 256: 368 and 387).
+// (With the 30 ns from 240 for SwiGLU too: 34816 x 5120, 1300 tokens 338 us in tiles of 224, 313 in the 192 taken now; 1830
+// tokens 480 and 462; 24576 x 4096, 1720 tokens 271 and 255.)
+constexpr double persist_kblock_ns(int tn, int epi) {
+  return 211. + 0.55 * tn + (persist_ring_bytes(epi) / (kWTileBytes + 128 * tn) < 5 ? 30. : 0.);
+}
 constexpr double kPersistTailNs = 30.;   // per token of the last tile, whose epilogue nothing overlaps
 
 template <int EPI>
@@ -1065,13 +1071,13 @@ __global__ void __launch_bounds__(kPersistThreads, 1) gemm_persist_kernel(const 
 // of weight rows times the token tiles are dealt out in rounds of one tile per SM; what a fixed 256 loses is the last
 // round (N = 5120, T = 2048: 320 tiles = 2.16 rounds, paid as 3; 192 tokens make it 2.97) or, with few tiles, the SMs that
 // get none (N = 264: 24 tiles of 256 against 96 of 64).
-int persist_tile_tokens(int T, int w_tiles, int num_kb, int sms) {
+int persist_tile_tokens(int T, int w_tiles, int num_kb, int sms, int epi) {
   int best = kPersistMaxTN;
   double best_ns = 0;
   for (int tn = kPersistMaxTN; tn >= kPersistMinTN; tn -= 16) {
     const long long tiles = static_cast<long long>(w_tiles) * ((T + tn - 1) / tn);
     const long long rounds = (tiles + sms - 1) / sms;
-    const double ns = static_cast<double>(rounds) * num_kb * persist_kblock_ns(tn) + kPersistTailNs * tn;
+    const double ns = static_cast<double>(rounds) * num_kb * persist_kblock_ns(tn, epi) + kPersistTailNs * tn;
     if (best_ns == 0 || ns < best_ns * 0.99) { best = tn; best_ns = ns; }
   }
   return best;
@@ -1353,7 +1359,9 @@ namespace {
 // Tokens per tile for 65 to 256 tokens.  With few tiles of weight rows a tile that holds all tokens leaves most SMs idle
 // (N = 2048: 16 CTAs walk the whole contraction), so the narrower of 32 and 64 whose tiles all run at once is taken: a k-block
 // of a narrower tile takes less time (persist_kblock_ns), its epilogue too, and the weights are read once from HBM and again
-// from L2.  The contraction is not cut: a row's sums keep one order whatever the number of rows beside it.
+// from L2.  The contraction is not cut: a row's sums keep one order whatever the number of rows beside it.  One tile of 128 or
+// 256 tokens -> now, us: 128 tokens 2048 x 4096 33 -> 25, 264 x 2048 22 -> 16, 5120 x 17408 78 -> 70; 256 tokens 49 -> 25,
+// 33 -> 16, 125 -> 76.
 int narrow_tile(int T, int w_tiles, int tn) {
   for (int n = 32; n <= 64; n *= 2)
     if (static_cast<long long>(w_tiles) * ((T + n - 1) / n) <= device_sm_count()) return n;
@@ -1486,7 +1494,8 @@ const char* gemm_bf16(const GemmArgs& a) {
   const bool needs_out = !all32 && (a.epi == kEpiStore || a.epi == kEpiResidual || a.epi == kEpiSwiglu);
   if (needs_out && a.out == nullptr) return "gemm_bf16: no output";
 
-  // More than 128 tokens and a plain epilogue: persistent kernel, epilogue overlapped with the next main loop
+  // More than 128 tokens (that no narrow tile takes) and a plain epilogue: persistent kernel, epilogue overlapped with the next
+  // main loop
   // (NFB_GEMM_PERSISTENT=0 keeps the one-tile-per-CTA kernel for every size)
   static const bool persistent_enabled = [] {
     const char* e = getenv("NFB_GEMM_PERSISTENT");
@@ -1501,7 +1510,7 @@ const char* gemm_bf16(const GemmArgs& a) {
   const bool stream = tn <= 64 && a.epi == kEpiSwiglu && w_tiles > device_sm_count() &&
                       (last_round == 0 || 4 * last_round >= 3 * device_sm_count());
   const bool persistent = (tn == 256 || stream) && splits == 1 && persistent_enabled && !g_trace_enabled && plain;
-  const int box_tokens = persistent && !stream ? persist_tile_tokens(kp.T, w_tiles, kp.num_kb, device_sm_count()) : tn;
+  const int box_tokens = persistent && !stream ? persist_tile_tokens(kp.T, w_tiles, kp.num_kb, device_sm_count(), a.epi) : tn;
   kp.tn = box_tokens;
 
   CUtensorMap tw, tx;
