@@ -155,8 +155,9 @@ def pick_attention_split(max_kv_len: int, n_work: int, sm_count: int = 148, max_
     Aim for about `waves` items per SM: two for the scalar kernel (one CTA per item), four for the tensor-core kernel (two
     CTAs per SM at a time, so that with two the last round of them was often half empty: 8 sequences of 32,000 nvfp4 keys
     189 -> 173 us, of 26,000 bf16 keys 243 -> 205; eight cost 185 and 210), eight for the persistent tcgen05 kernel (its
-    CTAs walk a list of items, so many small items balance better than few large ones).  The split size only depends on the
-    context bucket, so decode and verify of the same position use the same ranges."""
+    CTAs walk a list of items, so many small items balance better than few large ones).  The split depends on the context's
+    power-of-two bucket and on `n_work`: a sequence's ranges stay while its context grows inside a bucket, and differ between
+    steps of unlike token counts."""
     bucket = 128
     while bucket < max_kv_len:
         bucket *= 2
@@ -167,6 +168,13 @@ def pick_attention_split(max_kv_len: int, n_work: int, sm_count: int = 148, max_
         split *= 2
     n_splits = (max_kv_len + split - 1) // split
     return split, max(1, n_splits)
+
+
+def attention_waves(fmt: int, head_dim: int, page_size: int, n_q_heads: int, n_kv_heads: int, impl: int = 0) -> int:
+    """`waves` of `pick_attention_split` for the kernel that the split attention takes (`impl` 0: by itself)."""
+    if fmt == 1 and head_dim == 256 and page_size % 64 == 0 and impl in (0, 3) and os.environ.get("NFB_ATTN_TC", "1") != "0":
+        return 8    # persistent tcgen05 kernel
+    return 4 if head_dim == 256 and n_q_heads <= 16 * n_kv_heads and impl != 1 else 2   # tensor-core kernel, scalar kernel
 
 
 class LaunchCounter:
@@ -484,13 +492,10 @@ class HybridModel:
                                         planes.v_scales, kv.page_size, planes.fmt, planes.group, self.sm_scale, gate,
                                         out, self.pdl, 0, tiers, self.status.tensor)
             return out, self.w[f"{prefix}/attn/o_proj"]
-        persistent = (planes.fmt == 1 and D == 256 and kv.page_size % 64 == 0 and self.attn_impl in (0, 3)
-                      and os.environ.get("NFB_ATTN_TC", "1") != "0")
-        tensor = D == 256 and g.n_q_heads <= 16 * g.n_kv_heads and self.attn_impl != 1   # what the mma kernel takes
-        split, n_splits = pick_attention_split(b.max_kv_len, T * g.n_kv_heads, max_splits=ws.max_splits_attn,
-                                               waves=8 if persistent else 4 if tensor else 2)
-        if persistent:
-            n_splits = max(n_splits, 2)   # the kernel cuts rows at CTA boundaries: a row needs a second result slot
+        waves = attention_waves(planes.fmt, D, kv.page_size, g.n_q_heads, g.n_kv_heads, self.attn_impl)
+        split, n_splits = pick_attention_split(b.max_kv_len, T * g.n_kv_heads, max_splits=ws.max_splits_attn, waves=waves)
+        if waves == 8:
+            n_splits = max(n_splits, 2)   # the persistent kernel cuts rows at CTA boundaries: a row needs a second result slot
         chunk = max(1, ws.part_rows // n_splits)
         w_out = self.w[f"{prefix}/attn/o_proj"]
         qc, qs = self._next_operand(T, w_out, q_dim) if chunk >= T else (None, None)   # nvfp4: merge quantises its rows

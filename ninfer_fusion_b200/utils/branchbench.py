@@ -184,8 +184,8 @@ def _attention(k: _Kernels, model, ws, cfg, hyb, batch: int, new: int, total: in
         k.add(f"attention {tag}", "hybrid", lambda: ops.paged_attention_prefill(qh, Hh, Gh, Dh, row, kv, bs, bc, table, kh, vh, None, None, P, 0, Dh, Dh ** -0.5,
                                                                                 gh, oh, False, 0, None), hb, hm)
     else:
-        from ..models.hybrid import pick_attention_split
-        sp, ns = pick_attention_split(total, T * Gh)
+        from ..models.hybrid import attention_waves, pick_attention_split
+        sp, ns = pick_attention_split(total, T * Gh, waves=attention_waves(0, Dh, P, Hh, Gh))
         po2, ml2 = torch.empty(T * ns * Hh * Dh, device="cuda"), torch.empty(T * ns * Hh * 2, device="cuda")
         k.add(f"attention {tag}", "hybrid", lambda: ops.paged_attention(qh, Hh, Gh, Dh, row, kv, table, kh, vh, None, None, P, 0, Dh, Dh ** -0.5, sp, ns, po2, ml2,
                                                                         gh, oh, None, None, 0, False), hb, hm)

@@ -195,8 +195,8 @@ def _attention_rows(k: _Kernels, ops, model, ws, cfg, hyb, batch: int, new: int,
                                                                                 Dh ** -0.5, gh, oh, False, 0, None),
               batch * tot * Gh * Dh * 4 + T * Hh * Dh * 6, batch * _pairs(new, tot, 0) * Hh * 2 * Dh)
     else:
-        from ..models.hybrid import pick_attention_split
-        sp, ns = pick_attention_split(tot, T * Gh)
+        from ..models.hybrid import attention_waves, pick_attention_split
+        sp, ns = pick_attention_split(tot, T * Gh, waves=attention_waves(0, Dh, P, Hh, Gh))
         po2, ml2 = torch.empty(T * ns * Hh * Dh, device="cuda"), torch.empty(T * ns * Hh * 2, device="cuda")
         k.add(f"attention {tag}", "hybrid", lambda: ops.paged_attention(qh, Hh, Gh, Dh, row, kv, table2, kh, vh, None, None, P, 0, Dh, Dh ** -0.5, sp, ns,
                                                                         po2, ml2, gh, oh, None, None, 0, False),

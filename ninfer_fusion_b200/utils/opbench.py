@@ -135,8 +135,8 @@ def bench_attn(ops, batch, ctx, kv, hq=24, hkv=4, D=256, P=64, iters=20, impl=0)
         vs = torch.full((n_pages, hkv, P, sb), 0x20, dtype=torch.uint8, device="cuda")
     table = torch.randperm(n_pages, device="cuda").int().view(batch, pages_per)
     q = torch.randn(batch, hq, D, device="cuda").to(torch.bfloat16)
-    from ..models.hybrid import pick_attention_split
-    split, n_splits = pick_attention_split(ctx, batch * hkv, waves={3: 8, 2: 4}.get(impl, 2))
+    from ..models.hybrid import attention_waves, pick_attention_split
+    split, n_splits = pick_attention_split(ctx, batch * hkv, waves=attention_waves(fmt, D, P, hq, hkv, impl))
     part_o = torch.empty(batch * hq * n_splits * D, device="cuda")
     part_ml = torch.empty(batch * hq * n_splits * 2, device="cuda")
     out = torch.empty((batch, hq * D), dtype=torch.bfloat16, device="cuda")

@@ -5,7 +5,7 @@ import torch
 
 from ninfer_fusion_b200.kv import codec_report
 from ninfer_fusion_b200.models.config import QWEN36_27B, QWEN36_35B_A3B, TINY_DENSE, TINY_MOE
-from ninfer_fusion_b200.models.hybrid import pick_attention_split
+from ninfer_fusion_b200.models.hybrid import attention_waves, pick_attention_split
 from ninfer_fusion_b200.models.reference_model import ReferenceModel, ReferenceSequence
 from ninfer_fusion_b200.models.weights import random_weights, weight_shapes
 from ninfer_fusion_b200.ops import reference as R
@@ -121,3 +121,11 @@ def test_attention_split_geometry_is_bucketed():
     assert pick_attention_split(2048, 100000)[1] == 1  # prefill: plenty of parallelism, no split
     s, n = pick_attention_split(131072, 8, max_splits=64)
     assert n <= 64 and s * n >= 131072
+
+
+def test_attention_waves_follow_the_kernel():
+    assert attention_waves(1, 256, 64, 24, 4) == 8 and attention_waves(1, 256, 64, 24, 4, 3) == 8   # persistent, fp8 pages
+    assert attention_waves(1, 256, 64, 24, 4, 2) == 4 and attention_waves(1, 256, 16, 24, 4) == 4   # tensor-core kernel
+    assert attention_waves(0, 256, 64, 24, 4) == 4 and attention_waves(3, 256, 64, 16, 1) == 4
+    assert attention_waves(0, 256, 64, 24, 4, 1) == 2 and attention_waves(0, 128, 64, 8, 2) == 2    # scalar kernel
+    assert attention_waves(0, 256, 64, 17, 1) == 2
