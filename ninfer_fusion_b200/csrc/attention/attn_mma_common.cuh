@@ -1,5 +1,5 @@
-// Shared pieces of the mma.sync attention kernels (decode split-KV and prefill): tile geometry,
-// ldmatrix / mma wrappers and the raw-unit loader that dequantises 16 cache values to fp16 pairs.
+// Shared pieces of the tensor-core attention kernels over pages: tile geometry and ldmatrix / mma wrappers of the split-KV
+// decode kernel, and the raw-unit loader that dequantises 16 cache values to fp16 pairs, which the prefill kernel takes too.
 #pragma once
 #include <cuda_fp16.h>
 #include <cuda_fp4.h>
@@ -14,7 +14,6 @@ namespace attn_mma {
 constexpr int D = 256;
 constexpr int kTileKeys = 64;
 constexpr int kLdK = D + 8;          // halves per K-tile row
-constexpr int kLdV = kTileKeys + 8;  // halves per V^T-tile row
 constexpr int kLdP = kTileKeys + 8;
 constexpr int kLdQ = D + 8;
 

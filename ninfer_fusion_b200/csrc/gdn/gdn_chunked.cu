@@ -31,6 +31,7 @@
 
 #include <math_constants.h>
 
+#include "../common/device.h"
 #include "../common/ptx.cuh"
 
 namespace nfb {
@@ -664,16 +665,6 @@ __global__ void __launch_bounds__(256) gdn_gated_norm_kernel(const GdnParams p) 
   }
 }
 
-int sm_count() {
-  static int n = 0;
-  if (n == 0) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
-  }
-  return n;
-}
-
 }  // namespace
 
 size_t gdn_chunked_workspace_bytes(int max_chunks, int n_v_heads) {
@@ -721,7 +712,7 @@ const char* gdn_chunked(const GdnParams& p, void* workspace, size_t workspace_by
   // The scan is serial over the chunks and one CTA fills an SM: quarters of dv when all of them fit the GPU at once (32 heads:
   // 128 CTAs), else halves (48 heads: 96; quarters would run in two rounds).  With the prepare kernel's changes this took
   // 4096 tokens of the 32-head decoder with experts from 12.81 to 12.39 ms, eight layers.
-  if (static_cast<long long>(p.n_v_heads) * 4 * p.n_seq <= sm_count())
+  if (static_cast<long long>(p.n_v_heads) * 4 * p.n_seq <= device_sm_count())
     gdn_chunk_scan_kernel<32><<<dim3(p.n_v_heads, 4, p.n_seq), kScanThreads, sizeof(ScanSmem<32>), stream>>>(cp);
   else
     gdn_chunk_scan_kernel<64><<<dim3(p.n_v_heads, 2, p.n_seq), kScanThreads, sizeof(ScanSmem<64>), stream>>>(cp);

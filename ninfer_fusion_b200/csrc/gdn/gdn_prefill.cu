@@ -14,6 +14,7 @@
 // so prefill, decode and replay stay bit-consistent with one another).
 #include "gdn.h"
 
+#include "../common/device.h"
 #include "../common/ptx.cuh"
 
 namespace nfb {
@@ -628,16 +629,6 @@ cudaError_t launch_split(const GdnParams& p, cudaStream_t stream, bool pdl) {
   return cudaLaunchKernelEx(&cfg, kern, p);
 }
 
-int sm_count_cached() {
-  static int n = 0;
-  if (n == 0) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
-  }
-  return n;
-}
-
 }  // namespace
 
 void gdn_prefill_trace(bool enable, long long* host5) {
@@ -654,7 +645,7 @@ const char* gdn_prefill(const GdnParams& p, cudaStream_t stream, bool pdl) {
   // few (head, sequence) pairs: spread each head's independent state rows over a cluster of CTAs
   {
     const int work = p.n_v_heads * p.n_seq;
-    const int sms = sm_count_cached();
+    const int sms = device_sm_count();
     cudaError_t e = cudaSuccess;
     bool done = true;
     // (measured on the 27B geometry, 2048 tokens of one sequence: 48 heads split 4 ways = 1.0 ms against 1.5 ms

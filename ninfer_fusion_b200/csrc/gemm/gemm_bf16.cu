@@ -20,6 +20,7 @@
 #include <cstdlib>
 
 #include "../comm/peer_sync.cuh"
+#include "../common/device.h"
 #include "../common/ptx.cuh"
 #include "../common/tensor_map.h"
 #include "persist_epilogue.cuh"
@@ -748,8 +749,6 @@ __global__ void __launch_bounds__(128) gemm_ws_kernel(const __grid_constant__ CU
   stamp(6);
 }
 
-int device_sm_count();
-
 // ------------------------------------------------------------------------------------------------------------
 // Persistent kernel for more than 128 tokens, and for SwiGLU of up to 64 whose weight tiles fill whole rounds: one CTA per SM
 // walks output tiles of 128 weight rows x `tn` tokens, with the roles split over ten warps so that the epilogue of tile i
@@ -1139,16 +1138,6 @@ cudaError_t launch_one(const CUtensorMap& tw, const CUtensorMap& tx, const Kerne
   cfg.attrs = attr;
   cfg.numAttrs = n_attr;
   return cudaLaunchKernelEx(&cfg, kern, tw, tx, kp);
-}
-
-int device_sm_count() {
-  static int n = 0;
-  if (n == 0) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
-  }
-  return n;
 }
 
 // One CTA per SM with the deep pipeline when the whole grid fits in one wave.  NFB_GEMM_DEEP=0 keeps the shallow

@@ -23,6 +23,7 @@
 #include <unordered_map>
 
 #include "../comm/peer_sync.cuh"
+#include "../common/device.h"
 #include "../common/launch.h"
 #include "../common/ptx.cuh"
 #include "../common/tensor_map.h"
@@ -316,16 +317,6 @@ __global__ void __launch_bounds__(kThreads, 1) moe_gemm_kernel(const __grid_cons
   if (warp == 1) tmem_dealloc(tmem_base, 512);
 }
 
-int sm_count() {
-  static int n = 0;
-  if (n == 0) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
-  }
-  return n;
-}
-
 template <int EPI>
 cudaError_t launch(const CUtensorMap& tw, const CUtensorMap& tx, const MoeKernelParams& kp, long long max_items,
                    cudaStream_t stream, bool pdl) {
@@ -336,7 +327,7 @@ cudaError_t launch(const CUtensorMap& tw, const CUtensorMap& tx, const MoeKernel
     if (e != cudaSuccess) return e;
     attr_set = true;
   }
-  const dim3 grid(static_cast<unsigned>(max_items < sm_count() ? max_items : sm_count()));
+  const dim3 grid(static_cast<unsigned>(max_items < device_sm_count() ? max_items : device_sm_count()));
   return launch_kernel(kern, grid, dim3(kThreads), kSmemBytes, stream, pdl, 1, tw, tx, kp);
 }
 
