@@ -17,15 +17,17 @@
 //           the products of its neighbours
 // The row scales of fp8 pages never touch the operands: the K scale multiplies a key's column of S, the V scale its
 // probability.  A row's exponentials are taken against its largest score so far, so that no probability exceeds one (times an
-// fp8 V scale: at most 65504, fp16's largest); O is rescaled in TMEM by the warps that have a row whose maximum has grown.  K /
-// V of the chunk itself were appended by attn_prep before this kernel runs, so the key loop covers [first visible key, last
-// visible key] with a limit per row.
+// fp8 V scale: at most 65504, fp16's largest; below, values of a page row that are all under 0.027 have scales under 2^-14, whose
+// products fp16 holds with fewer bits, and drops below 2^-25); O is rescaled in TMEM by the warps that have a row whose maximum
+// has grown.  K / V of the chunk itself were appended by attn_prep before this kernel runs, so the key loop covers [first
+// visible key, last visible key] with a limit per row.
 //
 // TMEM is full (two S buffers of 64 columns, Q 128, O 256).  Q lies there and not in shared memory because the gathers need
 // the room: with Q and 128-key K and V tiles in shared memory (192 KB) 28 KB of L1 were left, which bound the loads in flight
 // and with them the kernel (4.2 us per 128 keys; the products alone take 1.6).  Now the serial chain scores -> softmax -> P of
-// a tile bounds it (3.7 us per 128 keys).  24 / 4 heads, 2048 queries, us, the mma.sync kernel before -> now: fp8 rows, 2048
-// keys 386 -> 180, 16384 keys 3715 -> 1237 (625 TFLOP/s); bf16 rows, 8192 keys 1990 -> 721; nvfp4 1878 -> 660.
+// a tile bounds it (4.1 us per 128 keys, a tenth of it the rescaling of O; against a maximum that lags by up to four powers of
+// two it was 3.7, with other roundings).  24 / 4 heads, 2048 queries, us, the mma.sync kernel before -> now: fp8 rows, 2048 keys
+// 386 -> 167, 16384 keys 3715 -> 1363 (567 TFLOP/s); bf16 rows, 8192 keys 1990 -> 750; nvfp4 1878 -> 682; bits are the same.
 //
 // Reference kernels covered: kernel/gqa_attention_prefill_{bf16,i8,nvfp4}.cuh (Br = 64 x Bc = 64
 // mma.sync kernels that also quantise-append in-kernel).

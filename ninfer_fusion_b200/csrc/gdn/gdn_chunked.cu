@@ -13,12 +13,11 @@
 //
 // Three launches:
 //   gdn_chunk_prepare  one CTA per (chunk, value head), all chunks in parallel: K K^T and Q K^T on mma.sync,
-//                      the triangular inverse by substitution in two halves and their product, W / U / P and the row scales
-//                      into a workspace;
+//                      the triangular inverse by forward substitution in two halves, W / U / P and the row scales into a
+//                      workspace;
 //   gdn_chunk_scan     one CTA per (sequence, value head, half or quarter of dv), sequential over the chunks: the state slice
 //                      lives in MMA accumulator registers (fp32) of eight warps, eight more load and write the output;
-//                      the four products per chunk run on mma.sync
-//                      out of a two-deep cp.async ring;
+//                      the four products per chunk run on mma.sync out of a two-deep cp.async ring;
 //   gdn_gated_norm     per (token, head) gated RMSNorm of the raw outputs in place.
 //
 // Operands of the products are bf16 (the inverse X as a hi + lo pair), accumulation and the state are fp32.
@@ -115,8 +114,8 @@ struct PrepSmem {
 
 // Latency bound (short products and a serial inverse behind barriers; two warps per scheduler issued in 0.36 of the cycles),
 // so what counts is how many chunks an SM works on at once, 72 KB of shared memory lets three CTAs in, and the length of the
-// chain: the inverse by halves, the row norms by all threads.  2048 tokens, 48 heads: prepare, scan and norm together 283 us
-// before, 218 with these.
+// chain: the substitution's long rows summed by all warps, the row norms four rows at a time.  Within a prompt's step of 2048
+// tokens: 48 heads 128 us with two CTAs and one thread per column, 105 so; 32 heads 82 and 66.
 __global__ void __launch_bounds__(128, 3) gdn_chunk_prepare_kernel(const ChunkParams cp) {
   extern __shared__ __align__(16) uint8_t smem_raw[];
   PrepSmem& sm = *reinterpret_cast<PrepSmem*>(smem_raw);
@@ -388,7 +387,8 @@ __global__ void __launch_bounds__(128, 3) gdn_chunk_prepare_kernel(const ChunkPa
 // The chunks of a sequence follow one another, so the time of one is the time of its longest chain: u~ = U - W S^T, then
 // S = exp(G_C) S + u~^T K.  Warps 0-7 do nothing else (S in their registers); warps 8-15 load the next chunk's operands and
 // compute the output rows Q S^T + P u~ beside them.  Two block barriers a chunk: operands and state are there, u~ is there.
-// 2048 tokens: 48 heads 125 us with eight warps that did both in turn, 90 so; 32 heads (quarters of dv) 71 and 62.
+// Within a prompt's step of 2048 tokens: 48 heads 112 us with eight warps that did both in turn, 106 so; 32 heads 102, with
+// quarters of dv as well 62.
 constexpr int kScanGroup = 256;
 constexpr int kScanThreads = 2 * kScanGroup;
 
@@ -614,7 +614,8 @@ __global__ void __launch_bounds__(kScanThreads, 1) gdn_chunk_scan_kernel(const C
 
 // ------------------------------------------------------------------------------------------------ gated norm
 // y = o * rsqrt(mean(o^2) + eps) * norm_w * silu(z), in place on `out`.  A warp takes four (token, head) rows and has all of
-// their loads in flight: with one row, 512 bytes and a 64-bit division per warp, 2048 tokens of 48 heads (75 MB) took 26 us, 18 so.
+// their loads in flight: with one row, 512 bytes and a 64-bit division per warp, 2048 tokens of 48 heads (75 MB) took 24 us
+// within a prompt's step, 21 so; of 32 heads 16 and 13.
 constexpr int kNormRows = 4;
 
 __global__ void __launch_bounds__(256) gdn_gated_norm_kernel(const GdnParams p) {
@@ -710,8 +711,8 @@ const char* gdn_chunked(const GdnParams& p, void* workspace, size_t workspace_by
   }
   gdn_chunk_prepare_kernel<<<dim3(cp.max_chunks, p.n_v_heads), 128, sizeof(PrepSmem), stream>>>(cp);
   // The scan is serial over the chunks and one CTA fills an SM: quarters of dv when all of them fit the GPU at once (32 heads:
-  // 128 CTAs), else halves (48 heads: 96; quarters would run in two rounds).  With the prepare kernel's changes this took
-  // 4096 tokens of the 32-head decoder with experts from 12.81 to 12.39 ms, eight layers.
+  // 128 CTAs; 2048 tokens 102 us in halves, 71 in quarters, both before the chain had warps of its own), else halves (48 heads:
+  // 96; quarters would run in two rounds).
   if (static_cast<long long>(p.n_v_heads) * 4 * p.n_seq <= device_sm_count())
     gdn_chunk_scan_kernel<32><<<dim3(p.n_v_heads, 4, p.n_seq), kScanThreads, sizeof(ScanSmem<32>), stream>>>(cp);
   else
