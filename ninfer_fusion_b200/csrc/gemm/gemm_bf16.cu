@@ -750,39 +750,48 @@ __global__ void __launch_bounds__(128) gemm_ws_kernel(const __grid_constant__ CU
 }
 
 // ------------------------------------------------------------------------------------------------------------
-// Persistent kernel for more than 128 tokens, and for SwiGLU of up to 64 whose weight tiles fill whole rounds: one CTA per SM
-// walks output tiles of 128 weight rows x `tn` tokens, with the roles split over ten warps so that the epilogue of tile i
-// overlaps the main loop of tile i + 1:
-//   warp 0  TMA producer (as many stages of 16 KB weights + tn x 128 B tokens as fit, one running counter over tiles)
+// Persistent kernel for more than 32 tokens, and for SwiGLU of up to 32 whose weight tiles fill whole rounds.  A walker, one
+// CTA or a pair of CTAs (a cluster of two), goes over output tiles of 128 weight rows a CTA x `tn` tokens, with the roles split
+// over ten warps so that the epilogue of tile i overlaps the main loop of tile i + 1:
+//   warp 0  TMA producer (as many stages as fit, one running counter over tiles)
 //   warp 1  MMA issuer; the fp32 accumulator alternates between TMEM columns [0, 256) and [256, 512)
 //   warps 2..9  epilogue: warp w drains TMEM lanes 32 (w % 4) .., every second chunk of 16 tokens; tcgen05.ld -> bias /
 //               activation / residual / SwiGLU -> bf16
 // Two warps per lane group, because with short contractions (K = 2048: 13 us per 128 x 256 tile) one warp per group took
 // longer to drain a tile than the tensor core to fill the next.  Tiles are numbered token-tile fastest, so the CTAs
-// running at one time share a few weight tiles and all token tiles through L2.  The main loop is bound by the tensor
-// rate at 256 tokens and by the operands' latency from L2 below (five stages or more from 224 tokens down, with SwiGLU's
-// exchange from 192).
-// T = 2048, us, before (256 tokens always, four epilogue warps) -> now: 5120 x 6144 residual 131 -> 94, 5120 x 17408
-// residual 332 -> 251, 34816 x 5120 SwiGLU 514 -> 461, 14336 x 5120 219 -> 204, 12352 x 2048 125 -> 84; and with fewer tiles
-// than SMs (one-tile-per-CTA kernel before) 2048 x 4096 55 -> 40, 264 x 2048 33 -> 17.
+// running at one time share a few weight tiles and all token tiles through L2.
+//
+// A single CTA is bound by its shared memory: a k-block of 128 x 64 weights and 256 x 64 tokens is 48 KB written by TMA and
+// 48 KB read by the tensor core at 128 bytes a clock, 390 ns, where the products take 260.  A pair shares the tokens: each CTA
+// loads its own weight rows and half of the tile's tokens (32 KB a k-block, seven stages instead of four), and the even CTA's
+// instruction multiplies 256 weight rows by all tokens.  That is less traffic from L2 as well, and under the power cap less
+// traffic is more clock.  Both forms give the same bits.  Back to back, weights from HBM, us, one CTA a tile -> pair: 2048 tokens
+// 34816 x 5120 SwiGLU 488 -> 463, 5120 x 17408 residual 283 -> 251, 5120 x 6144 97 -> 89, 12352 x 2048 82 -> 75, 8192 x 2048
+// 55 -> 51; 300 tokens 34816 x 5120 107 -> 99, 5120 x 17408 70 -> 63; for seconds at the power cap 34816 x 5120 573 -> 543,
+// 14336 x 5120 262 -> 226.
 constexpr int kPersistMaxTN = 256;
-constexpr int kPersistMinTN = 64;   // narrowest that persist_tile_tokens weighs (SwiGLU of up to 64 tokens: 16, 32 or 64)
+constexpr int kPersistMinTN = 64;   // narrowest single-CTA tile that pick_persist weighs (SwiGLU of up to 32 tokens: 16 or 32)
+constexpr int kPairMinTN = 32;      // narrowest tile of a pair
 constexpr int kPersistMaxStages = 12;
 constexpr int kPersistEpiWarps = 8;
 constexpr int kPersistThreads = 64 + 32 * kPersistEpiWarps;
 constexpr int kPersistSmemBytes = 226 * 1024;
 constexpr int kPersistExchangeBytes = 4 * 2 * 2 * 8 * 32 * 4;   // SwiGLU: per warp pair two buffers x two directions x 8 x 32
 constexpr int persist_ring_bytes(int epi) { return kPersistSmemBytes - 1024 - (epi == kEpiSwiglu ? kPersistExchangeBytes : 0); }
-// Time of one k-block of 64 by tokens per tile, all SMs busy: a line through what widths of 64 to 224 took (246 to 334 ns);
-// where only four stages fit, from 240 tokens or, beside SwiGLU's exchange, from 208, another 30 ns (240 and 256: 368 and 387).
-// (With the 30 ns from 240 for SwiGLU too: 34816 x 5120, 1300 tokens 338 us in tiles of 224, 313 in the 192 taken now; 1830
-// tokens 480 and 462; 24576 x 4096, 1720 tokens 271 and 255.)
+// Time of one k-block of 64 by tokens per tile, all SMs busy, through widths of 64 (one CTA) or 32 (pair) to 256 tokens on
+// weights of 5120 x 17408 and 34816 x 5120.  One CTA: 245 ns at 64, 311 at 128, 350 at 192, 400 at 256; where only four stages
+// fit, from 240 tokens or, beside SwiGLU's exchange, from 208, another 20 ns.  Pair: 192 ns at 32, 218 at 64, 265 at 128 and
+// 160 (weights from L2), then by the products: 300 at 192, 374 at 256.
 constexpr double persist_kblock_ns(int tn, int epi) {
-  return 211. + 0.55 * tn + (persist_ring_bytes(epi) / (kWTileBytes + 128 * tn) < 5 ? 30. : 0.);
+  return 215. + 0.65 * tn + (persist_ring_bytes(epi) / (kWTileBytes + 128 * tn) < 5 ? 20. : 0.);
 }
+constexpr double pair_kblock_ns(int tn) {
+  return tn >= 160 ? 264. + 1.18 * (tn - 160) : tn >= 128 ? 264. : 264. - 0.81 * (128 - tn);
+}
+constexpr double kPairStartNs = 1500.;    // cluster launch, its barriers and the farther commit
 constexpr double kPersistTailNs = 30.;   // per token of the last tile, whose epilogue nothing overlaps
 
-template <int EPI>
+template <int EPI, bool PAIR>
 __global__ void __launch_bounds__(kPersistThreads, 1) gemm_persist_kernel(const __grid_constant__ CUtensorMap tmap_w,
                                                                            const __grid_constant__ CUtensorMap tmap_x,
                                                                            const KernelParams p) {
@@ -799,11 +808,17 @@ __global__ void __launch_bounds__(kPersistThreads, 1) gemm_persist_kernel(const 
   const int lane = threadIdx.x & 31;
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const int TN = p.tn;
-  const int stage_bytes = kWTileBytes + TN * 128;
+  // PAIR: the two CTAs of a cluster work on one tile of twice the weight rows; each loads its own rows and half of the tokens
+  const int crank = PAIR ? static_cast<int>(blockIdx.x & 1) : 0;
+  const int walker = PAIR ? static_cast<int>(blockIdx.x >> 1) : static_cast<int>(blockIdx.x);
+  const int walkers = PAIR ? static_cast<int>(gridDim.x >> 1) : static_cast<int>(gridDim.x);
+  const int x_rows = PAIR ? TN / 2 : TN;
+  const int stage_bytes = kWTileBytes + x_rows * 128;
   constexpr int kRingBytes = persist_ring_bytes(EPI);
   const int n_stages = min(kPersistMaxStages, kRingBytes / stage_bytes);
-  const int w_rows = (EPI == kEpiSwiglu) ? 64 : kTileN;                 // output rows per tile
-  const int n_w_tiles = (EPI == kEpiSwiglu) ? (p.swiglu_half + 63) / 64 : (p.N + kTileN - 1) / kTileN;
+  const int w_rows = (EPI == kEpiSwiglu) ? 64 : kTileN;                 // output rows per CTA and tile
+  const int tile_rows = PAIR ? 2 * w_rows : w_rows;
+  const int n_w_tiles = ((EPI == kEpiSwiglu ? p.swiglu_half : p.N) + tile_rows - 1) / tile_rows;
   const int n_t_tiles = (p.T + TN - 1) / TN;
   const int n_tiles = n_w_tiles * n_t_tiles;
   const int num_kb = p.num_kb;
@@ -817,18 +832,24 @@ __global__ void __launch_bounds__(kPersistThreads, 1) gemm_persist_kernel(const 
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(smem_u32(&bar_acc_full[a]), 1);
-      mbar_init(smem_u32(&bar_acc_empty[a]), kPersistEpiWarps);
+      mbar_init(smem_u32(&bar_acc_empty[a]), PAIR ? 2 * kPersistEpiWarps : kPersistEpiWarps);
     }
     mbar_fence_init();
     tma_prefetch_desc(&tmap_w);
     tma_prefetch_desc(&tmap_x);
   }
   if (warp == 1) {
-    tmem_alloc(smem_u32(&tmem_base_slot), 512);
-    tmem_relinquish();
+    if constexpr (PAIR) {
+      tmem_alloc_pair(smem_u32(&tmem_base_slot), 512);
+      tmem_relinquish_pair();
+    } else {
+      tmem_alloc(smem_u32(&tmem_base_slot), 512);
+      tmem_relinquish();
+    }
   }
   tc_fence_before();
-  __syncthreads();
+  if constexpr (PAIR) cluster_sync_all();   // (the other CTA's barriers are initialised before anything counts on them)
+  else __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = tmem_base_slot;
   pdl_launch_next();
@@ -841,20 +862,23 @@ __global__ void __launch_bounds__(kPersistThreads, 1) gemm_persist_kernel(const 
       int s = 0;
       uint32_t ph = 1;      // the first pass over the ring finds every stage free
       uint32_t issued = 0;
-      auto load_w = [&](int n0, int kb) {
+      // (a pair's stage is counted by the even CTA's barrier, for both halves)
+      auto load = [&](uint32_t dst, const CUtensorMap* map, int kb, int row, uint64_t pol) {
         const uint32_t full = smem_u32(&bar_full[s]);
+        if constexpr (PAIR) tma_load_2d_pair(dst, map, mapa_shared(full, 0), kb * kBlockK, row, pol);
+        else tma_load_2d(dst, map, full, kb * kBlockK, row, pol);
+      };
+      auto load_w = [&](int n0, int kb) {
         const uint32_t dst = smem_base + s * stage_bytes;
-        mbar_expect_tx(full, stage_bytes);
-        tma_load_2d(dst, &tmap_w, full, kb * kBlockK, n0, pol_w);
-        tma_load_2d(dst + 64 * 128, &tmap_w, full, kb * kBlockK, (EPI == kEpiSwiglu) ? p.swiglu_half + n0 : n0 + 64, pol_w);
+        if (crank == 0) mbar_expect_tx(smem_u32(&bar_full[s]), PAIR ? 2 * stage_bytes : stage_bytes);
+        load(dst, &tmap_w, kb, n0, pol_w);
+        load(dst + 64 * 128, &tmap_w, kb, (EPI == kEpiSwiglu) ? p.swiglu_half + n0 : n0 + 64, pol_w);
       };
-      auto load_x = [&](int t0, int kb) {
-        tma_load_2d(smem_base + s * stage_bytes + kWTileBytes, &tmap_x, smem_u32(&bar_full[s]), kb * kBlockK, t0, pol_x);
-      };
+      auto load_x = [&](int t0, int kb) { load(smem_base + s * stage_bytes + kWTileBytes, &tmap_x, kb, t0, pol_x); };
       // Weights do not depend on the previous kernel: the ring is filled with them before it is waited for.
       const int primed = min(n_stages, num_kb);
       {
-        const int n0 = static_cast<int>(blockIdx.x) / n_t_tiles * w_rows, t0 = static_cast<int>(blockIdx.x) % n_t_tiles * TN;
+        const int n0 = walker / n_t_tiles * tile_rows + crank * w_rows, t0 = walker % n_t_tiles * TN + crank * x_rows;
         for (s = 0; s < primed; ++s) load_w(n0, s);
         pdl_wait_prior();  // activations are produced by the previous kernel
         for (s = 0; s < primed; ++s) load_x(t0, s);
@@ -862,9 +886,9 @@ __global__ void __launch_bounds__(kPersistThreads, 1) gemm_persist_kernel(const 
         if (s == n_stages) { s = 0; ph ^= 1; }
       }
       int kb0 = primed;
-      for (int tile = blockIdx.x; tile < n_tiles && !*abortp; tile += gridDim.x) {
-        const int n0 = (tile / n_t_tiles) * w_rows;
-        const int t0 = (tile % n_t_tiles) * TN;
+      for (int tile = walker; tile < n_tiles && !*abortp; tile += walkers) {
+        const int n0 = (tile / n_t_tiles) * tile_rows + crank * w_rows;
+        const int t0 = (tile % n_t_tiles) * TN + crank * x_rows;
         bool ok = true;
         for (int kb = kb0; kb < num_kb; ++kb, ++issued) {
           if (!mbar_wait(smem_u32(&bar_empty[s]), ph, &abort_flag, p.status, kStatusEmptyWaitTimeout)) {
@@ -888,7 +912,8 @@ __global__ void __launch_bounds__(kPersistThreads, 1) gemm_persist_kernel(const 
         }
       }
       if (*abortp) {
-        // Unwinding: let copies that were already issued land before the CTA exits.
+        // Unwinding: let copies that were already issued land before the CTA exits.  (The odd CTA of a pair has no barrier to
+        // see them by: its own never completes, and the polls are the pause.)
         const uint32_t depth = static_cast<uint32_t>(n_stages);
         for (uint32_t j = issued > depth ? issued - depth : 0; j < issued; ++j) {
           const uint32_t bar = smem_u32(&bar_full[j % depth]);
@@ -899,13 +924,17 @@ __global__ void __launch_bounds__(kPersistThreads, 1) gemm_persist_kernel(const 
     }
     __syncwarp();
   } else if (warp == 1) {
-    if (elect_one()) {
-      // ---------------- MMA issuer ----------------
-      const uint32_t idesc = umma_idesc(kTileN, TN, 1, 1);
+    if (crank == 0 && elect_one()) {
+      // ---------------- MMA issuer (of both CTAs of a pair) ----------------
+      const uint32_t idesc = umma_idesc(PAIR ? 2 * kTileN : kTileN, TN, 1, 1);
       int s = 0;
       uint32_t ph = 0;
       int tile_i = 0;
-      for (int tile = blockIdx.x; tile < n_tiles && !*abortp; tile += gridDim.x, ++tile_i) {
+      auto commit = [](uint32_t bar) {
+        if constexpr (PAIR) tc_commit_pair(bar);
+        else tc_commit(bar);
+      };
+      for (int tile = walker; tile < n_tiles && !*abortp; tile += walkers, ++tile_i) {
         const int a = tile_i & 1;
         const uint32_t aph = (tile_i >> 1) & 1;
         // the epilogue has drained this accumulator's previous tile
@@ -925,13 +954,16 @@ __global__ void __launch_bounds__(kPersistThreads, 1) gemm_persist_kernel(const 
           const uint64_t a_desc = umma_desc_k_sw128(a_addr);
           const uint64_t b_desc = umma_desc_k_sw128(a_addr + kWTileBytes);
 #pragma unroll
-          for (int k = 0; k < kBlockK / 16; ++k)
-            tc_mma_f16(acc, a_desc + 2 * k, b_desc + 2 * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
-          tc_commit(smem_u32(&bar_empty[s]));
+          for (int k = 0; k < kBlockK / 16; ++k) {
+            const uint32_t accumulate = (kb > 0 || k > 0) ? 1u : 0u;
+            if constexpr (PAIR) tc_mma_f16_pair(acc, a_desc + 2 * k, b_desc + 2 * k, idesc, accumulate);
+            else tc_mma_f16(acc, a_desc + 2 * k, b_desc + 2 * k, idesc, accumulate);
+          }
+          commit(smem_u32(&bar_empty[s]));
           if (++s == n_stages) { s = 0; ph ^= 1; }
         }
         if (!ok) break;
-        tc_commit(smem_u32(&bar_acc_full[a]));
+        commit(smem_u32(&bar_acc_full[a]));
       }
     }
     __syncwarp();
@@ -944,14 +976,14 @@ __global__ void __launch_bounds__(kPersistThreads, 1) gemm_persist_kernel(const 
     float* const xch_s = reinterpret_cast<float*>(smem_raw + (smem_base - smem_u32(smem_raw)) + kRingBytes);
     const int pair = (lg & 1) + 2 * half;
     int tile_i = 0, xch_i = 0;
-    for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x, ++tile_i) {
+    for (int tile = walker; tile < n_tiles; tile += walkers, ++tile_i) {
       const int a = tile_i & 1;
       const uint32_t ph = (tile_i >> 1) & 1;
       const bool have = mbar_wait(smem_u32(&bar_acc_full[a]), ph, &abort_flag, p.status, kStatusAccumWaitTimeout);
       // one verdict for the eight warps, so that the pair barriers below are never divergent
       if (!epi_all(have && !*abortp)) break;
       tc_fence_after();
-      const int n0 = (tile / n_t_tiles) * w_rows;
+      const int n0 = (tile / n_t_tiles) * tile_rows + crank * w_rows;
       const int t0 = (tile % n_t_tiles) * TN;
       const int cols = min(TN, p.T - t0);     // live tokens of the tile
       const uint32_t lane_taddr = tmem_base + a * kPersistMaxTN + (static_cast<uint32_t>(lg * 32) << 16);
@@ -1057,35 +1089,52 @@ __global__ void __launch_bounds__(kPersistThreads, 1) gemm_persist_kernel(const 
       // this warp is done with the accumulator: hand it back to the MMA issuer
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(smem_u32(&bar_acc_empty[a]));
+      if (lane == 0) {
+        if constexpr (PAIR) mbar_arrive_cluster(mapa_shared(smem_u32(&bar_acc_empty[a]), 0));
+        else mbar_arrive(smem_u32(&bar_acc_empty[a]));
+      }
     }
   }
 
   tc_fence_before();
-  __syncthreads();
-  if (warp == 1) tmem_dealloc(tmem_base, 512);
+  if constexpr (PAIR) {
+    cluster_sync_all();   // (the other CTA neither reads this one's operands nor arrives on its barriers any more)
+    if (warp == 1) tmem_dealloc_pair(tmem_base, 512);
+  } else {
+    __syncthreads();
+    if (warp == 1) tmem_dealloc(tmem_base, 512);
+  }
 }
 
-// Tokens per tile of the persistent kernel: the width (a multiple of 16) with the least estimated time.  `w_tiles` tiles
-// of weight rows times the token tiles are dealt out in rounds of one tile per SM; what a fixed 256 loses is the last
-// round (N = 5120, T = 2048: 320 tiles = 2.16 rounds, paid as 3; 192 tokens make it 2.97) or, with few tiles, the SMs that
-// get none (N = 264: 24 tiles of 256 against 96 of 64).
-int persist_tile_tokens(int T, int w_tiles, int num_kb, int sms, int epi) {
-  int best = kPersistMaxTN;
+// Tokens per tile of the persistent kernel and whether pairs of CTAs walk them: the width (a multiple of 16) and form with the
+// least estimated time.  `rows` output rows in tiles of 128 a CTA (64 beside SwiGLU) times the token tiles are dealt out in
+// rounds of one tile per walker; what a fixed 256 loses is the last round (N = 5120, T = 2048: 160 tiles of 74 pairs = 2.16
+// rounds, paid as 3; 192 tokens make it 2.97) or, with few tiles, the SMs that get none (N = 264: 16 tiles of 256 tokens
+// against 64 of 64).  One CTA a tile is left with short contractions in one round (us, one CTA and pair: 2048 x 512 9.3 and
+// 10.7, 2048 x 2048 16.9 and 17.9, 2048 tokens), and is not weighed up to 128 tokens, where pairs were the faster at every size
+// tried.
+struct PersistPlan { int tn; bool pair; };
+PersistPlan pick_persist(int T, int rows, int num_kb, int sms, int epi) {
+  PersistPlan best = {kPersistMaxTN, true};
   double best_ns = 0;
-  for (int tn = kPersistMaxTN; tn >= kPersistMinTN; tn -= 16) {
-    const long long tiles = static_cast<long long>(w_tiles) * ((T + tn - 1) / tn);
-    const long long rounds = (tiles + sms - 1) / sms;
-    const double ns = static_cast<double>(rounds) * num_kb * persist_kblock_ns(tn, epi) + kPersistTailNs * tn;
-    if (best_ns == 0 || ns < best_ns * 0.99) { best = tn; best_ns = ns; }
+  const int cta_rows = epi == kEpiSwiglu ? 64 : kTileN;
+  for (int pair = 1; pair >= (T > 128 ? 0 : 1); --pair) {
+    const int w_tiles = (rows + (cta_rows << pair) - 1) / (cta_rows << pair);
+    for (int tn = kPersistMaxTN; tn >= (pair ? kPairMinTN : kPersistMinTN); tn -= 16) {
+      const long long tiles = static_cast<long long>(w_tiles) * ((T + tn - 1) / tn);
+      const long long rounds = (tiles + (sms >> pair) - 1) / (sms >> pair);
+      const double ns = static_cast<double>(rounds) * num_kb * (pair ? pair_kblock_ns(tn) : persist_kblock_ns(tn, epi)) +
+                        kPersistTailNs * tn + (pair ? kPairStartNs : 0.);
+      if (best_ns == 0 || ns < best_ns * 0.99) { best = {tn, pair != 0}; best_ns = ns; }
+    }
   }
   return best;
 }
 
-template <int EPI>
-cudaError_t launch_persist(const CUtensorMap& tw, const CUtensorMap& tx, const KernelParams& kp, int n_tiles,
+template <int EPI, bool PAIR>
+cudaError_t launch_walkers(const CUtensorMap& tw, const CUtensorMap& tx, const KernelParams& kp, int n_tiles,
                            cudaStream_t stream, bool pdl) {
-  auto kern = gemm_persist_kernel<EPI>;
+  auto kern = gemm_persist_kernel<EPI, PAIR>;
   static bool attr_set = false;
   if (!attr_set) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kPersistSmemBytes);
@@ -1093,16 +1142,35 @@ cudaError_t launch_persist(const CUtensorMap& tw, const CUtensorMap& tx, const K
     attr_set = true;
   }
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(n_tiles < device_sm_count() ? n_tiles : device_sm_count());
+  constexpr int kCtas = PAIR ? 2 : 1;
+  const int walkers = device_sm_count() / kCtas;
+  cfg.gridDim = dim3(kCtas * (n_tiles < walkers ? n_tiles : walkers));
   cfg.blockDim = dim3(kPersistThreads);
   cfg.dynamicSmemBytes = kPersistSmemBytes;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchAttribute attr[2];
+  int n_attr = 0;
+  if (PAIR) {
+    attr[n_attr].id = cudaLaunchAttributeClusterDimension;
+    attr[n_attr].val.clusterDim.x = kCtas;
+    attr[n_attr].val.clusterDim.y = 1;
+    attr[n_attr].val.clusterDim.z = 1;
+    ++n_attr;
+  }
+  if (pdl) {
+    attr[n_attr].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[n_attr].val.programmaticStreamSerializationAllowed = 1;
+    ++n_attr;
+  }
   cfg.attrs = attr;
-  cfg.numAttrs = pdl ? 1 : 0;
+  cfg.numAttrs = n_attr;
   return cudaLaunchKernelEx(&cfg, kern, tw, tx, kp);
+}
+
+template <int EPI>
+cudaError_t launch_persist(bool pair, const CUtensorMap& tw, const CUtensorMap& tx, const KernelParams& kp, int n_tiles,
+                           cudaStream_t stream, bool pdl) {
+  return pair ? launch_walkers<EPI, true>(tw, tx, kp, n_tiles, stream, pdl) : launch_walkers<EPI, false>(tw, tx, kp, n_tiles, stream, pdl);
 }
 
 template <int TN, int EPI, bool DEEP>
@@ -1343,22 +1411,6 @@ int gemm_pick_splits(int T, int N, int K, int epi, int sm_count) {
   return s < 1 ? 1 : s;
 }
 
-namespace {
-
-// Tokens per tile for 65 to 256 tokens.  With few tiles of weight rows a tile that holds all tokens leaves most SMs idle
-// (N = 2048: 16 CTAs walk the whole contraction), so the narrower of 32 and 64 whose tiles all run at once is taken: a k-block
-// of a narrower tile takes less time (persist_kblock_ns), its epilogue too, and the weights are read once from HBM and again
-// from L2.  The contraction is not cut: a row's sums keep one order whatever the number of rows beside it.  One tile of 128 or
-// 256 tokens -> now, us: 128 tokens 2048 x 4096 33 -> 25, 264 x 2048 22 -> 16, 5120 x 17408 78 -> 70; 256 tokens 49 -> 25,
-// 33 -> 16, 125 -> 76.
-int narrow_tile(int T, int w_tiles, int tn) {
-  for (int n = 32; n <= 64; n *= 2)
-    if (static_cast<long long>(w_tiles) * ((T + n - 1) / n) <= device_sm_count()) return n;
-  return tn;
-}
-
-}  // namespace
-
 const char* gemm_bf16(const GemmArgs& a) {
   if (a.T <= 0 || a.N <= 0 || a.K <= 0) return "gemm_bf16: empty problem";
   if ((a.K % 8) || (a.ldw % 8) || (a.ldx % 8)) return "gemm_bf16: K and leading dims must be multiples of 8";
@@ -1372,7 +1424,7 @@ const char* gemm_bf16(const GemmArgs& a) {
         a.ldo32 < a.N - a.out32_from || (reinterpret_cast<uintptr_t>(a.out32) & 7))
       return "gemm_bf16: fp32 columns must start at an even column and have an even leading dimension";
   }
-  int tn = gemm_tile_tokens(static_cast<int>(a.T));
+  const int tn = gemm_tile_tokens(static_cast<int>(a.T));
   const bool global_split = a.epi == kEpiPartial || a.epi == kEpiPushPartial;
   const bool plain = (a.epi == kEpiStore || a.epi == kEpiResidual || a.epi == kEpiSwiglu) && a.gather.flag == nullptr &&
                      a.conv.state == nullptr;
@@ -1385,7 +1437,6 @@ const char* gemm_bf16(const GemmArgs& a) {
   int splits = a.splits < 1 ? 1 : a.splits;
   if (splits > kp.num_kb) splits = kp.num_kb;
   if (splits != (a.splits < 1 ? 1 : a.splits)) return "gemm_bf16: split count leaves an empty split";
-  if (splits == 1 && plain && tn >= 128 && kp.T <= 256) tn = narrow_tile(kp.T, w_tiles, tn);
   kp.kb_per_split = (kp.num_kb + splits - 1) / splits;
   if ((kp.num_kb + kp.kb_per_split - 1) / kp.kb_per_split != splits) return "gemm_bf16: split count leaves an empty split";
   kp.cluster = 1;
@@ -1483,35 +1534,39 @@ const char* gemm_bf16(const GemmArgs& a) {
   const bool needs_out = !all32 && (a.epi == kEpiStore || a.epi == kEpiResidual || a.epi == kEpiSwiglu);
   if (needs_out && a.out == nullptr) return "gemm_bf16: no output";
 
-  // More than 128 tokens (that no narrow tile takes) and a plain epilogue: persistent kernel, epilogue overlapped with the next
-  // main loop
+  // More than 32 tokens and a plain epilogue: persistent kernel, epilogue overlapped with the next main loop.  One tile of 64,
+  // 128 or 256 tokens per CTA, or narrower ones, before -> pairs now, us: 48 tokens 16480 x 5120 28.0 -> 26.9, 24576 x 4096
+  // SwiGLU 42.0 -> 38.1; 80 tokens 34816 x 5120 SwiGLU 90 -> 54; 128 tokens 12352 x 2048 18.5 -> 14.0, 1024 x 2048 SwiGLU
+  // 12.1 -> 9.6, 248320 x 2048 278 -> 166; 256 tokens 5120 x 17408 residual 67 -> 58.  Up to 32 tokens pairs lose what the
+  // cluster costs (one token: 12352 x 2048 11.3 and 11.7, the language-model head 355 and 374) or, with a split contraction, more.
   // (NFB_GEMM_PERSISTENT=0 keeps the one-tile-per-CTA kernel for every size)
   static const bool persistent_enabled = [] {
     const char* e = getenv("NFB_GEMM_PERSISTENT");
     return !(e != nullptr && e[0] == '0');
   }();
-  // Up to 64 tokens, SwiGLU with more weight tiles than SMs and at least three quarters of them busy in the last round: the
-  // same kernel streams the weights in whole rounds of one tile per SM, where two CTAs per SM run them in one.  34816 x 5120,
-  // 272 tiles, 1.84 rounds: 37 tokens 75.8 -> 67.6 us, one token 70.1 -> 69.6; 24576 x 4096, 192 tiles, whose second round would
+  // Up to 32 tokens, SwiGLU with more weight tiles than SMs and at least three quarters of them busy in the last round: the
+  // same kernel, one CTA a tile, streams the weights in whole rounds of one tile per SM, where two CTAs per SM run them in one.
+  // 34816 x 5120, 272 tiles, 1.84 rounds: one token 70.1 -> 69.6 us; 24576 x 4096, 192 tiles, whose second round would
   // leave 104 SMs idle: one token 47.1 us with two CTAs per SM, 50.1 in rounds.  (The plain store gained nothing, the
   // language-model head lost 1 %.)
   const int last_round = w_tiles % device_sm_count();
-  const bool stream = tn <= 64 && a.epi == kEpiSwiglu && w_tiles > device_sm_count() &&
+  const bool stream = tn <= 32 && a.epi == kEpiSwiglu && w_tiles > device_sm_count() &&
                       (last_round == 0 || 4 * last_round >= 3 * device_sm_count());
-  const bool persistent = (tn == 256 || stream) && splits == 1 && persistent_enabled && !g_trace_enabled && plain;
-  const int box_tokens = persistent && !stream ? persist_tile_tokens(kp.T, w_tiles, kp.num_kb, device_sm_count(), a.epi) : tn;
-  kp.tn = box_tokens;
+  const bool persistent = (tn > 32 || stream) && splits == 1 && persistent_enabled && !g_trace_enabled && plain;
+  const int out_rows = a.epi == kEpiSwiglu ? kp.N / 2 : kp.N;
+  const PersistPlan plan = persistent && !stream ? pick_persist(kp.T, out_rows, kp.num_kb, device_sm_count(), a.epi) : PersistPlan{tn, false};
+  kp.tn = plan.tn;
 
   CUtensorMap tw, tx;
   if (!cached_tmap(&tw, a.w, a.N, a.K, a.ldw, 64)) return "gemm_bf16: weight tensor map rejected";
-  if (!cached_tmap(&tx, a.x, a.T, a.K, a.ldx, box_tokens)) return "gemm_bf16: activation tensor map rejected";
+  if (!cached_tmap(&tx, a.x, a.T, a.K, a.ldx, plan.pair ? plan.tn / 2 : plan.tn)) return "gemm_bf16: activation tensor map rejected";
 
   dim3 grid;
-  grid.x = w_tiles;
-  grid.y = (kp.T + box_tokens - 1) / box_tokens;
+  grid.x = plan.pair ? (w_tiles + 1) / 2 : w_tiles;
+  grid.y = (kp.T + plan.tn - 1) / plan.tn;
   grid.z = splits;
   if (a.prefetch != nullptr && a.prefetch_bytes > 0 && (reinterpret_cast<uintptr_t>(a.prefetch) & 15) == 0) {
-    long long ctas = static_cast<long long>(grid.x) * grid.y * grid.z;
+    long long ctas = static_cast<long long>(grid.x) * grid.y * grid.z * (plan.pair ? 2 : 1);
     if (persistent && ctas > device_sm_count()) ctas = device_sm_count();
     long long per = (a.prefetch_bytes + ctas - 1) / ctas;
     per = (per + 4095) & ~4095LL;                 // whole 4 KB pieces per CTA
@@ -1524,9 +1579,9 @@ const char* gemm_bf16(const GemmArgs& a) {
   if (persistent) {
     const int n_tiles = static_cast<int>(grid.x * grid.y);
     switch (a.epi) {
-      case kEpiStore: e = launch_persist<kEpiStore>(tw, tx, kp, n_tiles, a.stream, a.pdl); break;
-      case kEpiResidual: e = launch_persist<kEpiResidual>(tw, tx, kp, n_tiles, a.stream, a.pdl); break;
-      default: e = launch_persist<kEpiSwiglu>(tw, tx, kp, n_tiles, a.stream, a.pdl); break;
+      case kEpiStore: e = launch_persist<kEpiStore>(plan.pair, tw, tx, kp, n_tiles, a.stream, a.pdl); break;
+      case kEpiResidual: e = launch_persist<kEpiResidual>(plan.pair, tw, tx, kp, n_tiles, a.stream, a.pdl); break;
+      default: e = launch_persist<kEpiSwiglu>(plan.pair, tw, tx, kp, n_tiles, a.stream, a.pdl); break;
     }
     return e == cudaSuccess ? nullptr : cudaGetErrorString(e);
   }

@@ -178,6 +178,33 @@ def test_gemm_persistent_prefill_kernel(ops, status, T):
     status.check("persistent gemm")
 
 
+@pytest.mark.parametrize("T", [33, 48, 64, 65, 97, 128, 200])
+@pytest.mark.parametrize("N,K", [(64, 1024), (128, 72), (130, 1096), (384, 4096), (20040, 512)])
+def test_gemm_cta_pairs(ops, status, T, N, K):
+    """Tiles of a pair of CTAs: weight rows that leave the second CTA without any, token halves that lie past the last token,
+    more tiles than pairs, contractions shorter than the ring; nothing is written beside the output."""
+    x, w = _mk(T, N, K, seed=6)
+    ref = x.float() @ w.float().t()
+    wide = torch.full((T + 1, N + 2), float("nan"), device="cuda", dtype=torch.bfloat16)
+    ops.gemm_bf16(x, w, wide[:T, :N], EPI_STORE, None, None, None, 1, status.tensor, False)
+    # one rounding to bf16 (2^-9) and fp32 sums of K products in another order
+    assert (wide[:T, :N].float() - ref).abs().max() <= ref.abs().max() * 2.0 ** -8
+    assert wide[T].isnan().all() and wide[:, N:].isnan().all()
+    resid = torch.randn(T, N, device="cuda").to(torch.bfloat16)
+    got = resid.clone()
+    ops.gemm_bf16(x, w, got, EPI_RESIDUAL, got, None, None, 1, status.tensor, True)
+    want = resid.float() + ref
+    assert (got.float() - want).abs().max() <= want.abs().max() * 2.0 ** -8
+    if N % 4 == 0:
+        act = torch.full((T + 1, N // 2), float("nan"), device="cuda", dtype=torch.bfloat16)
+        ops.gemm_bf16(x, w, act[:T], EPI_SWIGLU, None, None, None, 1, status.tensor, True)
+        want = torch.nn.functional.silu(ref[:, : N // 2]) * ref[:, N // 2:]
+        # (the sigmoid's hardware exponential and quotient beside the rounding: 2^-7 of the largest unit)
+        assert (act[:T].float() - want).abs().max() <= want.abs().max() * 2.0 ** -7
+        assert act[T].isnan().all()
+    status.check("pairs")
+
+
 @pytest.mark.parametrize("T", [65, 128, 129, 160, 256, 257, 300, 1873])
 @pytest.mark.parametrize("N,K", [(264, 2048), (2048, 520), (2048, 4096), (5120, 128)])
 def test_gemm_token_tiles(ops, status, T, N, K):
