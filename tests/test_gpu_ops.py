@@ -247,6 +247,40 @@ def test_conv_and_gdn_recurrent(ops, lens, heads):
         assert torch.equal(ssm_g[s].cpu(), ssm[s])
 
 
+@pytest.mark.parametrize("heads", [(16, 48), (16, 32)])
+@pytest.mark.parametrize("pdl", [False, True])
+@pytest.mark.parametrize("ragged", [False, True])
+def test_gdn_step_of_many_states(ops, heads, pdl, ragged):
+    """Enough states for the streaming kernel, the last round of a part of the CTAs; `commit` of ones takes the general kernel.
+    Ragged: as many tokens as sequences, but sequences of none and of several."""
+    torch.manual_seed(3)
+    (hk, hv), d = heads, 128
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    B = -(-13 * sms // (2 * hv)) + 1
+    qk, vd = hk * d, hv * d
+    C = 2 * qk + vd
+    ld = C + vd + 2 * hv
+    conv = torch.randn(B, C, device="cuda").to(torch.bfloat16)
+    proj = torch.randn(B, ld, device="cuda").to(torch.bfloat16)
+    A_log, dt_bias = torch.rand(hv, device="cuda") * 2 - 1, torch.rand(hv, device="cuda") * 2 - 1.5
+    nw = (1 + 0.1 * torch.randn(d, device="cuda")).to(torch.bfloat16)
+    lens = [1] * B
+    if ragged:
+        lens[0], lens[1], lens[5], lens[6], lens[7], lens[B - 1] = 0, 2, 0, 3, 0, 1
+        assert sum(lens) == B
+    cu = torch.tensor([0] + lens, device="cuda").cumsum(0).int()
+    slot = torch.randperm(B + 1, device="cuda")[:B].int()
+    states = torch.randn(B + 1, hv, d, d, device="cuda") * 0.2
+    got = []
+    for commit in (torch.ones(B, dtype=torch.uint8, device="cuda"), None):
+        s, out = states.clone(), torch.full((B, vd), float("nan"), dtype=torch.bfloat16, device="cuda")
+        ops.gdn_recurrent(conv, 0, qk, 2 * qk, proj, C, C + vd, C + vd + hv, hk, hv, A_log, dt_bias, nw, 1e-6, cu, slot, s, True, out,
+                          pdl, None, commit)
+        got.append((s, out))
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
+    assert not got[1][1].isnan().any() and not torch.equal(got[1][0], states)
+
+
 @pytest.mark.parametrize("T", [9, 200])
 def test_embed_rmsnorm(ops, T):
     torch.manual_seed(0)
