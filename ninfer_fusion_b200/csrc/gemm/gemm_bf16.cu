@@ -975,6 +975,7 @@ __global__ void __launch_bounds__(kPersistThreads, 1) gemm_persist_kernel(const 
     constexpr int kChunk = 16;
     float* const xch_s = reinterpret_cast<float*>(smem_raw + (smem_base - smem_u32(smem_raw)) + kRingBytes);
     const int pair = (lg & 1) + 2 * half;
+    const uint32_t select = swap_select(lane);
     int tile_i = 0, xch_i = 0;
     for (int tile = walker; tile < n_tiles; tile += walkers, ++tile_i) {
       const int a = tile_i & 1;
@@ -1005,6 +1006,7 @@ __global__ void __launch_bounds__(kPersistThreads, 1) gemm_persist_kernel(const 
           for (int j = 0; j < 8; ++j) mine[j * 32 + lane] = __uint_as_float(is_up ? v[j] : v[8 + j]);
           epi_pair_sync(pair);
           const int tb = t0 + c + (is_up ? 8 : 0);
+          uint32_t w[4];
 #pragma unroll
           for (int m = 0; m < 4; ++m) {
             float o2[2];
@@ -1015,14 +1017,11 @@ __global__ void __launch_bounds__(kPersistThreads, 1) gemm_persist_kernel(const 
               const float got = other[j * 32 + lane];
               o2[h] = gated_unit(is_up ? got : own, is_up ? own : got, p.glu);
             }
-            const float send = (lane & 1) ? o2[0] : o2[1];
-            const float recv = __shfl_xor_sync(0xffffffffu, send, 1);
-            const int t = tb + 2 * m + (lane & 1);
-            if (t < p.T && ne < p.swiglu_half) {
-              const uint32_t packed = (lane & 1) ? pack_bf16x2(recv, o2[1]) : pack_bf16x2(o2[0], recv);
-              *reinterpret_cast<uint32_t*>(p.out + static_cast<long long>(t) * p.ldo + ne) = packed;
-            }
+            const __nv_bfloat162 units = __floats2bfloat162_rn(o2[0], o2[1]);
+            w[m] = swap_pair(*reinterpret_cast<const uint32_t*>(&units), select);
           }
+          const int live = ne < p.swiglu_half ? (p.T - tb - (lane & 1) + 1) >> 1 : 0;
+          store_rows<4>({p.out + static_cast<long long>(tb + (lane & 1)) * p.ldo + ne, 2 * p.ldo, live}, w);
         }
       } else {
         const int n = n0 + lg * 32 + lane;
@@ -1030,22 +1029,16 @@ __global__ void __launch_bounds__(kPersistThreads, 1) gemm_persist_kernel(const 
         const float bias = (p.bias != nullptr && n < p.N) ? p.bias[n] : 0.f;
         const float act_a = EPI == kEpiStore && p.act_params != nullptr ? p.act_params[0] : 0.f;
         const float act_b = EPI == kEpiStore && p.act_params != nullptr ? p.act_params[1] : 0.f;
-        const bool to32 = EPI == kEpiStore && p.out32 != nullptr && ne >= p.out32_from;
+        const bool has32 = EPI == kEpiStore && p.out32 != nullptr && n0 + kTileN > p.out32_from;   // (of the tile)
+        const long long row0 = t0 + (lane & 1);
+        auto live = [&](int c) { return ne < p.N ? min(8, (p.T - t0 - c - (lane & 1) + 1) >> 1) : 0; };
         // The residual may alias the output (in-place update): a chunk's values are fetched one chunk ahead, so that
         // their latency runs beside the chunk before and no load waits for a store.
-        __nv_bfloat162 r2[kChunk / 2];
-        auto fetch = [&](int c) {
-#pragma unroll
-          for (int m = 0; m < kChunk / 2; ++m) {
-            const int t = t0 + c + 2 * m + (lane & 1);
-            r2[m] = (t < p.T && ne < p.N)
-                        ? *reinterpret_cast<const __nv_bfloat162*>(p.resid + static_cast<long long>(t) * p.ldr + ne)
-                        : __nv_bfloat162();
-          }
-        };
+        uint32_t r2[kChunk / 2];
+        auto fetch = [&](int c) { load_rows8({p.resid + (row0 + c) * p.ldr + ne, 2 * p.ldr, live(c)}, r2); };
         if constexpr (EPI == kEpiResidual) fetch(half * kChunk);
         for (int c = half * kChunk; c < cols; c += 2 * kChunk) {
-          __nv_bfloat162 r[kChunk / 2];
+          uint32_t r[kChunk / 2];
           if constexpr (EPI == kEpiResidual) {
 #pragma unroll
             for (int m = 0; m < kChunk / 2; ++m) r[m] = r2[m];
@@ -1066,22 +1059,20 @@ __global__ void __launch_bounds__(kPersistThreads, 1) gemm_persist_kernel(const 
               for (int j = 0; j < kChunk; ++j) f[j] = activate(f[j], p.act, act_a, act_b);
             }
           }
+          if (!has32) {
+            store_chunk<EPI == kEpiResidual>({p.out + (row0 + c) * p.ldo + ne, 2 * p.ldo, live(c)}, f, r, select);
+          } else {
+            // columns from out32_from on as fp32: pairs swapped in full
+            const int n_live = live(c);
 #pragma unroll
-          for (int m = 0; m < kChunk / 2; ++m) {
-            const float send = (lane & 1) ? f[2 * m] : f[2 * m + 1];
-            const float recv = __shfl_xor_sync(0xffffffffu, send, 1);
-            const int t = t0 + c + 2 * m + (lane & 1);
-            if (t < p.T && ne < p.N) {
-              float lo = (lane & 1) ? recv : f[2 * m];
-              float hi = (lane & 1) ? f[2 * m + 1] : recv;
-              if constexpr (EPI == kEpiResidual) {
-                lo += __bfloat162float(r[m].x);
-                hi += __bfloat162float(r[m].y);
+            for (int m = 0; m < kChunk / 2; ++m) {
+              const float recv = __shfl_xor_sync(0xffffffffu, (lane & 1) ? f[2 * m] : f[2 * m + 1], 1);
+              const float lo = (lane & 1) ? recv : f[2 * m], hi = (lane & 1) ? f[2 * m + 1] : recv;
+              const long long t = row0 + c + 2 * m;
+              if (m < n_live) {
+                if (ne >= p.out32_from) *reinterpret_cast<float2*>(p.out32 + t * p.ldo32 + ne - p.out32_from) = make_float2(lo, hi);
+                else *reinterpret_cast<uint32_t*>(p.out + t * p.ldo + ne) = pack_bf16x2(lo, hi);
               }
-              if (to32)
-                *reinterpret_cast<float2*>(p.out32 + static_cast<long long>(t) * p.ldo32 + ne - p.out32_from) = make_float2(lo, hi);
-              else
-                *reinterpret_cast<uint32_t*>(p.out + static_cast<long long>(t) * p.ldo + ne) = pack_bf16x2(lo, hi);
             }
           }
         }
