@@ -31,6 +31,7 @@
 #include "../common/ptx.cuh"
 #include "../common/tensor_map.h"
 #include "../kv/codec.cuh"
+#include "persist_epilogue.cuh"
 
 namespace nfb {
 
@@ -514,36 +515,43 @@ __global__ void __launch_bounds__(256) quant_act_nvfp4_kernel(const __nv_bfloat1
 }
 
 // ------------------------------------------------------------------------------------------------------------
-// Persistent prefill kernel for quantised weights: the same role split as the bf16 one (gemm_bf16.cu) -- warp 0 TMA,
-// warp 1 MMA with the accumulator alternating between two TMEM column ranges, warps 2..5 epilogue -- so the epilogue
-// of tile i overlaps the main loop of tile i + 1.  With fp8 / nvfp4 the main loop is 2-4 x shorter than in bf16 while
-// the epilogue is the same size, so the one-tile-per-CTA kernel spends most of its time in epilogues.
-//   fp8 row-scale: 256-token tiles, accumulators at TMEM columns [0, 256) and [256, 512)
-//   nvfp4:         128-token tiles, accumulators at [0, 128) and [128, 256), scale factors at [256, 288)
-template <int QT>
+// Persistent kernel for quantised weights and more than 64 tokens: the same role split as the bf16 one (gemm_bf16.cu) -- warp 0
+// TMA, warp 1 MMA, warps 2..9 epilogue -- so the epilogue of tile i overlaps the main loop of tile i + 1.  With fp8 / nvfp4 the
+// main loop is 2-4 x shorter than in bf16 while the epilogue is the same size, so the one-tile-per-CTA kernel spends most of its
+// time in epilogues.
+//   fp8 row-scale: tiles of 128 or 256 tokens, two accumulators
+//   nvfp4:         128 tokens, accumulators at TMEM columns [0, 128) and [128, 256), scale factors behind them; or 256 tokens,
+//                  one accumulator at [0, 256), scale factors behind it
+// The nvfp4 main loop is bound by shared memory, not by the tensor cores: a k-block of 128 rows and 128 tokens is 36 KB
+// written and 32 KB read, 530 clocks at 128 bytes each, for 256 clocks of products; 256 tokens are 102 KB, 800 clocks, so the
+// wide tile saves a quarter and pays with an epilogue that overlaps only the loads of the next tile (two accumulators of 256
+// columns leave no room for the scales).
+template <int QT, int TILE>
 struct QPersist {
   static constexpr bool kBS = QT == kQNvfp4;
-  static constexpr int TN = kBS ? 128 : 256;
+  static constexpr int TN = TILE;
   static constexpr int kXTileBytes = TN * kKBytes;
   static constexpr int kSfaBytes = kBS ? 4 * kSfTileBytes : 0;
-  static constexpr int kSfbBytes = kBS ? 4 * kSfTileBytes : 0;
+  static constexpr int kSfbStep = TN <= 128 ? 4 : 8;              // TMEM columns of the token scales of one MMA
+  static constexpr int kSfbBytes = kBS ? kSfbStep * kSfTileBytes : 0;
   static constexpr int kStageBytes = kWTileBytes + kXTileBytes + kSfaBytes + kSfbBytes;
-  static constexpr int kStages = kBS ? 5 : 4;
-  static constexpr int kExchangeBytes = 2 * 16 * 64 * 4;
+  static constexpr int kStages = TN == 128 ? (kBS ? 5 : 6) : 4;
+  static constexpr int kExchangeBytes = 4 * 2 * 8 * 32 * 4;       // SwiGLU: per warp pair two directions x 8 x 32
   static constexpr int kSmemBytes = kStages * kStageBytes + kExchangeBytes + 1024;
-  static constexpr int kSfaCol = 2 * TN;
-  static constexpr int kSfbCol = 2 * TN + 16;
+  static constexpr int kAccs = kBS && TN == 256 ? 1 : 2;
+  static constexpr int kSfaCol = kAccs * TN;
+  static constexpr int kSfbCol = kAccs * TN + 16;
+  static_assert(kSmemBytes <= 227 * 1024 && (!kBS || kSfbCol + 4 * kSfbStep <= 512), "does not fit an SM");
 };
-constexpr int kQPersistThreads = 192;
+constexpr int kQPersistThreads = 64 + 256;
 
-__device__ __forceinline__ void q_epi_bar_sync() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
-
-template <int QT, int EPI>
+template <int QT, int EPI, int TILE>
 __global__ void __launch_bounds__(kQPersistThreads, 1) gemm_q_persist_kernel(const __grid_constant__ CUtensorMap tmap_w,
                                                                               const __grid_constant__ CUtensorMap tmap_x,
                                                                               const QParams p) {
   static_assert(EPI == kEpiStore || EPI == kEpiResidual || EPI == kEpiSwiglu, "persistent kernel: plain epilogues only");
-  using Cfg = QPersist<QT>;
+  using Cfg = QPersist<QT, TILE>;
+  constexpr int kAccs = Cfg::kAccs;
   constexpr int TN = Cfg::TN;
   constexpr int kStages = Cfg::kStages;
   constexpr bool kBS = Cfg::kBS;
@@ -554,7 +562,6 @@ __global__ void __launch_bounds__(kQPersistThreads, 1) gemm_q_persist_kernel(con
   __shared__ __align__(8) uint64_t bar_acc_empty[2];
   __shared__ uint32_t tmem_base_slot;
   __shared__ int abort_flag;
-  __shared__ int epi_verdict[4];
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -573,7 +580,7 @@ __global__ void __launch_bounds__(kQPersistThreads, 1) gemm_q_persist_kernel(con
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(smem_u32(&bar_acc_full[a]), 1);
-      mbar_init(smem_u32(&bar_acc_empty[a]), 4);
+      mbar_init(smem_u32(&bar_acc_empty[a]), 8);
     }
     mbar_fence_init();
     tma_prefetch_desc(&tmap_w);
@@ -628,6 +635,8 @@ __global__ void __launch_bounds__(kQPersistThreads, 1) gemm_q_persist_kernel(con
             const uint32_t sfb_dst = dst + kWTileBytes + Cfg::kXTileBytes + Cfg::kSfaBytes;
             const long long tile0 = t0 / 128;
             bulk_load(sfb_dst, p.x_sf + (tile0 * p.k_tiles + 4 * kb) * kSfTileBytes, 4 * kSfTileBytes, full);
+            if constexpr (TN > 128)
+              bulk_load(sfb_dst + 4 * kSfTileBytes, p.x_sf + ((tile0 + 1) * p.k_tiles + 4 * kb) * kSfTileBytes, 4 * kSfTileBytes, full);
           }
         }
         if (!ok) break;
@@ -646,13 +655,15 @@ __global__ void __launch_bounds__(kQPersistThreads, 1) gemm_q_persist_kernel(con
   } else if (warp == 1) {
     if (elect_one()) {
       // ---------------- MMA issuer ----------------
-      constexpr uint32_t idesc = kBS ? idesc_nvfp4(kTileN, TN) : umma_idesc(kTileN, TN, 0, 0);
       uint32_t it = 0;
       int tile_i = 0;
       for (int tile = blockIdx.x; tile < n_tiles && !*abortp; tile += gridDim.x, ++tile_i) {
-        const int a = tile_i & 1;
-        const uint32_t aph = (tile_i >> 1) & 1;
-        if (tile_i >= 2 &&
+        const int a = tile_i % kAccs;
+        const uint32_t aph = (tile_i / kAccs) & 1;
+        // (a ragged last tile: as many columns as it has tokens, in sixteens)
+        const int live = min(TN, (p.T - (tile % n_t_tiles) * TN + 15) & ~15);
+        const uint32_t idesc = kBS ? idesc_nvfp4(kTileN, live) : umma_idesc(kTileN, live, 0, 0);
+        if (tile_i >= kAccs &&
             !mbar_wait(smem_u32(&bar_acc_empty[a]), aph ^ 1, &abort_flag, p.status, kStatusAccumWaitTimeout))
           break;
         tc_fence_after();
@@ -675,12 +686,13 @@ __global__ void __launch_bounds__(kQPersistThreads, 1) gemm_q_persist_kernel(con
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
               tc_cp_sf(tmem_base + Cfg::kSfaCol + 4 * k, sf_desc(sfa_s + k * kSfTileBytes));
-              tc_cp_sf(tmem_base + Cfg::kSfbCol + 4 * k, sf_desc(sfb_s + k * kSfTileBytes));
+              tc_cp_sf(tmem_base + Cfg::kSfbCol + Cfg::kSfbStep * k, sf_desc(sfb_s + k * kSfTileBytes));
+              if constexpr (TN > 128) tc_cp_sf(tmem_base + Cfg::kSfbCol + Cfg::kSfbStep * k + 4, sf_desc(sfb_s + (4 + k) * kSfTileBytes));
             }
 #pragma unroll
             for (int k = 0; k < 4; ++k)
               tc_mma_nvfp4(acc, a_desc + 2 * k, b_desc + 2 * k, idesc, tmem_base + Cfg::kSfaCol + 4 * k,
-                           tmem_base + Cfg::kSfbCol + 4 * k, (kb > 0 || k > 0) ? 1u : 0u);
+                           tmem_base + Cfg::kSfbCol + Cfg::kSfbStep * k, (kb > 0 || k > 0) ? 1u : 0u);
           } else {
 #pragma unroll
             for (int k = 0; k < 4; ++k)
@@ -696,30 +708,31 @@ __global__ void __launch_bounds__(kQPersistThreads, 1) gemm_q_persist_kernel(con
   } else {
     // ---------------- epilogue warps ----------------
     pdl_wait_prior();
-    const int lg = warp & 3;
+    const int lg = warp & 3;          // TMEM lane group this warp may read
+    const int half = (warp - 2) >> 2; // which chunks: half, half + 2, ...
     constexpr int kChunk = 16;
-    float* up_s = reinterpret_cast<float*>(smem_raw + (smem_base - smem_u32(smem_raw)) + kStages * Cfg::kStageBytes);
+    float* const xch_s = reinterpret_cast<float*>(smem_raw + (smem_base - smem_u32(smem_raw)) + kStages * Cfg::kStageBytes);
+    const int pair = (lg & 1) + 2 * half;
+    const uint32_t select = swap_select(lane);
     int tile_i = 0;
     for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x, ++tile_i) {
-      const int a = tile_i & 1;
-      const uint32_t ph = (tile_i >> 1) & 1;
+      const int a = tile_i % kAccs;
+      const uint32_t ph = (tile_i / kAccs) & 1;
       const bool have = mbar_wait(smem_u32(&bar_acc_full[a]), ph, &abort_flag, p.status, kStatusAccumWaitTimeout);
-      if (lane == 0) epi_verdict[warp - 2] = (have && !*abortp) ? 1 : 0;
-      q_epi_bar_sync();
-      const bool go = epi_verdict[0] && epi_verdict[1] && epi_verdict[2] && epi_verdict[3];
-      q_epi_bar_sync();
-      if (!go) break;
+      // one verdict for the eight warps, so that the pair barriers below are never divergent
+      if (!epi_all(have && !*abortp)) break;
       tc_fence_after();
       const int w_tile = tile / n_t_tiles;
       const int n0 = w_tile * kTileN;
       const int t0 = (tile % n_t_tiles) * TN;
+      const int cols = min(TN, p.T - t0);     // live tokens of the tile
       const uint32_t lane_taddr = tmem_base + a * TN + (static_cast<uint32_t>(lg * 32) << 16);
       const int n = n0 + lg * 32 + lane;
       const float row_scale = kBS ? p.out_scale : ((n < p.N) ? p.w_scale[n] : 0.f);
       auto load_acc = [&](int c, float* acc) {
         uint32_t v[kChunk];
         tmem_ld_x16(lane_taddr + c, v);
-        tmem_ld_wait();
+        tmem_ld_wait_x16(v);
 #pragma unroll
         for (int j = 0; j < kChunk; ++j) {
           float sc = row_scale;
@@ -728,73 +741,52 @@ __global__ void __launch_bounds__(kQPersistThreads, 1) gemm_q_persist_kernel(con
         }
       };
       if constexpr (EPI == kEpiSwiglu) {
-        // rows are tile-interleaved: lane groups 0, 1 = gate rows, 2, 3 = the matching up rows
+        // Rows are tile-interleaved: lane groups 0, 1 = gate rows, 2, 3 = the matching up rows.  The two warps of a pair swap
+        // eight of a chunk's sixteen columns, so that both finish half of the units.
         const bool is_up = lg >= 2;
-        const int r = (lg & 1) * 32 + lane;
-        const int col = w_tile * 64 + r;
-        for (int c = 0, ci = 0; c < TN; c += kChunk, ++ci) {
-          float* buf = up_s + (ci & 1) * (kChunk * 64);
+        const int col = w_tile * 64 + (lg & 1) * 32 + lane;
+        const int ce = col & ~1;
+        float* const buf = xch_s + pair * (2 * 8 * 32);
+        float* const mine = buf + (is_up ? 8 * 32 : 0);
+        const float* const other = buf + (is_up ? 0 : 8 * 32);
+        for (int c = half * kChunk; c < cols; c += 2 * kChunk) {
           float v[kChunk];
           load_acc(c, v);
-          if (is_up) {
+          // (selects, not indices: the chunk stays in registers)
 #pragma unroll
-            for (int j = 0; j < kChunk; ++j) buf[j * 64 + r] = v[j];
-          }
-          q_epi_bar_sync();
-          if (!is_up && t0 + c < p.T) {
+          for (int j = 0; j < 8; ++j) mine[j * 32 + lane] = is_up ? v[j] : v[8 + j];
+          epi_pair_sync(pair);
+          const int tb = t0 + c + (is_up ? 8 : 0);
+          uint32_t w[4];
 #pragma unroll
-            for (int m = 0; m < kChunk / 2; ++m) {
-              float o2[2];
+          for (int m = 0; m < 4; ++m) {
+            float o2[2];
 #pragma unroll
-              for (int h = 0; h < 2; ++h) {
-                const int j = 2 * m + h;
-                const float g = v[j];
-                o2[h] = g / (1.f + __expf(-g)) * buf[j * 64 + r];
-              }
-              const float send = (lane & 1) ? o2[0] : o2[1];
-              const float recv = __shfl_xor_sync(0xffffffffu, send, 1);
-              const int t = t0 + c + 2 * m + (lane & 1);
-              const int ce = col & ~1;
-              if (t < p.T && ce < p.N / 2) {
-                const uint32_t packed = (lane & 1) ? pack_bf16x2(recv, o2[1]) : pack_bf16x2(o2[0], recv);
-                *reinterpret_cast<uint32_t*>(p.out + static_cast<long long>(t) * p.ldo + ce) = packed;
-              }
+            for (int h = 0; h < 2; ++h) {
+              const int j = 2 * m + h;
+              const float own = is_up ? v[8 + j] : v[j];
+              const float got = other[j * 32 + lane];
+              const float g = is_up ? got : own, u = is_up ? own : got;
+              o2[h] = g / (1.f + __expf(-g)) * u;
             }
+            const __nv_bfloat162 units = __floats2bfloat162_rn(o2[0], o2[1]);
+            w[m] = swap_pair(*reinterpret_cast<const uint32_t*>(&units), select);
           }
+          const int live = ce < p.N / 2 ? (p.T - tb - (lane & 1) + 1) >> 1 : 0;
+          store_rows<4>({p.out + static_cast<long long>(tb + (lane & 1)) * p.ldo + ce, 2 * p.ldo, live}, w);
+          epi_pair_sync(pair);   // the other warp has read this one's values
         }
       } else {
-        for (int c = 0; c < TN; c += kChunk) {
-          if (t0 + c >= p.T) break;
+        const int ne = n & ~1;
+        const long long row0 = t0 + (lane & 1);
+        for (int c = half * kChunk; c < cols; c += 2 * kChunk) {
+          const int live = ne < p.N ? min(8, (cols - c - (lane & 1) + 1) >> 1) : 0;
+          // (the residual may alias the output: a chunk's values are fetched before its first store)
+          uint32_t r2[kChunk / 2];
+          if constexpr (EPI == kEpiResidual) load_rows8({p.resid + (row0 + c) * p.ldr + ne, 2 * p.ldr, live}, r2);
           float v[kChunk];
           load_acc(c, v);
-          __nv_bfloat162 r2[kChunk / 2];
-          if constexpr (EPI == kEpiResidual) {
-#pragma unroll
-            for (int m = 0; m < kChunk / 2; ++m) {
-              const int t = t0 + c + 2 * m + (lane & 1);
-              const int ne = n & ~1;
-              r2[m] = (t < p.T && ne < p.N)
-                          ? *reinterpret_cast<const __nv_bfloat162*>(p.resid + static_cast<long long>(t) * p.ldr + ne)
-                          : __nv_bfloat162();
-            }
-          }
-#pragma unroll
-          for (int m = 0; m < kChunk / 2; ++m) {
-            const float a0 = v[2 * m], a1 = v[2 * m + 1];
-            const float send = (lane & 1) ? a0 : a1;
-            const float recv = __shfl_xor_sync(0xffffffffu, send, 1);
-            const int t = t0 + c + 2 * m + (lane & 1);
-            const int ne = n & ~1;
-            if (t < p.T && ne < p.N) {
-              float lo = (lane & 1) ? recv : a0;
-              float hi = (lane & 1) ? a1 : recv;
-              if constexpr (EPI == kEpiResidual) {
-                lo += __bfloat162float(r2[m].x);
-                hi += __bfloat162float(r2[m].y);
-              }
-              *reinterpret_cast<uint32_t*>(p.out + static_cast<long long>(t) * p.ldo + ne) = pack_bf16x2(lo, hi);
-            }
-          }
+          store_chunk<EPI == kEpiResidual>({p.out + (row0 + c) * p.ldo + ne, 2 * p.ldo, live}, v, r2, select);
         }
       }
       tc_fence_before();
@@ -810,20 +802,20 @@ __global__ void __launch_bounds__(kQPersistThreads, 1) gemm_q_persist_kernel(con
 
 int q_sm_count();
 
-template <int QT, int EPI>
+template <int QT, int EPI, int TILE>
 cudaError_t launch_q_persist(const CUtensorMap& tw, const CUtensorMap& tx, const QParams& kp, int n_tiles,
                              cudaStream_t stream, bool pdl) {
-  auto kern = gemm_q_persist_kernel<QT, EPI>;
+  auto kern = gemm_q_persist_kernel<QT, EPI, TILE>;
   static bool attr_set = false;
   if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, QPersist<QT>::kSmemBytes);
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, QPersist<QT, TILE>::kSmemBytes);
     if (e != cudaSuccess) return e;
     attr_set = true;
   }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(n_tiles < q_sm_count() ? n_tiles : q_sm_count());
   cfg.blockDim = dim3(kQPersistThreads);
-  cfg.dynamicSmemBytes = QPersist<QT>::kSmemBytes;
+  cfg.dynamicSmemBytes = QPersist<QT, TILE>::kSmemBytes;
   cfg.stream = stream;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -833,13 +825,13 @@ cudaError_t launch_q_persist(const CUtensorMap& tw, const CUtensorMap& tx, const
   return cudaLaunchKernelEx(&cfg, kern, tw, tx, kp);
 }
 
-template <int QT>
+template <int QT, int TILE>
 cudaError_t launch_q_persist_epi(int epi, const CUtensorMap& tw, const CUtensorMap& tx, const QParams& kp, int n_tiles,
                                  cudaStream_t stream, bool pdl) {
   switch (epi) {
-    case kEpiResidual: return launch_q_persist<QT, kEpiResidual>(tw, tx, kp, n_tiles, stream, pdl);
-    case kEpiSwiglu: return launch_q_persist<QT, kEpiSwiglu>(tw, tx, kp, n_tiles, stream, pdl);
-    default: return launch_q_persist<QT, kEpiStore>(tw, tx, kp, n_tiles, stream, pdl);
+    case kEpiResidual: return launch_q_persist<QT, kEpiResidual, TILE>(tw, tx, kp, n_tiles, stream, pdl);
+    case kEpiSwiglu: return launch_q_persist<QT, kEpiSwiglu, TILE>(tw, tx, kp, n_tiles, stream, pdl);
+    default: return launch_q_persist<QT, kEpiStore, TILE>(tw, tx, kp, n_tiles, stream, pdl);
   }
 }
 
@@ -941,6 +933,16 @@ bool cached_tmap(CUtensorMap* out, const void* base, uint64_t rows, uint64_t col
   cache.emplace(key, m);
   *out = m;
   return true;
+}
+
+// Tokens per tile of the persistent kernel, 128 or 256, by the least estimated time: rounds of one tile per SM times the time of
+// a tile.  A k-block takes (fits to 34816 x 5120 and 5120 x 17408 with all SMs busy) 305 ns at 128 tokens and 385 at 256 with
+// nvfp4, 300 and 400 with fp8; the wide nvfp4 tile adds its epilogue of 2.5 us, which nothing overlaps.
+int q_persist_tile(bool nvfp4, int T, int w_tiles, int num_kb) {
+  auto rounds = [&](int tn) { return (static_cast<long long>(w_tiles) * ((T + tn - 1) / tn) + q_sm_count() - 1) / q_sm_count(); };
+  const double narrow = rounds(128) * num_kb * (nvfp4 ? 305. : 300.);
+  const double wide = rounds(256) * (num_kb * (nvfp4 ? 385. : 400.) + (nvfp4 ? 2500. : 0.));
+  return wide < narrow ? 256 : 128;
 }
 
 int q_tile_tokens(int T) { return T <= 32 ? 32 : (T <= 64 ? 64 : (T <= 128 ? 128 : 256)); }
@@ -1049,20 +1051,25 @@ const char* gemm_quant(const QGemmArgs& a) {
   }
   CUtensorMap tw, tx;
   if (!cached_tmap(&tw, a.w, a.N, k_bytes, a.ldw, 64)) return "gemm_quant: weight tensor map rejected";
-  // prefill-sized problems with more tiles than SMs: persistent kernel (NFB_GEMM_PERSISTENT=0 switches it off)
+  // More than 64 tokens: persistent kernel (NFB_GEMM_PERSISTENT=0 switches it off).  One tile of 128 or 256 tokens per CTA, or
+  // the persistent kernel with four epilogue warps where there were more tiles than SMs, before -> now, us, nvfp4: 34816 x 5120,
+  // 128 tokens 28.0 -> 19.8, 256 32 -> 26.9, 2048 200 -> 158; 5120 x 17408, 256 tokens 38.5 -> 24.6; 1024 x 2048, 256 tokens
+  // 12.1 -> 5.4.
   static const bool persistent_enabled = [] {
     const char* e = getenv("NFB_GEMM_PERSISTENT");
     return !(e != nullptr && e[0] == '0');
   }();
-  if (persistent_enabled && tn == 256 && splits == 1 && !push) {
-    const int ptn = bs ? 128 : 256;
-    const long long n_tiles = static_cast<long long>((kp.N + kTileN - 1) / kTileN) * ((kp.T + ptn - 1) / ptn);
-    if (n_tiles > q_sm_count()) {
-      if (!cached_tmap(&tx, a.x, a.T, k_bytes, a.ldx, ptn)) return "gemm_quant: activation tensor map rejected";
-      cudaError_t e = bs ? launch_q_persist_epi<kQNvfp4>(a.epi, tw, tx, kp, static_cast<int>(n_tiles), a.stream, a.pdl)
-                         : launch_q_persist_epi<kQFp8Row>(a.epi, tw, tx, kp, static_cast<int>(n_tiles), a.stream, a.pdl);
-      return e == cudaSuccess ? nullptr : cudaGetErrorString(e);
-    }
+  if (persistent_enabled && tn > 64 && splits == 1 && !push && kp.next_codes == nullptr) {
+    const int w_tiles = (kp.N + kTileN - 1) / kTileN;
+    const int ptn = q_persist_tile(bs, kp.T, w_tiles, kp.num_kb);
+    const int n = w_tiles * ((kp.T + ptn - 1) / ptn);
+    if (!cached_tmap(&tx, a.x, a.T, k_bytes, a.ldx, ptn)) return "gemm_quant: activation tensor map rejected";
+    cudaError_t e;
+    if (bs) e = ptn == 256 ? launch_q_persist_epi<kQNvfp4, 256>(a.epi, tw, tx, kp, n, a.stream, a.pdl)
+                           : launch_q_persist_epi<kQNvfp4, 128>(a.epi, tw, tx, kp, n, a.stream, a.pdl);
+    else e = ptn == 256 ? launch_q_persist_epi<kQFp8Row, 256>(a.epi, tw, tx, kp, n, a.stream, a.pdl)
+                        : launch_q_persist_epi<kQFp8Row, 128>(a.epi, tw, tx, kp, n, a.stream, a.pdl);
+    return e == cudaSuccess ? nullptr : cudaGetErrorString(e);
   }
   if (!cached_tmap(&tx, a.x, a.T, k_bytes, a.ldx, tn)) return "gemm_quant: activation tensor map rejected";
   dim3 grid((kp.N + kTileN - 1) / kTileN, (kp.T + tn - 1) / tn, splits);

@@ -12,6 +12,18 @@ namespace nfb {
 
 constexpr int kNvfp4SfTileBytes = 512;   // 128 rows x 4 scales
 
+// e2m1 code of v / s, to nearest, ties to even, for a bf16 v and an e4m3 s > 0.  The boundaries lie midway between the grid's
+// values; a boundary times s has six bits at most and v eight, so that v is on the boundary or 2^-9 of it away: comparing products
+// gives what comparing the quotient, rounded to fp32, gives, at a third of the instructions (quantiser, 2048 x 17408: 55 -> 33 us;
+// 256 x 5120: 6.9 -> 4.6).
+__device__ __forceinline__ uint32_t e2m1_code(float v, float s) {
+  const float a = fabsf(v);
+  // (as negations: a NaN takes the largest code)
+  const uint32_t m = !(a <= 0.25f * s) + !(a < 0.75f * s) + !(a <= 1.25f * s) + !(a < 1.75f * s) + !(a <= 2.5f * s) +
+                     !(a < 3.5f * s) + !(a <= 5.f * s);
+  return m | (v < 0.f ? 8u : 0u);
+}
+
 // `v`: the block's sixteen values as the consumer would read them from a bf16 tensor (already rounded to bf16);
 // token row t, block g of the row (K / 16 blocks per row).
 __device__ __forceinline__ void nvfp4_store_block(const float* v, int t, int g, int K, uint8_t* codes, uint8_t* sf_plane) {
@@ -23,9 +35,10 @@ __device__ __forceinline__ void nvfp4_store_block(const float* v, int t, int g, 
   uint32_t lo = 0, hi = 0;
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
-    lo |= float_to_e2m1(sf > 0.f ? __fdiv_rn(v[i], sf) : 0.f) << (4 * i);
-    hi |= float_to_e2m1(sf > 0.f ? __fdiv_rn(v[8 + i], sf) : 0.f) << (4 * i);
+    lo |= e2m1_code(v[i], sf) << (4 * i);
+    hi |= e2m1_code(v[8 + i], sf) << (4 * i);
   }
+  if (!(sf > 0.f)) lo = hi = 0;
   *reinterpret_cast<uint2*>(codes + static_cast<long long>(t) * (K / 2) + g * 8) = make_uint2(lo, hi);
   const int k_tiles = K / 64;
   const long long off = (static_cast<long long>(t / 128) * k_tiles + g / 4) * kNvfp4SfTileBytes + (t % 32) * 16 +
