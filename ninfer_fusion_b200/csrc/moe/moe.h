@@ -135,6 +135,13 @@ struct MoeGemmArgs {
   int* status = nullptr;
   cudaStream_t stream = nullptr;
   bool pdl = false;         // bf16 experts: launch with programmatic stream serialization
+  // bf16 experts, optional: an expert that every token of this rank meets, beside the routed ones in the same launch.  It reads
+  // `dense_x` [dense_T, dense_K] and dense_w [dense_rows, dense_K], both contiguous, and stores its unit (kMoeEpiSwiglu,
+  // [dense_T, dense_rows / 2]) or its rows (kMoeEpiReturn, [dense_T, dense_rows]) in dense_out.
+  const void* dense_w = nullptr;
+  const void* dense_x = nullptr;
+  __nv_bfloat16* dense_out = nullptr;
+  int64_t dense_T = 0, dense_rows = 0, dense_K = 0;
   // fp8 block-scaled experts (moe_gemm_fp8): w / x are e4m3 codes, scales are fp32
   const float* w_scale = nullptr;   // [experts, rows_per_expert / 128, K / 128]
   const float* x_scale = nullptr;   // [cap, K / 128]

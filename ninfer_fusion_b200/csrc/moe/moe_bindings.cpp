@@ -111,7 +111,7 @@ void moe_push(int64_t world, int64_t rank, int64_t E, int64_t cap, const Tensor&
 // x: [cap, K] expert-sorted rows; w: [local experts, rows per expert, K], bf16, or fp32 for 32-bit runs (one GPU).
 void moe_gemm(const Tensor& x, const Tensor& w, int64_t epi, int64_t tile_tokens, int64_t max_tiles, const Tensor& tiles,
               const Tensor& state, OptT out, int64_t world, OptT recv_meta, at::IntArrayRef peer_bases, int64_t ret_off,
-              int64_t ret_flag_off, OptT status, at::ArrayRef<double> glu, bool pdl) {
+              int64_t ret_flag_off, OptT status, at::ArrayRef<double> glu, bool pdl, OptT dense_x, OptT dense_w, OptT dense_out) {
   const auto dt = w.scalar_type();
   TORCH_CHECK(dt == at::kBFloat16 || dt == at::kFloat, "moe_gemm: bf16 or fp32 experts");
   const bool f32 = dt == at::kFloat;
@@ -149,6 +149,16 @@ void moe_gemm(const Tensor& x, const Tensor& w, int64_t epi, int64_t tile_tokens
   if (!glu.empty()) {
     TORCH_CHECK(glu.size() == 3, "moe_gemm: glu = limit, slope, shift");
     a.glu.limit = static_cast<float>(glu[0]); a.glu.slope = static_cast<float>(glu[1]); a.glu.shift = static_cast<float>(glu[2]);
+  }
+  if (dense_w.has_value() && dense_w->defined()) {
+    TORCH_CHECK(!f32 && dense_x.has_value() && dense_out.has_value(), "moe_gemm: a dense expert needs bf16 x, w and out");
+    need(*dense_w, dt, "dense_w"); need(*dense_x, dt, "dense_x"); need(*dense_out, dt, "dense_out");
+    TORCH_CHECK(dense_w->dim() == 2 && dense_x->dim() == 2 && dense_out->dim() == 2 && dense_w->is_contiguous() &&
+                dense_x->is_contiguous() && dense_out->is_contiguous() && dense_x->size(1) == dense_w->size(1) &&
+                dense_out->size(0) == dense_x->size(0) &&
+                dense_out->size(1) == (epi == nfb::kMoeEpiSwiglu ? dense_w->size(0) / 2 : dense_w->size(0)), "moe_gemm: dense shapes");
+    a.dense_w = dense_w->data_ptr(); a.dense_x = dense_x->data_ptr(); a.dense_out = static_cast<__nv_bfloat16*>(dense_out->data_ptr());
+    a.dense_T = dense_x->size(0); a.dense_rows = dense_w->size(0); a.dense_K = dense_w->size(1);
   }
   a.stream = cur_stream();
   a.pdl = pdl;
@@ -199,7 +209,7 @@ TORCH_LIBRARY_FRAGMENT(nfb200, m) {
   m.def("moe_route(Tensor logits, int E, int k, bool norm_topk, bool has_shared_gate, Tensor hist, Tensor ids, Tensor weights, Tensor pos, Tensor? shared_gate, bool pdl=False) -> ()", &moe_route);
   m.def("moe_plan(int world, int rank, int E, int tile_tokens, int cap, Tensor hist, int[] peer_bases, int counts_off, int count_flag_off, Tensor send_base, Tensor tiles, Tensor state, Tensor? status, bool pdl=False) -> ()", &moe_plan);
   m.def("moe_push(int world, int rank, int E, int cap, Tensor x, Tensor ids, Tensor pos, Tensor send_base, int[] peer_bases, int recv_x_off, int recv_meta_off, int arrive_flag_off, Tensor state, Tensor? status, bool pdl=False) -> ()", &moe_push);
-  m.def("moe_gemm(Tensor x, Tensor w, int epi, int tile_tokens, int max_tiles, Tensor tiles, Tensor state, Tensor? out, int world, Tensor? recv_meta, int[] peer_bases, int ret_off, int ret_flag_off, Tensor? status, float[] glu=[], bool pdl=False) -> ()", &moe_gemm);
+  m.def("moe_gemm(Tensor x, Tensor w, int epi, int tile_tokens, int max_tiles, Tensor tiles, Tensor state, Tensor? out, int world, Tensor? recv_meta, int[] peer_bases, int ret_off, int ret_flag_off, Tensor? status, float[] glu=[], bool pdl=False, Tensor? dense_x=None, Tensor? dense_w=None, Tensor? dense_out=None) -> ()", &moe_gemm);
   m.def("moe_route_scored(Tensor logits, int E, int identity, int k, Tensor? correction, float scale, Tensor hist, Tensor ids, Tensor weights, Tensor pos, bool pdl, bool sigmoid=False, bool renormalise=False, int groups=0, int keep=0) -> ()", &moe_route_scored);
   m.def("moe_combine(Tensor x, Tensor weights, Tensor ret, int my_base, int ret_flag_off, Tensor? shared, Tensor? shared_gate, Tensor? norm_w, Tensor? normed, float eps, Tensor state, Tensor? status, bool pdl=False) -> ()", &moe_combine);
   m.def("moe_state_bytes() -> int", &moe_state_bytes);

@@ -38,10 +38,10 @@ constexpr int kTileN = 128;
 constexpr int kWTileBytes = kTileN * 128;
 
 constexpr int kMaxTN = 256;
-constexpr int kMaxStages = 8;
+constexpr int kMaxStages = 12;
 constexpr int kEpiWarps = 8;
 constexpr int kThreads = 64 + 32 * kEpiWarps;
-constexpr int kSmemBytes = 224 * 1024;   // (2 KB of static tables beside it)
+constexpr int kSmemBytes = 221 * 1024;   // (4.5 KB of static tables beside it)
 constexpr int kExchangeBytes = 4 * 2 * 2 * 8 * 32 * 4;   // gated unit: per warp pair two buffers x two directions x 8 x 32
 
 struct MoeKernelParams {
@@ -61,11 +61,34 @@ struct MoeKernelParams {
   unsigned int* peer_ret_flag[kMoeMaxRanks];
   int* status;
   GluParams glu;
+  // the dense expert: its items come first
+  int dense_items, dense_tn, dense_row_tiles, dense_num_kb, dense_T, dense_rows;
+  __nv_bfloat16* dense_out;
 };
+
+// Gated unit: the two CTAs of a cluster work on one item of twice the weight rows; each loads its own 128 rows and half of the
+// tokens (see gemm_bf16.cu).  256 experts of 1024 x 2048, 2048 tokens, top-8, 181 us either way, bound by the weights from HBM,
+// but the dense expert's tokens beside them cost 3 us so and 16 with one CTA an item, whose shared memory they fill.  The return
+// form has contractions of a few k-blocks, where handing an accumulator over between two CTAs shows (103 us, pairs 119).
+template <int EPI>
+constexpr bool kPair = EPI == kMoeEpiSwiglu;
+
+// (token tile, row tile) of the walk
+struct MoeItem {
+  bool dense;
+  int tile, xt;
+};
+__device__ __forceinline__ MoeItem moe_item(const MoeKernelParams& p, int item) {
+  if (item < p.dense_items) return {true, item / p.dense_row_tiles, item % p.dense_row_tiles};
+  item -= p.dense_items;
+  return {false, item / p.n_row_tiles, item % p.n_row_tiles};
+}
 
 template <int EPI>
 __global__ void __launch_bounds__(kThreads, 1) moe_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w,
                                                                const __grid_constant__ CUtensorMap tmap_x,
+                                                               const __grid_constant__ CUtensorMap tmap_dense_w,
+                                                               const __grid_constant__ CUtensorMap tmap_dense_x,
                                                                const MoeKernelParams p) {
   constexpr int kRingBytes = kSmemBytes - 1024 - (EPI == kMoeEpiSwiglu ? kExchangeBytes : 0);
   extern __shared__ uint8_t smem_raw[];
@@ -75,17 +98,21 @@ __global__ void __launch_bounds__(kThreads, 1) moe_gemm_kernel(const __grid_cons
   __shared__ __align__(8) uint64_t bar_acc_empty[2];
   __shared__ uint32_t tmem_base_slot;
   __shared__ int abort_flag;
-  __shared__ int meta_s[2][kMaxTN];            // return: where the rows of an item go
+  __shared__ __nv_bfloat16* dst_s[2][kMaxTN];  // return: where the rows of an item go
   __shared__ int src_cnt[2][kMoeMaxRanks];     // return, several ranks: rows of an item per source
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const int TN = p.tn;
-  const int stage_bytes = kWTileBytes + TN * 128;
+  constexpr bool PAIR = kPair<EPI>;
+  const int crank = PAIR ? static_cast<int>(blockIdx.x & 1) : 0;
+  const int walker = PAIR ? static_cast<int>(blockIdx.x >> 1) : static_cast<int>(blockIdx.x);
+  const int walkers = PAIR ? static_cast<int>(gridDim.x >> 1) : static_cast<int>(gridDim.x);
+  constexpr int kCtas = PAIR ? 2 : 1;
+  const int stage_bytes = kWTileBytes + (p.dense_items > 0 ? max(TN, p.dense_tn) : TN) * 128 / kCtas;
   const int n_stages = min(kMaxStages, kRingBytes / stage_bytes);
   const int half = p.rows_per_expert / 2;
-  const int num_kb = p.num_kb, n_row_tiles = p.n_row_tiles;
   volatile int* abortp = &abort_flag;
 
   if (threadIdx.x == 0) {
@@ -96,7 +123,7 @@ __global__ void __launch_bounds__(kThreads, 1) moe_gemm_kernel(const __grid_cons
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(smem_u32(&bar_acc_full[a]), 1);
-      mbar_init(smem_u32(&bar_acc_empty[a]), kEpiWarps);
+      mbar_init(smem_u32(&bar_acc_empty[a]), (PAIR ? 2 : 1) * kEpiWarps);
     }
     mbar_fence_init();
     tma_prefetch_desc(&tmap_w);
@@ -104,16 +131,22 @@ __global__ void __launch_bounds__(kThreads, 1) moe_gemm_kernel(const __grid_cons
   }
   if (threadIdx.x < 2 * kMoeMaxRanks) (&src_cnt[0][0])[threadIdx.x] = 0;
   if (warp == 1) {
-    tmem_alloc(smem_u32(&tmem_base_slot), 512);
-    tmem_relinquish();
+    if constexpr (PAIR) {
+      tmem_alloc_pair(smem_u32(&tmem_base_slot), 512);
+      tmem_relinquish_pair();
+    } else {
+      tmem_alloc(smem_u32(&tmem_base_slot), 512);
+      tmem_relinquish();
+    }
   }
   tc_fence_before();
-  __syncthreads();
+  if constexpr (PAIR) cluster_sync_all();   // (the other CTA's barriers are initialised before anything counts on them)
+  else __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = tmem_base_slot;
   pdl_launch_next();
   pdl_wait_prior();   // the tile table and the rows come from earlier kernels
-  const int n_items = p.state->n_tiles * n_row_tiles;
+  const int n_items = p.dense_items + p.state->n_tiles * p.n_row_tiles;
 
   if (warp == 0) {
     if (elect_one()) {
@@ -123,22 +156,29 @@ __global__ void __launch_bounds__(kThreads, 1) moe_gemm_kernel(const __grid_cons
       int s = 0;
       uint32_t ph = 1;      // the first pass over the ring finds every stage free
       uint32_t issued = 0;
-      int item = blockIdx.x;
+      int item = walker;
       int expert = 0, row0 = 0;
-      if (item < n_items) {
-        expert = p.tile_expert[item / n_row_tiles];
-        row0 = p.tile_row0[item / n_row_tiles];
-      }
-      while (item < n_items && !*abortp) {
-        const int wrow = expert * p.rows_per_expert;
-        const int xt = item % n_row_tiles, x_row = row0;
-        const int row_a = EPI == kMoeEpiSwiglu ? wrow + xt * 64 : wrow + xt * kTileN;
-        const int row_b = EPI == kMoeEpiSwiglu ? wrow + half + xt * 64 : row_a + 64;
-        item += gridDim.x;
-        if (item < n_items) {   // the next item's entry, in flight beside this item's loads
-          expert = p.tile_expert[item / n_row_tiles];
-          row0 = p.tile_row0[item / n_row_tiles];
+      auto look_up = [&] {
+        const MoeItem it = moe_item(p, item);
+        if (item < n_items && !it.dense) {
+          expert = p.tile_expert[it.tile];
+          row0 = p.tile_row0[it.tile];
         }
+      };
+      look_up();
+      while (item < n_items && !*abortp) {
+        const MoeItem it = moe_item(p, item);
+        const CUtensorMap* const map_w = it.dense ? &tmap_dense_w : &tmap_w;
+        const CUtensorMap* const map_x = it.dense ? &tmap_dense_x : &tmap_x;
+        const int wrow = it.dense ? 0 : expert * p.rows_per_expert;
+        const int tn = it.dense ? p.dense_tn : TN;
+        const int x_row = (it.dense ? it.tile * tn : row0) + crank * (tn / 2);
+        const int row_a = wrow + (kCtas * it.xt + crank) * (EPI == kMoeEpiSwiglu ? 64 : kTileN);
+        const int row_b = EPI == kMoeEpiSwiglu ? row_a + (it.dense ? p.dense_rows / 2 : half) : row_a + 64;
+        const int num_kb = it.dense ? p.dense_num_kb : p.num_kb;
+        const int bytes = kCtas * kWTileBytes + tn * 128;   // (of a pair, counted by the even CTA's barrier)
+        item += walkers;
+        look_up();   // the next item's entry, in flight beside this item's loads
         bool ok = true;
         for (int kb = 0; kb < num_kb; ++kb, ++issued) {
           if (!mbar_wait(smem_u32(&bar_empty[s]), ph, abortp, p.status, kStatusEmptyWaitTimeout)) {
@@ -147,16 +187,21 @@ __global__ void __launch_bounds__(kThreads, 1) moe_gemm_kernel(const __grid_cons
           }
           const uint32_t full = smem_u32(&bar_full[s]);
           const uint32_t dst = smem_base + s * stage_bytes;
-          mbar_expect_tx(full, stage_bytes);
-          tma_load_2d(dst, &tmap_w, full, kb * kBlockK, row_a, pol_w);
-          tma_load_2d(dst + 64 * 128, &tmap_w, full, kb * kBlockK, row_b, pol_w);
-          tma_load_2d(dst + kWTileBytes, &tmap_x, full, kb * kBlockK, x_row, pol_x);
+          if (crank == 0) mbar_expect_tx(full, bytes);
+          auto load = [&](uint32_t to, const CUtensorMap* map, int row, uint64_t pol) {
+            if constexpr (PAIR) tma_load_2d_pair(to, map, mapa_shared(full, 0), kb * kBlockK, row, pol);
+            else tma_load_2d(to, map, full, kb * kBlockK, row, pol);
+          };
+          load(dst, map_w, row_a, pol_w);
+          load(dst + 64 * 128, map_w, row_b, pol_w);
+          load(dst + kWTileBytes, map_x, x_row, pol_x);
           if (++s == n_stages) { s = 0; ph ^= 1; }
         }
         if (!ok) break;
       }
       if (*abortp) {
-        // Unwinding: let copies that were already issued land before the CTA exits.
+        // Unwinding: let copies that were already issued land before the CTA exits.  (The odd CTA of a pair has no barrier
+        // to see them by: its own never completes, and the polls are the pause.)
         const uint32_t depth = static_cast<uint32_t>(n_stages);
         for (uint32_t j = issued > depth ? issued - depth : 0; j < issued; ++j)
           for (uint32_t spin = 0; spin < (1u << 20); ++spin)
@@ -165,14 +210,20 @@ __global__ void __launch_bounds__(kThreads, 1) moe_gemm_kernel(const __grid_cons
     }
     __syncwarp();
   } else if (warp == 1) {
-    if (elect_one()) {
-      // ---------------- MMA issuer ----------------
-      const uint32_t idesc = umma_idesc(kTileN, TN, 1, 1);
+    if (crank == 0 && elect_one()) {
+      // ---------------- MMA issuer (of both CTAs of a pair) ----------------
       int s = 0;
       uint32_t ph = 0;
       int n = 0;
-      for (int item = blockIdx.x; item < n_items && !*abortp; item += gridDim.x, ++n) {
+      auto commit = [](uint32_t bar) {
+        if constexpr (PAIR) tc_commit_pair(bar);
+        else tc_commit(bar);
+      };
+      for (int item = walker; item < n_items && !*abortp; item += walkers, ++n) {
         const int a = n & 1;
+        const bool dense = item < p.dense_items;
+        const int num_kb = dense ? p.dense_num_kb : p.num_kb;
+        const uint32_t idesc = umma_idesc(kCtas * kTileN, dense ? p.dense_tn : TN, 1, 1);
         // the epilogue has drained this accumulator's previous item
         if (n >= 2 && !mbar_wait(smem_u32(&bar_acc_empty[a]), ((n >> 1) & 1) ^ 1, abortp, p.status, kStatusAccumWaitTimeout)) break;
         tc_fence_after();
@@ -189,12 +240,16 @@ __global__ void __launch_bounds__(kThreads, 1) moe_gemm_kernel(const __grid_cons
           const uint64_t b_desc = umma_desc_k_sw128(a_addr + kWTileBytes);
 #pragma unroll
           for (int k = 0; k < kBlockK / 16; ++k)
-            tc_mma_f16(acc, a_desc + 2 * k, b_desc + 2 * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
-          tc_commit(smem_u32(&bar_empty[s]));
+          {
+            const uint32_t accumulate = (kb > 0 || k > 0) ? 1u : 0u;
+            if constexpr (PAIR) tc_mma_f16_pair(acc, a_desc + 2 * k, b_desc + 2 * k, idesc, accumulate);
+            else tc_mma_f16(acc, a_desc + 2 * k, b_desc + 2 * k, idesc, accumulate);
+          }
+          commit(smem_u32(&bar_empty[s]));
           if (++s == n_stages) { s = 0; ph ^= 1; }
         }
         if (!ok) break;
-        tc_commit(smem_u32(&bar_acc_full[a]));
+        commit(smem_u32(&bar_acc_full[a]));
       }
     }
     __syncwarp();
@@ -206,17 +261,24 @@ __global__ void __launch_bounds__(kThreads, 1) moe_gemm_kernel(const __grid_cons
     constexpr int kChunk = 16;
     float* const xch_s = reinterpret_cast<float*>(smem_raw + (smem_base - smem_u32(smem_raw)) + kRingBytes);
     const int pair = (lg & 1) + 2 * hf;
+    const uint32_t select = swap_select(lane);
     int n = 0, xch_i = 0;
     uint32_t returned = 0;            // one GPU: rows this CTA has returned
-    for (int item = blockIdx.x; item < n_items; item += gridDim.x, ++n) {
-      const int tile = item / n_row_tiles, xt = item % n_row_tiles;
-      const int row0 = p.tile_row0[tile], rows = p.tile_rows[tile];
+    for (int item = walker; item < n_items; item += walkers, ++n) {
+      const MoeItem it = moe_item(p, item);
+      const int row0 = it.dense ? it.tile * p.dense_tn : p.tile_row0[it.tile];
+      const int rows = it.dense ? min(p.dense_tn, p.dense_T - row0) : p.tile_rows[it.tile];
+      const int N = it.dense ? p.dense_rows : p.rows_per_expert;
       const int a = n & 1;
       if constexpr (EPI == kMoeEpiReturn) {
         if (etid < rows) {
-          const int meta = p.recv_meta[row0 + etid];
-          meta_s[a][etid] = meta;
-          if (p.world > 1) atomicAdd(&src_cnt[a][meta >> 24], 1);
+          if (it.dense) {
+            dst_s[a][etid] = p.dense_out + static_cast<long long>(row0 + etid) * N;
+          } else {
+            const int meta = p.recv_meta[row0 + etid];
+            dst_s[a][etid] = p.peer_ret[meta >> 24] + static_cast<long long>(meta & 0xffffff) * N;
+            if (p.world > 1) atomicAdd(&src_cnt[a][meta >> 24], 1);
+          }
         }
       }
       const bool have = mbar_wait(smem_u32(&bar_acc_full[a]), (n >> 1) & 1, abortp, p.status, kStatusAccumWaitTimeout);
@@ -228,7 +290,9 @@ __global__ void __launch_bounds__(kThreads, 1) moe_gemm_kernel(const __grid_cons
         // Lane groups 0, 1 hold gate rows, 2, 3 the matching up rows.  The two warps of a pair swap eight of a chunk's
         // sixteen columns, so that both finish half of the units.
         const bool is_up = lg >= 2;
-        const int ne = (xt * 64 + (lg & 1) * 32 + lane) & ~1;
+        const int ne = ((kCtas * it.xt + crank) * 64 + (lg & 1) * 32 + lane) & ~1;
+        __nv_bfloat16* const out = it.dense ? p.dense_out : p.out;
+        const long long ldo = it.dense ? N / 2 : p.ldo;
         for (int c = hf * kChunk; c < rows; c += 2 * kChunk, ++xch_i) {
           float* buf = xch_s + (pair * 2 + (xch_i & 1)) * (2 * 8 * 32);
           float* mine = buf + (is_up ? 8 * 32 : 0);
@@ -240,6 +304,7 @@ __global__ void __launch_bounds__(kThreads, 1) moe_gemm_kernel(const __grid_cons
           for (int j = 0; j < 8; ++j) mine[j * 32 + lane] = __uint_as_float(is_up ? v[j] : v[8 + j]);
           epi_pair_sync(pair);
           const int cb = c + (is_up ? 8 : 0);
+          uint32_t w[4];
 #pragma unroll
           for (int m = 0; m < 4; ++m) {
             float o2[2];
@@ -250,47 +315,40 @@ __global__ void __launch_bounds__(kThreads, 1) moe_gemm_kernel(const __grid_cons
               const float got = other[j * 32 + lane];
               o2[h] = gated_unit(is_up ? got : own, is_up ? own : got, p.glu);
             }
-            const float send = (lane & 1) ? o2[0] : o2[1];
-            const float recv = __shfl_xor_sync(0xffffffffu, send, 1);
-            const int tl = cb + 2 * m + (lane & 1);
-            if (tl < rows && ne < half) {
-              const uint32_t packed = (lane & 1) ? pack_bf16x2(recv, o2[1]) : pack_bf16x2(o2[0], recv);
-              *reinterpret_cast<uint32_t*>(p.out + static_cast<long long>(row0 + tl) * p.ldo + ne) = packed;
-            }
+            const __nv_bfloat162 units = __floats2bfloat162_rn(o2[0], o2[1]);
+            w[m] = swap_pair(*reinterpret_cast<const uint32_t*>(&units), select);
           }
+          const int live = ne < N / 2 ? (rows - cb - (lane & 1) + 1) >> 1 : 0;
+          store_rows<4>({out + static_cast<long long>(row0 + cb + (lane & 1)) * ldo + ne, 2 * ldo, live}, w);
         }
       } else {
-        const int N = p.rows_per_expert;
-        const int ne = (xt * kTileN + lg * 32 + lane) & ~1;
+        const int ne = ((kCtas * it.xt + crank) * kTileN + lg * 32 + lane) & ~1;
         for (int c = hf * kChunk; c < rows; c += 2 * kChunk) {
           uint32_t v[kChunk];
           tmem_ld_x16(lane_taddr + c, v);
           tmem_ld_wait_x16(v);
+          __nv_bfloat16* const* dst = &dst_s[a][c + (lane & 1)];
+          const int live = ne < N ? (rows - c - (lane & 1) + 1) >> 1 : 0;
 #pragma unroll
           for (int m = 0; m < kChunk / 2; ++m) {
-            const float a0 = __uint_as_float(v[2 * m]), a1 = __uint_as_float(v[2 * m + 1]);
-            const float send = (lane & 1) ? a0 : a1;
-            const float recv = __shfl_xor_sync(0xffffffffu, send, 1);
-            const int tl = c + 2 * m + (lane & 1);
-            if (tl < rows && ne < N) {
-              const int meta = meta_s[a][tl];
-              const float lo = (lane & 1) ? recv : a0;
-              const float hi = (lane & 1) ? a1 : recv;
-              *reinterpret_cast<uint32_t*>(p.peer_ret[meta >> 24] + static_cast<long long>(meta & 0xffffff) * N + ne) = pack_bf16x2(lo, hi);
-            }
+            const uint32_t w = swap_pair(pack_bf16x2(__uint_as_float(v[2 * m]), __uint_as_float(v[2 * m + 1])), select);
+            if (m < live) *reinterpret_cast<uint32_t*>(dst[2 * m] + ne) = w;
           }
         }
       }
       // this warp is done with the accumulator: hand it back to the MMA issuer
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(smem_u32(&bar_acc_empty[a]));
+      if (lane == 0) {
+        if constexpr (PAIR) mbar_arrive_cluster(mapa_shared(smem_u32(&bar_acc_empty[a]), 0));
+        else mbar_arrive(smem_u32(&bar_acc_empty[a]));
+      }
       if constexpr (EPI == kMoeEpiReturn) {
         // One arrival unit per returned row of a 128-column tile.  Several ranks: signalled per item, so that the owners can
         // start early (the barrier orders all stores before the signalling threads, whose system-scope fence + release is
         // cumulative over them).  One GPU: the kernel's end orders the stores, the counter is advanced once per CTA.
         if (p.world == 1) {
-          returned += static_cast<uint32_t>(rows);
+          if (!it.dense) returned += static_cast<uint32_t>(rows);
         } else {
           epi_all(true);
           if (etid < p.world) {
@@ -313,13 +371,18 @@ __global__ void __launch_bounds__(kThreads, 1) moe_gemm_kernel(const __grid_cons
   }
 
   tc_fence_before();
-  __syncthreads();
-  if (warp == 1) tmem_dealloc(tmem_base, 512);
+  if constexpr (PAIR) {
+    cluster_sync_all();   // (the other CTA neither reads this one's operands nor arrives on its barriers any more)
+    if (warp == 1) tmem_dealloc_pair(tmem_base, 512);
+  } else {
+    __syncthreads();
+    if (warp == 1) tmem_dealloc(tmem_base, 512);
+  }
 }
 
 template <int EPI>
-cudaError_t launch(const CUtensorMap& tw, const CUtensorMap& tx, const MoeKernelParams& kp, long long max_items,
-                   cudaStream_t stream, bool pdl) {
+cudaError_t launch(const CUtensorMap& tw, const CUtensorMap& tx, const CUtensorMap& dw, const CUtensorMap& dx,
+                   const MoeKernelParams& kp, long long max_items, cudaStream_t stream, bool pdl) {
   auto kern = moe_gemm_kernel<EPI>;
   static bool attr_set = false;
   if (!attr_set) {
@@ -327,8 +390,10 @@ cudaError_t launch(const CUtensorMap& tw, const CUtensorMap& tx, const MoeKernel
     if (e != cudaSuccess) return e;
     attr_set = true;
   }
-  const dim3 grid(static_cast<unsigned>(max_items < device_sm_count() ? max_items : device_sm_count()));
-  return launch_kernel(kern, grid, dim3(kThreads), kSmemBytes, stream, pdl, 1, tw, tx, kp);
+  constexpr int kCtas = kPair<EPI> ? 2 : 1;
+  const long long walkers = device_sm_count() / kCtas;
+  const dim3 grid(static_cast<unsigned>(kCtas * (max_items < walkers ? max_items : walkers)));
+  return launch_kernel(kern, grid, dim3(kThreads), kSmemBytes, stream, pdl, kCtas, tw, tx, dw, dx, kp);
 }
 
 struct Key {
@@ -396,7 +461,7 @@ const char* moe_gemm(const MoeGemmArgs& a) {
     if (a.rows_per_expert % 128) return "moe_gemm: SwiGLU needs expert rows in multiples of 128 (64 gate + 64 up per tile)";
     if (a.out == nullptr || (a.ldo & 1)) return "moe_gemm: no output";
     kp.out = static_cast<__nv_bfloat16*>(a.out); kp.ldo = a.ldo;
-    kp.n_row_tiles = static_cast<int>(a.rows_per_expert / 2 / 64);
+    kp.n_row_tiles = static_cast<int>((a.rows_per_expert / 2 + 127) / 128);
   } else if (a.epi == kMoeEpiReturn) {
     if (a.rows_per_expert % 8) return "moe_gemm: expert rows must be a multiple of 8";
     if (a.world < 1 || a.world > kMoeMaxRanks || a.recv_meta == nullptr) return "moe_gemm: bad return set-up";
@@ -412,10 +477,30 @@ const char* moe_gemm(const MoeGemmArgs& a) {
   CUtensorMap tw, tx;
   if (!cached_tmap(&tw, a.w, static_cast<uint64_t>(a.n_local_experts) * a.rows_per_expert, a.K, a.ldw, 64))
     return "moe_gemm: weight tensor map rejected";
-  if (!cached_tmap(&tx, a.x, a.cap, a.K, a.ldx, tn)) return "moe_gemm: activation tensor map rejected";
-  const long long max_items = static_cast<long long>(a.max_tiles) * kp.n_row_tiles;
-  cudaError_t e = a.epi == kMoeEpiSwiglu ? launch<kMoeEpiSwiglu>(tw, tx, kp, max_items, a.stream, a.pdl)
-                                         : launch<kMoeEpiReturn>(tw, tx, kp, max_items, a.stream, a.pdl);
+  if (!cached_tmap(&tx, a.x, a.cap, a.K, a.ldx, a.epi == kMoeEpiSwiglu ? tn / 2 : tn)) return "moe_gemm: activation tensor map rejected";
+  CUtensorMap dw = tw, dx = tx;
+  if (a.dense_w != nullptr) {
+    const bool swiglu = a.epi == kMoeEpiSwiglu;
+    if (a.dense_x == nullptr || a.dense_out == nullptr || a.dense_T <= 0 || a.dense_K <= 0 || a.dense_K % 8 ||
+        a.dense_rows <= 0 || a.dense_rows % (swiglu ? 128 : 8))
+      return "moe_gemm: bad dense expert";
+    if ((reinterpret_cast<uintptr_t>(a.dense_w) | reinterpret_cast<uintptr_t>(a.dense_x)) & 15 || reinterpret_cast<uintptr_t>(a.dense_out) & 3)
+      return "moe_gemm: dense operands must be 16-byte aligned";
+    // its own token tile: the routed one follows the few rows of an expert, and 128 tokens of a pair or 64 fit eight stages
+    const int few = static_cast<int>((a.dense_T + 15) / 16 * 16), wide = swiglu ? 128 : 64;
+    kp.dense_tn = tn > wide ? tn : (few < wide ? (few > tn ? few : tn) : wide);
+    kp.dense_T = static_cast<int>(a.dense_T);
+    kp.dense_rows = static_cast<int>(a.dense_rows);
+    kp.dense_num_kb = static_cast<int>((a.dense_K + kBlockK - 1) / kBlockK);
+    kp.dense_row_tiles = swiglu ? (kp.dense_rows / 2 + 127) / 128 : (kp.dense_rows + kTileN - 1) / kTileN;
+    kp.dense_items = kp.dense_row_tiles * ((kp.dense_T + kp.dense_tn - 1) / kp.dense_tn);
+    kp.dense_out = a.dense_out;
+    if (!cached_tmap(&dw, a.dense_w, a.dense_rows, a.dense_K, a.dense_K, 64)) return "moe_gemm: dense weight tensor map rejected";
+    if (!cached_tmap(&dx, a.dense_x, a.dense_T, a.dense_K, a.dense_K, swiglu ? kp.dense_tn / 2 : kp.dense_tn)) return "moe_gemm: dense activation tensor map rejected";
+  }
+  const long long max_items = static_cast<long long>(a.max_tiles) * kp.n_row_tiles + kp.dense_items;
+  cudaError_t e = a.epi == kMoeEpiSwiglu ? launch<kMoeEpiSwiglu>(tw, tx, dw, dx, kp, max_items, a.stream, a.pdl)
+                                         : launch<kMoeEpiReturn>(tw, tx, dw, dx, kp, max_items, a.stream, a.pdl);
   return e == cudaSuccess ? nullptr : cudaGetErrorString(e);
 }
 

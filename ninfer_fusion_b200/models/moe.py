@@ -175,15 +175,20 @@ class MoeBlock:
             ops.moe_quant_rows_block128(self.act[:rb], self.act_q[:rb], self.act_qs[:rb], self.state)
             ops.moe_gemm_fp8(self.act_q, self.act_qs, dn_q, dn_s, MOE_EPI_RETURN, tn, max_tiles, self.tiles, self.state,
                              None, W, self.recv_meta, self.peer_bases, self.off["ret"], self.off["ret_flag"], status)
-        else:
+        sact, sout = self.shared_act[:T], self.shared_out[:T]
+        up_s, down_s = model.w[f"{prefix}/moe/shared_gate_up"], model.w[f"{prefix}/moe/shared_down"]
+        # the shared expert (replicated): a dense SwiGLU MLP on the local tokens, beside the routed ones where its weights are bf16 too
+        dense = self.expert_format != "fp8_block" and all(isinstance(w, torch.Tensor) and w.dtype == torch.bfloat16 and w.is_contiguous()
+                                                          for w in (up_s, down_s))
+        if self.expert_format != "fp8_block":
             gate_up, down = self._experts(model.w, prefix)
             ops.moe_gemm(self.recv_x, gate_up, MOE_EPI_SWIGLU, tn, max_tiles, self.tiles, self.state, self.act, W, None,
-                         self.peer_bases, 0, 0, status, [], pdl)
+                         self.peer_bases, 0, 0, status, [], pdl, *((normed, up_s, sact) if dense else ()))
             ops.moe_gemm(self.act, down, MOE_EPI_RETURN, tn, max_tiles, self.tiles, self.state, None, W, self.recv_meta,
-                         self.peer_bases, self.off["ret"], self.off["ret_flag"], status, [], pdl)
-        # shared expert (replicated): dense SwiGLU MLP on the local tokens
-        sact, sout = self.shared_act[:T], self.shared_out[:T]
-        model._gemm(normed, model.w[f"{prefix}/moe/shared_gate_up"], sact, EPI_SWIGLU)
-        model._gemm(sact, model.w[f"{prefix}/moe/shared_down"], sout)
+                         self.peer_bases, self.off["ret"], self.off["ret_flag"], status, [], pdl,
+                         *((sact, down_s, sout) if dense else ()))
+        if not dense:
+            model._gemm(normed, up_s, sact, EPI_SWIGLU)
+            model._gemm(sact, down_s, sout)
         ops.moe_combine(ws.x[:T], wts, self.ret, self.peer_bases[self.rank], self.off["ret_flag"], sout, sgate,
                         next_norm_w, normed_out, cfg.rms_eps, self.state, status, pdl)
