@@ -66,7 +66,10 @@ class MoeBlock:
             self.off[name] = off
             off += _align(nbytes)
         self.total_bytes = off
-        self.local, handle = self.ops.symm_alloc(off)
+        if world > 1:
+            self.local, handle = self.ops.symm_alloc(off)
+        else:   # nobody else maps it: from the allocator's pool, where a device allocation in the first step took up to 80 ms
+            self.local, handle = torch.zeros(off, dtype=torch.uint8, device=self.device), None
         self.peer_bases: List[int] = [self.local.data_ptr()]
         if world > 1:
             import torch.distributed as dist
