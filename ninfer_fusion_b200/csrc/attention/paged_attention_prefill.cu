@@ -35,6 +35,7 @@
 
 #include <math_constants.h>
 
+#include "../common/quotient.cuh"
 #include "attn_mma_common.cuh"
 
 namespace nfb {
@@ -337,8 +338,8 @@ __global__ void __launch_bounds__(kThreads, 1) paged_attn_prefill_kernel(const P
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
             const __nv_bfloat162 v = *reinterpret_cast<const __nv_bfloat162*>(&ow[e]);
-            ow[e] = pack_bf16x2(__bfloat162float(v.x) / (1.f + __expf(-__bfloat162float(g2[e].x))),
-                                __bfloat162float(v.y) / (1.f + __expf(-__bfloat162float(g2[e].y))));
+            ow[e] = pack_bf16x2(gate_by(__bfloat162float(v.x), __bfloat162float(g2[e].x)),
+                                gate_by(__bfloat162float(v.y), __bfloat162float(g2[e].y)));
           }
         }
         store_row16(p.out + (static_cast<long long>(t0 + r / G) * p.n_q_heads + kvh * G + r % G) * D + c * 8, o, wide);

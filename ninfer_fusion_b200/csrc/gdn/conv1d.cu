@@ -8,6 +8,7 @@
 #include "gdn.h"
 
 #include "../common/ptx.cuh"
+#include "../common/quotient.cuh"
 
 namespace nfb {
 
@@ -64,113 +65,152 @@ __global__ void __launch_bounds__(128) conv1d_silu_kernel(const ConvParams p) {
   *reinterpret_cast<uint32_t*>(p.out + static_cast<long long>(t) * p.C + c) = pack_bf16x2(a0, a1);
 }
 
-// Prefill variant: one thread owns 8 channels of a run of 16 consecutive tokens and slides the three previous
-// inputs through registers, so every input row is read once (16-byte loads) instead of four times, and the grid is
-// T / 16 x C / 1024 CTAs instead of T x C / 256.  Sequence boundaries inside a run reload the window from the new
-// sequence's history.  (2048 tokens x 10240 channels: 97 us with the per-token kernel against 13 us of traffic.)
+// Prefill variant: one thread owns 4 channels of a run of 16 consecutive tokens and slides the three previous
+// inputs through registers, so every input row is read once instead of four times, and the grid is T / 16 x C / 512 CTAs instead
+// of T x C / 256.  Sequence boundaries inside a run reload the window from the new sequence's history.  Bound by what the SM can
+// issue next to memory: two channels per multiplication, the quotient without a branch, four channels a thread so that seven CTAs
+// fit (eight took 130 registers and three).  2048 tokens x 10240 channels, 13 us of traffic: 97 us with the per-token kernel, 36
+// with one channel per instruction, 20 now; 1873 tokens of six sequences x 8192 36 -> 18.
 constexpr int kConvRun = 16;
 
-__device__ __forceinline__ void ld8(const __nv_bfloat16* p, float* v) {
-  const uint4 u = *reinterpret_cast<const uint4*>(p);
-  const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&u);
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    v[2 * i] = __bfloat162float(h[i].x);
-    v[2 * i + 1] = __bfloat162float(h[i].y);
+// two channels side by side: one instruction multiplies and adds both
+struct Pair {
+  unsigned long long v;
+  __device__ __forceinline__ static Pair of(float x, float y) {
+    Pair p;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(p.v) : "f"(x), "f"(y));
+    return p;
   }
+  __device__ __forceinline__ void get(float& x, float& y) const { asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(v)); }
+};
+__device__ __forceinline__ Pair mul2(Pair a, Pair b) {
+  Pair r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ Pair fma2(Pair a, Pair b, Pair c) {
+  Pair r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+  return r;
+}
+__device__ __forceinline__ void unpack4(const uint2& u, Pair* v) {
+  const uint32_t w[2] = {u.x, u.y};
+#pragma unroll
+  for (int i = 0; i < 2; ++i) v[i] = Pair::of(__uint_as_float(w[i] << 16), __uint_as_float(w[i] & 0xffff0000u));
 }
 
-__global__ void __launch_bounds__(128) conv1d_silu_rows_kernel(const ConvParams p) {
-  pdl_launch_next();
-  pdl_wait_prior();
-  const int c = (blockIdx.y * blockDim.x + threadIdx.x) * 8;
-  if (c >= p.C) return;
-  const int t0 = blockIdx.x * kConvRun, t1 = min(p.T, t0 + kConvRun);
-  float w[8][4];
+// four channels from c on: taps, the last three inputs, one token
+struct ConvLane {
+  Pair w[4][2];     // [tap][channel pair]
+  Pair win[3][2];
+  __device__ __forceinline__ void load_taps(const ConvParams& p, int c) {
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {   // 8 channels x 4 taps = 64 bytes
-    float v[8];
-    ld8(p.w + static_cast<long long>(c) * 4 + i * 8, v);
+    for (int i = 0; i < 2; ++i) {   // 4 channels x 4 taps = 32 bytes
+      const uint4 u = *reinterpret_cast<const uint4*>(p.w + static_cast<long long>(c) * 4 + i * 8);
+      const uint32_t a[2] = {u.x, u.y}, b[2] = {u.z, u.w};   // taps 0, 1 and 2, 3 of channels 2 i and 2 i + 1
 #pragma unroll
-    for (int j = 0; j < 8; ++j) w[(i * 8 + j) >> 2][(i * 8 + j) & 3] = v[j];
+      for (int j = 0; j < 2; ++j) {
+        w[2 * j][i] = Pair::of(__uint_as_float(a[j] << 16), __uint_as_float(b[j] << 16));
+        w[2 * j + 1][i] = Pair::of(__uint_as_float(a[j] & 0xffff0000u), __uint_as_float(b[j] & 0xffff0000u));
+      }
+    }
   }
-  float win[3][8];
-  auto open_window = [&](int t, int s) {   // the three inputs before token t of sequence s
+  __device__ __forceinline__ void open_window(const ConvParams& p, int c, int t, int s) {   // before token t of sequence s
     const int start = p.cu_seqlens[s];
     const int slot = p.state_slot[s];
 #pragma unroll
     for (int j = 0; j < 3; ++j) {
       const int tau = t - 3 + j;
-      if (tau >= start) ld8(p.x + static_cast<long long>(tau) * p.ld_x + p.c_off + c, win[j]);
-      else ld8(p.conv_state + (static_cast<long long>(slot) * 3 + (tau - start + 3)) * p.C + c, win[j]);
+      unpack4(*reinterpret_cast<const uint2*>(tau >= start ? p.x + static_cast<long long>(tau) * p.ld_x + p.c_off + c
+                                                           : p.conv_state + (static_cast<long long>(slot) * 3 + (tau - start + 3)) * p.C + c),
+              win[j]);
     }
-  };
-  auto token = [&](int t, const uint4& raw) {
-    float cur[8];
-    const __nv_bfloat162* h2 = reinterpret_cast<const __nv_bfloat162*>(&raw);
+  }
+  __device__ __forceinline__ void token(const ConvParams& p, int c, int t, const uint2& raw) {
+    Pair cur[2];
+    unpack4(raw, cur);
+    uint32_t o[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      float a, b;
+      fma2(w[3][i], cur[i], fma2(w[2][i], win[2][i], fma2(w[1][i], win[1][i], mul2(w[0][i], win[0][i])))).get(a, b);
+      o[i] = pack_bf16x2(gate_by(a, a), gate_by(b, b));
+    }
+    *reinterpret_cast<uint2*>(p.out + static_cast<long long>(t) * p.C + c) = make_uint2(o[0], o[1]);
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      win[0][i] = win[1][i];
+      win[1][i] = win[2][i];
+      win[2][i] = cur[i];
+    }
+  }
+};
+__device__ __forceinline__ uint2 conv_row(const ConvParams& p, int c, int t) {
+  return *reinterpret_cast<const uint2*>(p.x + static_cast<long long>(t) * p.ld_x + p.c_off + c);
+}
+
+// A run with a boundary or an end in it: four rows at a time, and the window anew where a sequence starts.  (A function of its own:
+// its registers do not weigh on the usual run.)
+__device__ __noinline__ void conv_mixed_run(const ConvParams& p, int c, int t0, int t1) {
+  ConvLane lane;
+  lane.load_taps(p, c);
+  int seq = -2;
+#pragma unroll 1
+  for (int t = t0; t < t1; t += 4) {
+    uint2 raw[4];
+    int of[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      cur[2 * i] = __bfloat162float(h2[i].x);
-      cur[2 * i + 1] = __bfloat162float(h2[i].y);
+      of[i] = t + i < t1 ? p.token_seq[t + i] : -1;
+      raw[i] = conv_row(p, c, min(t + i, t1 - 1));
     }
-    uint32_t o[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      float a[2];
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int ch = 2 * i + h;
-        const float v = w[ch][0] * win[0][ch] + w[ch][1] * win[1][ch] + w[ch][2] * win[2][ch] + w[ch][3] * cur[ch];
-        a[h] = v / (1.f + __expf(-v));
+      if (of[i] < 0) {
+        seq = -2;
+        continue;
       }
-      o[i] = pack_bf16x2(a[0], a[1]);
+      if (of[i] != seq) {   // first token of this run, or a new sequence starts here
+        seq = of[i];
+        lane.open_window(p, c, t + i, seq);
+      }
+      lane.token(p, c, t + i, raw[i]);
     }
-    *reinterpret_cast<uint4*>(p.out + static_cast<long long>(t) * p.C + c) = make_uint4(o[0], o[1], o[2], o[3]);
-#pragma unroll
-    for (int ch = 0; ch < 8; ++ch) {
-      win[0][ch] = win[1][ch];
-      win[1][ch] = win[2][ch];
-      win[2][ch] = cur[ch];
-    }
-  };
-  const auto row = [&](int t) { return *reinterpret_cast<const uint4*>(p.x + static_cast<long long>(t) * p.ld_x + p.c_off + c); };
+  }
+}
+
+__global__ void __launch_bounds__(128, 7) conv1d_silu_rows_kernel(const __grid_constant__ ConvParams p) {
+  pdl_launch_next();
+  pdl_wait_prior();
+  const int c = (blockIdx.y * blockDim.x + threadIdx.x) * 4;
+  if (c >= p.C) return;
+  const int t0 = blockIdx.x * kConvRun, t1 = min(p.T, t0 + kConvRun);
   // A full run of one sequence, the usual case: nothing between the loads depends on the data, so eight rows are in flight at
-  // a time.  (Row by row behind the sequence test, a thread waited for sixteen loads in turn: 2048 tokens x 10240 channels 53 us,
-  // 45 so.)
-  int first = p.token_seq[t0];
+  // a time (row by row behind the sequence test, a thread waited for sixteen loads in turn).
+  const int first = p.token_seq[t0];
   bool one = first >= 0 && t1 - t0 == kConvRun;
   if (one) {
 #pragma unroll
     for (int i = 1; i < kConvRun; ++i) one &= p.token_seq[t0 + i] == first;
   }
-  if (one) {
-    uint4 raw[kConvRun / 2];
-#pragma unroll
-    for (int i = 0; i < kConvRun / 2; ++i) raw[i] = row(t0 + i);
-    open_window(t0, first);
-#pragma unroll
-    for (int i = 0; i < kConvRun / 2; ++i) {
-      const uint4 r = raw[i];
-      raw[i] = row(t0 + kConvRun / 2 + i);
-      token(t0 + i, r);
-    }
-#pragma unroll
-    for (int i = 0; i < kConvRun / 2; ++i) token(t0 + kConvRun / 2 + i, raw[i]);
+  if (!one) {
+    conv_mixed_run(p, c, t0, t1);
     return;
   }
-  int seq = -2;
-  for (int t = t0; t < t1; ++t) {
-    const int s = p.token_seq[t];
-    if (s < 0) {
-      seq = -2;
-      continue;
-    }
-    if (s != seq) {   // first token of this run, or a new sequence starts here
-      seq = s;
-      open_window(t, s);
-    }
-    token(t, row(t));
+  uint2 raw[kConvRun / 2];
+#pragma unroll
+  for (int i = 0; i < kConvRun / 2; ++i) raw[i] = conv_row(p, c, t0 + i);
+  ConvLane lane;
+  lane.load_taps(p, c);
+  lane.open_window(p, c, t0, first);
+#pragma unroll
+  for (int i = 0; i < kConvRun / 2; ++i) {
+    const uint2 r = raw[i];
+    raw[i] = conv_row(p, c, t0 + kConvRun / 2 + i);
+    lane.token(p, c, t0 + i, r);
   }
+#pragma unroll
+  for (int i = 0; i < kConvRun / 2; ++i) lane.token(p, c, t0 + kConvRun / 2 + i, raw[i]);
 }
 
 __global__ void __launch_bounds__(128) conv1d_state_kernel(const ConvParams p) {
@@ -247,7 +287,7 @@ const char* causal_conv1d_silu(const ConvParams& p, cudaStream_t stream, bool pd
                        ((reinterpret_cast<uintptr_t>(p.x) | reinterpret_cast<uintptr_t>(p.out) |
                          reinterpret_cast<uintptr_t>(p.conv_state) | reinterpret_cast<uintptr_t>(p.w)) & 15) == 0;
   if (!p.state_only && rows_ok) {
-    cfg.gridDim = dim3((p.T + kConvRun - 1) / kConvRun, (p.C / 8 + 127) / 128);
+    cfg.gridDim = dim3((p.T + kConvRun - 1) / kConvRun, (p.C / 4 + 127) / 128);
     e = cudaLaunchKernelEx(&cfg, conv1d_silu_rows_kernel, p);
     cfg.gridDim = dim3(p.T, (p.C / 2 + 127) / 128);
   } else if (!p.state_only) {

@@ -32,6 +32,7 @@
 
 #include "../common/device.h"
 #include "../common/ptx.cuh"
+#include "../common/quotient.cuh"
 
 namespace nfb {
 
@@ -658,7 +659,7 @@ __global__ void __launch_bounds__(256) gdn_gated_norm_kernel(const GdnParams p) 
     const float inv = rsqrtf(sq / kD + p.eps);
     float y[4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) y[i] = of[i] * inv * wf[i] * (zf[i] / (1.f + __expf(-zf[i])));
+    for (int i = 0; i < 4; ++i) y[i] = of[i] * inv * wf[i] * gate_by(zf[i], zf[i]);
     uint2 out;
     out.x = pack_bf16x2(y[0], y[1]);
     out.y = pack_bf16x2(y[2], y[3]);

@@ -29,6 +29,7 @@
 #include <unordered_map>
 
 #include "../common/ptx.cuh"
+#include "../common/quotient.cuh"
 #include "../common/tensor_map.h"
 #include "../kv/codec.cuh"
 #include "persist_epilogue.cuh"
@@ -767,7 +768,7 @@ __global__ void __launch_bounds__(kQPersistThreads, 1) gemm_q_persist_kernel(con
               const float own = is_up ? v[8 + j] : v[j];
               const float got = other[j * 32 + lane];
               const float g = is_up ? got : own, u = is_up ? own : got;
-              o2[h] = g / (1.f + __expf(-g)) * u;
+              o2[h] = gate_by(g, g) * u;
             }
             const __nv_bfloat162 units = __floats2bfloat162_rn(o2[0], o2[1]);
             w[m] = swap_pair(*reinterpret_cast<const uint32_t*>(&units), select);

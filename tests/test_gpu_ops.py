@@ -247,6 +247,36 @@ def test_conv_and_gdn_recurrent(ops, lens, heads):
         assert torch.equal(ssm_g[s].cpu(), ssm[s])
 
 
+@pytest.mark.parametrize("lens", [[64], [16, 16, 32], [1, 3, 60, 200], [79], [130, 2, 1, 1]])
+def test_conv_runs_match_single_tokens(ops, lens):
+    """The kernel for runs of tokens (two channels an instruction, quotient by residual) against the per-token one, which takes
+    steps of fewer than 64 tokens and divides: the same bits, infinities, NaN, large and tiny values among them."""
+    torch.manual_seed(6)
+    T, B, C = sum(lens), len(lens), 1032
+    x = torch.randn(T, C + 8).bfloat16()
+    for k, v in enumerate((float("inf"), float("-inf"), float("nan"), 3e38, -3e38, -1000.0, 1000.0, -87.5, -89.0, 1e-38, -1e-38, -0.0)):
+        x[(7 * k + 3) % T, k::101] = v
+    x = x.cuda()
+    w = (torch.randn(C, 4) * 0.5).bfloat16().cuda()
+    hist = torch.randn(B, 3, C).bfloat16().cuda()
+    slot = torch.randperm(B).int().cuda()
+    tok = torch.cat([torch.full((n,), b) for b, n in enumerate(lens)]).int().cuda()
+    cu = torch.tensor([0] + lens).cumsum(0).int().cuda()
+    want_hist, got_hist = hist.clone(), hist.clone()
+    got = torch.full((T, C), 7.0, dtype=torch.bfloat16, device="cuda")
+    ops.causal_conv1d_silu(x, 0, C, w, cu, tok, slot, got_hist, got, True, False, True)
+    want = torch.empty_like(got)
+    for b, n in enumerate(lens):
+        for o in range(0, n, 48):
+            m, s = min(48, n - o), int(cu[b]) + o
+            out = torch.empty((m, C), dtype=torch.bfloat16, device="cuda")
+            ops.causal_conv1d_silu(x[s:s + m], 0, C, w, torch.tensor([0, m]).int().cuda(), torch.zeros(m).int().cuda(), slot[b:b + 1],
+                                   want_hist, out, True, False, False)
+            want[s:s + m] = out
+    assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.nan_to_num(5.0), want.nan_to_num(5.0))
+    assert torch.equal(got_hist.view(torch.int16), want_hist.view(torch.int16))
+
+
 @pytest.mark.parametrize("heads", [(16, 48), (16, 32)])
 @pytest.mark.parametrize("pdl", [False, True])
 @pytest.mark.parametrize("ragged", [False, True])
