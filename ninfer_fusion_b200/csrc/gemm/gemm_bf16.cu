@@ -1030,6 +1030,7 @@ __global__ void __launch_bounds__(kPersistThreads, 1) gemm_persist_kernel(const 
         const float act_a = EPI == kEpiStore && p.act_params != nullptr ? p.act_params[0] : 0.f;
         const float act_b = EPI == kEpiStore && p.act_params != nullptr ? p.act_params[1] : 0.f;
         const bool has32 = EPI == kEpiStore && p.out32 != nullptr && n0 + kTileN > p.out32_from;   // (of the tile)
+        const bool all32 = has32 && n0 >= p.out32_from;
         const long long row0 = t0 + (lane & 1);
         auto live = [&](int c) { return ne < p.N ? min(8, (p.T - t0 - c - (lane & 1) + 1) >> 1) : 0; };
         // The residual may alias the output (in-place update): a chunk's values are fetched one chunk ahead, so that
@@ -1061,8 +1062,20 @@ __global__ void __launch_bounds__(kPersistThreads, 1) gemm_persist_kernel(const 
           }
           if (!has32) {
             store_chunk<EPI == kEpiResidual>({p.out + (row0 + c) * p.ldo + ne, 2 * p.ldo, live(c)}, f, r, select);
+          } else if (all32) {
+            // fp32 columns: a warp's 32 of a token are a line of 128 bytes as they are
+            float* at = p.out32 + (t0 + c) * static_cast<long long>(p.ldo32) + n - p.out32_from;
+            const int n_live = n < p.N ? p.T - t0 - c : 0;
+            if (n_live >= kChunk) {
+#pragma unroll
+              for (int j = 0; j < kChunk; ++j, at += p.ldo32) *at = f[j];
+            } else {
+#pragma unroll
+              for (int j = 0; j < kChunk; ++j, at += p.ldo32)
+                if (j < n_live) *at = f[j];
+            }
           } else {
-            // columns from out32_from on as fp32: pairs swapped in full
+            // columns from out32_from on as fp32, those before as bf16: pairs swapped in full
             const int n_live = live(c);
 #pragma unroll
             for (int m = 0; m < kChunk / 2; ++m) {

@@ -205,6 +205,24 @@ def test_gemm_cta_pairs(ops, status, T, N, K):
     status.check("pairs")
 
 
+@pytest.mark.parametrize("T", [33, 65, 128, 300])
+@pytest.mark.parametrize("first", [0, 128, 130, 250])
+def test_gemm_fp32_columns_of_persistent_tiles(ops, status, T, first):
+    """Columns from `first` on as fp32: whole tiles, one that begins inside a tile, ragged tokens and columns; guards beside both."""
+    N, K = 270, 320
+    x, w = _mk(T, N, K, seed=8)
+    ref = x.float() @ w.float().t()
+    out = torch.full((T + 1, N), float("nan"), device="cuda", dtype=torch.bfloat16)
+    o32 = torch.full((T + 1, N - first + 2), float("nan"), device="cuda")
+    ops.gemm_bf16(x, w, out[:T] if first else None, EPI_STORE, None, None, None, 1, status.tensor, True, 0, out32=o32[:T, : N - first],
+                  out32_from=first)
+    assert (o32[:T, : N - first] - ref[:, first:]).abs().max() <= ref.abs().max() * 2.0 ** -18   # fp32 sums of 320 products
+    assert o32[T].isnan().all() and o32[:, N - first:].isnan().all()
+    if first:
+        assert (out[:T, :first].float() - ref[:, :first]).abs().max() <= ref.abs().max() * 2.0 ** -8
+        assert out[T].isnan().all() and out[:, first:].isnan().all()
+
+
 @pytest.mark.parametrize("T", [65, 128, 129, 160, 256, 257, 300, 1873])
 @pytest.mark.parametrize("N,K", [(264, 2048), (2048, 520), (2048, 4096), (5120, 128)])
 def test_gemm_token_tiles(ops, status, T, N, K):
