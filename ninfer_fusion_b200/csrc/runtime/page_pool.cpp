@@ -70,6 +70,13 @@ NFB_API int32_t nfb200_pool_release(void* h, int32_t page) {
   return c;
 }
 
+// Releases pages[0], pages[1], ..; stops at one that is not allocated.  Returns how many were released.
+NFB_API int32_t nfb200_pool_release_many(void* h, int32_t n, const int32_t* pages) {
+  for (int32_t i = 0; i < n; ++i)
+    if (nfb200_pool_release(h, pages[i]) < 0) return i;
+  return n;
+}
+
 NFB_API int32_t nfb200_pool_refcount(void* h, int32_t page) {
   Pool* p = static_cast<Pool*>(h);
   if (page < 0 || page >= static_cast<int32_t>(p->refcount.size())) return -1;

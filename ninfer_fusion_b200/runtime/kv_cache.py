@@ -17,6 +17,7 @@ from __future__ import annotations
 from dataclasses import dataclass
 from typing import Dict, List, Optional, Sequence
 
+import numpy as np
 import torch
 
 from ..models.config import ModelConfig
@@ -175,6 +176,9 @@ def _load_pool_lib():
         for name in ("retain", "release", "refcount"):
             getattr(lib, f"nfb200_pool_{name}").restype = ctypes.c_int32
             getattr(lib, f"nfb200_pool_{name}").argtypes = [ctypes.c_void_p, ctypes.c_int32]
+        for name in ("alloc_many", "release_many"):
+            getattr(lib, f"nfb200_pool_{name}").restype = ctypes.c_int32
+            getattr(lib, f"nfb200_pool_{name}").argtypes = [ctypes.c_void_p, ctypes.c_int32, ctypes.c_void_p]
         return lib
     except (OSError, AttributeError):
         return None
@@ -219,6 +223,30 @@ class PagePool:
         p = self._free.pop()
         self._ref[p] = 1
         return p
+
+    def alloc_many(self, n: int) -> np.ndarray:
+        """`n` pages as n times `alloc` (int32), or none of them."""
+        out = np.empty(n, dtype=np.int32)
+        if self._h is not None:
+            if self._lib.nfb200_pool_alloc_many(self._h, n, out.ctypes.data) < 0:
+                raise MemoryError("KV page pool exhausted")
+            return out
+        if len(self._free) < n:
+            raise MemoryError("KV page pool exhausted")
+        for i in range(n):
+            out[i] = self.alloc()
+        return out
+
+    def release_many(self, pages: Sequence[int]) -> None:
+        """`release` of each, in order; the first one that is not allocated ends it."""
+        if self._h is None:
+            for p in pages:
+                self.release(p)
+            return
+        a = np.array(pages, dtype=np.int32)
+        done = self._lib.nfb200_pool_release_many(self._h, len(a), a.ctypes.data)
+        if done < len(a):
+            raise RuntimeError(f"page {pages[done]} released twice")
 
     def retain(self, page: int) -> None:
         if self._h is not None:
@@ -305,6 +333,7 @@ class PagedKvCache:
         self.max_pages_per_row = max_pages_per_row
         pin = self.device.type == "cuda"
         self.table_host = torch.full((max_rows, max_pages_per_row), -1, dtype=torch.int32, pin_memory=pin)
+        self._table_np = self.table_host.numpy()
         self.table = torch.full((max_rows, max_pages_per_row), -1, dtype=torch.int32, device=self.device)
         self.row_pages: Dict[int, List[int]] = {}
         self._dirty_rows: set[int] = set()
@@ -387,6 +416,12 @@ class PagedKvCache:
         need = (n_tokens + self.page_size - 1) // self.page_size
         if need > self.max_pages_per_row:
             raise MemoryError(f"row {row}: {n_tokens} tokens exceed the block-table width")
+        have = len(pages)
+        if need - have > 1 and not self.mixed and self.pool.free_pages >= need - have:
+            new = self.pool.alloc_many(need - have)
+            self._table_np[row, have:need] = new
+            pages.extend(new.tolist())
+            self._dirty_rows.add(row)
         while len(pages) < need:
             p = self._page_alloc()
             self.table_host[row, len(pages)] = p
@@ -443,10 +478,13 @@ class PagedKvCache:
         return n
 
     def free_row(self, row: int) -> None:
-        for p in self.row_pages.pop(row, []):
-            if p >= 0:
+        pages = [p for p in self.row_pages.pop(row, []) if p >= 0]
+        if self.mixed:
+            for p in pages:
                 self._page_release(p)
-        self.table_host[row].fill_(-1)
+        else:
+            self.pool.release_many(pages)
+        self._table_np[row].fill(-1)
         self._dirty_rows.add(row)
 
     def fork_row(self, src: int, dst: int, n_tokens: int) -> None:
@@ -593,7 +631,8 @@ class PagedKvCache:
             l.publish()
         if not self._dirty_rows:
             return
-        if len(self._dirty_rows) > 8:
+        # (a copy costs some 7 us of the host's time whatever its size: a small table goes as one)
+        if len(self._dirty_rows) > (1 if self.table.numel() <= 65536 else 8):
             self.table.copy_(self.table_host, non_blocking=True)
         else:
             for r in self._dirty_rows:
@@ -669,10 +708,12 @@ class RecurrentStatePool:
         arrays = self.tensors()
         if n and arrays:   # (a decoder without recurrent layers has no arrays)
             lo = min(slots)
-            if max(slots) - lo + 1 == n:   # neighbours: one view per array, all arrays in a few launches
-                torch._foreach_zero_([t[lo:lo + n] for t in arrays])
+            if max(slots) - lo + 1 == n:   # neighbours: one view per array
+                views = [t[lo:lo + n] for t in arrays]
             else:
-                torch._foreach_zero_([t[s] for t in arrays for s in slots])
+                views = [t[s] for t in arrays for s in slots]
+            for dt in {t.dtype for t in views}:   # (arrays of one type go in a few launches, of several types in one each)
+                torch._foreach_zero_([t for t in views if t.dtype == dt])
         return slots
 
     def release(self, slot: int) -> None:

@@ -64,3 +64,42 @@ def test_alloc_many_is_alloc_n_times(taken, n, shapes):
     with pytest.raises(MemoryError):
         pools[1].alloc_many(7)
     assert pools[1].alloc_many(6 - len(taken) - n) == [pools[0].alloc() for _ in range(6 - len(taken) - n)]
+
+
+@pytest.mark.parametrize("native", [True, False])
+def test_pages_in_one_go(native):
+    """Pages for many positions, and rows given back, as page by page: the same numbers, the same free list, the same state when
+    the pool runs out."""
+    from ninfer_fusion_b200.models.config import TINY_DENSE
+    from ninfer_fusion_b200.runtime.kv_cache import PagedKvCache, PagePool
+    caches = [PagedKvCache(TINY_DENSE, 12, 16, 3, 9, "cpu") for _ in range(2)]
+    for c in caches:
+        c.pool = PagePool(12, use_native=native)
+    bulk, single = caches
+
+    def one_by_one(cache, row, tokens):
+        for n in range(1, tokens + 1):
+            cache.ensure(row, n)
+
+    def same():
+        assert torch.equal(bulk.table_host, single.table_host) and bulk.row_pages == single.row_pages
+        assert bulk._dirty_rows == single._dirty_rows and bulk.pool.free_pages == single.pool.free_pages
+        bulk.publish(), single.publish()
+        assert torch.equal(bulk.table, bulk.table_host) and torch.equal(single.table, single.table_host)
+    for row, n in ((0, 50), (1, 16), (2, 33), (0, 90)):
+        bulk.ensure(row, n)
+        one_by_one(single, row, n)
+        same()
+    for c in caches:
+        c.free_row(1)
+        c.free_row(0)
+    same()
+    bulk.ensure(1, 9 * 16)
+    one_by_one(single, 1, 9 * 16)
+    same()
+    for grow in (lambda: bulk.ensure(0, 40), lambda: one_by_one(single, 0, 40)):   # three pages wanted, none or few left
+        with pytest.raises(MemoryError):
+            grow()
+    same()
+    with pytest.raises(RuntimeError):
+        bulk.pool.release_many([bulk.row_pages[1][0], 11 if bulk.pool.refcount_of(11) == 0 else bulk.row_pages[1][0]])
