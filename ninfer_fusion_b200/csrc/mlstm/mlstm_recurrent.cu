@@ -7,6 +7,7 @@
 
 #include <cooperative_groups.h>
 
+#include "../common/device.h"
 #include "../common/elem.cuh"
 #include "../common/launch.h"
 
@@ -311,6 +312,217 @@ __global__ void __launch_bounds__(kThreads, 3) mlstm_decode_kernel(const MlstmAr
   if (n_cta > 1) cluster.sync();   // nobody leaves while a neighbour may still read its sum
 }
 
+// The same step where there are many states: one CTA per SM walks its (sequence, head) pairs, whole rows of the state in a ring of
+// three buffers that bulk copies fill and empty while the rows in the third are updated.  A thread holds four columns and the
+// sums of four of the sixteen row groups of the kernel above, whose order of summation (rows of a group, pairs of groups, slices
+// of 64 columns) it keeps: the same bits, and a head's norm needs no cluster.
+constexpr int kRing = 3, kChunkRows = 32, kStreamCols = 512, kStreamMaxDim = 512;
+constexpr int kStreamWorkers = 512;
+constexpr int kChunkBytes = kChunkRows * kStreamCols * 4;
+constexpr int kSlices = kStreamCols / 64;
+constexpr int kStreamSmem = kRing * kChunkBytes + 128;
+
+__device__ __forceinline__ void bulk_load(uint32_t smem, const void* src, uint32_t bytes, uint32_t bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+               ::"r"(smem), "l"(src), "r"(bytes), "r"(bar) : "memory");
+}
+__device__ __forceinline__ void bulk_store(void* dst, uint32_t smem, uint32_t bytes) {
+  asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(smem), "r"(bytes) : "memory");
+  asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+}
+
+template <typename A>
+__global__ void __launch_bounds__(kStreamWorkers + 32, 1) mlstm_stream_kernel(const MlstmArgs p) {
+  extern __shared__ __align__(16) uint8_t smem_b[];
+  __shared__ __align__(8) uint64_t bar_full[kRing], bar_done[kRing];
+  __shared__ float qs[kStreamMaxDim], ks[kStreamMaxDim], ns[kStreamMaxDim];
+  __shared__ __align__(16) float part[8][kStreamCols];   // sums of two row groups each
+  __shared__ float den_s[16], ss_s[kSlices];
+  __shared__ int abort_flag;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int D = p.dim, V = p.vdim, H = p.n_heads;
+  const uint32_t ring = (smem_u32(smem_b) + 127u) & ~127u;
+  uint8_t* const ring_gen = smem_b + (ring - smem_u32(smem_b));
+  pdl_launch_next();
+  if (tid == 0) {
+    abort_flag = 0;
+    for (int b = 0; b < kRing; ++b) {
+      mbar_init(smem_u32(&bar_full[b]), 1);
+      mbar_init(smem_u32(&bar_done[b]), kStreamWorkers / 32);
+    }
+    mbar_fence_init();
+  }
+  __syncthreads();
+  volatile int* abortp = &abort_flag;
+  const int chunks = (D + kChunkRows - 1) / kChunkRows;
+  const int items = p.n_seq * H, mine = (items - static_cast<int>(blockIdx.x) + static_cast<int>(gridDim.x) - 1) / static_cast<int>(gridDim.x);
+  const int total = mine * chunks;
+  if (warp == kStreamWorkers / 32) {
+    // ---- copies, one thread.  States and the step's description depend on no kernel of this step: no wait before the first loads ----
+    if (lane == 0) {
+      auto rows = [&](int n, uint32_t& bytes) {
+        const int i = static_cast<int>(blockIdx.x) + n / chunks * static_cast<int>(gridDim.x), c = n % chunks;
+        bytes = static_cast<uint32_t>(min(kChunkRows, D - c * kChunkRows)) * V * 4;
+        return p.S + ((static_cast<long long>(p.state_slot[i / H]) * H + i % H) * D + c * kChunkRows) * V;
+      };
+      int loaded = 0;
+      auto load = [&](int n) {
+        uint32_t bytes;
+        const float* src = rows(n, bytes);
+        const uint32_t bar = smem_u32(&bar_full[n % kRing]);
+        mbar_expect_tx(bar, bytes);
+        bulk_load(ring + (n % kRing) * kChunkBytes, src, bytes, bar);
+        loaded = n + 1;
+      };
+      for (int n = 0; n < min(total, kRing); ++n) load(n);
+      for (int n = 0; n < total; ++n) {
+        if (!mbar_wait(smem_u32(&bar_done[n % kRing]), (n / kRing) & 1, abortp, nullptr, 0)) break;
+        uint32_t bytes;
+        float* dst = rows(n, bytes);
+        bulk_store(dst, ring + (n % kRing) * kChunkBytes, bytes);
+        if (n + kRing < total) {
+          asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");   // the buffer has been read
+          load(n + kRing);
+        }
+      }
+      if (*abortp) {   // unwinding: copies in flight land before the CTA leaves
+        for (int j = max(0, loaded - kRing); j < loaded; ++j)
+          for (uint32_t spin = 0; spin < (1u << 20); ++spin)
+            if (mbar_try_wait(smem_u32(&bar_full[j % kRing]), (j / kRing) & 1)) break;
+      }
+      asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+    }
+    __syncwarp();
+    pdl_wait_prior();   // every warp waits before it leaves: a later kernel's wait then still implies all earlier ones
+    return;
+  }
+  const auto sync = [] { asm volatile("bar.sync 1, 512;" ::: "memory"); };
+  const int cg = tid & 127, quarter = tid >> 7, col = cg * 4;
+  const bool col_ok = col < V;
+  const float inv_cap = 1.f / p.gate_cap;
+  pdl_wait_prior();
+  int n = 0;
+  for (int it = 0; it < mine; ++it) {
+    const int i = static_cast<int>(blockIdx.x) + it * static_cast<int>(gridDim.x), seq = i / H, h = i % H;
+    const int t = p.cu_seqlens[seq];
+    const long long slot = p.state_slot[seq];
+    float* ng = p.n + (slot * H + h) * D;
+    float* mg = p.m + slot * H + h;
+    const A* row = static_cast<const A*>(p.proj) + t * p.ldp;
+    float v4[4] = {0.f, 0.f, 0.f, 0.f};
+    if (col_ok) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) v4[j] = elem_to_f(row[p.v_off + h * V + col + j]);
+    }
+    const float ig = p.gate_cap * tanhf(p.gates[t * p.ldg + p.i_off + h] * inv_cap);
+    const float fr = p.gate_cap * tanhf(p.gates[t * p.ldg + p.f_off + h] * inv_cap);
+    const float fg = fminf(fr, 0.f) - log1pf(expf(-fabsf(fr)));      // log sigmoid
+    const float m_old = *mg;
+    const float m = fmaxf(fg + m_old, ig);
+    const float da = expf(fg + m_old - m), db = expf(ig - m);
+    for (int r = tid; r < D; r += kStreamWorkers) {
+      const float k = elem_to_f(row[p.k_off + h * D + r]) * db;
+      qs[r] = elem_to_f(row[p.q_off + h * D + r]) * p.q_scale;
+      ks[r] = k;
+      ns[r] = fmaf(da, ng[r], k);
+    }
+    sync();
+    if (tid < 16) {
+      float d = 0.f;
+      for (int r = tid; r < D; r += 16) d = fmaf(ns[r], qs[r], d);
+      den_s[tid] = d;
+    }
+    float acc[4][4];
+#pragma unroll
+    for (int g = 0; g < 4; ++g)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) acc[g][e] = 0.f;
+    for (int c = 0; c < chunks; ++c, ++n) {
+      const bool ok = mbar_wait(smem_u32(&bar_full[n % kRing]), (n / kRing) & 1, abortp, nullptr, 0);
+      if (!ok) break;   // (the barriers below are reached all the same)
+      float* const buf = reinterpret_cast<float*>(ring_gen + (n % kRing) * kChunkBytes) + col;
+      if (col_ok) {
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+          if (c * kChunkRows + half * 16 >= D) break;
+          float4 s[4];
+#pragma unroll
+          for (int g = 0; g < 4; ++g) s[g] = *reinterpret_cast<const float4*>(buf + (half * 16 + quarter * 4 + g) * V);
+#pragma unroll
+          for (int g = 0; g < 4; ++g) {
+            const int lr = half * 16 + quarter * 4 + g, r = c * kChunkRows + lr;
+            const float kb = ks[r], qr = qs[r];
+            s[g].x = fmaf(da, s[g].x, kb * v4[0]);
+            s[g].y = fmaf(da, s[g].y, kb * v4[1]);
+            s[g].z = fmaf(da, s[g].z, kb * v4[2]);
+            s[g].w = fmaf(da, s[g].w, kb * v4[3]);
+            *reinterpret_cast<float4*>(buf + lr * V) = s[g];
+            acc[g][0] = fmaf(s[g].x, qr, acc[g][0]);
+            acc[g][1] = fmaf(s[g].y, qr, acc[g][1]);
+            acc[g][2] = fmaf(s[g].z, qr, acc[g][2]);
+            acc[g][3] = fmaf(s[g].w, qr, acc[g][3]);
+          }
+        }
+        fence_proxy_async_smem();
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(smem_u32(&bar_done[n % kRing]));
+    }
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+      *reinterpret_cast<float4*>(&part[2 * quarter + j][col]) =
+          make_float4(acc[2 * j][0] + acc[2 * j + 1][0], acc[2 * j][1] + acc[2 * j + 1][1], acc[2 * j][2] + acc[2 * j + 1][2],
+                      acc[2 * j][3] + acc[2 * j + 1][3]);
+    for (int r = tid; r < D; r += kStreamWorkers) ng[r] = ns[r];
+    if (tid == 0) *mg = m;
+    sync();
+    float o4[4] = {0.f, 0.f, 0.f, 0.f};
+    if (tid < 128) {
+      float den = 0.f, sq = 0.f;
+#pragma unroll
+      for (int w = 0; w < 8; ++w) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) o4[e] += part[w][col + e];
+        den += den_s[2 * w] + den_s[2 * w + 1];
+      }
+      const float inv = 1.f / (fmaxf(fabsf(den), expf(-m)) + 1e-6f);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        o4[e] *= inv;
+        sq += o4[e] * o4[e];
+      }
+#pragma unroll
+      for (int o = 8; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
+      if ((lane & 15) == 0) ss_s[tid >> 4] = sq;
+    }
+    sync();
+    if (tid < 128 && col_ok) {
+      float sum = 0.f;
+      for (int r = 0; r < (V + 63) / 64; ++r) sum += ss_s[r];
+      const float inv = 1.f / sqrtf(sum / static_cast<float>(p.vdim_true) + p.eps);
+      const A* gr = row + p.g_off + h * V + col;
+      A* dst = static_cast<A*>(p.out) + t * p.ldo + h * V + col;
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        dst[e] = elem_from_f<A>(o4[e] * inv * p.norm[h * V + col + e] * sigmoid_of<A>(elem_to_f(gr[e])));
+    }
+  }
+}
+
+template <typename A>
+cudaError_t launch_stream(const MlstmArgs& a) {
+  auto kern = mlstm_stream_kernel<A>;
+  static bool attr_set = false;
+  if (!attr_set) {
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kStreamSmem);
+    if (e != cudaSuccess) return e;
+    attr_set = true;
+  }
+  const long long items = static_cast<long long>(a.n_seq) * a.n_heads;
+  const unsigned int ctas = static_cast<unsigned int>(items < device_sm_count() ? items : device_sm_count());
+  return launch_kernel(kern, dim3(ctas), dim3(kStreamWorkers + 32), kStreamSmem, a.stream, a.pdl, 1, a);
+}
+
 template <typename A, int VC>
 cudaError_t launch_decode(const MlstmArgs& a) {
   const size_t smem = sizeof(float) * (3 * static_cast<size_t>(a.dim) + kThreads / 32 * (VC / 4) * 5);
@@ -331,6 +543,16 @@ cudaError_t launch(const MlstmArgs& a) {
 template <typename A>
 const char* dispatch(const MlstmArgs& a) {
   cudaError_t e;
+  // States of 256 KB and more, and two for every five SMs at least: below, the CTAs of a head's cluster read a state faster than one
+  // CTA does.  Step of the 1 B layer-list decoder, twelve layers of four heads of 256 x 512 (512 KB), us, clusters -> streamed:
+  // 12 sequences 1039 and 1089, 16 1157 -> 1110, 24 1359 -> 1232, 32 1570 -> 1359 (a layer 40 -> 23, 21 at the copy rate),
+  // 64 2072 -> 1846.
+  if (a.one_token && a.write_state && a.vdim <= kStreamCols && a.dim <= kStreamMaxDim &&
+      static_cast<long long>(a.dim) * a.vdim * 4 >= 256 * 1024 &&
+      5LL * a.n_seq * a.n_heads >= 2LL * device_sm_count() && (reinterpret_cast<uintptr_t>(a.S) & 15) == 0) {
+    e = launch_stream<A>(a);
+    return e == cudaSuccess ? nullptr : cudaGetErrorString(e);
+  }
   if (a.one_token) {
     e = a.vdim <= 8 * 64 ? launch_decode<A, 64>(a) : launch_decode<A, 128>(a);
     return e == cudaSuccess ? nullptr : cudaGetErrorString(e);

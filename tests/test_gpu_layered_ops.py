@@ -294,6 +294,37 @@ def test_matrix_memory(ops, geo, dt, i_shift, f_shift):
             assert rel(a, b) < 3e-5
 
 
+@pytest.mark.parametrize("geo", [(4, 256, 512), (3, 272, 496), (5, 512, 240), (2, 144, 512)])
+@pytest.mark.parametrize("dt", DTYPES)
+@pytest.mark.parametrize("pdl", [False, True])
+def test_matrix_memory_step_of_many_states(ops, geo, dt, pdl):
+    """Enough large states for the streaming kernel (more than one a CTA in the largest case) against the cluster kernel that a few
+    sequences at a time take: outputs and states bit for bit, ragged last chunks and column slices, slots in any order."""
+    H, D, V = geo
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    B = (sms + H) // H + 2 if H == 4 else 2 * sms // (5 * H) + 1
+    assert D * V * 4 >= 256 * 1024 and 5 * B * H >= 2 * sms
+    few = max(1, 2 * sms // (5 * H) - 1)
+    torch.manual_seed(9)
+    proj = torch.randn(B, H * (2 * D + 2 * V), device="cuda").to(dt)
+    gates = torch.randn(B, 2 * H, device="cuda") * 3 + torch.tensor([0.0] * H + [2.0] * H, device="cuda")
+    norm = 1 + 0.3 * torch.randn(H * V, device="cuda")
+    slot = torch.randperm(B + 1, device="cuda")[:B].int()
+    first = [torch.randn(B + 1, H, D, V, device="cuda") * 0.2, torch.randn(B + 1, H, D, device="cuda"), torch.rand(B + 1, H, device="cuda")]
+    got = []
+    for size in (few, B):
+        S, n, m = (t.clone() for t in first)
+        out = torch.full((B, H * V), float("nan"), dtype=dt, device="cuda")
+        for b in range(0, B, size):
+            e = min(B, b + size)
+            ops.mlstm(proj[b:e], 0, H * D, 2 * H * D, H * (2 * D + V), gates[b:e], 0, H, V, D ** -0.5, 8.0, 1e-3, norm,
+                      torch.arange(e - b + 1, dtype=torch.int32, device="cuda"), slot[b:e], S, n, m, out[b:e], True, None, pdl, True)
+        got.append((out, S, n, m))
+    for a, b in zip(*got):
+        assert torch.equal(a, b) and not a.isnan().any()
+    assert not torch.equal(got[0][1], first[0])
+
+
 @pytest.mark.parametrize("dt", DTYPES)
 def test_token_selection_on_both_logit_types(ops, dt):
     lg = rnd(3, 5, 301).to(dt)
