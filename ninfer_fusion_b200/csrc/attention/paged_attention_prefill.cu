@@ -7,13 +7,13 @@
 //   O[128 rows, 256 d]  += P . V       P in TMEM (fp16, over the S it came from), V in shared memory as it lies in the
 //                                      page ([key][d] = an MN-major operand: no transpose), O in TMEM
 //
-// Thirteen warps:
-//   0..3    softmax, one row per thread: Q into TMEM, then per tile the row maximum, exp2, P back to TMEM, the row sum in a
-//           register; at the end the normalised row
-//   4..7    K: rows of a tile gathered from their pages into registers up to two tiles ahead of their use, dequantised once
+// Seventeen warps:
+//   0..7    softmax, two threads per row: Q into TMEM, then per tile the row maximum, exp2, P back to TMEM, the row sum in
+//           registers; at the end the normalised row.  Of every eight keys one thread takes the first four and the other the rest
+//   8..11   K: rows of a tile gathered from their pages into registers up to two tiles ahead of their use, dequantised once
 //           (bf16 / fp8-row / int8-group / nvfp4 -> fp16) into one of two shared-memory slots
-//   8..11   V, the same way; 4..11 also load the output gate beside the last products and store the result
-//   12      issues the products: S of tile i + 1 goes in front of P V of tile i, so that the softmax of one tile runs beside
+//   12..15  V, the same way; 8..15 also load the output gate beside the last products and store the result
+//   16      issues the products: S of tile i + 1 goes in front of P V of tile i, so that the softmax of one tile runs beside
 //           the products of its neighbours
 // The row scales of fp8 pages never touch the operands: the K scale multiplies a key's column of S, the V scale its
 // probability.  A row's exponentials are taken against its largest score so far, so that no probability exceeds one (times an
@@ -24,16 +24,23 @@
 //
 // TMEM is full (two S buffers of 64 columns, Q 128, O 256).  Q lies there and not in shared memory because the gathers need
 // the room: with Q and 128-key K and V tiles in shared memory (192 KB) 28 KB of L1 were left, which bound the loads in flight
-// and with them the kernel (4.2 us per 128 keys; the products alone take 1.6).  Now the serial chain scores -> softmax -> P of
-// a tile bounds it (4.1 us per 128 keys, a tenth of it the rescaling of O; against a maximum that lags by up to four powers of
-// two it was 3.7, with other roundings).  24 / 4 heads, 2048 queries, us, the mma.sync kernel before -> now: fp8 rows, 2048 keys
-// 386 -> 167, 16384 keys 3715 -> 1363 (567 TFLOP/s); bf16 rows, 8192 keys 1990 -> 750; nvfp4 1878 -> 682; bits are the same.
+// and with them the kernel (4.2 us per 128 keys; the products alone take 1.6).  Then the serial chain scores -> softmax -> P of
+// a tile bounds it, with one thread per row, and instructions: of the four schedulers one had the issuer, a softmax, a K and a V
+// warp to choose from, and divisions by the page size, selects per row and stores with two-way conflicts to issue (issue slots
+// 54 %, the integer units 45 %, a fifth of the stalls for instructions not yet fetched).  Two threads per row, pages walked
+// without a division, row numbers of 32 bits, the check for keys without a row once per tile and conflict-free stores: 24 / 4
+// heads, 2048 queries, us, before -> now: 2048 keys, fp8 rows 161 -> 125, bf16 164 -> 130, nvfp4 152 -> 118, int8 174 -> 143;
+// 16384 keys, fp8 rows 1367 -> 1122 (689 TFLOP/s), bf16 1526 -> 1258, nvfp4 1337 -> 1067, int8 1696 -> 1453; 300 queries, 1500
+// keys 68 -> 55; 37 tokens, of which a launch is the most, 21.5 -> 15.7; bits are the same.  Left: 3.4 us per 128 keys, the
+// chain of a tile still (a maximum that lags by up to four powers of two would spare a tenth of it, with other roundings).
 //
 // Reference kernels covered: kernel/gqa_attention_prefill_{bf16,i8,nvfp4}.cuh (Br = 64 x Bc = 64
 // mma.sync kernels that also quantise-append in-kernel).
 #include "attention.h"
 
 #include <math_constants.h>
+
+#include <type_traits>
 
 #include "../common/quotient.cuh"
 #include "attn_mma_common.cuh"
@@ -51,8 +58,11 @@ constexpr int kKeys = 64;                    // keys per tile
 constexpr int kAtomBytes = kKeys * 128;      // 64 columns of d: [64 keys][128 bytes], 8-row swizzle atoms of 1024 bytes
 constexpr int kTileBytes = 4 * kAtomBytes;   // one [64][256] fp16 operand
 constexpr int kSmemBytes = 4 * kTileBytes + 1024;   // two slots of K, two of V
-constexpr int kGroup = 128;                  // threads of the softmax, K and V groups
-constexpr int kThreads = 3 * kGroup + 32;
+constexpr int kGroup = 128;                  // threads of the K and V groups, and of each half of the softmax
+constexpr int kSoftmax = 2 * kGroup;
+constexpr int kThreads = kSoftmax + 2 * kGroup + 32;
+constexpr int kIssuer = kThreads / 32 - 1;   // warp that issues the products
+constexpr int kHalfKeys = kKeys / 2;
 constexpr int kUnits = kKeys * 16 / kGroup;  // 16-value units per thread and tile
 constexpr int kStagePitch = 2 * D + 16;      // bytes per row of the output tile: neighbouring rows start in other banks
 constexpr uint32_t kColQ = 128, kColO = 256; // TMEM: S / P of even tiles at 0, of odd tiles at 64, then Q and O
@@ -97,12 +107,11 @@ __device__ __forceinline__ void tmem_ld_wait_x32(uint32_t* r) {
   asm volatile("" : "+r"(r[16]), "+r"(r[17]), "+r"(r[18]), "+r"(r[19]), "+r"(r[20]), "+r"(r[21]), "+r"(r[22]), "+r"(r[23]),
                "+r"(r[24]), "+r"(r[25]), "+r"(r[26]), "+r"(r[27]), "+r"(r[28]), "+r"(r[29]), "+r"(r[30]), "+r"(r[31]));
 }
-__device__ __forceinline__ void tmem_ld_wait_x32(uint32_t* a, uint32_t* b) {
-  tmem_ld_wait_x32(a);
-  asm volatile("" : "+r"(b[0]), "+r"(b[1]), "+r"(b[2]), "+r"(b[3]), "+r"(b[4]), "+r"(b[5]), "+r"(b[6]), "+r"(b[7]), "+r"(b[8]),
-               "+r"(b[9]), "+r"(b[10]), "+r"(b[11]), "+r"(b[12]), "+r"(b[13]), "+r"(b[14]), "+r"(b[15]));
-  asm volatile("" : "+r"(b[16]), "+r"(b[17]), "+r"(b[18]), "+r"(b[19]), "+r"(b[20]), "+r"(b[21]), "+r"(b[22]), "+r"(b[23]),
-               "+r"(b[24]), "+r"(b[25]), "+r"(b[26]), "+r"(b[27]), "+r"(b[28]), "+r"(b[29]), "+r"(b[30]), "+r"(b[31]));
+__device__ __forceinline__ void tmem_ld_x4(uint32_t taddr, uint32_t* r) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(taddr));
+}
+__device__ __forceinline__ void tmem_st_x2(uint32_t taddr, uint32_t a, uint32_t b) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x2.b32 [%0], {%1,%2};" ::"r"(taddr), "r"(a), "r"(b) : "memory");
 }
 __device__ __forceinline__ void tmem_st_x16(uint32_t taddr, const uint32_t* r) {
   asm volatile(
@@ -116,6 +125,15 @@ __device__ __forceinline__ float ex2(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
+}
+// two floats in one instruction
+__device__ __forceinline__ void mul2(uint32_t& x, uint32_t& y, float a, float b) {
+  asm("{\n\t.reg .b64 u, w;\n\tmov.b64 u, {%0, %1};\n\tmov.b64 w, {%2, %3};\n\tmul.rn.f32x2 u, u, w;\n\tmov.b64 {%0, %1}, u;\n\t}"
+      : "+r"(x), "+r"(y) : "f"(a), "f"(b));
+}
+__device__ __forceinline__ void add2(float& x, float& y, float a, float b) {
+  asm("{\n\t.reg .b64 u, w;\n\tmov.b64 u, {%0, %1};\n\tmov.b64 w, {%2, %3};\n\tadd.rn.f32x2 u, u, w;\n\tmov.b64 {%0, %1}, u;\n\t}"
+      : "+f"(x), "+f"(y) : "f"(a), "f"(b));
 }
 __device__ __forceinline__ void group_bar(int id) { asm volatile("bar.sync %0, 128;" ::"r"(id) : "memory"); }
 // 16 bytes of a bf16 row: rows at any even element address are accepted, 16-byte accesses are used where all of them are aligned
@@ -133,22 +151,18 @@ __device__ __forceinline__ void store_row16(__nv_bfloat16* dst, uint4 v, bool wi
   }
 }
 
-// Converts this thread's units of a tile into the operand at `dst`.  Lanes whose unit lies in an odd group of 64 columns
-// store their halves in the other order: eight neighbouring lanes then hit eight bank groups.
-template <int FORMAT, int N>
-__device__ __forceinline__ void store_units(const RawUnit<FORMAT>* raw, uint32_t live, int gtid, uint8_t* dst) {
-#pragma unroll
-  for (int i = 0; i < N; ++i) {
-    const int u = i * kGroup + gtid;
-    const int r = u >> 4, part = u & 15, chunk = (part & 3) * 2, swap = (part >> 2) & 1;
-    uint32_t h[8];
-    raw[i].convert(h, (live >> i) & 1u);
-    uint8_t* row = dst + (part >> 2) * kAtomBytes + r * 128;
-    const uint4 lo = make_uint4(h[0], h[1], h[2], h[3]), hi = make_uint4(h[4], h[5], h[6], h[7]);
-    *reinterpret_cast<uint4*>(row + (((chunk + swap) ^ (r & 7)) << 4)) = swap ? hi : lo;
-    *reinterpret_cast<uint4*>(row + (((chunk + 1 - swap) ^ (r & 7)) << 4)) = swap ? lo : hi;
+// The page of a key and its place there, for keys that come a tile apart (page sizes need not divide a tile or be divided by it).
+struct PageWalk {
+  int page, at;
+  __device__ __forceinline__ PageWalk(int key, int size) : page(key / size), at(key - key / size * size) {}
+  __device__ __forceinline__ void next_tile(int size) {
+    at += kKeys;
+    while (at >= size) {
+      at -= size;
+      ++page;
+    }
   }
-}
+};
 
 template <int FORMAT>
 __global__ void __launch_bounds__(kThreads, 1) paged_attn_prefill_kernel(const PrefillAttnParams p) {
@@ -156,8 +170,12 @@ __global__ void __launch_bounds__(kThreads, 1) paged_attn_prefill_kernel(const P
   __shared__ __align__(8) Bars bars;
   __shared__ uint32_t tmem_base_slot;
   __shared__ int abort_flag;
-  __shared__ long long rows_s[2][4][kKeys];                  // [K, V][tile mod 4]: cache rows of the tile's keys
+  // (rows have 144 bytes or more: 2^31 of them are more than the memory; a mixed layer's carry their tier in the top bits)
+  using Row = std::conditional_t<FORMAT == kKvMixed, long long, int>;
+  __shared__ Row rows_s[2][4][kKeys];                        // [K, V][tile mod 4]: cache rows of the tile's keys, -1: none
+  __shared__ uint32_t all_s[2][4][2];                        // whether all keys of a half tile have rows
   __shared__ __align__(16) float scale_s[2][2][kKeys];       // [tile parity][K, V]
+  __shared__ float half_s[2][2][kRows];                      // [tile parity][half]: what the halves of a row tell one another
   constexpr bool kScaled = FORMAT == kKvFp8Row || FORMAT == kKvMixed;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -173,12 +191,12 @@ __global__ void __launch_bounds__(kThreads, 1) paged_attn_prefill_kernel(const P
       mbar_init(smem_u32(&bars.v_full[b]), 4);
       mbar_init(smem_u32(&bars.v_empty[b]), 1);
       mbar_init(smem_u32(&bars.s_full[b]), 1);
-      mbar_init(smem_u32(&bars.p_full[b]), 4);
+      mbar_init(smem_u32(&bars.p_full[b]), kSoftmax / 32);
     }
     mbar_init(smem_u32(&bars.o_done), 1);
     mbar_fence_init();
   }
-  if (warp == 12) {
+  if (warp == kIssuer) {
     tmem_alloc(smem_u32(&tmem_base_slot), 512);
     tmem_relinquish();
   }
@@ -208,7 +226,7 @@ __global__ void __launch_bounds__(kThreads, 1) paged_attn_prefill_kernel(const P
                       static_cast<uintptr_t>(p.ld_gate * 2)) & 15) == 0;
   uint8_t* const stage = smem_gen;   // output tile, over the K and V slots once every product has retired
 
-  if (warp == 12) {
+  if (warp == kIssuer) {
     // =========================== issuer of the products ===========================
     if (elect_one()) {
       auto scores = [&](int i) {
@@ -249,31 +267,60 @@ __global__ void __launch_bounds__(kThreads, 1) paged_attn_prefill_kernel(const P
       }
     }
     __syncwarp();
-  } else if (warp >= 4) {
-    // =========================== K (warps 4..7) and V (warps 8..11) ===========================
+  } else if (warp >= kSoftmax / 32) {
+    // =========================== K (warps 8..11) and V (warps 12..15) ===========================
     // A wait that runs out sets the abort word and the status; the loop goes on, so that the group's barriers stay uniform.
-    const int which = warp >= 8 ? 1 : 0, gtid = threadIdx.x & (kGroup - 1);
+    const int which = warp >= 12 ? 1 : 0, gtid = threadIdx.x & (kGroup - 1);
     // tiles in registers: the gathers of a tile are issued when the tile `kSets` before it has been converted (bf16 units are
     // 32 bytes each: one tile fits)
     constexpr int kSets = FORMAT == kKvBf16 || FORMAT == kKvMixed ? 1 : 2;
     RawUnit<FORMAT> raw[kSets][kUnits];
     uint32_t live[kSets];   // bit per unit: its row exists
-    // page of this thread's key of tile i (-1: none, or released: its rows are zero), and the row behind it
-    auto page_of = [&](int i) {
-      const int key = k_first + i * kKeys + gtid;
-      return gtid < kKeys && key < k_end ? table[key / P] : -1;
+    // page of this thread's key of the next tile asked for (-1: none, or released: its rows are zero), and the row behind it
+    PageWalk ask(k_first + (gtid & (kKeys - 1)), P), place = ask;
+    int ask_key = k_first + gtid;
+    auto next_page = [&] {
+      const int page = gtid < kKeys && ask_key < k_end ? table[ask.page] : -1;
+      ask_key += kKeys;
+      ask.next_tile(P);
+      return page;
     };
     auto publish_row = [&](int i, int page) {
-      if (gtid < kKeys) rows_s[which][i & 3][gtid] = kv_row_of(p.kv, page, kvh, (k_first + i * kKeys + gtid) % P);
+      if (gtid < kKeys) {
+        const long long r = kv_row_of(p.kv, page, kvh, place.at);
+        rows_s[which][i & 3][gtid] = static_cast<Row>(r);
+        const bool all = __all_sync(0xffffffffu, r >= 0);
+        if (lane == 0) all_s[which][i & 3][gtid >> 5] = all;
+      }
+      place.next_tile(P);
     };
-    auto load = [&](int i, RawUnit<FORMAT>* dst) {
-      uint32_t m = 0;
-#pragma unroll
-      for (int j = 0; j < kUnits; ++j) {
-        const int u = j * kGroup + gtid;
-        const long long r = rows_s[which][i & 3][u >> 4];
-        dst[j].load_row(p.kv, which, r, u & 15);
-        m |= static_cast<uint32_t>(r >= 0) << j;
+    const uint8_t* const codes = which ? p.kv.v_codes : p.kv.k_codes;
+    const uint8_t* const scales = which ? p.kv.v_scales : p.kv.k_scales;
+    // Eight neighbouring lanes have four units of an even row and of the odd one behind it: the swizzle puts their halves into
+    // eight bank groups.
+    const int r0 = (gtid >> 5) * 2 + ((gtid >> 2) & 1), part = ((gtid >> 3) & 3) * 4 + (gtid & 3);
+    const int chunk = (part & 3) * 2;
+    uint8_t* const place0 = smem_gen + 2 * which * kTileBytes + (part >> 2) * kAtomBytes + r0 * 128;
+    uint8_t* const lo0 = place0 + ((chunk ^ r0) << 4);
+    uint8_t* const hi0 = place0 + (((chunk + 1) ^ r0) << 4);
+    // unit j of a tile: this thread's sixteen columns of its key in the j-th eight
+    auto load_unit = [&](int i, int j, RawUnit<FORMAT>& dst) {
+      const Row r = rows_s[which][i & 3][8 * j + r0];
+      if constexpr (FORMAT == kKvMixed) dst.load_row(p.kv, which, r, part);
+      else dst.load(p.kv, codes, scales, max(r, 0), part);
+    };
+    auto store_unit = [&](const RawUnit<FORMAT>& src, uint32_t exists, int b, int j) {
+      uint32_t h[8];
+      src.convert(h, exists);
+      *reinterpret_cast<uint4*>(lo0 + b * kTileBytes + j * 1024) = make_uint4(h[0], h[1], h[2], h[3]);
+      *reinterpret_cast<uint4*>(hi0 + b * kTileBytes + j * 1024) = make_uint4(h[4], h[5], h[6], h[7]);
+    };
+    auto live_units = [&](int i) {
+      uint32_t m = (1u << kUnits) - 1;
+      if (!(all_s[which][i & 3][0] & all_s[which][i & 3][1])) {
+        m = 0;
+#pragma unroll 1
+        for (int j = 0; j < kUnits; ++j) m |= static_cast<uint32_t>(rows_s[which][i & 3][8 * j + r0] >= 0) << j;
       }
       return m;
     };
@@ -281,27 +328,52 @@ __global__ void __launch_bounds__(kThreads, 1) paged_attn_prefill_kernel(const P
     if (n_tiles > 0) {
       int pages[3];
 #pragma unroll
-      for (int i = 0; i < 3; ++i) pages[i] = page_of(i);
-      page_next = page_of(3);
+      for (int i = 0; i < 3; ++i) pages[i] = next_page();
+      page_next = next_page();
 #pragma unroll
       for (int i = 0; i < 3; ++i) publish_row(i, pages[i]);
       group_bar(2 + which);
 #pragma unroll
-      for (int i = 0; i < kSets; ++i) live[i] = load(i, raw[i]);
+      for (int i = 0; i < kSets; ++i) {
+        live[i] = live_units(i);
+#pragma unroll
+        for (int j = 0; j < kUnits; ++j) load_unit(i, j, raw[i][j]);
+      }
     }
     auto step = [&](int i, RawUnit<FORMAT>* set, uint32_t& mask) {
       const int b = i & 1;
       const uint32_t freed = smem_u32(which ? &bars.v_empty[b] : &bars.k_empty[b]);
       if (i >= 2) mbar_wait(freed, ((i >> 1) - 1) & 1, abortp, p.status, kStatusPrefillWait);
-      store_units<FORMAT, kUnits>(set, mask, gtid, smem_gen + (2 * which + b) * kTileBytes);
+      // With one set a unit's registers take the next tile as soon as it is converted (its rows were published long ago); with two
+      // the loads wait for the last conversion, since one that waits for its data waits for the loads issued before it too
+      // (2048 queries, 16384 keys: int8, interleaved, 3052 us where 1453; bf16, not, 1550 where 1258).
+      uint32_t next_mask = 0;
+      if constexpr (kSets == 1) {
+        const bool more = i + 1 < n_tiles;
+        if (more) next_mask = live_units(i + 1);
+#pragma unroll
+        for (int j = 0; j < kUnits; ++j) {
+          store_unit(set[j], (mask >> j) & 1u, b, j);
+          if (more) load_unit(i + 1, j, set[j]);
+        }
+      } else {
+#pragma unroll
+        for (int j = 0; j < kUnits; ++j) store_unit(set[j], (mask >> j) & 1u, b, j);
+      }
       fence_proxy_async_smem();
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(which ? &bars.v_full[b] : &bars.k_full[b]));
-      // rows of tile i + 3 from the page asked for a tile ago; rows of tile i + kSets were published before this barrier
+      // rows of tile i + 3 from the page asked for a tile ago
       publish_row(i + 3, page_next);
-      page_next = page_of(i + 4);
+      page_next = next_page();
       group_bar(2 + which);
-      if (i + kSets < n_tiles) mask = load(i + kSets, set);
+      if constexpr (kSets == 1) {
+        mask = next_mask;
+      } else if (i + 2 < n_tiles) {
+#pragma unroll
+        for (int j = 0; j < kUnits; ++j) load_unit(i + 2, j, set[j]);
+        mask = live_units(i + 2);
+      }
     };
     for (int i = 0; i < n_tiles; i += kSets) {
       step(i, raw[0], live[0]);
@@ -313,7 +385,7 @@ __global__ void __launch_bounds__(kThreads, 1) paged_attn_prefill_kernel(const P
     //      one key tile, took 59 us a layer so, 39 in a loop.) ----
     constexpr int kOut = kRows * (D / 8) / (2 * kGroup), kBatch = 4;   // 16-byte pieces per thread, and at a time
     uint4 gate[kBatch];
-    const int otid = threadIdx.x - kGroup;
+    const int otid = threadIdx.x - kSoftmax;
     auto load_gates = [&](int j0) {
 #pragma unroll
       for (int j = 0; j < kBatch; ++j) {
@@ -324,7 +396,7 @@ __global__ void __launch_bounds__(kThreads, 1) paged_attn_prefill_kernel(const P
       }
     };
     load_gates(0);
-    asm volatile("bar.sync 4, 384;" ::: "memory");
+    asm volatile("bar.sync 4, 512;" ::: "memory");
 #pragma unroll 1
     for (int j0 = 0; j0 < kOut && (j0 * 2 * kGroup >> 5) < n_rows; j0 += kBatch) {
 #pragma unroll
@@ -347,27 +419,30 @@ __global__ void __launch_bounds__(kThreads, 1) paged_attn_prefill_kernel(const P
       if (j0 + kBatch < kOut) load_gates(j0 + kBatch);
     }
   } else {
-    // =========================== softmax: thread = row = TMEM lane ===========================
-    const int row = threadIdx.x;
-    const uint32_t lane_sel = static_cast<uint32_t>(warp * 32) << 16;
+    // =========================== softmax: two threads per row = TMEM lane ===========================
+    // Warps w and w + 4 share 32 rows: of every eight keys the first half takes the first four, the second the others, and
+    // each half of the columns of Q and O.  (The row sum's four parts go by pairs of keys, so that each has two of them.)
+    const int row = threadIdx.x & (kRows - 1), half = threadIdx.x / kRows;
+    const uint32_t lane_sel = static_cast<uint32_t>((warp & 3) * 32) << 16;
+    const auto row_bar = [&] { asm volatile("bar.sync %0, 64;" ::"r"(5 + (warp & 3)) : "memory"); };   // both halves of 32 rows
     // ---- this row of Q, (token row / G, head row % G), pre-scaled for exp2 softmax; rows past the block are zero ----
     if (n_tiles > 0) {
       const float qscale = p.sm_scale * 1.4426950408889634f;
       const __nv_bfloat16* src = p.q + (static_cast<long long>(t0 + row / G) * p.n_q_heads + kvh * G + row % G) * D;
 #pragma unroll
-      for (int c = 0; c < D; c += 64) {
-        uint4 raw[8];
+      for (int c0 = 0; c0 < D / 2; c0 += 32) {
+        const int c = half * (D / 2) + c0;
+        uint4 raw[4];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) raw[j] = row < n_rows ? load_row16(src + c + 8 * j, wide) : make_uint4(0, 0, 0, 0);
-        uint32_t h[32];
+        for (int j = 0; j < 4; ++j) raw[j] = row < n_rows ? load_row16(src + c + 8 * j, wide) : make_uint4(0, 0, 0, 0);
+        uint32_t h[16];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
+        for (int j = 0; j < 4; ++j) {
           const __nv_bfloat162* v = reinterpret_cast<const __nv_bfloat162*>(&raw[j]);
 #pragma unroll
           for (int e = 0; e < 4; ++e) h[4 * j + e] = pack_half2(__bfloat162float(v[e].x) * qscale, __bfloat162float(v[e].y) * qscale);
         }
         tmem_st_x16(tmem + lane_sel + kColQ + c / 2, h);
-        tmem_st_x16(tmem + lane_sel + kColQ + c / 2 + 16, h + 16);
       }
       tmem_st_wait();
       tc_fence_before();
@@ -380,18 +455,22 @@ __global__ void __launch_bounds__(kThreads, 1) paged_attn_prefill_kernel(const P
       lim = p.q_kv_len[t0 + row / G];
       if (p.window > 0) lo = max(0, lim - p.window);
     }
-    // Scales of a tile: threads 0..63 fetch the K scales, 64..127 the V scales, the page two tiles and the scale one tile
-    // ahead of their use.
+    // Scales of a tile: of the first half threads 0..63 fetch the K scales, 64..127 the V scales, the page two tiles and the
+    // scale one tile ahead of their use.
     const int sv = row >> 6, skey = row & 63;
     int page_next = -1;
     uint32_t scale_raw = 0;    // fp8: the fp16 bits as loaded (decoded where they are used); mixed: the value's bits
     bool scale_live = false;
-    auto fetch_page = [&](int i) {
-      const int key = k_first + i * kKeys + skey;
-      page_next = key < k_end ? table[key / P] : -1;
+    PageWalk ask(k_first + skey, P), place = ask;
+    int ask_key = k_first + skey;
+    auto fetch_page = [&] {
+      page_next = ask_key < k_end ? table[ask.page] : -1;
+      ask_key += kKeys;
+      ask.next_tile(P);
     };
-    auto fetch_scale = [&](int i) {
-      const long long r = kv_row_of(p.kv, page_next, kvh, (k_first + i * kKeys + skey) % P);
+    auto fetch_scale = [&] {
+      const long long r = kv_row_of(p.kv, page_next, kvh, place.at);
+      place.next_tile(P);
       scale_live = r >= 0;
       if (FORMAT == kKvFp8Row) {
         scale_raw = reinterpret_cast<const uint16_t*>(sv ? p.kv.v_scales : p.kv.k_scales)[scale_live ? r : 0];
@@ -402,57 +481,63 @@ __global__ void __launch_bounds__(kThreads, 1) paged_attn_prefill_kernel(const P
         scale_raw = __float_as_uint(f);
       }
     };
-    if (kScaled && n_tiles > 0) {
-      fetch_page(0);
-      fetch_scale(0);
-      fetch_page(1);
+    if (kScaled && half == 0 && n_tiles > 0) {
+      fetch_page();
+      fetch_scale();
+      fetch_page();
     }
     float top = -CUDART_INF_F;   // the row's largest score so far
-    // The row sum in four parts, by pairs of keys: a row's parts are summed in key order whatever the block it is in.
-    float l4[4] = {0.f, 0.f, 0.f, 0.f};
+    // This half's two of the row sum's four parts: a row's parts are summed in key order whatever the block it is in.
+    float l2[2] = {0.f, 0.f};
     for (int i = 0; i < n_tiles; ++i) {
-      const int b = i & 1, kb = k_first + i * kKeys;
-      const float* ks = scale_s[b][0];
-      const float* vs = scale_s[b][1];
+      const int b = i & 1, kb = k_first + i * kKeys + half * 4;   // key of value j: kb + j / 4 * 8 + j % 4
+      const float* ks = scale_s[b][0] + half * 4;
+      const float* vs = scale_s[b][1] + half * 4;
       if constexpr (kScaled) {
-        const float value = FORMAT == kKvFp8Row ? __half2float(__ushort_as_half(static_cast<unsigned short>(scale_raw))) : __uint_as_float(scale_raw);
-        const float scale = scale_live ? value : 0.f;
-        scale_s[b][sv][skey] = scale;
-        group_bar(1);
-        fetch_scale(i + 1);
-        fetch_page(i + 2);
+        if (half == 0) {
+          const float value = FORMAT == kKvFp8Row ? __half2float(__ushort_as_half(static_cast<unsigned short>(scale_raw))) : __uint_as_float(scale_raw);
+          scale_s[b][sv][skey] = scale_live ? value : 0.f;
+        }
+        asm volatile("bar.sync 1, 256;" ::: "memory");
+        if (half == 0) {
+          fetch_scale();
+          fetch_page();
+        }
       }
       mbar_wait(smem_u32(&bars.s_full[b]), (i >> 1) & 1, abortp, p.status, kStatusPrefillWait);
       __syncwarp();
       tc_fence_after();
       const uint32_t s_addr = tmem + lane_sel + b * kKeys;
       // (nothing stands between a load from TMEM and its wait: the registers must not be touched, copied or spilled before)
-      uint32_t v[kKeys];
-      tmem_ld_x32(s_addr, v);
-      tmem_ld_x32(s_addr + 32, v + 32);
-      tmem_ld_wait_x32(v, v + 32);
+      uint32_t v[kHalfKeys];
+#pragma unroll
+      for (int j = 0; j < kHalfKeys; j += 4) tmem_ld_x4(s_addr + 2 * j + half * 4, v + j);
+      tmem_ld_wait_x32(v);
       // scores: scaled, keys out of sight at -inf
       if constexpr (kScaled) {
 #pragma unroll
-        for (int j = 0; j < kKeys; j += 4) {
-          const float4 k4 = *reinterpret_cast<const float4*>(ks + j);
-          v[j] = __float_as_uint(__uint_as_float(v[j]) * k4.x);
-          v[j + 1] = __float_as_uint(__uint_as_float(v[j + 1]) * k4.y);
-          v[j + 2] = __float_as_uint(__uint_as_float(v[j + 2]) * k4.z);
-          v[j + 3] = __float_as_uint(__uint_as_float(v[j + 3]) * k4.w);
+        for (int j = 0; j < kHalfKeys; j += 4) {
+          const float4 k4 = *reinterpret_cast<const float4*>(ks + 2 * j);
+          mul2(v[j], v[j + 1], k4.x, k4.y);
+          mul2(v[j + 2], v[j + 3], k4.z, k4.w);
         }
       }
-      if (!__all_sync(0xffffffffu, kb + kKeys <= lim && kb >= lo)) {
+      if (!__all_sync(0xffffffffu, kb - half * 4 + kKeys <= lim && kb - half * 4 >= lo)) {
 #pragma unroll
-        for (int j = 0; j < kKeys; ++j)
-          if (kb + j >= lim || kb + j < lo) v[j] = __float_as_uint(-CUDART_INF_F);
+        for (int j = 0; j < kHalfKeys; ++j) {
+          const int key = kb + j / 4 * 8 + j % 4;
+          if (key >= lim || key < lo) v[j] = __float_as_uint(-CUDART_INF_F);
+        }
       }
       float m4[4];
 #pragma unroll
       for (int j = 0; j < 4; ++j) m4[j] = __uint_as_float(v[j]);
 #pragma unroll
-      for (int j = 4; j < kKeys; ++j) m4[j & 3] = fmaxf(m4[j & 3], __uint_as_float(v[j]));
-      const float mx = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3]));
+      for (int j = 4; j < kHalfKeys; ++j) m4[j & 3] = fmaxf(m4[j & 3], __uint_as_float(v[j]));
+      const float own = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3]));
+      half_s[b][half][row] = own;
+      row_bar();   // (also: both halves have their scores, so that P may go over them)
+      const float mx = fmaxf(own, half_s[b][half ^ 1][row]);
       const bool move = mx > top;
       const float corr = move ? ex2(top - mx) : 1.f;   // (a row's first keys: exp2(-inf) = 0)
       if (__any_sync(0xffffffffu, move)) {
@@ -462,37 +547,39 @@ __global__ void __launch_bounds__(kThreads, 1) paged_attn_prefill_kernel(const P
           __syncwarp();
           tc_fence_after();
 #pragma unroll 1
-          for (int c = 0; c < D; c += 32) {
+          for (int c = half * (D / 2); c < half * (D / 2) + D / 2; c += 32) {
             uint32_t o[32];
             tmem_ld_x32(tmem + lane_sel + kColO + c, o);
             tmem_ld_wait_x32(o);
 #pragma unroll
-            for (int j = 0; j < 32; ++j) o[j] = __float_as_uint(__uint_as_float(o[j]) * corr);
+            for (int j = 0; j < 32; j += 2) mul2(o[j], o[j + 1], corr, corr);
             tmem_st_x16(tmem + lane_sel + kColO + c, o);
             tmem_st_x16(tmem + lane_sel + kColO + c + 16, o + 16);
           }
         }
       }
       const float at = top == -CUDART_INF_F ? 0.f : top;   // (a row that has seen no key yet)
-      uint32_t pk[kKeys / 4];
 #pragma unroll
-      for (int j = 0; j < kKeys; j += 4) {
+      for (int j = 0; j < kHalfKeys; j += 4) {
         float e[4];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          e[q] = ex2(__uint_as_float(v[j + q]) - at);
-          float& part = l4[((j + q) >> 1) & 3];
-          part = j + q < 8 && (q & 1) == 0 ? fmaf(part, corr, e[q]) : part + e[q];   // (a part's first key of the tile)
+        for (int q = 0; q < 4; ++q) e[q] = __uint_as_float(v[j + q]);
+        add2(e[0], e[1], -at, -at);
+        add2(e[2], e[3], -at, -at);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) e[q] = ex2(e[q]);
+        if (j == 0) {   // (a part's first key of the tile)
+          l2[0] = fmaf(l2[0], corr, e[0]);
+          l2[1] = fmaf(l2[1], corr, e[2]);
+        } else {
+          add2(l2[0], l2[1], e[0], e[2]);
         }
+        add2(l2[0], l2[1], e[1], e[3]);
         if constexpr (kScaled) {
-          const float4 v4 = *reinterpret_cast<const float4*>(vs + j);
+          const float4 v4 = *reinterpret_cast<const float4*>(vs + 2 * j);
           e[0] *= v4.x; e[1] *= v4.y; e[2] *= v4.z; e[3] *= v4.w;
         }
-        pk[(j / 2) % (kKeys / 4)] = pack_half2(e[0], e[1]);
-        pk[(j / 2) % (kKeys / 4) + 1] = pack_half2(e[2], e[3]);
-        // over the scores, which this lane holds in registers
-        if (j == kKeys / 2 - 4) tmem_st_x16(s_addr, pk);
-        if (j == kKeys - 4) tmem_st_x16(s_addr + 16, pk);
+        tmem_st_x2(s_addr + j + half * 2, pack_half2(e[0], e[1]), pack_half2(e[2], e[3]));
       }
       tmem_st_wait();
       tc_fence_before();
@@ -500,14 +587,16 @@ __global__ void __launch_bounds__(kThreads, 1) paged_attn_prefill_kernel(const P
       if (lane == 0) mbar_arrive(smem_u32(&bars.p_full[b]));
     }
     // ---- normalised rows to the stage ----
+    half_s[n_tiles & 1][half][row] = l2[0] + l2[1];
     if (n_tiles > 0) {
       mbar_wait(smem_u32(&bars.o_done), 0, abortp, p.status, kStatusPrefillWait);
       tc_fence_after();
     }
-    const float l = (l4[0] + l4[1]) + (l4[2] + l4[3]);
+    row_bar();
+    const float l = half_s[n_tiles & 1][0][row] + half_s[n_tiles & 1][1][row];
     const float inv = l > 0.f ? 1.f / l : 0.f;
 #pragma unroll 1
-    for (int c = 0; c < D; c += 32) {
+    for (int c = half * (D / 2); c < half * (D / 2) + D / 2; c += 32) {
       uint32_t o[32];
       if (n_tiles > 0) {
         tmem_ld_x32(tmem + lane_sel + kColO + c, o);
@@ -526,12 +615,12 @@ __global__ void __launch_bounds__(kThreads, 1) paged_attn_prefill_kernel(const P
         dst[j] = make_uint4(w[0], w[1], w[2], w[3]);
       }
     }
-    asm volatile("bar.sync 4, 384;" ::: "memory");
+    asm volatile("bar.sync 4, 512;" ::: "memory");
   }
 
   tc_fence_before();
   __syncthreads();
-  if (warp == 12) tmem_dealloc(tmem, 512);
+  if (warp == kIssuer) tmem_dealloc(tmem, 512);
 }
 
 template <int FORMAT>

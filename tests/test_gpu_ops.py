@@ -496,6 +496,38 @@ def test_prefill_attention_tile_edges(ops, status, name, fmt, group, hq, hkv, n,
     status.check("prefill attention")
 
 
+@pytest.mark.parametrize("name,fmt,group", FORMATS)
+def test_prefill_attention_does_not_depend_on_pages(ops, status, name, fmt, group):
+    """The same rows in pages of a tile, of sizes that neither divide a tile nor are divided by one, and with the pages behind a
+    window released: the same bits, with the window and without."""
+    torch.manual_seed(9)
+    D, hq, hkv, n, T = 256, 6, 2, 333, 70
+    ld, k_off, v_off = (2 * hq + 2 * hkv) * D, hq * D, 2 * hq * D + hkv * D
+    proj = torch.randn(n, ld).to(torch.bfloat16).cuda()
+    pos, seq = torch.arange(n).int().cuda(), torch.zeros(n, dtype=torch.int32, device="cuda")
+    qt = int(ops.prefill_attn_block_tokens(hq, hkv))
+    starts = list(range(0, T, qt))
+    counts = torch.tensor([min(qt, T - o) for o in starts]).int().cuda()
+    outs = {}
+    for P in (64, 7, 48, 160):
+        pages = (n + P - 1) // P
+        table = torch.randperm(pages + 1)[:pages].int().view(1, pages).cuda()
+        planes = _planes(pages + 1, hkv, P, D, fmt, group)
+        q = torch.empty((n, hq, D), dtype=torch.bfloat16, device="cuda")
+        ops.attn_prep(proj, 0, k_off, v_off, hq, hkv, D, None, None, 1e-6, True, 0, R.rope_inv_freq(64, 1e7).cuda(), 1.0, pos,
+                      seq, pos, table, q, *planes, P, fmt, group, False)
+        for window, released in ((0, 0), (100, 0), (100, (n - T + 1 - 100) // P)):
+            used = table.clone()
+            used[:, :released] = -1
+            out = torch.full((T, hq * D), float("nan"), dtype=torch.bfloat16, device="cuda")
+            ops.paged_attention_prefill(q[n - T:].contiguous(), hq, hkv, D, seq[:T], (pos[n - T:] + 1).contiguous(),
+                                        torch.tensor(starts).int().cuda(), counts, used, *planes, P, fmt, group, 1 / 16, None, out,
+                                        False, window, None, status.tensor)
+            assert torch.equal(out, outs.setdefault(window, out)), (P, window, released)
+    assert not outs[0].isnan().any() and not torch.equal(outs[0], outs[100])
+    status.check("prefill attention")
+
+
 def test_prefill_attention_largest_key_weighs_one(ops, status):
     """The 64 keys of the first tile score 0, one key of the second 2.03125 (in powers of two): that key's probability against
     the row's largest score is one, exactly, so outputs are its value times an fp32 factor.  Against the first tile's frame it
