@@ -36,13 +36,33 @@ __device__ __forceinline__ uint32_t pack_half2(float a, float b) {
   const __half2 h = __floats2half2_rn(a, b);
   return *reinterpret_cast<const uint32_t*>(&h);
 }
+// Codes to fp16 pairs, all of a word in one statement: bytes taken from it one by one, as the conversion functions take them, are
+// shifted and masked before each conversion (a word of e2m1 codes and its four products 21 cycles of a scheduler, so 11).
+__device__ __forceinline__ void e2m1_pairs(uint32_t w, uint32_t* out) {
+  asm("{\n\t.reg .b8 a, b, c, d;\n\tmov.b32 {a, b, c, d}, %4;\n\t"
+      "cvt.rn.f16x2.e2m1x2 %0, a;\n\tcvt.rn.f16x2.e2m1x2 %1, b;\n\tcvt.rn.f16x2.e2m1x2 %2, c;\n\tcvt.rn.f16x2.e2m1x2 %3, d;\n\t}"
+      : "=r"(out[0]), "=r"(out[1]), "=r"(out[2]), "=r"(out[3]) : "r"(w));
+}
+__device__ __forceinline__ void e4m3_pairs(uint32_t w, uint32_t* out) {
+  asm("{\n\t.reg .b16 a, b;\n\tmov.b32 {a, b}, %2;\n\tcvt.rn.f16x2.e4m3x2 %0, a;\n\tcvt.rn.f16x2.e4m3x2 %1, b;\n\t}"
+      : "=r"(out[0]), "=r"(out[1]) : "r"(w));
+}
+// an e4m3 scale, twice
+__device__ __forceinline__ __half2 e4m3_twice(uint32_t code) {
+  const __half2_raw r = __nv_cvt_fp8x2_to_halfraw2(static_cast<__nv_fp8x2_storage_t>(code * 0x101u), __NV_E4M3);
+  return *reinterpret_cast<const __half2*>(&r);
+}
+__device__ __forceinline__ uint32_t mul_h2(uint32_t a, __half2 b) {
+  const __half2 r = __hmul2(*reinterpret_cast<const __half2*>(&a), b);
+  return *reinterpret_cast<const uint32_t*>(&r);
+}
 
 // One "unit" = 16 consecutive values [16*part, 16*part+16) of a cache row.  Loading (raw bytes into
 // registers) and converting (to 8 packed fp16 pairs) are separate so that a thread can put all of a
 // tile's loads in flight before it converts the first one.  For that the loads are unconditional and nothing is done with
 // their results before `convert`: a load under a condition, or a scale decoded where it is loaded, makes the thread wait
 // for each unit in turn (128-key tiles of the prefill kernel: 3500 ns per tile so, 1700 without the wait).  A row that does
-// not exist (r < 0) is read as row 0 and converted to zeros (`live`).  The fp8-row scale is NOT applied here (it
+// not exist (r < 0) is read as row 0 and `clear`ed before it is converted.  The fp8-row scale is NOT applied here (it
 // multiplies scores / probabilities instead).
 template <int FORMAT>
 struct RawUnit {
@@ -92,32 +112,31 @@ struct RawUnit {
       scale = scales[r * (D / 16) + part];
     }
   }
-  __device__ __forceinline__ void convert(uint32_t* out, bool live) const {
+  // the unit of a row that does not exist: codes and a scale whose values are zeros
+  __device__ __forceinline__ void clear() {
+    a = b = make_uint4(0, 0, 0, 0);
+    scale = 0;
+  }
+  __device__ __forceinline__ void convert(uint32_t* out) const {
     if constexpr (FORMAT == kKvMixed) {
       // one of the three tier codecs, chosen per unit
       if (tier == 0) {
         RawUnit<kKvBf16> u;
         u.a = a; u.b = b;
-        u.convert(out, live);
+        u.convert(out);
       } else if (tier == 1) {
         RawUnit<kKvFp8Row> u;
         u.a = a;
-        u.convert(out, live);
+        u.convert(out);
       } else {
         RawUnit<kKvNvfp4> u;
         u.a = a; u.scale = scale;
-        u.convert(out, live);
+        u.convert(out);
       }
-      return;
     } else if constexpr (FORMAT == kKvFp8Row) {
       const uint32_t w[4] = {a.x, a.y, a.z, a.w};
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const __half2_raw lo = __nv_cvt_fp8x2_to_halfraw2(static_cast<__nv_fp8x2_storage_t>(w[i] & 0xffff), __NV_E4M3);
-        const __half2_raw hi = __nv_cvt_fp8x2_to_halfraw2(static_cast<__nv_fp8x2_storage_t>(w[i] >> 16), __NV_E4M3);
-        out[2 * i] = *reinterpret_cast<const uint32_t*>(&lo);
-        out[2 * i + 1] = *reinterpret_cast<const uint32_t*>(&hi);
-      }
+      for (int i = 0; i < 4; ++i) e4m3_pairs(w[i], out + 2 * i);
     } else if constexpr (FORMAT == kKvBf16) {
       const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
 #pragma unroll
@@ -140,19 +159,11 @@ struct RawUnit {
     } else {
       // two e2m1 codes per byte -> fp16 pair in one conversion instruction, then the block scale (the product of an
       // e2m1 value and an e4m3 scale is exact in fp16, so this equals the fp32 route bit for bit)
-      const uint32_t w[2] = {a.x, a.y};
-      const __half2 s2 = __float2half2_rn(e4m3_to_float(static_cast<uint8_t>(scale)));
+      const __half2 s2 = e4m3_twice(scale);
+      e2m1_pairs(a.x, out);
+      e2m1_pairs(a.y, out + 4);
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const __nv_fp4x2_storage_t pair = static_cast<__nv_fp4x2_storage_t>((w[i / 4] >> (8 * (i % 4))) & 0xff);
-        const __half2_raw hr = __nv_cvt_fp4x2_to_halfraw2(pair, __NV_E2M1);
-        const __half2 h = __hmul2(*reinterpret_cast<const __half2*>(&hr), s2);
-        out[i] = *reinterpret_cast<const uint32_t*>(&h);
-      }
-    }
-    if (!live) {
-#pragma unroll
-      for (int i = 0; i < 8; ++i) out[i] = 0u;
+      for (int i = 0; i < 8; ++i) out[i] = mul_h2(out[i], s2);
     }
   }
 };

@@ -19,8 +19,10 @@
 //   are staged in the same order, and an output column is put back where it belongs when it is written;
 // * groups of at most 8 query heads (kRows = 8) read only the eight rows of Q and P that exist;
 // * S is summed from two accumulators: one chain of sixteen dependent MMAs took longer than their operands.
-// 8 sequences of 32,000 nvfp4 keys, 24 heads in 4 groups: 236 -> 189 us at the same split (295 MB: 44 us of traffic), of
-// 26,000 int8 keys 220 -> 171, of bf16 keys 288 -> 243; one sequence of 2048 keys 19.5 -> 17.4.
+// 8 sequences of 26,000 keys, 24 heads in 4 groups: int8 220 -> 171 us at the same split, bf16 288 -> 243; one sequence of 2048
+// nvfp4 keys 19.5 -> 17.4.  nvfp4 pages and groups of up to eight heads are paged_attention_fp4.cu's.  (Its scheme, with every
+// format through shared memory: int8 158 -> 155 us, bf16 203 -> 224, whose conversions are few and whose raw rows fill the
+// registers; these stay here.)
 // Splits cover absolute key ranges and tiles start at split boundaries, so the
 // reduction order for a query depends only on key positions.  Output partials
 // (m, l, un-normalised O) use the same layout as the SIMT kernel and are
@@ -174,11 +176,19 @@ __global__ void __launch_bounds__(kThreads, 2) paged_attn_mma_kernel(const Paged
   };
   // Dequantise to fp16, K and V both as [key][d] rows in the order of `place`: 16-byte stores, neighbouring lanes side by side.
   auto store_tile = [&]() {
+    if (live != (1u << kUnits) - 1) {
+#pragma unroll
+      for (int it = 0; it < kUnits; ++it) {
+        if (live >> it & 1u) continue;
+        rawk[it].clear();
+        rawv[it].clear();
+      }
+    }
 #pragma unroll
     for (int it = 0; it < kUnits; ++it) {
       const int u = it * kThreads + threadIdx.x;
       uint32_t h[8];
-      rawk[it].convert(h, (live >> it) & 1u);
+      rawk[it].convert(h);
       uint4* dst = reinterpret_cast<uint4*>(&sm.k[u >> 4][(u & 15) * 8]);
       dst[0] = make_uint4(h[0], h[1], h[2], h[3]);
       dst[D / 16] = make_uint4(h[4], h[5], h[6], h[7]);
@@ -187,7 +197,7 @@ __global__ void __launch_bounds__(kThreads, 2) paged_attn_mma_kernel(const Paged
     for (int it = 0; it < kUnits; ++it) {
       const int u = it * kThreads + threadIdx.x;
       uint32_t h[8];
-      rawv[it].convert(h, (live >> it) & 1u);
+      rawv[it].convert(h);
       uint4* dst = reinterpret_cast<uint4*>(&sm.v[u >> 4][(u & 15) * 8]);
       dst[0] = make_uint4(h[0], h[1], h[2], h[3]);
       dst[D / 16] = make_uint4(h[4], h[5], h[6], h[7]);
@@ -393,7 +403,10 @@ cudaError_t paged_attention_mma_split(const PagedAttnParams& p, cudaStream_t str
     case kKvBf16: return launch_fmt<kKvBf16>(p, stream, pdl);
     case kKvFp8Row: return launch_fmt<kKvFp8Row>(p, stream, pdl);
     case kKvInt8Group: return launch_fmt<kKvInt8Group>(p, stream, pdl);
-    case kKvNvfp4: return launch_fmt<kKvNvfp4>(p, stream, pdl);
+    case kKvNvfp4: {
+      const cudaError_t e = paged_attention_fp4_split(p, stream, pdl);
+      return e == cudaErrorNotSupported ? launch_fmt<kKvNvfp4>(p, stream, pdl) : e;
+    }
     case kKvMixed: return launch_fmt<kKvMixed>(p, stream, pdl);
     default: return cudaErrorNotSupported;
   }

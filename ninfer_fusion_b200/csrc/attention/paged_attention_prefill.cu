@@ -29,9 +29,9 @@
 // warp to choose from, and divisions by the page size, selects per row and stores with two-way conflicts to issue (issue slots
 // 54 %, the integer units 45 %, a fifth of the stalls for instructions not yet fetched).  Two threads per row, pages walked
 // without a division, row numbers of 32 bits, the check for keys without a row once per tile and conflict-free stores: 24 / 4
-// heads, 2048 queries, us, before -> now: 2048 keys, fp8 rows 161 -> 125, bf16 164 -> 130, nvfp4 152 -> 118, int8 174 -> 143;
-// 16384 keys, fp8 rows 1367 -> 1122 (689 TFLOP/s), bf16 1526 -> 1258, nvfp4 1337 -> 1067, int8 1696 -> 1453; 300 queries, 1500
-// keys 68 -> 55; 37 tokens, of which a launch is the most, 21.5 -> 15.7; bits are the same.  Left: 3.4 us per 128 keys, the
+// heads, 2048 queries, us, before -> now: 2048 keys, fp8 rows 161 -> 123, bf16 164 -> 131, nvfp4 152 -> 110, int8 174 -> 141;
+// 16384 keys, fp8 rows 1367 -> 1097 (705 TFLOP/s), bf16 1526 -> 1265, nvfp4 1337 -> 952, int8 1696 -> 1454; 300 queries, 1500
+// keys 68 -> 55; 37 tokens, of which a launch is the most, 21.5 -> 15.7; bits are the same.  Left: 3.3 us per 128 keys, the
 // chain of a tile still (a maximum that lags by up to four powers of two would spare a tenth of it, with other roundings).
 //
 // Reference kernels covered: kernel/gqa_attention_prefill_{bf16,i8,nvfp4}.cuh (Br = 64 x Bc = 64
@@ -309,9 +309,9 @@ __global__ void __launch_bounds__(kThreads, 1) paged_attn_prefill_kernel(const P
       if constexpr (FORMAT == kKvMixed) dst.load_row(p.kv, which, r, part);
       else dst.load(p.kv, codes, scales, max(r, 0), part);
     };
-    auto store_unit = [&](const RawUnit<FORMAT>& src, uint32_t exists, int b, int j) {
+    auto store_unit = [&](const RawUnit<FORMAT>& src, int b, int j) {
       uint32_t h[8];
-      src.convert(h, exists);
+      src.convert(h);
       *reinterpret_cast<uint4*>(lo0 + b * kTileBytes + j * 1024) = make_uint4(h[0], h[1], h[2], h[3]);
       *reinterpret_cast<uint4*>(hi0 + b * kTileBytes + j * 1024) = make_uint4(h[4], h[5], h[6], h[7]);
     };
@@ -346,19 +346,24 @@ __global__ void __launch_bounds__(kThreads, 1) paged_attn_prefill_kernel(const P
       if (i >= 2) mbar_wait(freed, ((i >> 1) - 1) & 1, abortp, p.status, kStatusPrefillWait);
       // With one set a unit's registers take the next tile as soon as it is converted (its rows were published long ago); with two
       // the loads wait for the last conversion, since one that waits for its data waits for the loads issued before it too
-      // (2048 queries, 16384 keys: int8, interleaved, 3052 us where 1453; bf16, not, 1550 where 1258).
+      // (2048 queries, 16384 keys: int8, interleaved, 3052 us where 1454; bf16, not, 1550 where 1265).
       uint32_t next_mask = 0;
+      if (mask != (1u << kUnits) - 1) {
+#pragma unroll
+        for (int j = 0; j < kUnits; ++j)
+          if (!(mask >> j & 1u)) set[j].clear();
+      }
       if constexpr (kSets == 1) {
         const bool more = i + 1 < n_tiles;
         if (more) next_mask = live_units(i + 1);
 #pragma unroll
         for (int j = 0; j < kUnits; ++j) {
-          store_unit(set[j], (mask >> j) & 1u, b, j);
+          store_unit(set[j], b, j);
           if (more) load_unit(i + 1, j, set[j]);
         }
       } else {
 #pragma unroll
-        for (int j = 0; j < kUnits; ++j) store_unit(set[j], (mask >> j) & 1u, b, j);
+        for (int j = 0; j < kUnits; ++j) store_unit(set[j], b, j);
       }
       fence_proxy_async_smem();
       __syncwarp();

@@ -496,6 +496,42 @@ def test_prefill_attention_tile_edges(ops, status, name, fmt, group, hq, hkv, n,
     status.check("prefill attention")
 
 
+@pytest.mark.parametrize("hq,hkv", [(1, 1), (6, 2), (24, 4), (8, 1)])
+@pytest.mark.parametrize("P,window,tree", [(64, 0, False), (7, 0, True), (48, 100, False), (160, 300, False)])
+def test_nvfp4_decode_attention_of_aligned_scales(ops, hq, hkv, P, window, tree):
+    """Row scales at a 16-byte boundary are read sixteen at once, by a kernel whose products and sums are those of the general
+    one, which takes scales at any address: the same bits, for any page size, released pages, windows, tree masks and lengths at
+    the edges of tiles and splits."""
+    torch.manual_seed(P)
+    D, lens, split, ns = 256, [1, 63, 64, 65, 129, 700, 128, 511], 128, 6
+    B, pages = len(lens), (max(lens) + P - 1) // P
+    table = torch.randperm(B * pages + 1)[: B * pages].int().view(B, pages).cuda()
+    k, v, ks, vs = _planes(B * pages + 1, hkv, P, D, R.KV_NVFP4, 16)
+    for codes, scales in ((k, ks), (v, vs)):
+        codes.copy_(torch.randint(0, 256, codes.shape, dtype=torch.uint8))
+        scales.copy_(torch.randint(0, 0x7f, scales.shape, dtype=torch.uint8))
+    if window:
+        for b, n in enumerate(lens):
+            table[b, : max(0, n - window) // P] = -1
+    elsewhere = torch.empty(ks.numel() + 16, dtype=torch.uint8, device="cuda")[8:8 + ks.numel()].view(ks.shape)
+    elsewhere.copy_(ks)
+    q = torch.randn(B, hq, D).to(torch.bfloat16).cuda()
+    kv_len, seq = torch.tensor(lens).int().cuda(), torch.arange(B).int().cuda()
+    seq[2] = -1
+    mask = torch.randint(0, 2 ** 62, (B,)).cuda() if tree else None
+    base = (kv_len - 60).clamp(min=0).int() if tree else None
+    got = []
+    for scales in (ks, elsewhere):
+        po, pm = torch.zeros(B * hq * ns * D, device="cuda"), torch.zeros(B * hq * ns * 2, device="cuda")
+        out = torch.full((B, hq * D), float("nan"), dtype=torch.bfloat16, device="cuda")
+        ops.paged_attention(q, hq, hkv, D, seq, kv_len, table, k, v, scales, vs, P, R.KV_NVFP4, 16, 1 / 16, split, ns, po, pm, None,
+                            out, mask, base, 2, False, window)
+        got.append((po, pm, out))
+    for a, b in zip(*got):
+        assert torch.equal(a.view(torch.uint8), b.view(torch.uint8))
+    assert got[0][1].isfinite().any() and not got[0][2].isnan().any()
+
+
 @pytest.mark.parametrize("name,fmt,group", FORMATS)
 def test_prefill_attention_does_not_depend_on_pages(ops, status, name, fmt, group):
     """The same rows in pages of a tile, of sizes that neither divide a tile nor are divided by one, and with the pages behind a
