@@ -100,9 +100,8 @@ __device__ __forceinline__ bool find_chunk(const int* cu, int n_seq, int ci, int
 
 // ------------------------------------------------------------------------------------------------ prepare
 struct PrepSmem {
-  __nv_bfloat16 k[kC][kLdR];    // raw k rows (zero past the chunk's end)
+  __nv_bfloat16 k[kC][kLdR];    // raw k rows (zero past the chunk's end); running sums; at last beta v
   __nv_bfloat16 q[kC][kLdR];    // raw q rows; once Q K^T is done, beta exp(G) k / |k|
-  __nv_bfloat16 v[kC][kLdR];    // raw v, scaled in place to beta v
   union {                       // A and the pieces of its inverse in fp32, then the inverse as a bf16 pair
     float a[kC][kLdA];
     struct {
@@ -114,10 +113,12 @@ struct PrepSmem {
 };
 
 // Latency bound (short products and a serial inverse behind barriers; two warps per scheduler issued in 0.36 of the cycles),
-// so what counts is how many chunks an SM works on at once, 72 KB of shared memory lets three CTAs in, and the length of the
-// chain: the substitution's long rows summed by all warps, the row norms four rows at a time.  Within a prompt's step of 2048
-// tokens: 48 heads 128 us with two CTAs and one thread per column, 105 so; 32 heads 82 and 66.
-__global__ void __launch_bounds__(128, 3) gdn_chunk_prepare_kernel(const ChunkParams cp) {
+// so what counts is how many chunks an SM works on at once and the length of the chain: the substitution's long rows summed by
+// all warps, the row norms four rows at a time.  v is wanted last and comes into registers beside the end of the substitution, so
+// that 54 KB of shared memory and 128 registers let four CTAs in.  Within a prompt's step of 2048 tokens: 48 heads 128 us with two
+// CTAs and one thread per column, 105 with three; by itself 89 with three and 80 with four, 32 heads 66 and 57 (2.7 and 1.8
+// rounds of the grid).
+__global__ void __launch_bounds__(128, 4) gdn_chunk_prepare_kernel(const ChunkParams cp) {
   extern __shared__ __align__(16) uint8_t smem_raw[];
   PrepSmem& sm = *reinterpret_cast<PrepSmem*>(smem_raw);
   const GdnParams& p = cp.g;
@@ -129,12 +130,11 @@ __global__ void __launch_bounds__(128, 3) gdn_chunk_prepare_kernel(const ChunkPa
   const long long item = static_cast<long long>(blockIdx.x) * p.n_v_heads + hv;
 
   // ---- raw rows by cp.async (zero-filled past the chunk), gates by the first 64 threads ----
-  for (int i = tid; i < 3 * kC * (kD / 8); i += blockDim.x) {
+  for (int i = tid; i < 2 * kC * (kD / 8); i += blockDim.x) {
     const int which = i / (kC * (kD / 8)), r = (i / (kD / 8)) % kC, c = i % (kD / 8);
     const bool ok = r < n_tok;
-    const int off = which == 0 ? p.k_off + hk * kD : (which == 1 ? p.q_off + hk * kD : p.v_off + hv * kD);
-    const __nv_bfloat16* src = p.qkv + static_cast<long long>(t0 + (ok ? r : 0)) * p.ld_qkv + off + c * 8;
-    __nv_bfloat16(*dst)[kLdR] = which == 0 ? sm.k : (which == 1 ? sm.q : sm.v);
+    const __nv_bfloat16* src = p.qkv + static_cast<long long>(t0 + (ok ? r : 0)) * p.ld_qkv + (which ? p.q_off : p.k_off) + hk * kD + c * 8;
+    __nv_bfloat16(*dst)[kLdR] = which ? sm.q : sm.k;
     cp_async_16(smem_u32(&dst[r][c * 8]), src, ok ? 16 : 0);
   }
   cp_async_commit();
@@ -251,7 +251,7 @@ __global__ void __launch_bounds__(128, 3) gdn_chunk_prepare_kernel(const ChunkPa
   // ---- X = (I + A)^-1 by forward substitution, each entry's terms in the order of its row (four running sums, by column mod
   //      4).  Columns 0..31: warp 0 takes rows 0..31; then all warps take the terms of rows 32..63 with those; then warp 0 the
   //      rest of rows 32..63.  Columns 32..63 start at row 32 and are warp 1's meanwhile.  Lane c owns a column; the other two
-  //      warps scale the right-hand sides ----
+  //      warps scale k, and beside the last part v comes into registers ----
   constexpr int kH = kC / 2;
   auto substitute = [&](int o, const float4* start, float* x) {   // rows o .. o + 31 and as many columns of A
 #pragma unroll
@@ -276,11 +276,9 @@ __global__ void __launch_bounds__(128, 3) gdn_chunk_prepare_kernel(const ChunkPa
   } else {
     for (int i = tid - kC; i < kC * (kD / 2); i += blockDim.x - kC) {
       const int r = i / (kD / 2), c2 = (i % (kD / 2)) * 2;
-      const float sk = sm.beta[r] * __expf(sm.G[r]) * sm.rk[r], sv = sm.beta[r];
+      const float sk = sm.beta[r] * __expf(sm.G[r]) * sm.rk[r];
       const __nv_bfloat162 kv = *reinterpret_cast<const __nv_bfloat162*>(&sm.k[r][c2]);
-      const __nv_bfloat162 vv = *reinterpret_cast<const __nv_bfloat162*>(&sm.v[r][c2]);
       *reinterpret_cast<uint32_t*>(&sm.q[r][c2]) = pack_bf16x2(__bfloat162float(kv.x) * sk, __bfloat162float(kv.y) * sk);
-      *reinterpret_cast<uint32_t*>(&sm.v[r][c2]) = pack_bf16x2(__bfloat162float(vv.x) * sv, __bfloat162float(vv.y) * sv);
     }
   }
   __syncthreads();
@@ -312,8 +310,35 @@ __global__ void __launch_bounds__(128, 3) gdn_chunk_prepare_kernel(const ChunkPa
   }
   __syncthreads();
   float x21[kH];
-  if (warp == 0) substitute(kH, sums, x21);
-  __syncthreads();   // (the bf16 pair lies over A)
+  constexpr int kVLoads = (kC * (kD / 8) + 95) / 96;   // 16-byte pieces of v per thread of warps 1..3
+  uint4 v[kVLoads];
+  if (warp == 0) {
+    substitute(kH, sums, x21);
+  } else {
+#pragma unroll
+    for (int j = 0; j < kVLoads; ++j) {
+      const int i = j * 96 + tid - 32, r = i / (kD / 8), c = i % (kD / 8);
+      v[j] = make_uint4(0, 0, 0, 0);
+      if (r < n_tok)
+        v[j] = *reinterpret_cast<const uint4*>(p.qkv + static_cast<long long>(t0 + r) * p.ld_qkv + p.v_off + hv * kD + c * 8);
+    }
+  }
+  __syncthreads();   // (the bf16 pair lies over A, v over the running sums)
+  if (warp != 0) {
+#pragma unroll
+    for (int j = 0; j < kVLoads; ++j) {
+      const int i = j * 96 + tid - 32, r = i / (kD / 8), c = i % (kD / 8);
+      if (r >= kC) break;
+      const float sv = sm.beta[r];
+      uint32_t* w = reinterpret_cast<uint32_t*>(&v[j]);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const __nv_bfloat162 vv = *reinterpret_cast<const __nv_bfloat162*>(&w[e]);
+        w[e] = pack_bf16x2(__bfloat162float(vv.x) * sv, __bfloat162float(vv.y) * sv);
+      }
+      *reinterpret_cast<uint4*>(&sm.k[r][c * 8]) = v[j];
+    }
+  }
   {
     auto put = [&](int i, int c, float v) {
       const __nv_bfloat16 hi = __float2bfloat16(v);
@@ -342,7 +367,7 @@ __global__ void __launch_bounds__(128, 3) gdn_chunk_prepare_kernel(const ChunkPa
     for (int n = 0; n < 16; ++n)
 #pragma unroll
       for (int j = 0; j < 4; ++j) acc[n][j] = 0.f;
-    __nv_bfloat16(*rhs)[kLdR] = pass == 0 ? sm.q : sm.v;
+    __nv_bfloat16(*rhs)[kLdR] = pass == 0 ? sm.q : sm.k;
 #pragma unroll
     for (int kk = 0; kk < 4; ++kk) {
       if (kk <= warp) {
