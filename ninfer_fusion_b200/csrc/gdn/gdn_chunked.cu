@@ -172,18 +172,21 @@ __global__ void __launch_bounds__(128, 4) gdn_chunk_prepare_kernel(const ChunkPa
         sq[m] = fmaf(qf.y, qf.y, fmaf(qf.x, qf.x, sq[m]));
       }
     }
+    // The sums of a warp's eight values, pairs of lanes 16, 8, 4, 2 and 1 apart as warp_sum adds them: after each of the first three
+    // steps a lane goes on with the half of the values that its bit names.
+    float s[8] = {sk[0], sk[1], sk[2], sk[3], sq[0], sq[1], sq[2], sq[3]};
 #pragma unroll
-    for (int m = 0; m < 4; ++m) {
-      sk[m] = warp_sum(sk[m]);
-      sq[m] = warp_sum(sq[m]);
-    }
-    if (lane == 0) {
+    for (int n = 4, o = 16; n > 0; n /= 2, o /= 2) {
+      const bool upper = lane & o;
 #pragma unroll
-      for (int m = 0; m < 4; ++m) {
-        sm.rk[r0 + m] = rsqrtf(sk[m] + 1e-6f);
-        sm.rq[r0 + m] = rsqrtf(sq[m] + 1e-6f);
+      for (int m = 0; m < n; ++m) {
+        const float other = __shfl_xor_sync(0xffffffffu, upper ? s[m] : s[m + n], o);
+        s[m] = (upper ? s[m + n] : s[m]) + other;
       }
     }
+    s[0] += __shfl_xor_sync(0xffffffffu, s[0], 2);
+    s[0] += __shfl_xor_sync(0xffffffffu, s[0], 1);
+    if ((lane & 3) == 0) (lane & 16 ? sm.rq : sm.rk)[r0 + (lane >> 2 & 3)] = rsqrtf(s[0] + 1e-6f);
   }
   if (warp == 0) {
     float a = sm.g[lane], b = sm.g[lane + 32];
@@ -228,7 +231,12 @@ __global__ void __launch_bounds__(128, 4) gdn_chunk_prepare_kernel(const ChunkPa
     const float qscale = rsqrtf(static_cast<float>(kD));
     __nv_bfloat16* Pg = cp.ws.P + item * (kC * kC);
 #pragma unroll
-    for (int n = 0; n < 8; ++n)
+    for (int n = 0; n < 8; ++n) {
+      if (n / 2 > warp) {   // (of A nothing above the diagonal tile is read)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) *reinterpret_cast<uint32_t*>(Pg + (warp * 16 + row0 + 8 * h) * kC + n * 8 + 2 * cq) = 0u;
+        continue;
+      }
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         const int i = warp * 16 + row0 + 8 * h;
@@ -245,6 +253,7 @@ __global__ void __launch_bounds__(128, 4) gdn_chunk_prepare_kernel(const ChunkPa
         *reinterpret_cast<float2*>(&sm.a[i][j]) = make_float2(av[0], av[1]);
         *reinterpret_cast<uint32_t*>(Pg + i * kC + j) = pack_bf16x2(pv[0], pv[1]);
       }
+    }
   }
   __syncthreads();
 
@@ -274,11 +283,18 @@ __global__ void __launch_bounds__(128, 4) gdn_chunk_prepare_kernel(const ChunkPa
       for (int i = 0; i < kH; ++i) sm.a[i][kH + lane] = x[i];
     }
   } else {
-    for (int i = tid - kC; i < kC * (kD / 2); i += blockDim.x - kC) {
-      const int r = i / (kD / 2), c2 = (i % (kD / 2)) * 2;
+#pragma unroll 4
+    for (int i = tid - kC; i < kC * (kD / 8); i += 128 - kC) {
+      const int r = i / (kD / 8), c = i % (kD / 8) * 8;
       const float sk = sm.beta[r] * __expf(sm.G[r]) * sm.rk[r];
-      const __nv_bfloat162 kv = *reinterpret_cast<const __nv_bfloat162*>(&sm.k[r][c2]);
-      *reinterpret_cast<uint32_t*>(&sm.q[r][c2]) = pack_bf16x2(__bfloat162float(kv.x) * sk, __bfloat162float(kv.y) * sk);
+      uint4 k = *reinterpret_cast<const uint4*>(&sm.k[r][c]);
+      uint32_t* w = reinterpret_cast<uint32_t*>(&k);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const __nv_bfloat162 kv = *reinterpret_cast<const __nv_bfloat162*>(&w[e]);
+        w[e] = pack_bf16x2(__bfloat162float(kv.x) * sk, __bfloat162float(kv.y) * sk);
+      }
+      *reinterpret_cast<uint4*>(&sm.q[r][c]) = k;
     }
   }
   __syncthreads();
@@ -359,44 +375,48 @@ __global__ void __launch_bounds__(128, 4) gdn_chunk_prepare_kernel(const ChunkPa
   }
   __syncthreads();
 
-  // ---- W = X (beta exp(G) k^), U = X (beta v); X is lower triangular, so k-steps past the diagonal are skipped ----
+  // ---- W = X (beta exp(G) k^), U = X (beta v); X is lower triangular, so k-steps past the diagonal are skipped.  A warp has 32
+  //      columns of all rows: with sixteen rows each the last warp had four times the first one's products ----
 #pragma unroll 1
   for (int pass = 0; pass < 2; ++pass) {
-    float acc[16][4];
+    float acc[4][4][4];   // [row tile][8 columns]
 #pragma unroll
-    for (int n = 0; n < 16; ++n)
+    for (int m = 0; m < 4; ++m)
 #pragma unroll
-      for (int j = 0; j < 4; ++j) acc[n][j] = 0.f;
+      for (int n = 0; n < 4; ++n)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[m][n][j] = 0.f;
     __nv_bfloat16(*rhs)[kLdR] = pass == 0 ? sm.q : sm.k;
+    const int xr = (lane & 7) + 8 * ((lane >> 3) & 1), xc = 8 * (lane >> 4);
 #pragma unroll
     for (int kk = 0; kk < 4; ++kk) {
-      if (kk <= warp) {
-        uint32_t h[4], l[4];
-        const int xr = warp * 16 + (lane & 7) + 8 * ((lane >> 3) & 1), xc = kk * 16 + 8 * (lane >> 4);
-        ldsm_x4(smem_u32(&sm.xh[xr][xc]), h[0], h[1], h[2], h[3]);
-        ldsm_x4(smem_u32(&sm.xl[xr][xc]), l[0], l[1], l[2], l[3]);
-        const int br = kk * 16 + (lane & 7) + 8 * ((lane >> 3) & 1);
+      uint32_t b[2][4];
 #pragma unroll
-        for (int np = 0; np < 8; ++np) {
-          uint32_t b0, b1, b2, b3;
-          ldsm_x4_trans(smem_u32(&rhs[br][np * 16 + 8 * (lane >> 4)]), b0, b1, b2, b3);
-          mma_bf16(acc[2 * np], h[0], h[1], h[2], h[3], b0, b1);
-          mma_bf16(acc[2 * np + 1], h[0], h[1], h[2], h[3], b2, b3);
-          mma_bf16(acc[2 * np], l[0], l[1], l[2], l[3], b0, b1);
-          mma_bf16(acc[2 * np + 1], l[0], l[1], l[2], l[3], b2, b3);
-        }
+      for (int np = 0; np < 2; ++np)
+        ldsm_x4_trans(smem_u32(&rhs[kk * 16 + xr][warp * 32 + np * 16 + xc]), b[np][0], b[np][1], b[np][2], b[np][3]);
+#pragma unroll
+      for (int m = kk; m < 4; ++m) {
+        uint32_t h[4], l[4];
+        ldsm_x4(smem_u32(&sm.xh[m * 16 + xr][kk * 16 + xc]), h[0], h[1], h[2], h[3]);
+        ldsm_x4(smem_u32(&sm.xl[m * 16 + xr][kk * 16 + xc]), l[0], l[1], l[2], l[3]);
+#pragma unroll
+        for (int n = 0; n < 4; ++n) mma_bf16(acc[m][n], h[0], h[1], h[2], h[3], b[n / 2][n % 2 * 2], b[n / 2][n % 2 * 2 + 1]);
+#pragma unroll
+        for (int n = 0; n < 4; ++n) mma_bf16(acc[m][n], l[0], l[1], l[2], l[3], b[n / 2][n % 2 * 2], b[n / 2][n % 2 * 2 + 1]);
       }
     }
 #pragma unroll
-    for (int n = 0; n < 16; ++n)
+    for (int m = 0; m < 4; ++m)
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int i = warp * 16 + row0 + 8 * h, j = n * 8 + 2 * cq;
-        if (pass == 0)
-          *reinterpret_cast<uint32_t*>(cp.ws.W + item * (kC * kD) + i * kD + j) = pack_bf16x2(acc[n][2 * h], acc[n][2 * h + 1]);
-        else
-          *reinterpret_cast<float2*>(cp.ws.U + item * (kC * kD) + i * kD + j) = make_float2(acc[n][2 * h], acc[n][2 * h + 1]);
-      }
+      for (int n = 0; n < 4; ++n)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int i = m * 16 + row0 + 8 * h, j = warp * 32 + n * 8 + 2 * cq;
+          if (pass == 0)
+            *reinterpret_cast<uint32_t*>(cp.ws.W + item * (kC * kD) + i * kD + j) = pack_bf16x2(acc[m][n][2 * h], acc[m][n][2 * h + 1]);
+          else
+            *reinterpret_cast<float2*>(cp.ws.U + item * (kC * kD) + i * kD + j) = make_float2(acc[m][n][2 * h], acc[m][n][2 * h + 1]);
+        }
   }
 
   // ---- row scales for the scan ----
