@@ -435,8 +435,8 @@ __global__ void __launch_bounds__(128, 4) gdn_chunk_prepare_kernel(const ChunkPa
 // compute the output rows Q S^T + P u~ beside them.  Two block barriers a chunk: operands and state are there, u~ is there.
 // Within a prompt's step of 2048 tokens: 48 heads 112 us with eight warps that did both in turn, 106 so; 32 heads 102, with
 // quarters of dv as well 62.
-constexpr int kScanGroup = 256;
-constexpr int kScanThreads = 2 * kScanGroup;
+constexpr int kScanGroup = 128;                  // threads of the chain, of the output and of the loads
+constexpr int kScanThreads = 3 * kScanGroup;
 
 // DV: dv columns per CTA, 64 or 32
 template <int DV>
@@ -467,8 +467,8 @@ __global__ void __launch_bounds__(kScanThreads, 1) gdn_chunk_scan_kernel(const C
   const int hk = hv / (p.n_v_heads / p.n_qk_heads);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int row0 = lane >> 2, cq = lane & 3;
-  const bool chain = warp < 8;               // (the warps' other half: loads and output)
-  const int mt = warp & 3, nh = (warp >> 2) & 1;   // products with 64 x DV outputs: row tile, half of the columns
+  const bool chain = warp < 4, loads = warp >= 8;
+  const int mt = warp & 1, nh = (warp >> 1) & 1;   // products with 64 x DV outputs: half of the rows, half of the columns
 
   const int seq_b = p.cu_seqlens[seq], seq_e = p.cu_seqlens[seq + 1];
   if (seq_e <= seq_b) return;
@@ -476,7 +476,7 @@ __global__ void __launch_bounds__(kScanThreads, 1) gdn_chunk_scan_kernel(const C
   int chunk0 = 0;
   for (int s = 0; s < seq; ++s) chunk0 += (max(p.cu_seqlens[s + 1] - p.cu_seqlens[s], 0) + kC - 1) / kC;
 
-  const int ltid = tid - kScanGroup;         // of the loading warps
+  const int ltid = tid - 2 * kScanGroup;     // of the loading warps
   auto load_stage = [&](int c, int stg) {
     ScanStage<DV>& st = sm.st[stg];
     const int t0 = seq_b + c * kC;
@@ -502,22 +502,22 @@ __global__ void __launch_bounds__(kScanThreads, 1) gdn_chunk_scan_kernel(const C
     if (ltid < 3 * kC / 4) cp_async_16(smem_u32(&st.vec[0][ltid * 4]), Vg + ltid * 4, 16);
   };
 
-  if (!chain) {
+  if (loads) {
     load_stage(0, 0);
     cp_async_commit();
   }
 
-  // state slice S[dv DV*slice ..][dk] in accumulator layout: warp w owns dk columns 16w..16w+15
+  // state slice S[dv DV*slice ..][dk] in accumulator layout: warp w owns dk columns 32w..32w+31
   float* sbase = p.state + ((static_cast<long long>(p.state_slot[seq]) * p.n_v_heads + hv) * kD + slice * DV) * kD;
-  float S[kMt][2][4];
+  float S[kMt][4][4];
   if (chain) {
 #pragma unroll
     for (int mi = 0; mi < kMt; ++mi)
 #pragma unroll
-      for (int n = 0; n < 2; ++n)
+      for (int n = 0; n < 4; ++n)
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-          const int dv = mi * 16 + row0 + 8 * h, dk = warp * 16 + n * 8 + 2 * cq;
+          const int dv = mi * 16 + row0 + 8 * h, dk = warp * 32 + n * 8 + 2 * cq;
           const float2 v = *reinterpret_cast<const float2*>(sbase + dv * kD + dk);
           S[mi][n][2 * h] = v.x;
           S[mi][n][2 * h + 1] = v.y;
@@ -528,120 +528,143 @@ __global__ void __launch_bounds__(kScanThreads, 1) gdn_chunk_scan_kernel(const C
   for (int c = 0; c < n_chunks; ++c) {
     const int stg = c & 1;
     ScanStage<DV>& st = sm.st[stg];
-    if (!chain) cp_async_wait<0>();
+    if (loads) cp_async_wait<0>();
     __syncthreads();   // this chunk's operands and the bf16 state are visible; everyone is done with the other stage and vn / vnd
-    if (!chain && c + 1 < n_chunks) {
-      load_stage(c + 1, stg ^ 1);
-      cp_async_commit();
+    if (loads) {
+      if (c + 1 < n_chunks) {
+        load_stage(c + 1, stg ^ 1);
+        cp_async_commit();
+      }
+      __syncthreads();
+      continue;
     }
 
-    // ---- M1 = W S^T (chain) or O1 = Q S^T: rows 16 mt.., dv columns DV / 2 nh.. ----
-    float acc[kMt][4];
+    // ---- M1 = W S^T (chain) or O1 = Q S^T: rows 32 mt.., dv columns DV / 2 nh.. ----
+    float acc[2][kMt][4];
 #pragma unroll
-    for (int n = 0; n < kMt; ++n)
+    for (int m = 0; m < 2; ++m)
 #pragma unroll
-      for (int j = 0; j < 4; ++j) acc[n][j] = 0.f;
+      for (int n = 0; n < kMt; ++n)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[m][n][j] = 0.f;
     {
       const __nv_bfloat16(*left)[kLdR] = chain ? st.w : st.q;
-      const uint32_t al = smem_u32(&left[mt * 16 + (lane & 7) + 8 * ((lane >> 3) & 1)][8 * (lane >> 4)]);
+      const uint32_t al = smem_u32(&left[mt * 32 + (lane & 7) + 8 * ((lane >> 3) & 1)][8 * (lane >> 4)]);
       const uint32_t bs = smem_u32(&sm.sb[nh * (DV / 2) + (lane & 7) + 8 * (lane >> 4)][8 * ((lane >> 3) & 1)]);
 #pragma unroll
       for (int ks = 0; ks < kD / 16; ++ks) {
-        uint32_t a[4];
-        ldsm_x4(al + ks * 32, a[0], a[1], a[2], a[3]);
+        uint32_t a[2][4];
+#pragma unroll
+        for (int m = 0; m < 2; ++m) ldsm_x4(al + m * 16 * kLdR * 2 + ks * 32, a[m][0], a[m][1], a[m][2], a[m][3]);
 #pragma unroll
         for (int np = 0; np < kMt / 2; ++np) {
           uint32_t c0, c1, c2, c3;
           ldsm_x4(bs + np * 16 * kLdR * 2 + ks * 32, c0, c1, c2, c3);
-          mma_bf16(acc[2 * np], a[0], a[1], a[2], a[3], c0, c1);
-          mma_bf16(acc[2 * np + 1], a[0], a[1], a[2], a[3], c2, c3);
+#pragma unroll
+          for (int m = 0; m < 2; ++m) {
+            mma_bf16(acc[m][2 * np], a[m][0], a[m][1], a[m][2], a[m][3], c0, c1);
+            mma_bf16(acc[m][2 * np + 1], a[m][0], a[m][1], a[m][2], a[m][3], c2, c3);
+          }
         }
       }
     }
     if (chain) {
       // ---- u~ = U - M1 (fp32), published as bf16 twice: plain and row-scaled for the state update ----
 #pragma unroll
-      for (int n = 0; n < kMt; ++n)
+      for (int m = 0; m < 2; ++m)
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const int r = mt * 16 + row0 + 8 * h, col = nh * (DV / 2) + n * 8 + 2 * cq;
-          const float2 u = *reinterpret_cast<const float2*>(&st.u[r][col]);
-          const float v0 = u.x - acc[n][2 * h], v1 = u.y - acc[n][2 * h + 1];
-          const float dk = st.vec[1][r];
-          *reinterpret_cast<uint32_t*>(&sm.vn[r][col]) = pack_bf16x2(v0, v1);
-          *reinterpret_cast<uint32_t*>(&sm.vnd[r][col]) = pack_bf16x2(v0 * dk, v1 * dk);
-        }
+        for (int n = 0; n < kMt; ++n)
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const int r = mt * 32 + m * 16 + row0 + 8 * h, col = nh * (DV / 2) + n * 8 + 2 * cq;
+            const float2 u = *reinterpret_cast<const float2*>(&st.u[r][col]);
+            const float v0 = u.x - acc[m][n][2 * h], v1 = u.y - acc[m][n][2 * h + 1];
+            const float dk = st.vec[1][r];
+            *reinterpret_cast<uint32_t*>(&sm.vn[r][col]) = pack_bf16x2(v0, v1);
+            *reinterpret_cast<uint32_t*>(&sm.vnd[r][col]) = pack_bf16x2(v0 * dk, v1 * dk);
+          }
     } else {
 #pragma unroll
-      for (int n = 0; n < kMt; ++n)
+      for (int m = 0; m < 2; ++m)
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const float dq = st.vec[0][mt * 16 + row0 + 8 * h];
-          acc[n][2 * h] *= dq;
-          acc[n][2 * h + 1] *= dq;
-        }
+        for (int n = 0; n < kMt; ++n)
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const float dq = st.vec[0][mt * 32 + m * 16 + row0 + 8 * h];
+            acc[m][n][2 * h] *= dq;
+            acc[m][n][2 * h + 1] *= dq;
+          }
     }
     __syncthreads();   // u~ is visible; everyone is done with the bf16 state
 
     if (chain) {
-      // ---- S = exp(G_C) S + (scaled u~)^T K: all DV rows, dk columns 16 warp.. ----
+      // ---- S = exp(G_C) S + (scaled u~)^T K: all DV rows, dk columns 32 warp.. ----
       const float gamma = st.vec[2][0];
 #pragma unroll
       for (int mi = 0; mi < kMt; ++mi)
 #pragma unroll
-        for (int n = 0; n < 2; ++n)
+        for (int n = 0; n < 4; ++n)
 #pragma unroll
           for (int j = 0; j < 4; ++j) S[mi][n][j] *= gamma;
 #pragma unroll
       for (int kk = 0; kk < kC / 16; ++kk) {
-        uint32_t b0, b1, b2, b3;
-        ldsm_x4_trans(smem_u32(&st.k[kk * 16 + (lane & 7) + 8 * ((lane >> 3) & 1)][warp * 16 + 8 * (lane >> 4)]), b0, b1, b2, b3);
+        uint32_t b[2][4];
+#pragma unroll
+        for (int np = 0; np < 2; ++np)
+          ldsm_x4_trans(smem_u32(&st.k[kk * 16 + (lane & 7) + 8 * ((lane >> 3) & 1)][warp * 32 + np * 16 + 8 * (lane >> 4)]),
+                        b[np][0], b[np][1], b[np][2], b[np][3]);
 #pragma unroll
         for (int mi = 0; mi < kMt; ++mi) {
           uint32_t a[4];
           ldsm_x4_trans(smem_u32(&sm.vnd[kk * 16 + (lane & 7) + 8 * (lane >> 4)][mi * 16 + 8 * ((lane >> 3) & 1)]),
                         a[0], a[1], a[2], a[3]);
-          mma_bf16(S[mi][0], a[0], a[1], a[2], a[3], b0, b1);
-          mma_bf16(S[mi][1], a[0], a[1], a[2], a[3], b2, b3);
+#pragma unroll
+          for (int n = 0; n < 4; ++n) mma_bf16(S[mi][n], a[0], a[1], a[2], a[3], b[n / 2][n % 2 * 2], b[n / 2][n % 2 * 2 + 1]);
         }
       }
 #pragma unroll
       for (int mi = 0; mi < kMt; ++mi)
 #pragma unroll
-        for (int n = 0; n < 2; ++n)
+        for (int n = 0; n < 4; ++n)
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
-            const int dv = mi * 16 + row0 + 8 * h, dk = warp * 16 + n * 8 + 2 * cq;
+            const int dv = mi * 16 + row0 + 8 * h, dk = warp * 32 + n * 8 + 2 * cq;
             *reinterpret_cast<uint32_t*>(&sm.sb[dv][dk]) = pack_bf16x2(S[mi][n][2 * h], S[mi][n][2 * h + 1]);
           }
     } else {
       // ---- O = O1 + P u~ ----
-      const uint32_t ap = smem_u32(&st.p[mt * 16 + (lane & 7) + 8 * ((lane >> 3) & 1)][8 * (lane >> 4)]);
+      const uint32_t ap = smem_u32(&st.p[mt * 32 + (lane & 7) + 8 * ((lane >> 3) & 1)][8 * (lane >> 4)]);
 #pragma unroll
       for (int kk = 0; kk < kC / 16; ++kk) {
-        uint32_t a[4];
-        ldsm_x4(ap + kk * 32, a[0], a[1], a[2], a[3]);
+        uint32_t a[2][4];
+#pragma unroll
+        for (int m = 0; m < 2; ++m) ldsm_x4(ap + m * 16 * kLdP * 2 + kk * 32, a[m][0], a[m][1], a[m][2], a[m][3]);
         const int br = kk * 16 + (lane & 7) + 8 * ((lane >> 3) & 1);
 #pragma unroll
         for (int np = 0; np < kMt / 2; ++np) {
           uint32_t c0, c1, c2, c3;
           ldsm_x4_trans(smem_u32(&sm.vn[br][nh * (DV / 2) + np * 16 + 8 * (lane >> 4)]), c0, c1, c2, c3);
-          mma_bf16(acc[2 * np], a[0], a[1], a[2], a[3], c0, c1);
-          mma_bf16(acc[2 * np + 1], a[0], a[1], a[2], a[3], c2, c3);
+#pragma unroll
+          for (int m = 0; m < 2; ++m) {
+            mma_bf16(acc[m][2 * np], a[m][0], a[m][1], a[m][2], a[m][3], c0, c1);
+            mma_bf16(acc[m][2 * np + 1], a[m][0], a[m][1], a[m][2], a[m][3], c2, c3);
+          }
         }
       }
       const int t0 = seq_b + c * kC;
       const int n_tok = min(kC, seq_e - t0);
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int r = mt * 16 + row0 + 8 * h;
-        if (r < n_tok) {
-          __nv_bfloat16* dst = p.out + static_cast<long long>(t0 + r) * (p.n_v_heads * kD) + hv * kD + slice * DV + nh * (DV / 2) + 2 * cq;
+      for (int m = 0; m < 2; ++m)
 #pragma unroll
-          for (int n = 0; n < kMt; ++n)
-            *reinterpret_cast<uint32_t*>(dst + n * 8) = pack_bf16x2(acc[n][2 * h], acc[n][2 * h + 1]);
+        for (int h = 0; h < 2; ++h) {
+          const int r = mt * 32 + m * 16 + row0 + 8 * h;
+          if (r < n_tok) {
+            __nv_bfloat16* dst = p.out + static_cast<long long>(t0 + r) * (p.n_v_heads * kD) + hv * kD + slice * DV + nh * (DV / 2) + 2 * cq;
+#pragma unroll
+            for (int n = 0; n < kMt; ++n)
+              *reinterpret_cast<uint32_t*>(dst + n * 8) = pack_bf16x2(acc[m][n][2 * h], acc[m][n][2 * h + 1]);
+          }
         }
-      }
     }
   }
 
@@ -649,10 +672,10 @@ __global__ void __launch_bounds__(kScanThreads, 1) gdn_chunk_scan_kernel(const C
 #pragma unroll
     for (int mi = 0; mi < kMt; ++mi)
 #pragma unroll
-      for (int n = 0; n < 2; ++n)
+      for (int n = 0; n < 4; ++n)
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-          const int dv = mi * 16 + row0 + 8 * h, dk = warp * 16 + n * 8 + 2 * cq;
+          const int dv = mi * 16 + row0 + 8 * h, dk = warp * 32 + n * 8 + 2 * cq;
           *reinterpret_cast<float2*>(sbase + dv * kD + dk) = make_float2(S[mi][n][2 * h], S[mi][n][2 * h + 1]);
         }
   }
