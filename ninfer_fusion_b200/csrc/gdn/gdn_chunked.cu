@@ -16,7 +16,7 @@
 //                      the triangular inverse by forward substitution in two halves, W / U / P and the row scales into a
 //                      workspace;
 //   gdn_chunk_scan     one CTA per (sequence, value head, half or quarter of dv), sequential over the chunks: the state slice
-//                      lives in MMA accumulator registers (fp32) of eight warps, eight more load and write the output;
+//                      lives in MMA accumulator registers (fp32) of four warps, eight more load and write the output;
 //                      the four products per chunk run on mma.sync out of a two-deep cp.async ring;
 //   gdn_gated_norm     per (token, head) gated RMSNorm of the raw outputs in place.
 //
@@ -116,8 +116,9 @@ struct PrepSmem {
 // so what counts is how many chunks an SM works on at once and the length of the chain: the substitution's long rows summed by
 // all warps, the row norms four rows at a time.  v is wanted last and comes into registers beside the end of the substitution, so
 // that 54 KB of shared memory and 128 registers let four CTAs in.  Within a prompt's step of 2048 tokens: 48 heads 128 us with two
-// CTAs and one thread per column, 105 with three; by itself 89 with three and 80 with four, 32 heads 66 and 57 (2.7 and 1.8
-// rounds of the grid).
+// CTAs and one thread per column, 105 with three; by itself 89 with three, 80 with four, 32 heads 66 and 57 (2.7 and 1.8 rounds
+// of the grid).  Then shared memory was busy 60 % of the time; with norms that are reduced together, k scaled eight values at a
+// time and even shares of the last products 73 and 51, one chunk 13 for 17.
 __global__ void __launch_bounds__(128, 4) gdn_chunk_prepare_kernel(const ChunkParams cp) {
   extern __shared__ __align__(16) uint8_t smem_raw[];
   PrepSmem& sm = *reinterpret_cast<PrepSmem*>(smem_raw);
@@ -431,10 +432,11 @@ __global__ void __launch_bounds__(128, 4) gdn_chunk_prepare_kernel(const ChunkPa
 
 // ------------------------------------------------------------------------------------------------ scan
 // The chunks of a sequence follow one another, so the time of one is the time of its longest chain: u~ = U - W S^T, then
-// S = exp(G_C) S + u~^T K.  Warps 0-7 do nothing else (S in their registers); warps 8-15 load the next chunk's operands and
-// compute the output rows Q S^T + P u~ beside them.  Two block barriers a chunk: operands and state are there, u~ is there.
-// Within a prompt's step of 2048 tokens: 48 heads 112 us with eight warps that did both in turn, 106 so; 32 heads 102, with
-// quarters of dv as well 62.
+// S = exp(G_C) S + u~^T K.  Warps 0-3 do nothing else (S in their registers); warps 4-7 compute the output rows Q S^T + P u~
+// beside them, warps 8-11 load the next chunk's operands.  Two block barriers a chunk: operands and state are there, u~ is there.
+// Within a prompt's step of 2048 tokens: 48 heads 112 us with eight warps that did both in turn, 106 with two groups of eight;
+// by itself 91 with those, whose tiles of sixteen rows read 2560 wavefronts of shared memory per chunk (of 5400 cycles), and 84 with
+// tiles of 32 rows (1660); 32 heads 63 and 58, in quarters of dv.  (Q S^T after u~, beside the state's update: 89.)
 constexpr int kScanGroup = 128;                  // threads of the chain, of the output and of the loads
 constexpr int kScanThreads = 3 * kScanGroup;
 
