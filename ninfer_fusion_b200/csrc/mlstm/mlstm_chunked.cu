@@ -2,7 +2,7 @@
 // m_0 the running maximum at the chunk's start and S_0, n_0 the state there, the recurrence unrolls to
 //   m_t   = F_t + max(m_0, max_{s <= t} (i_s - F_s))
 //   S_t^T q = exp(F_t + m_0 - m_t) S_0^T q  +  sum_{s <= t} exp(F_t - F_s + i_s - m_t) (k_s . q) v_s
-// and n_t . q is the same with v_s = 1; every exponent is <= 0.  Four kernels:
+// and n_t . q is the same with v_s = 1; every exponent is <= 0.  Four kernels, or three (contrib and scan in one, see below):
 //   gates    one CTA per (sequence, head): log gates, F, m per token, and m at every chunk boundary
 //   contrib  one CTA per (chunk, head, value slice): what a chunk adds to the state, U = sum_s w_s k_s v_s^T
 //   scan     elementwise over the chunks of a sequence: the state at every chunk's start, kept in fp32 and handed to
@@ -13,6 +13,7 @@
 
 #include <math_constants.h>
 
+#include "../common/device.h"
 #include "../common/elem.cuh"
 #include "../common/launch.h"
 #include "../common/mma_sync.cuh"
@@ -310,6 +311,210 @@ __global__ void __launch_bounds__(256) mlstm_scan_kernel(const MlstmArgs p, cons
   if (p.write_state) {
     s_state[0] = s0;
     s_state[V] = s1;
+  }
+}
+
+// The two kernels above in one, which walks the chunks of a sequence with a 64 x 64 block of a head's state in registers: what a
+// chunk adds never goes through memory (2048 tokens, 4 heads of 256 x 512: 67 MB written and read again).  Of such heads three
+// sequences of 1138, 683 and 227 tokens 65 -> 54 us, seven of 300 76 -> 51, one of 2048 69 -> 57, one of 100 14 -> 6; bound by the
+// chain of a chunk, a third of it issue (eight warps with twice the values each: 62 for 54).  The contributions'
+// products and sums and the order of the state's updates are theirs: the same bits.  Sixteen warps of 16 x 16, whose loads run two
+// chunks ahead; a seventeenth makes the weights and keeps n in the blocks of the first columns.
+// Columns of a weighted key row lie in the order even, odd within sixteen: a thread's two rows of a product are then neighbours and
+// a pair of a state word.
+constexpr int kBlock = 64;                       // state rows and columns per CTA
+constexpr int kLdB = kBlock + 8;
+constexpr int kWalkers = 16 * 32, kWalkThreads = kWalkers + 32;
+constexpr int kAheadChunks = 3;                  // chunks whose rows are in shared memory or on their way
+constexpr size_t kWalkSmem = sizeof(bf16) * (2 * kAheadChunks + 2) * L * kLdB;
+__global__ void __launch_bounds__(kWalkThreads) mlstm_walk_kernel(const MlstmArgs p, const ChunkWs w) {
+  extern __shared__ __align__(16) bf16 smem_b[];
+  __shared__ __align__(16) float wt[2][L];
+  __shared__ float fade[2];
+  bf16* const raw_k = smem_b;                    // [kAheadChunks][L][kLdB]
+  bf16* const raw_v = raw_k + kAheadChunks * L * kLdB;
+  bf16* const kh = raw_v + kAheadChunks * L * kLdB;         // [L][kLdB] weighted keys, high part
+  bf16* const kl = kh + L * kLdB;                // low part
+  pdl_launch_next();
+  pdl_wait_prior();
+  const int H = p.n_heads, D = p.dim, V = p.vdim, h = blockIdx.y, seq = blockIdx.z;
+  const int n_vb = (V + kBlock - 1) / kBlock;
+  const int v0 = static_cast<int>(blockIdx.x) % n_vb * kBlock, d0 = static_cast<int>(blockIdx.x) / n_vb * kBlock;
+  const int tb = p.cu_seqlens[seq], te = p.cu_seqlens[seq + 1];
+  const int nc = (te - tb + L - 1) / L, base = chunk_base(p.cu_seqlens, seq);
+  if (nc <= 0) return;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, r4 = lane >> 2, c4 = lane & 3;
+  const long long sh = static_cast<long long>(p.state_slot[seq]) * H + h;
+  const bf16* proj = static_cast<const bf16*>(p.proj);
+  const uint32_t k_a = smem_u32(raw_k), v_a = smem_u32(raw_v), kh_a = smem_u32(kh), kl_a = smem_u32(kl);
+  auto load = [&](int c) {   // by the sixteen warps
+    if (c >= nc) {
+      cp_async_commit();
+      return;
+    }
+    const int t0 = tb + c * L, len = min(L, te - t0);
+    for (int i = tid; i < L * (kBlock / 8); i += kWalkers) {
+      const int s = i / (kBlock / 8), e = (i % (kBlock / 8)) * 8, at = ((c % kAheadChunks * L + s) * kLdB + e) * 2;
+      const bf16* row = proj + (t0 + min(s, len - 1)) * p.ldp;
+      const bool k_ok = s < len && d0 + e < D, v_ok = s < len && v0 + e < V;
+      cp_async16(k_a + at, k_ok ? row + p.k_off + h * D + d0 + e : proj, k_ok);
+      cp_async16(v_a + at, v_ok ? row + p.v_off + h * V + v0 + e : proj, v_ok);
+    }
+    cp_async_commit();
+  };
+  // by the last warp: the weights of a chunk's keys, and what its state before fades to, from gates asked for a chunk earlier
+  float g_F[2], g_i[2], g_end, g_m0, g_m1;
+  auto ask = [&](int c) {
+    if (c >= nc) return;
+    const int t0 = tb + c * L, len = min(L, te - t0);
+    const long long ch = static_cast<long long>(base + c) * H + h;
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const long long at = static_cast<long long>(t0 + min(lane + 32 * j, len - 1)) * H + h;
+      g_F[j] = w.F[at];
+      g_i[j] = w.ig[at];
+    }
+    g_end = w.c_F[ch];
+    g_m0 = w.c_m0[ch];
+    g_m1 = w.c_m1[ch];
+  };
+  auto weigh = [&](int c) {
+    if (c >= nc) return;
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+      wt[c & 1][lane + 32 * j] = lane + 32 * j < te - tb - c * L ? expf(g_end - g_F[j] + g_i[j] - g_m1) : 0.f;
+    if (lane == 0) fade[c & 1] = expf(g_end + g_m0 - g_m1);
+  };
+  if (warp == kWalkers / 32) {
+    const int d = d0 + 2 * lane;   // this thread's two entries of n
+    const bool keep_n = v0 == 0 && d < D;
+    float2 n = make_float2(0.f, 0.f);
+    if (keep_n) n = *reinterpret_cast<const float2*>(p.n + sh * D + d);
+    ask(0);
+    weigh(0);
+    ask(1);
+    __syncthreads();
+    for (int c = 0; c < nc; ++c) {
+      weigh(c + 1);
+      ask(c + 2);
+      __syncthreads();   // the weighted keys are there
+      if (keep_n) {
+        float2 a = make_float2(0.f, 0.f);
+        const bf16* k = raw_k + c % kAheadChunks * L * kLdB + 2 * lane;
+#pragma unroll
+        for (int s = 0; s < L; s += 4) {
+          const float4 x = *reinterpret_cast<const float4*>(&wt[c & 1][s]);
+          const float y[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const float2 k2 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(k + (s + j) * kLdB));
+            a.x = fmaf(y[j], k2.x, a.x);
+            a.y = fmaf(y[j], k2.y, a.y);
+          }
+        }
+        *reinterpret_cast<float2*>(w.Sn + (static_cast<long long>(base + c) * H + h) * D + d) = n;
+        n.x = fmaf(fade[c & 1], n.x, a.x);
+        n.y = fmaf(fade[c & 1], n.y, a.y);
+      }
+      __syncthreads();   // everyone is done with the chunk's rows
+    }
+    if (keep_n && p.write_state) *reinterpret_cast<float2*>(p.n + sh * D + d) = n;
+    return;
+  }
+  load(0);
+  load(1);
+  const int mt = warp & 3, nh = warp >> 2;   // rows 16 mt .., columns 16 nh ..
+  const int d = d0 + mt * 16 + 2 * r4, v = v0 + nh * 16 + 2 * c4;   // rows d, d + 1; columns v, v + 1 and eights on
+  const bool rows_ok = d0 + mt * 16 < D;     // (widths are multiples of 16)
+  float S[2][4];   // [8 columns][row d: v, v + 1; row d + 1: v, v + 1]
+#pragma unroll
+  for (int n = 0; n < 2; ++n)
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      float2 x = make_float2(0.f, 0.f);
+      if (rows_ok && v + n * 8 < V) x = *reinterpret_cast<const float2*>(p.S + (sh * D + d + r) * V + v + n * 8);
+      S[n][2 * r] = x.x;
+      S[n][2 * r + 1] = x.y;
+    }
+  cp_async_wait<1>();
+  __syncthreads();
+  for (int c = 0; c < nc; ++c) {
+    const long long ch = static_cast<long long>(base + c) * H + h;
+    const int stage = c % kAheadChunks;
+    load(c + 2);
+    // weighted keys as hi + lo pairs: eight neighbouring columns of a row per thread
+    {
+      const int s = tid >> 3, e = (tid & 7) * 8;
+      const uint4 raw = *reinterpret_cast<const uint4*>(raw_k + (stage * L + s) * kLdB + e);
+      const uint32_t x[4] = {raw.x, raw.y, raw.z, raw.w};
+      const float weight = wt[c & 1][s];
+      uint32_t hi[2][2], lo[2][2];   // [even or odd column]
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&x[2 * j]));
+        const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&x[2 * j + 1]));
+        const float y[2][2] = {{a.x * weight, b.x * weight}, {a.y * weight, b.y * weight}};
+#pragma unroll
+        for (int o = 0; o < 2; ++o) {
+          hi[o][j] = pack_bf16x2(y[o][0], y[o][1]);
+          const float2 h2 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&hi[o][j]));
+          lo[o][j] = pack_bf16x2(y[o][0] - h2.x, y[o][1] - h2.y);
+        }
+      }
+      const int at = s * kLdB + (e & ~15) + (e & 8) / 2;
+#pragma unroll
+      for (int o = 0; o < 2; ++o) {
+        *reinterpret_cast<uint2*>(kh + at + 8 * o) = make_uint2(hi[o][0], hi[o][1]);
+        *reinterpret_cast<uint2*>(kl + at + 8 * o) = make_uint2(lo[o][0], lo[o][1]);
+      }
+    }
+    // the state before the chunk
+    if (rows_ok) {
+#pragma unroll
+      for (int n = 0; n < 2; ++n) {
+        if (v + n * 8 >= V) continue;
+        float hi[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) hi[e] = __bfloat162float(__float2bfloat16(S[n][e]));
+        const long long at = (ch * (D / 2) + d / 2) * V + v + n * 8;
+        *reinterpret_cast<uint2*>(w.Sh + at) = make_uint2(pack_bf16x2(hi[0], hi[2]), pack_bf16x2(hi[1], hi[3]));
+        *reinterpret_cast<uint2*>(w.Sl + at) = make_uint2(pack_bf16x2(S[n][0] - hi[0], S[n][2] - hi[2]), pack_bf16x2(S[n][1] - hi[1], S[n][3] - hi[3]));
+      }
+    }
+    __syncthreads();   // the weighted keys are there
+    float acc[2][4];
+#pragma unroll
+    for (int n = 0; n < 2; ++n)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) acc[n][e] = 0.f;
+#pragma unroll
+    for (int kk = 0; kk < L / 16; ++kk) {
+      uint32_t ah[4], al[4];
+      const uint32_t at = ((kk * 16 + (lane & 7) + ((lane >> 4) & 1) * 8) * kLdB + mt * 16 + ((lane >> 3) & 1) * 8) * 2;
+      ldsm_x4_trans(kh_a + at, ah);
+      ldsm_x4_trans(kl_a + at, al);
+      uint32_t b[4];
+      ldsm_x4_trans(v_a + ((stage * L + kk * 16 + (lane & 15)) * kLdB + nh * 16 + (lane >> 4) * 8) * 2, b);
+      mma_bf16_16816(acc[0], ah, b[0], b[1]);
+      mma_bf16_16816(acc[1], ah, b[2], b[3]);
+      mma_bf16_16816(acc[0], al, b[0], b[1]);
+      mma_bf16_16816(acc[1], al, b[2], b[3]);
+    }
+    const float f = fade[c & 1];
+#pragma unroll
+    for (int n = 0; n < 2; ++n)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) S[n][e] = fmaf(f, S[n][e], acc[n][e]);
+    cp_async_wait<1>();
+    __syncthreads();   // everyone is done with the chunk's rows; the next ones are there
+  }
+  if (p.write_state && rows_ok) {
+#pragma unroll
+    for (int n = 0; n < 2; ++n)
+#pragma unroll
+      for (int r = 0; r < 2; ++r)
+        if (v + n * 8 < V)
+          *reinterpret_cast<float2*>(p.S + (sh * D + d + r) * V + v + n * 8) = make_float2(S[n][2 * r], S[n][2 * r + 1]);
   }
 }
 
@@ -624,10 +829,21 @@ const char* mlstm_chunked(const MlstmArgs& a, void* workspace, int64_t workspace
   const int nc = a.T / L + a.n_seq;
   cudaError_t e = launch_kernel(mlstm_gates_kernel, dim3(a.n_seq, a.n_heads), dim3(a.T >= 8 * L * a.n_seq ? 1024 : 256), 0, a.stream, a.pdl, 1, a, w);
   if (e != cudaSuccess) return cudaGetErrorString(e);
-  e = launch_contrib(a, w, nc);
-  if (e != cudaSuccess) return cudaGetErrorString(e);
-  const int blocks = ((a.dim / 2) * a.vdim + 255) / 256 + 1;
-  e = launch_kernel(mlstm_scan_kernel, dim3(blocks, a.n_heads, a.n_seq), dim3(256), 0, a.stream, a.pdl, 1, a, w);
+  // The walk where the heads of a single sequence fill two thirds of the SMs: a chunk takes it 1.7 us whatever the width, so that one
+  // sequence of 2048 tokens is 55 us with 8 blocks or 128; the two kernels take 19 us for 8 or 16 blocks and 69 for 128.  (Lengths are
+  // not known here: one of many sequences may have most of the tokens.)  It reads state rows two values at a time.
+  const int state_blocks = ((a.dim + kBlock - 1) / kBlock) * ((a.vdim + kBlock - 1) / kBlock);
+  if (3LL * state_blocks * a.n_heads >= 2LL * device_sm_count() &&
+      (reinterpret_cast<uintptr_t>(a.S) | reinterpret_cast<uintptr_t>(a.n)) % 8 == 0) {
+    e = allow_smem(mlstm_walk_kernel, kWalkSmem);
+    if (e == cudaSuccess)
+      e = launch_kernel(mlstm_walk_kernel, dim3(state_blocks, a.n_heads, a.n_seq), dim3(kWalkThreads), kWalkSmem, a.stream, a.pdl, 1, a, w);
+  } else {
+    e = launch_contrib(a, w, nc);
+    if (e != cudaSuccess) return cudaGetErrorString(e);
+    const int blocks = ((a.dim / 2) * a.vdim + 255) / 256 + 1;
+    e = launch_kernel(mlstm_scan_kernel, dim3(blocks, a.n_heads, a.n_seq), dim3(256), 0, a.stream, a.pdl, 1, a, w);
+  }
   if (e != cudaSuccess) return cudaGetErrorString(e);
   const int nt = (a.vdim / 8 + 7) / 8;
   if (nt <= 1) e = launch_output<8, 1>(a, w, nc);

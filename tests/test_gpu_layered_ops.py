@@ -294,6 +294,35 @@ def test_matrix_memory(ops, geo, dt, i_shift, f_shift):
             assert rel(a, b) < 3e-5
 
 
+@pytest.mark.parametrize("geo", [(4, 256, 512), (5, 272, 496), (13, 80, 240), (2, 512, 496)])
+@pytest.mark.parametrize("lens", [[150, 1, 64, 77], [63], [200, 129]])
+@pytest.mark.parametrize("write", [True, False])
+def test_matrix_memory_states_of_wide_heads(ops, geo, lens, write):
+    """Heads that fill the GPU have their states walked by one kernel where the state starts at an 8-byte boundary, and else by the
+    two that any heads have: the same bits of outputs and states, at the edges of blocks and chunks."""
+    H, D, V = geo
+    T, B = sum(lens), len(lens)
+    g = torch.Generator().manual_seed(D + T)
+    proj = torch.randn(T, H * (2 * D + 2 * V), generator=g).to(torch.bfloat16).cuda()
+    gates = (torch.randn(T, 2 * H, generator=g) * 2 + torch.tensor([0.0] * H + [3.0] * H)).cuda()
+    S0, n0, m0 = torch.randn(B, H, D, V, generator=g) * 0.1, torch.rand(B, H, D, generator=g), torch.zeros(B, H).cuda()
+    norm = torch.rand(H * V, generator=g).cuda()
+    cu = torch.tensor([0] + list(torch.tensor(lens).cumsum(0)), dtype=torch.int32, device="cuda")
+    slots = torch.arange(B, dtype=torch.int32, device="cuda")
+    got = []
+    for offset in (0, 1):
+        S = torch.empty(S0.numel() + 1, device="cuda")[offset:offset + S0.numel()].view(S0.shape).copy_(S0)
+        n, m = n0.cuda(), m0.clone()
+        out = torch.full((T, H * V), float("nan"), dtype=torch.bfloat16, device="cuda")
+        ws = torch.empty(int(ops.mlstm_chunked_workspace_bytes(T, B, H, D, V)), dtype=torch.uint8, device="cuda").fill_(0xff)
+        ops.mlstm(proj, 0, H * D, 2 * H * D, H * (2 * D + V), gates, 0, H, V, D ** -0.5, 15.0, 1e-6, norm, cu, slots, S, n, m, out,
+                  write, ws, False, False)
+        got.append((out, S, n, m))
+    for a, b in zip(*got):
+        assert torch.equal(a, b) and not a.isnan().any()
+    assert torch.equal(got[0][1].cpu(), S0) != write
+
+
 @pytest.mark.parametrize("geo", [(4, 256, 512), (3, 272, 496), (5, 512, 240), (2, 144, 512)])
 @pytest.mark.parametrize("dt", DTYPES)
 @pytest.mark.parametrize("pdl", [False, True])
