@@ -17,6 +17,7 @@
 #include "../common/elem.cuh"
 #include "../common/launch.h"
 #include "../common/mma_sync.cuh"
+#include "../common/quotient.cuh"
 
 namespace nfb {
 
@@ -519,6 +520,10 @@ __global__ void __launch_bounds__(kWalkThreads) mlstm_walk_kernel(const MlstmArg
 }
 
 // NW warps, NT: 8-wide value tiles per warp (NW warps cover V).  grid: (chunk slot, head)
+// One round of CTAs and a chain each, so what counts is latency and, outside the products (9 us of a scheduler's tensor pipe for
+// 256 x 512), code: n_0 comes once for a warp's queries, a query's factors are made by one lane and not by the 64 that use them,
+// gates are asked for before the last barrier and opened without a division's branch, the first state rows beside the intra-chunk
+// weights.  Three sequences of 1138, 683 and 227 tokens 45 -> 34 us, one of 100 35 -> 30.
 template <int NW, int NT>
 __global__ void __launch_bounds__(NW * 32, NW == 8 ? 2 : 1) mlstm_output_kernel(const MlstmArgs p, const ChunkWs w) {
   extern __shared__ __align__(16) bf16 smem_b[];
@@ -564,6 +569,22 @@ __global__ void __launch_bounds__(NW * 32, NW == 8 ? 2 : 1) mlstm_output_kernel(
     ms[tid] = w.mt[at];
     inter[tid] = p.q_scale * expf(w.F[at] + w.c_m0[ch] - w.mt[at]);
   }
+  const int vt0 = warp * NT;
+  const int n_live = min(NT, V / 8 - vt0);
+  // The fragments of the next sixteen rows are loaded beside the products of these, without a condition: a dead tile reads the
+  // last live one and is not used (49 -> 47 us at the sizes above).
+  const uint32_t* sh = w.Sh + (ch * (D / 2) + c4) * V + vt0 * 8 + r4;
+  const uint32_t* sl = w.Sl + (ch * (D / 2) + c4) * V + vt0 * 8 + r4;
+  uint32_t bh[2][NT][2], bl[2][NT][2];
+  auto fetch = [&](int d, uint32_t (*fh)[2], uint32_t (*fl)[2]) {
+#pragma unroll
+    for (int n = 0; n < NT; ++n) {
+      const long long at = static_cast<long long>(d / 2) * V + min(n, n_live - 1) * 8;
+      fh[n][0] = sh[at]; fh[n][1] = sh[at + 4LL * V];
+      fl[n][0] = sl[at]; fl[n][1] = sl[at + 4LL * V];
+    }
+  };
+  if (n_live > 0) fetch(0, bh[0], bl[0]);   // beside the intra-chunk weights
   cp_async_wait<1>();
   __syncthreads();
   // ---- intra-chunk weights: warp = 16 queries x 8 kKn keys ----
@@ -605,19 +626,27 @@ __global__ void __launch_bounds__(NW * 32, NW == 8 ? 2 : 1) mlstm_output_kernel(
       if (c4 == 0) den_s[nh][mt * 16 + r4 + r * 8] = sum[r];
     }
   }
-  // ---- n_0 . q: warp = L / NW queries ----
-  for (int j = 0; j < L / NW; ++j) {
-    const int t = warp * (L / NW) + j;
-    float d = 0.f;
+  // ---- n_0 . q: warp = L / NW queries, whose sums take n_0 from registers ----
+  {
+    float d[L / NW];
+#pragma unroll
+    for (int j = 0; j < L / NW; ++j) d[j] = 0.f;
     for (int i = lane * 8; i < D; i += 256) {
-      float q[8], n[8];
-      load8(qs + t * ldq + i, q);
+      float n[8];
       load8(w.Sn + ch * D + i, n);
 #pragma unroll
-      for (int e = 0; e < 8; ++e) d = fmaf(q[e], n[e], d);
+      for (int j = 0; j < L / NW; ++j) {
+        float q[8];
+        load8(qs + (warp * (L / NW) + j) * ldq + i, q);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) d[j] = fmaf(q[e], n[e], d[j]);
+      }
     }
-    d = warp_sum(d);
-    if (lane == 0) den_state[t] = d;
+#pragma unroll
+    for (int j = 0; j < L / NW; ++j) {
+      d[j] = warp_sum(d[j]);
+      if (lane == 0) den_state[warp * (L / NW) + j] = d[j];
+    }
   }
   // ---- S_0^T q: all 64 queries x this warp's value tiles, S_0 fragments straight from global memory ----
   float acc[4][NT][4];
@@ -627,22 +656,7 @@ __global__ void __launch_bounds__(NW * 32, NW == 8 ? 2 : 1) mlstm_output_kernel(
     for (int n = 0; n < NT; ++n)
 #pragma unroll
       for (int e = 0; e < 4; ++e) acc[m][n][e] = 0.f;
-  const int vt0 = warp * NT;
-  const int n_live = min(NT, V / 8 - vt0);
   if (n_live > 0) {
-    const uint32_t* sh = w.Sh + (ch * (D / 2) + c4) * V + vt0 * 8 + r4;
-    const uint32_t* sl = w.Sl + (ch * (D / 2) + c4) * V + vt0 * 8 + r4;
-    // The fragments of the next sixteen rows are loaded beside the products of these, without a condition: a dead tile reads
-    // the last live one and is not used (49 -> 47 us at the sizes above).
-    uint32_t bh[2][NT][2], bl[2][NT][2];
-    auto fetch = [&](int d, uint32_t (*fh)[2], uint32_t (*fl)[2]) {
-#pragma unroll
-      for (int n = 0; n < NT; ++n) {
-        const long long at = static_cast<long long>(d / 2) * V + min(n, n_live - 1) * 8;
-        fh[n][0] = sh[at]; fh[n][1] = sh[at + 4LL * V];
-        fl[n][0] = sl[at]; fl[n][1] = sl[at + 4LL * V];
-      }
-    };
     auto multiply = [&](int d, const uint32_t (*fh)[2], const uint32_t (*fl)[2]) {
 #pragma unroll
       for (int m = 0; m < 4; ++m) {
@@ -655,7 +669,6 @@ __global__ void __launch_bounds__(NW * 32, NW == 8 ? 2 : 1) mlstm_output_kernel(
         }
       }
     };
-    fetch(0, bh[0], bl[0]);
     for (int d = 0; d < D; d += 32) {
       if (d + 16 < D) fetch(d + 16, bh[1], bl[1]);
       multiply(d, bh[0], bl[0]);
@@ -699,16 +712,22 @@ __global__ void __launch_bounds__(NW * 32, NW == 8 ? 2 : 1) mlstm_output_kernel(
       }
     }
   }
-  // ---- denominator, head norm, gate ----
+  // ---- denominator, head norm, gate: a lane has two queries' factors and hands them round ----
+  float inv_of[2];
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    const int t = lane + 32 * j;
+    float den = inter[t] * den_state[t];
+#pragma unroll
+    for (int i = 0; i < NW / 4; ++i) den += den_s[i][t];
+    inv_of[j] = 1.f / (fmaxf(fabsf(den), expf(-ms[t])) + 1e-6f);
+  }
 #pragma unroll
   for (int m = 0; m < 4; ++m) {
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
       const int t = m * 16 + r4 + r * 8;
-      float den = inter[t] * den_state[t];
-#pragma unroll
-      for (int i = 0; i < NW / 4; ++i) den += den_s[i][t];
-      const float inv = 1.f / (fmaxf(fabsf(den), expf(-ms[t])) + 1e-6f);
+      const float inv = __shfl_sync(0xffffffffu, inv_of[m / 2], t & 31);
       float sq = 0.f;
 #pragma unroll
       for (int n = 0; n < NT; ++n) {
@@ -723,29 +742,44 @@ __global__ void __launch_bounds__(NW * 32, NW == 8 ? 2 : 1) mlstm_output_kernel(
       if (c4 == 0) ss_s[warp][t] = sq;
     }
   }
+  const auto open = [](bf16 g) { return quotient(1.f, 1.f + exp_of<bf16>(-__bfloat162float(g))); };
+  // (the gates are asked for before the barrier)
+  __nv_bfloat162 gate[4][2][NT];
+  float2 scale[NT];
+#pragma unroll
+  for (int n = 0; n < NT; ++n) {
+    const int v = (vt0 + max(min(n, n_live - 1), 0)) * 8 + c4 * 2;
+    scale[n] = n_live > 0 ? *reinterpret_cast<const float2*>(p.norm + h * V + v) : make_float2(0.f, 0.f);
+#pragma unroll
+    for (int m = 0; m < 4; ++m)
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        const int t = min(m * 16 + r4 + r * 8, len - 1);
+        if (n_live > 0) gate[m][r][n] = *reinterpret_cast<const __nv_bfloat162*>(proj + (t0 + t) * p.ldp + p.g_off + h * V + v);
+      }
+  }
   __syncthreads();
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    float tot = 0.f;
+#pragma unroll
+    for (int i = 0; i < NW; ++i) tot += ss_s[i][lane + 32 * j];
+    inv_of[j] = 1.f / sqrtf(tot / static_cast<float>(p.vdim_true) + p.eps);
+  }
 #pragma unroll
   for (int m = 0; m < 4; ++m) {
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
       const int t = m * 16 + r4 + r * 8;
+      const float inv = __shfl_sync(0xffffffffu, inv_of[m / 2], t & 31);
       if (t >= len) continue;
-      float tot = 0.f;
-#pragma unroll
-      for (int i = 0; i < NW; ++i) tot += ss_s[i][t];
-      const float inv = 1.f / sqrtf(tot / static_cast<float>(p.vdim_true) + p.eps);
-      const bf16* gr = proj + (t0 + t) * p.ldp + p.g_off + h * V;
       bf16* dst = static_cast<bf16*>(p.out) + (t0 + t) * p.ldo + h * V;
 #pragma unroll
       for (int n = 0; n < NT; ++n) {
-        if (n < n_live) {
-          const int v = (vt0 + n) * 8 + c4 * 2;
-          const __nv_bfloat162 g2 = *reinterpret_cast<const __nv_bfloat162*>(gr + v);
-          const float2 nw = *reinterpret_cast<const float2*>(p.norm + h * V + v);
-          *reinterpret_cast<uint32_t*>(dst + v) =
-              pack_bf16x2(acc[m][n][2 * r] * inv * nw.x * sigmoid_of<bf16>(__bfloat162float(g2.x)),
-                          acc[m][n][2 * r + 1] * inv * nw.y * sigmoid_of<bf16>(__bfloat162float(g2.y)));
-        }
+        if (n < n_live)
+          *reinterpret_cast<uint32_t*>(dst + (vt0 + n) * 8 + c4 * 2) =
+              pack_bf16x2(acc[m][n][2 * r] * inv * scale[n].x * open(gate[m][r][n].x),
+                          acc[m][n][2 * r + 1] * inv * scale[n].y * open(gate[m][r][n].y));
       }
     }
   }
