@@ -358,8 +358,11 @@ __global__ void __launch_bounds__(kStreamWorkers + 32, 1) mlstm_stream_kernel(co
   const int items = p.n_seq * H, mine = (items - static_cast<int>(blockIdx.x) + static_cast<int>(gridDim.x) - 1) / static_cast<int>(gridDim.x);
   const int total = mine * chunks;
   if (warp == kStreamWorkers / 32) {
-    // ---- copies, one thread.  States and the step's description depend on no kernel of this step: no wait before the first loads ----
+    // ---- copies, one thread.  The call before may be a step of the same states, or a portion whose walk wrote them: it is waited
+    //      for before anything is read ----
     if (lane == 0) {
+      pdl_wait_prior();
+      asm volatile("fence.proxy.async.global;" ::: "memory");   // bulk copies read what ordinary stores have written
       auto rows = [&](int n, uint32_t& bytes) {
         const int i = static_cast<int>(blockIdx.x) + n / chunks * static_cast<int>(gridDim.x), c = n % chunks;
         bytes = static_cast<uint32_t>(min(kChunkRows, D - c * kChunkRows)) * V * 4;

@@ -354,6 +354,41 @@ def test_matrix_memory_step_of_many_states(ops, geo, dt, pdl):
     assert not torch.equal(got[0][1], first[0])
 
 
+@pytest.mark.parametrize("B", [15, 40])
+@pytest.mark.parametrize("portion", [0, 70])
+def test_matrix_memory_steps_of_the_same_states(ops, B, portion):
+    """Steps right behind one another on the same slots, and behind a portion that wrote them, with and without the early start of
+    a kernel: the same bits.  60 states leave SMs free on which the next step's CTAs start at once."""
+    H, D, V, steps = 4, 256, 512, 6
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    assert 5 * B * H >= 2 * sms
+    torch.manual_seed(B)
+    ldp = H * (2 * D + 2 * V)
+    proj = torch.randn(steps * B + portion * B, ldp, device="cuda").bfloat16()
+    gates = torch.randn(proj.shape[0], 2 * H, device="cuda") * 3 + torch.tensor([0.0] * H + [2.0] * H, device="cuda")
+    norm = 1 + 0.3 * torch.randn(H * V, device="cuda")
+    slot = torch.randperm(B + 1, device="cuda")[:B].int()
+    first = [torch.randn(B + 1, H, D, V, device="cuda") * 0.2, torch.randn(B + 1, H, D, device="cuda"), torch.rand(B + 1, H, device="cuda")]
+    one, many = (torch.arange(B + 1, dtype=torch.int32, device="cuda") * n for n in (1, portion))
+    ws = torch.empty(int(ops.mlstm_chunked_workspace_bytes(portion * B, B, H, D, V)), dtype=torch.uint8, device="cuda") if portion else None
+    got = []
+    for pdl in (False, True):
+        S, n, m = (t.clone() for t in first)
+        out = torch.full((proj.shape[0], H * V), float("nan"), dtype=torch.bfloat16, device="cuda")
+        torch.cuda.synchronize()
+
+        def call(rows, cu, chunk_ws, single):
+            ops.mlstm(proj[rows], 0, H * D, 2 * H * D, H * (2 * D + V), gates[rows], 0, H, V, D ** -0.5, 8.0, 1e-3, norm, cu, slot,
+                      S, n, m, out[rows], True, chunk_ws, pdl, single)
+        if portion:
+            call(slice(steps * B, None), many, ws, False)
+        for i in range(steps):
+            call(slice(i * B, (i + 1) * B), one, None, True)
+        got.append((out, S, n, m))
+    for a, b in zip(*got):
+        assert torch.equal(a, b) and not a.isnan().any()
+
+
 @pytest.mark.parametrize("dt", DTYPES)
 def test_token_selection_on_both_logit_types(ops, dt):
     lg = rnd(3, 5, 301).to(dt)
