@@ -63,6 +63,9 @@ class StatusWord:
         3: "epilogue waited for an accumulator that never committed",
         4: "a peer-rank flag never reached the expected epoch",
         5: "bad kernel argument",
+        6: "an attention kernel waited for an operand or a product that never came",
+        7: "a step waited for rows of a recurrent state that never landed",
+        8: "a step's rows of a recurrent state were never handed on to be stored",
     }
 
     def __init__(self, device):

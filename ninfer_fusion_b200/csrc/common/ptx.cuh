@@ -21,6 +21,9 @@ enum : int {
   kStatusAccumWaitTimeout = 3,  // epilogue waited for an accumulator that never committed
   kStatusPeerWaitTimeout = 4,   // a peer-rank flag never reached the expected epoch
   kStatusBadArgument = 5,
+  // 6: waits of the attention kernels (named in their files)
+  kStatusStateWaitTimeout = 7,  // a step waited for rows of a recurrent state that never landed
+  kStatusStateDoneTimeout = 8,  // a step's rows of a recurrent state were never handed on to be stored
 };
 
 __device__ __forceinline__ void report_status(int* status, int code) {

@@ -72,6 +72,7 @@ struct GdnParams {
   // codes [T][Hv * 64] bytes and the scale plane of T x (Hv * 128) values.
   uint8_t* q_codes = nullptr;
   uint8_t* q_sf = nullptr;
+  int* status = nullptr;     // optional status word: where the streaming step reports a wait that ran out
 };
 const char* gdn_recurrent(const GdnParams& p, cudaStream_t stream, bool pdl);
 // Multi-token variant (token groups staged in shared memory); gdn_recurrent dispatches to it when T > n_seq.

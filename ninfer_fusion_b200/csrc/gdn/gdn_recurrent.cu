@@ -361,7 +361,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) gdn_stream_kernel(const Gdn
       asm volatile("fence.proxy.async.global;" ::: "memory");
       for (int n = 0; n < primed; ++n) load_rows(n, item(n));
       for (int n = 0; n < mine; ++n) {
-        if (!mbar_wait(smem_u32(&bar_done[n % kRing]), (n / kRing) & 1, abortp, nullptr, 0)) break;
+        if (!mbar_wait(smem_u32(&bar_done[n % kRing]), (n / kRing) & 1, abortp, p.status, kStatusStateDoneTimeout)) break;
         const Item it = item(n);
         if (it.t1 > it.t0) bulk_store(state(it), ring + (n % kRing) * kSlotBytes, kStateBytes);
         if (n + kRing < mine) {
@@ -408,7 +408,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) gdn_stream_kernel(const Gdn
       fetch_gates(it);
     }
     // (one verdict for the warps: their barriers below are never divergent)
-    const bool ok = mbar_wait(smem_u32(&bar_full[n % kRing]), (n / kRing) & 1, abortp, nullptr, 0);
+    const bool ok = mbar_wait(smem_u32(&bar_full[n % kRing]), (n / kRing) & 1, abortp, p.status, kStatusStateWaitTimeout);
     uint32_t all;
     asm volatile(
         "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 q, %1, 0;\n\tbar.red.and.pred p, 1, 256, q;\n\tselp.u32 %0, 1, 0, p;\n\t}\n"

@@ -33,6 +33,7 @@ struct MlstmArgs {
   bool write_state = true;
   bool one_token = false;         // every sequence brings exactly one token
   bool f32 = false;
+  int* status = nullptr;          // optional status word: where the streaming step reports a wait that ran out
   cudaStream_t stream = nullptr;
   bool pdl = false;
 };

@@ -379,7 +379,7 @@ __global__ void __launch_bounds__(kStreamWorkers + 32, 1) mlstm_stream_kernel(co
       };
       for (int n = 0; n < min(total, kRing); ++n) load(n);
       for (int n = 0; n < total; ++n) {
-        if (!mbar_wait(smem_u32(&bar_done[n % kRing]), (n / kRing) & 1, abortp, nullptr, 0)) break;
+        if (!mbar_wait(smem_u32(&bar_done[n % kRing]), (n / kRing) & 1, abortp, p.status, kStatusStateDoneTimeout)) break;
         uint32_t bytes;
         float* dst = rows(n, bytes);
         bulk_store(dst, ring + (n % kRing) * kChunkBytes, bytes);
@@ -440,9 +440,10 @@ __global__ void __launch_bounds__(kStreamWorkers + 32, 1) mlstm_stream_kernel(co
     for (int g = 0; g < 4; ++g)
 #pragma unroll
       for (int e = 0; e < 4; ++e) acc[g][e] = 0.f;
+    bool ok = true;
     for (int c = 0; c < chunks; ++c, ++n) {
-      const bool ok = mbar_wait(smem_u32(&bar_full[n % kRing]), (n / kRing) & 1, abortp, nullptr, 0);
-      if (!ok) break;   // (the barriers below are reached all the same)
+      ok = mbar_wait(smem_u32(&bar_full[n % kRing]), (n / kRing) & 1, abortp, p.status, kStatusStateWaitTimeout);
+      if (!ok) break;
       float* const buf = reinterpret_cast<float*>(ring_gen + (n % kRing) * kChunkBytes) + col;
       if (col_ok) {
 #pragma unroll
@@ -476,9 +477,14 @@ __global__ void __launch_bounds__(kStreamWorkers + 32, 1) mlstm_stream_kernel(co
       *reinterpret_cast<float4*>(&part[2 * quarter + j][col]) =
           make_float4(acc[2 * j][0] + acc[2 * j + 1][0], acc[2 * j][1] + acc[2 * j + 1][1], acc[2 * j][2] + acc[2 * j + 1][2],
                       acc[2 * j][3] + acc[2 * j + 1][3]);
+    // (a barrier, and one verdict for the warps: where rows did not come, neither n, m nor an output is written)
+    uint32_t all;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 q, %1, 0;\n\tbar.red.and.pred p, 1, 512, q;\n\tselp.u32 %0, 1, 0, p;\n\t}\n"
+        : "=r"(all) : "r"(static_cast<uint32_t>(ok)) : "memory");
+    if (!all) break;
     for (int r = tid; r < D; r += kStreamWorkers) ng[r] = ns[r];
     if (tid == 0) *mg = m;
-    sync();
     float o4[4] = {0.f, 0.f, 0.f, 0.f};
     if (tid < 128) {
       float den = 0.f, sq = 0.f;

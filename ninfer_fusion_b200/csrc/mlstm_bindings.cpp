@@ -10,7 +10,7 @@ using namespace nfb_bind;
 void mlstm(const Tensor& proj, int64_t q_off, int64_t k_off, int64_t v_off, int64_t g_off, const Tensor& gates, int64_t i_off,
            int64_t f_off, int64_t vdim_true, double q_scale, double gate_cap, double eps, const Tensor& norm,
            const Tensor& cu_seqlens, const Tensor& state_slot, const Tensor& S, const Tensor& n, const Tensor& m,
-           const Tensor& out, bool write_state, OptT chunk_ws, bool pdl, bool one_token) {
+           const Tensor& out, bool write_state, OptT chunk_ws, bool pdl, bool one_token, OptT status) {
   nfb::MlstmArgs a;
   a.f32 = act_f32(proj, "proj");
   need_rows(proj, "proj"); need_rows(out, "out"); need(out, proj.scalar_type(), "out");
@@ -39,6 +39,8 @@ void mlstm(const Tensor& proj, int64_t q_off, int64_t k_off, int64_t v_off, int6
   a.out = out.data_ptr(); a.ldo = out.stride(0); a.write_state = write_state;
   TORCH_CHECK(!one_token || T == B, "mlstm: one token per sequence expected");
   a.one_token = one_token;
+  if (status.has_value() && status->defined()) need(*status, at::kInt, "status");
+  a.status = ptr_or_null<int>(status);
   c10::cuda::CUDAGuard guard(proj.device());
   a.stream = cur_stream(); a.pdl = pdl;
   if (chunk_ws.has_value() && chunk_ws->defined()) {
@@ -60,7 +62,7 @@ bool mlstm_chunked_supported(int64_t dim, int64_t vdim) {
 }  // namespace
 
 TORCH_LIBRARY_FRAGMENT(nfb200, m) {
-  m.def("mlstm(Tensor proj, int q_off, int k_off, int v_off, int g_off, Tensor gates, int i_off, int f_off, int vdim_true, float q_scale, float gate_cap, float eps, Tensor norm, Tensor cu_seqlens, Tensor state_slot, Tensor S, Tensor n, Tensor m, Tensor out, bool write_state, Tensor? chunk_ws, bool pdl, bool one_token=False) -> ()", &mlstm);
+  m.def("mlstm(Tensor proj, int q_off, int k_off, int v_off, int g_off, Tensor gates, int i_off, int f_off, int vdim_true, float q_scale, float gate_cap, float eps, Tensor norm, Tensor cu_seqlens, Tensor state_slot, Tensor S, Tensor n, Tensor m, Tensor out, bool write_state, Tensor? chunk_ws, bool pdl, bool one_token=False, Tensor? status=None) -> ()", &mlstm);
   m.def("mlstm_chunked_workspace_bytes(int T, int n_seq, int n_heads, int dim, int vdim) -> int", &mlstm_chunked_workspace_bytes);
   m.def("mlstm_chunked_supported(int dim, int vdim) -> bool", &mlstm_chunked_supported);
 }

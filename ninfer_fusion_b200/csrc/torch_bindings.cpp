@@ -377,7 +377,8 @@ void gdn_recurrent(const Tensor& qkv, int64_t q_off, int64_t k_off, int64_t v_of
                    int64_t a_off, int64_t b_off, int64_t n_qk_heads, int64_t n_v_heads, const Tensor& A_log,
                    const Tensor& dt_bias, const Tensor& norm_w, double eps, const Tensor& cu_seqlens,
                    const Tensor& state_slot, const Tensor& state, bool write_state, const Tensor& out, bool pdl,
-                   OptT seq_end, OptT commit, OptT chunk_ws, OptT conv_w, OptT conv_state, OptT q_codes, OptT q_sf) {
+                   OptT seq_end, OptT commit, OptT chunk_ws, OptT conv_w, OptT conv_state, OptT q_codes, OptT q_sf,
+                   OptT status) {
   need(qkv, at::kBFloat16, "qkv"); need_rows(qkv, "qkv"); need(proj, at::kBFloat16, "proj"); need_rows(proj, "proj");
   need(A_log, at::kFloat, "A_log"); need(dt_bias, at::kFloat, "dt_bias"); need(norm_w, at::kBFloat16, "norm_w");
   need(cu_seqlens, at::kInt, "cu_seqlens"); need(state_slot, at::kInt, "state_slot");
@@ -432,6 +433,8 @@ void gdn_recurrent(const Tensor& qkv, int64_t q_off, int64_t k_off, int64_t v_of
     p.q_codes = static_cast<uint8_t*>(q_codes->data_ptr());
     p.q_sf = static_cast<uint8_t*>(q_sf->data_ptr());
   }
+  if (status.has_value() && status->defined()) need(*status, at::kInt, "status");
+  p.status = ptr_or_null<int>(status);
   if (chunk_ws.has_value() && chunk_ws->defined()) {
     // chunked tensor-core formulation (long prefill chunks)
     need(*chunk_ws, at::kByte, "chunk_ws");
@@ -754,7 +757,7 @@ TORCH_LIBRARY(nfb200, m) {
   m.def("kv_requant(Tensor tiers, Tensor anchor, Tensor src_cell, Tensor dst_cell, int page_size, int n_kv_heads, int head_dim) -> ()", &kv_requant);
   m.def("prefill_attn_block_tokens(int n_q_heads, int n_kv_heads) -> int", &prefill_attn_block_tokens);
   m.def("causal_conv1d_silu(Tensor x, int c_off, int C, Tensor w, Tensor cu_seqlens, Tensor token_seq, Tensor state_slot, Tensor conv_state, Tensor out, bool update_state, bool one_token_per_seq, bool pdl, Tensor? seq_end=None, bool state_only=False, Tensor? parent=None, Tensor? last_token=None) -> ()", &causal_conv1d_silu);
-  m.def("gdn_recurrent(Tensor qkv, int q_off, int k_off, int v_off, Tensor proj, int z_off, int a_off, int b_off, int n_qk_heads, int n_v_heads, Tensor A_log, Tensor dt_bias, Tensor norm_w, float eps, Tensor cu_seqlens, Tensor state_slot, Tensor state, bool write_state, Tensor out, bool pdl, Tensor? seq_end=None, Tensor? commit=None, Tensor? chunk_ws=None, Tensor? conv_w=None, Tensor? conv_state=None, Tensor? q_codes=None, Tensor? q_sf=None) -> ()", &gdn_recurrent);
+  m.def("gdn_recurrent(Tensor qkv, int q_off, int k_off, int v_off, Tensor proj, int z_off, int a_off, int b_off, int n_qk_heads, int n_v_heads, Tensor A_log, Tensor dt_bias, Tensor norm_w, float eps, Tensor cu_seqlens, Tensor state_slot, Tensor state, bool write_state, Tensor out, bool pdl, Tensor? seq_end=None, Tensor? commit=None, Tensor? chunk_ws=None, Tensor? conv_w=None, Tensor? conv_state=None, Tensor? q_codes=None, Tensor? q_sf=None, Tensor? status=None) -> ()", &gdn_recurrent);
   m.def("gdn_chunked_workspace_bytes(int T, int n_seq, int n_v_heads) -> int", &gdn_chunked_workspace_bytes);
   m.def("gdn_prefill_trace(bool enable) -> Tensor", &gdn_prefill_trace);
   m.def("kv_move_rows(Tensor block_table, Tensor table_row, Tensor src_pos, Tensor dst_pos, Tensor k_codes, Tensor v_codes, Tensor? k_scales, Tensor? v_scales, int page_size, int n_kv_heads, int head_dim, int format, int group) -> ()", &kv_move_rows);

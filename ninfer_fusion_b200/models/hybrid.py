@@ -206,9 +206,9 @@ class LaunchCounter:
             else:
                 k = self.KERNELS.get(name, 1)
 
-                def fn(*a, _raw=raw, _k=k):
+                def fn(*a, _raw=raw, _k=k, **named):
                     self.count += _k
-                    return _raw(*a)
+                    return _raw(*a, **named)
             self._cache[name] = fn
         return fn
 
@@ -538,7 +538,7 @@ class HybridModel:
                                   g.gdn_qk_heads, g.gdn_v_heads, self.w[f"{prefix}/gdn/A_log"],
                                   self.w[f"{prefix}/gdn/dt_bias"], self.w[f"{prefix}/gdn/norm"], cfg.rms_eps, b.cu_seqlens,
                                   b.state_slot, st.ssm[gi], True, out, self.pdl, None, None, None,
-                                  self.w[f"{prefix}/gdn/conv_w"], st.conv[gi])
+                                  self.w[f"{prefix}/gdn/conv_w"], st.conv[gi], status=self.status.tensor)
                 return out, self.w[f"{prefix}/gdn/out_proj"]
             ops.causal_conv1d_silu(proj, 0, C, self.w[f"{prefix}/gdn/conv_w"], b.cu_seqlens, b.token_seq, b.state_slot,
                                    st.conv[gi], conv, write_state, decode, self.pdl, None, False, b.tree_parent, None)
@@ -561,7 +561,7 @@ class HybridModel:
         ops.gdn_recurrent(conv, 0, qk, 2 * qk, proj, C, C + g.gdn_v_dim, C + g.gdn_v_dim + g.gdn_v_heads,
                           g.gdn_qk_heads, g.gdn_v_heads, self.w[f"{prefix}/gdn/A_log"], self.w[f"{prefix}/gdn/dt_bias"],
                           self.w[f"{prefix}/gdn/norm"], cfg.rms_eps, b.cu_seqlens, b.state_slot, st.ssm[gi],
-                          write_state, out, self.pdl, None, b.tree_commit, chunk_ws, None, None, qc, qs)
+                          write_state, out, self.pdl, None, b.tree_commit, chunk_ws, None, None, qc, qs, self.status.tensor)
         if qc is not None:
             self._prequant = (out.data_ptr(), T, g.gdn_v_dim)
         return out, w_out
@@ -593,7 +593,7 @@ class HybridModel:
             ops.gdn_recurrent(conv, 0, qk, 2 * qk, proj, C, C + g.gdn_v_dim, C + g.gdn_v_dim + g.gdn_v_heads,
                               g.gdn_qk_heads, g.gdn_v_heads, self.w[f"{p}/gdn/A_log"], self.w[f"{p}/gdn/dt_bias"],
                               self.w[f"{p}/gdn/norm"], cfg.rms_eps, b.cu_seqlens, b.state_slot, st.ssm[gi], True,
-                              ws.mix_gdn[:T], self.pdl, None, accepted)
+                              ws.mix_gdn[:T], self.pdl, None, accepted, status=self.status.tensor)
 
     def fold_gdn(self, ws: Workspace, b: StepBatch, st: GdnStatePool, rec: GdnRecords, seq_end: torch.Tensor) -> None:
         """Replays tokens [cu_seqlens[s], seq_end[s]) of the recorded verify pass `b` into the conv history and the
@@ -611,7 +611,7 @@ class HybridModel:
             ops.gdn_recurrent(conv, 0, qk, 2 * qk, proj, C, C + g.gdn_v_dim, C + g.gdn_v_dim + g.gdn_v_heads,
                               g.gdn_qk_heads, g.gdn_v_heads, self.w[f"{p}/gdn/A_log"], self.w[f"{p}/gdn/dt_bias"],
                               self.w[f"{p}/gdn/norm"], cfg.rms_eps, b.cu_seqlens, b.state_slot, st.ssm[gi], True,
-                              ws.mix_gdn[:T], self.pdl, seq_end)
+                              ws.mix_gdn[:T], self.pdl, seq_end, status=self.status.tensor)
 
     def forward_mtp(self, ws: Workspace, b: StepBatch, kv_mtp: PagedKvCache, hidden_in: torch.Tensor,
                     next_ids: torch.Tensor) -> torch.Tensor:

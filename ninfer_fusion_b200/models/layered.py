@@ -576,7 +576,7 @@ class LayeredModel:
         out = ws.mix[:T, : H * Vp]
         self.ops.mlstm(proj, 0, H * Dp, 2 * H * Dp, H * (2 * Dp + Vp), gates, 0, H, m.vdim, m.dim ** -0.5, m.gate_cap,
                        self.cfg.rms_eps, self.w[f"{p}/mix/norm"], b.cu_seqlens, b.state_slot, S, n, mx, out, write_state,
-                       chunk_ws, self.pdl, b.one_token_per_seq)
+                       chunk_ws, self.pdl, b.one_token_per_seq, self.status.tensor)
         return out
 
     def _gated_memory(self, ws, b: StepBatch, states, run: int, T: int, p: str, m: GatedMemoryMixer, write_state: bool):
