@@ -183,9 +183,11 @@ class MoeBlock:
         # the shared expert (replicated): a dense SwiGLU MLP on the local tokens, beside the routed ones where its weights are bf16 too
         dense = self.expert_format != "fp8_block" and all(isinstance(w, torch.Tensor) and w.dtype == torch.bfloat16 and w.is_contiguous()
                                                           for w in (up_s, down_s))
-        # Up to 64 tokens its first product by itself: the dense kernel then cuts that contraction into parts, whose sum has other
-        # roundings (beside the routed experts a round of one sequence took 819 us, so 880, of 64 2941 and 3091).
-        dense_up = dense and T > 64
+        # Its products stand by themselves where the dense kernel cuts their contraction into parts, whose sum has other roundings: the
+        # first one up to 64 tokens (beside the routed experts a round of one sequence took 819 us, so 880, of 64 2941 and 3091), the
+        # second one there where `shared_inter` is long enough.  The grouped kernel's gated form takes rows in multiples of 128 only.
+        dense_up = dense and T > 64 and up_s.shape[0] % 128 == 0
+        dense_down = dense and (T > 64 or not model.cluster_splitk or int(ops.gemm_pick_splits(T, *down_s.shape, EPI_STORE)) == 1)
         if not dense_up:
             model._gemm(normed, up_s, sact, EPI_SWIGLU)
         if self.expert_format != "fp8_block":
@@ -194,8 +196,8 @@ class MoeBlock:
                          self.peer_bases, 0, 0, status, [], pdl, *((normed, up_s, sact) if dense_up else ()))
             ops.moe_gemm(self.act, down, MOE_EPI_RETURN, tn, max_tiles, self.tiles, self.state, None, W, self.recv_meta,
                          self.peer_bases, self.off["ret"], self.off["ret_flag"], status, [], pdl,
-                         *((sact, down_s, sout) if dense else ()))
-        if not dense:
+                         *((sact, down_s, sout) if dense_down else ()))
+        if not dense_down:
             model._gemm(sact, down_s, sout)
         ops.moe_combine(ws.x[:T], wts, self.ret, self.peer_bases[self.rank], self.off["ret_flag"], sout, sgate,
                         next_norm_w, normed_out, cfg.rms_eps, self.state, status, pdl)
