@@ -541,7 +541,11 @@ __global__ void __launch_bounds__(kThreads, 1) paged_attn_prefill_kernel(const P
       for (int j = 4; j < kHalfKeys; ++j) m4[j & 3] = fmaxf(m4[j & 3], __uint_as_float(v[j]));
       const float own = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3]));
       half_s[b][half][row] = own;
-      row_bar();   // (also: both halves have their scores, so that P may go over them)
+      // Both halves have their scores now, and either stores P over columns that the other has read: the fences put this warp's
+      // loads from TMEM before the barrier and the other's stores behind it.
+      tc_fence_before();
+      row_bar();
+      tc_fence_after();
       const float mx = fmaxf(own, half_s[b][half ^ 1][row]);
       const bool move = mx > top;
       const float corr = move ? ex2(top - mx) : 1.f;   // (a row's first keys: exp2(-inf) = 0)

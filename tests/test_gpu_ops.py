@@ -564,6 +564,42 @@ def test_prefill_attention_does_not_depend_on_pages(ops, status, name, fmt, grou
     status.check("prefill attention")
 
 
+@pytest.mark.parametrize("name,fmt,group", FORMATS)
+def test_prefill_attention_halves_of_a_row(ops, status, name, fmt, group):
+    """The two warps of a row store probabilities over each other's scores.  Scores that grow from tile to tile in one part of the
+    rows and not in the other, on all SMs at once: every run gives the same bits, and those of the queries by themselves."""
+    torch.manual_seed(11)
+    D, hq, hkv, n, T, P = 256, 8, 2, 1100, 600, 64
+    ld, k_off, v_off = (2 * hq + 2 * hkv) * D, hq * D, 2 * hq * D + hkv * D
+    proj = torch.randn(n, ld)
+    proj[:, k_off:k_off + hkv * D] *= torch.linspace(0.2, 3.0, n)[:, None]
+    proj[::3, :hq * D] *= -1
+    proj = proj.to(torch.bfloat16).cuda()
+    pos, seq = torch.arange(n).int().cuda(), torch.zeros(n, dtype=torch.int32, device="cuda")
+    pages = (n + P - 1) // P
+    table = torch.randperm(pages)[:pages].int().view(1, pages).cuda()
+    planes = _planes(pages, hkv, P, D, fmt, group)
+    q = torch.empty((n, hq, D), dtype=torch.bfloat16, device="cuda")
+    ops.attn_prep(proj, 0, k_off, v_off, hq, hkv, D, None, None, 1e-6, True, 0, R.rope_inv_freq(64, 1e7).cuda(), 1.0, pos, seq, pos,
+                  table, q, *planes, P, fmt, group, False)
+    qt = int(ops.prefill_attn_block_tokens(hq, hkv))
+
+    def run(first, count):
+        starts = list(range(0, count, qt))
+        out = torch.full((count, hq * D), float("nan"), dtype=torch.bfloat16, device="cuda")
+        ops.paged_attention_prefill(q[first:first + count].contiguous(), hq, hkv, D, seq[:count], (pos[first:first + count] + 1).contiguous(),
+                                    torch.tensor(starts).int().cuda(), torch.tensor([min(qt, count - o) for o in starts]).int().cuda(),
+                                    table, *planes, P, fmt, group, 1 / 16, None, out, False, 0, None, status.tensor)
+        return out
+    first = run(n - T, T)
+    assert not first.isnan().any()
+    for _ in range(6):
+        assert torch.equal(run(n - T, T), first)
+    for at in (n - T, n - T + 333, n - 2):
+        assert torch.equal(run(at, 2), first[at - n + T:at - n + T + 2])
+    status.check("prefill attention")
+
+
 def test_prefill_attention_largest_key_weighs_one(ops, status):
     """The 64 keys of the first tile score 0, one key of the second 2.03125 (in powers of two): that key's probability against
     the row's largest score is one, exactly, so outputs are its value times an fp32 factor.  Against the first tile's frame it
