@@ -549,16 +549,30 @@ cudaError_t launch(const MlstmArgs& a) {
                        n_cta, a);
 }
 
+// Streams take the states of 256 KB and more (below, all stay with the clusters) where there are too many for the clusters' CTAs, 64
+// columns each and three an SM, to be resident at once, or one for every second SM: below, a cluster reads a state faster than one
+// CTA does.  A second round of states that is nearly empty costs a stream as much as a full one: from 320 columns on it still pays,
+// heads of 192 and more then want the round two fifths full, and narrower ones, which leave most of a stream's threads without
+// columns, no second round at all.  Behind a GEMM, us, clusters and streamed, by states:
+//   256 x 512   48: 17.9, 18.0   52: 20.5, 18.2   148: 44.3, 28.4   160: 48.7, 42.2   296: 83.3, 52.6 (48 at the copy rate)
+//   512 x 384   60: 25.5, 27.6   72: 35.9, 27.8   148: 59.8, 40.8   160: 63.8, 64.1   296: 107.9, 78.4
+//   256 x 256   60: 13.6, 13.8   84: 14.4, 14.2   148: 24.0, 16.1   160: 25.0, 25.1   296: 40.2, 30.6
+//   512 x 256   60: 23.0, 23.6   84: 25.0, 23.6   148: 43.5, 28.9   176: 46.6, 48.5   208: 50.7, 49.5
+//   512 x 128   60: 19.1, 19.5   84: 20.2, 19.7   148: 22.6, 20.1   160: 23.1, 35.0   296: 38.1, 38.0   444: 48.3, 55.7
+// Rounds of the 1 B layer-list decoder, twelve layers of four heads of 256 x 512: 12 sequences 1046 and 1105, 13 1146 -> 1111,
+// 20 1346 -> 1245, 32 1525 -> 1347, 40 1734 -> 1712, 64 2137 -> 1931.
+bool stream_pays(const MlstmArgs& a) {
+  const long long states = static_cast<long long>(a.n_seq) * a.n_heads, sms = device_sm_count();
+  if (static_cast<long long>(a.dim) * a.vdim * 4 < 256 * 1024) return false;
+  const bool many = 10 * states * ((a.vdim + 63) / 64) >= 27 * sms || 2 * states >= sms;
+  return many && (a.vdim >= 320 || states <= sms || (a.vdim >= 192 && 5 * states >= 7 * sms));
+}
+
 template <typename A>
 const char* dispatch(const MlstmArgs& a) {
   cudaError_t e;
-  // States of 256 KB and more, and two for every five SMs at least: below, the CTAs of a head's cluster read a state faster than one
-  // CTA does.  Step of the 1 B layer-list decoder, twelve layers of four heads of 256 x 512 (512 KB), us, clusters -> streamed:
-  // 12 sequences 1039 and 1089, 16 1157 -> 1110, 24 1359 -> 1232, 32 1570 -> 1359 (a layer 40 -> 23, 21 at the copy rate),
-  // 64 2072 -> 1846.
-  if (a.one_token && a.write_state && a.vdim <= kStreamCols && a.dim <= kStreamMaxDim &&
-      static_cast<long long>(a.dim) * a.vdim * 4 >= 256 * 1024 &&
-      5LL * a.n_seq * a.n_heads >= 2LL * device_sm_count() && (reinterpret_cast<uintptr_t>(a.S) & 15) == 0) {
+  if (a.one_token && a.write_state && a.vdim <= kStreamCols && a.dim <= kStreamMaxDim && stream_pays(a) &&
+      (reinterpret_cast<uintptr_t>(a.S) & 15) == 0) {
     e = launch_stream<A>(a);
     return e == cudaSuccess ? nullptr : cudaGetErrorString(e);
   }

@@ -331,9 +331,9 @@ def test_matrix_memory_step_of_many_states(ops, geo, dt, pdl):
     sequences at a time take: outputs and states bit for bit, ragged last chunks and column slices, slots in any order."""
     H, D, V = geo
     sms = torch.cuda.get_device_properties(0).multi_processor_count
-    B = (sms + H) // H + 2 if H == 4 else 2 * sms // (5 * H) + 1
-    assert D * V * 4 >= 256 * 1024 and 5 * B * H >= 2 * sms
-    few = max(1, 2 * sms // (5 * H) - 1)
+    B = (sms + H) // H + 2 if H == 4 else sms // (2 * H) + 1
+    few = max(1, sms // (4 * H))
+    assert D * V * 4 >= 256 * 1024 and 2 * B * H >= sms and 10 * few * H * 8 < 27 * sms
     torch.manual_seed(9)
     proj = torch.randn(B, H * (2 * D + 2 * V), device="cuda").to(dt)
     gates = torch.randn(B, 2 * H, device="cuda") * 3 + torch.tensor([0.0] * H + [2.0] * H, device="cuda")
@@ -361,7 +361,7 @@ def test_matrix_memory_steps_of_the_same_states(ops, B, portion):
     a kernel: the same bits.  60 states leave SMs free on which the next step's CTAs start at once."""
     H, D, V, steps = 4, 256, 512, 6
     sms = torch.cuda.get_device_properties(0).multi_processor_count
-    assert 5 * B * H >= 2 * sms
+    assert 10 * B * H * (V // 64) >= 27 * sms
     torch.manual_seed(B)
     ldp = H * (2 * D + 2 * V)
     proj = torch.randn(steps * B + portion * B, ldp, device="cuda").bfloat16()
