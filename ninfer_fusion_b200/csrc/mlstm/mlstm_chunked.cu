@@ -328,6 +328,9 @@ constexpr int kLdB = kBlock + 8;
 constexpr int kWalkers = 16 * 32, kWalkThreads = kWalkers + 32;
 constexpr int kAheadChunks = 3;                  // chunks whose rows are in shared memory or on their way
 constexpr size_t kWalkSmem = sizeof(bf16) * (2 * kAheadChunks + 2) * L * kLdB;
+// More than half of an SM's: a CTA has it to itself.  Three fit with what they need, and behind a kernel that fills the SMs the first
+// ones that it leaves take three each: a chain's chunk then takes 3 us for 1.7, with two thirds of the SMs empty.
+constexpr size_t kWalkAloneSmem = 116 * 1024;
 __global__ void __launch_bounds__(kWalkThreads) mlstm_walk_kernel(const MlstmArgs p, const ChunkWs w) {
   extern __shared__ __align__(16) bf16 smem_b[];
   __shared__ __align__(16) float wt[2][L];
@@ -869,9 +872,15 @@ const char* mlstm_chunked(const MlstmArgs& a, void* workspace, int64_t workspace
   const int state_blocks = ((a.dim + kBlock - 1) / kBlock) * ((a.vdim + kBlock - 1) / kBlock);
   if (3LL * state_blocks * a.n_heads >= 2LL * device_sm_count() &&
       (reinterpret_cast<uintptr_t>(a.S) | reinterpret_cast<uintptr_t>(a.n)) % 8 == 0) {
-    e = allow_smem(mlstm_walk_kernel, kWalkSmem);
+    // An SM for each CTA where there are enough.  Prompts of the 1 B layer-list decoder (128 CTAs a sequence; twelve layers), us, two
+    // kernels, walks that share SMs, walks by themselves: 200 tokens 2357, 2266, 2222; 1024 3624, 3768, 3593; 2048 5708, 5940, 5512.
+    // With more CTAs than SMs rounds of one a SM are slower than three side by side: three sequences of 2048 in all 5406, 5097, 5205,
+    // six 5409, 5106, 5264 (two of unlike lengths 5496, 5409, 5270).
+    const bool alone = static_cast<long long>(state_blocks) * a.n_heads * a.n_seq <= device_sm_count();
+    const size_t smem = alone ? kWalkAloneSmem : kWalkSmem;
+    e = allow_smem(mlstm_walk_kernel, kWalkAloneSmem);
     if (e == cudaSuccess)
-      e = launch_kernel(mlstm_walk_kernel, dim3(state_blocks, a.n_heads, a.n_seq), dim3(kWalkThreads), kWalkSmem, a.stream, a.pdl, 1, a, w);
+      e = launch_kernel(mlstm_walk_kernel, dim3(state_blocks, a.n_heads, a.n_seq), dim3(kWalkThreads), smem, a.stream, a.pdl, 1, a, w);
   } else {
     e = launch_contrib(a, w, nc);
     if (e != cudaSuccess) return cudaGetErrorString(e);
