@@ -1114,15 +1114,15 @@ __global__ void __launch_bounds__(kPersistThreads, 1) gemm_persist_kernel(const 
 // least estimated time.  `rows` output rows in tiles of 128 a CTA (64 beside SwiGLU) times the token tiles are dealt out in
 // rounds of one tile per walker; what a fixed 256 loses is the last round (N = 5120, T = 2048: 160 tiles of 74 pairs = 2.16
 // rounds, paid as 3; 192 tokens make it 2.97) or, with few tiles, the SMs that get none (N = 264: 16 tiles of 256 tokens
-// against 64 of 64).  One CTA a tile is left with short contractions in one round (us, one CTA and pair: 2048 x 512 9.3 and
-// 10.7, 2048 x 2048 16.9 and 17.9, 2048 tokens), and is not weighed up to 128 tokens, where pairs were the faster at every size
-// tried.
+// against 64 of 64).  One CTA a tile is left with short contractions (us, one CTA and pair: 2048 tokens 2048 x 512 9.3 and
+// 10.7, 2048 x 2048 16.9 and 17.9; 64 tokens 34816 x 128 6.1 and 9.2, 8.7 before there were pairs; 96 tokens 12288 x 512 7.6 and
+// 9.0; 128 tokens 12288 x 1024 10.1 and 13.1); from K = 2048 on pairs were the faster at every size tried up to 128 tokens.
 struct PersistPlan { int tn; bool pair; };
 PersistPlan pick_persist(int T, int rows, int num_kb, int sms, int epi) {
   PersistPlan best = {kPersistMaxTN, true};
   double best_ns = 0;
   const int cta_rows = epi == kEpiSwiglu ? 64 : kTileN;
-  for (int pair = 1; pair >= (T > 128 ? 0 : 1); --pair) {
+  for (int pair = 1; pair >= 0; --pair) {
     const int w_tiles = (rows + (cta_rows << pair) - 1) / (cta_rows << pair);
     for (int tn = kPersistMaxTN; tn >= (pair ? kPairMinTN : kPersistMinTN); tn -= 16) {
       const long long tiles = static_cast<long long>(w_tiles) * ((T + tn - 1) / tn);

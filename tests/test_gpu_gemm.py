@@ -179,7 +179,7 @@ def test_gemm_persistent_prefill_kernel(ops, status, T):
 
 
 @pytest.mark.parametrize("T", [33, 48, 64, 65, 97, 128, 200])
-@pytest.mark.parametrize("N,K", [(64, 1024), (128, 72), (130, 1096), (384, 4096), (20040, 512)])
+@pytest.mark.parametrize("N,K", [(64, 1024), (128, 72), (130, 1096), (384, 4096), (20040, 512), (20040, 2056)])
 def test_gemm_cta_pairs(ops, status, T, N, K):
     """Tiles of a pair of CTAs: weight rows that leave the second CTA without any, token halves that lie past the last token,
     more tiles than pairs, contractions shorter than the ring; nothing is written beside the output."""
