@@ -31,6 +31,17 @@ class SeqChunk:
     positions: object = None   # optional int [n, 3] rope positions (multimodal prefill); default = cache positions
 
 
+def _token_array(tokens):
+    """What numpy makes 32-bit ids of.  (A list of 2048 Python integers: 65 us through the array module, 87 by numpy's conversion,
+    which takes what else a list may hold.)"""
+    if type(tokens) is list:
+        try:
+            return array("i", tokens)
+        except (TypeError, OverflowError):
+            pass
+    return tokens
+
+
 class StepBuffers:
     def __init__(self, max_tokens: int, max_seqs: int, device, mrope: bool = False, attn_block_tokens: int = 16,
                  max_logit_rows: int = 0):
@@ -145,8 +156,7 @@ class StepBuffers:
         cu[0] = 0
         for b, c in enumerate(chunks):
             n = len(c.tokens)
-            # (a list of 2048 Python integers: 65 us through the array module, 87 by numpy's conversion)
-            ids[t:t + n] = array("i", c.tokens) if type(c.tokens) is list else c.tokens
+            ids[t:t + n] = _token_array(c.tokens)
             tseq[t:t + n] = b
             trow[t:t + n] = c.table_row
             pos = np.arange(c.start_pos, c.start_pos + n, dtype=np.int32)

@@ -25,6 +25,19 @@ def test_build_decode_is_build_of_one_token_chunks(B, deltas, mrope):
         bufs[1].build_decode([0] * 9, [0] * 9, [0] * 9, [0] * 9, [])
 
 
+@pytest.mark.parametrize("tokens", [[3, 1, 2], [3.0, 1.0, 2.0], [np.int64(3), np.float32(1), True], (3, 1, 2), np.array([3, 1, 2]),
+                                    np.array([3.0, 1.0, 2.0], dtype=np.float32)])
+def test_tokens_of_any_kind(tokens):
+    """Whatever numpy assigns to 32-bit integers is taken as token ids; what it refuses is refused."""
+    bufs = StepBuffers(8, 8, "cpu")
+    batch = bufs.build([SeqChunk(0, 0, 0, tokens, True)])
+    want = np.zeros(3, dtype=np.int32)
+    want[:] = tokens
+    assert batch.ids.tolist() == want.tolist()
+    with pytest.raises(OverflowError):
+        bufs.build([SeqChunk(0, 0, 0, [2 ** 31], True)])
+
+
 def test_every_upload_is_waited_for_before_the_buffer_is_written(monkeypatch):
     """An upload by itself (a speculative round that is captured) counts like the one of `build`: the buffer is not written
     before the event behind it."""
