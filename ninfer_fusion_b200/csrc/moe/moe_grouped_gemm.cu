@@ -38,7 +38,9 @@ constexpr int kTileN = 128;
 constexpr int kWTileBytes = kTileN * 128;
 
 constexpr int kMaxTN = 256;
-constexpr int kMaxStages = 12;
+// Stages of the ring: a pair's of 24 KB fill the room; of one CTA's eight are enough, and with twelve small ones the weights come
+// more slowly from memory (256 experts of 1024 x 2048, 16 rows each: 164 us, 155 with eight).
+constexpr int kMaxStages = 12, kSingleStages = 8;
 constexpr int kEpiWarps = 8;
 constexpr int kThreads = 64 + 32 * kEpiWarps;
 constexpr int kSmemBytes = 221 * 1024;   // (4.5 KB of static tables beside it)
@@ -66,13 +68,12 @@ struct MoeKernelParams {
   __nv_bfloat16* dense_out;
 };
 
-// Gated unit: the two CTAs of a cluster work on one item of twice the weight rows; each loads its own 128 rows and half of the
-// tokens (see gemm_bf16.cu).  256 experts of 1024 x 2048, 2048 tokens, top-8, 181 us either way, bound by the weights from HBM,
-// but the dense expert's tokens beside them cost 3 us so and 16 with one CTA an item, whose shared memory they fill.  The return
-// form has contractions of a few k-blocks, where handing an accumulator over between two CTAs shows (103 us, pairs 119).
-template <int EPI>
-constexpr bool kPair = EPI == kMoeEpiSwiglu;
-
+// Gated unit beside a dense expert (PAIR): the two CTAs of a cluster work on one item of twice the weight rows; each loads its own
+// 128 rows and half of the tokens (see gemm_bf16.cu).  256 experts of 1024 x 2048, 2048 tokens, top-8: the dense expert's tokens
+// beside them cost 3 us so and 16 with one CTA an item, whose shared memory they fill.  Without a dense expert the kernel is bound by
+// the weights from HBM and one CTA an item is the faster or the same (us, pairs and one CTA: 16 rows an expert 162 and 155, 64 rows
+// 179 and 177; 128 experts of 640 x 1024, whose third row tile leaves the second CTA idle, 33 and 31).  The return form has
+// contractions of a few k-blocks, where handing an accumulator over between two CTAs shows (103 us, pairs 119).
 // (token tile, row tile) of the walk
 struct MoeItem {
   bool dense;
@@ -84,7 +85,7 @@ __device__ __forceinline__ MoeItem moe_item(const MoeKernelParams& p, int item) 
   return {false, item / p.n_row_tiles, item % p.n_row_tiles};
 }
 
-template <int EPI>
+template <int EPI, bool PAIR>
 __global__ void __launch_bounds__(kThreads, 1) moe_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w,
                                                                const __grid_constant__ CUtensorMap tmap_x,
                                                                const __grid_constant__ CUtensorMap tmap_dense_w,
@@ -105,13 +106,12 @@ __global__ void __launch_bounds__(kThreads, 1) moe_gemm_kernel(const __grid_cons
   const int lane = threadIdx.x & 31;
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const int TN = p.tn;
-  constexpr bool PAIR = kPair<EPI>;
   const int crank = PAIR ? static_cast<int>(blockIdx.x & 1) : 0;
   const int walker = PAIR ? static_cast<int>(blockIdx.x >> 1) : static_cast<int>(blockIdx.x);
   const int walkers = PAIR ? static_cast<int>(gridDim.x >> 1) : static_cast<int>(gridDim.x);
   constexpr int kCtas = PAIR ? 2 : 1;
   const int stage_bytes = kWTileBytes + (p.dense_items > 0 ? max(TN, p.dense_tn) : TN) * 128 / kCtas;
-  const int n_stages = min(kMaxStages, kRingBytes / stage_bytes);
+  const int n_stages = min(PAIR ? kMaxStages : kSingleStages, kRingBytes / stage_bytes);
   const int half = p.rows_per_expert / 2;
   volatile int* abortp = &abort_flag;
 
@@ -380,17 +380,17 @@ __global__ void __launch_bounds__(kThreads, 1) moe_gemm_kernel(const __grid_cons
   }
 }
 
-template <int EPI>
+template <int EPI, bool PAIR>
 cudaError_t launch(const CUtensorMap& tw, const CUtensorMap& tx, const CUtensorMap& dw, const CUtensorMap& dx,
                    const MoeKernelParams& kp, long long max_items, cudaStream_t stream, bool pdl) {
-  auto kern = moe_gemm_kernel<EPI>;
+  auto kern = moe_gemm_kernel<EPI, PAIR>;
   static bool attr_set = false;
   if (!attr_set) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
     if (e != cudaSuccess) return e;
     attr_set = true;
   }
-  constexpr int kCtas = kPair<EPI> ? 2 : 1;
+  constexpr int kCtas = PAIR ? 2 : 1;
   const long long walkers = device_sm_count() / kCtas;
   const dim3 grid(static_cast<unsigned>(kCtas * (max_items < walkers ? max_items : walkers)));
   return launch_kernel(kern, grid, dim3(kThreads), kSmemBytes, stream, pdl, kCtas, tw, tx, dw, dx, kp);
@@ -457,11 +457,13 @@ const char* moe_gemm(const MoeGemmArgs& a) {
   kp.tile_expert = a.tile_expert; kp.tile_row0 = a.tile_row0; kp.tile_rows = a.tile_rows; kp.state = a.state;
   kp.status = a.status; kp.glu = a.glu;
   kp.tn = tn;
-  if (a.epi == kMoeEpiSwiglu) {
+  const bool swiglu = a.epi == kMoeEpiSwiglu, pair = swiglu && a.dense_w != nullptr;
+  const int ctas = pair ? 2 : 1;
+  if (swiglu) {
     if (a.rows_per_expert % 128) return "moe_gemm: SwiGLU needs expert rows in multiples of 128 (64 gate + 64 up per tile)";
     if (a.out == nullptr || (a.ldo & 1)) return "moe_gemm: no output";
     kp.out = static_cast<__nv_bfloat16*>(a.out); kp.ldo = a.ldo;
-    kp.n_row_tiles = static_cast<int>((a.rows_per_expert / 2 + 127) / 128);
+    kp.n_row_tiles = static_cast<int>((a.rows_per_expert / 2 + 64 * ctas - 1) / (64 * ctas));
   } else if (a.epi == kMoeEpiReturn) {
     if (a.rows_per_expert % 8) return "moe_gemm: expert rows must be a multiple of 8";
     if (a.world < 1 || a.world > kMoeMaxRanks || a.recv_meta == nullptr) return "moe_gemm: bad return set-up";
@@ -477,30 +479,30 @@ const char* moe_gemm(const MoeGemmArgs& a) {
   CUtensorMap tw, tx;
   if (!cached_tmap(&tw, a.w, static_cast<uint64_t>(a.n_local_experts) * a.rows_per_expert, a.K, a.ldw, 64))
     return "moe_gemm: weight tensor map rejected";
-  if (!cached_tmap(&tx, a.x, a.cap, a.K, a.ldx, a.epi == kMoeEpiSwiglu ? tn / 2 : tn)) return "moe_gemm: activation tensor map rejected";
+  if (!cached_tmap(&tx, a.x, a.cap, a.K, a.ldx, tn / ctas)) return "moe_gemm: activation tensor map rejected";
   CUtensorMap dw = tw, dx = tx;
   if (a.dense_w != nullptr) {
-    const bool swiglu = a.epi == kMoeEpiSwiglu;
     if (a.dense_x == nullptr || a.dense_out == nullptr || a.dense_T <= 0 || a.dense_K <= 0 || a.dense_K % 8 ||
         a.dense_rows <= 0 || a.dense_rows % (swiglu ? 128 : 8))
       return "moe_gemm: bad dense expert";
     if ((reinterpret_cast<uintptr_t>(a.dense_w) | reinterpret_cast<uintptr_t>(a.dense_x)) & 15 || reinterpret_cast<uintptr_t>(a.dense_out) & 3)
       return "moe_gemm: dense operands must be 16-byte aligned";
     // its own token tile: the routed one follows the few rows of an expert, and 128 tokens of a pair or 64 fit eight stages
-    const int few = static_cast<int>((a.dense_T + 15) / 16 * 16), wide = swiglu ? 128 : 64;
+    const int few = static_cast<int>((a.dense_T + 15) / 16 * 16), wide = 64 * ctas;
     kp.dense_tn = tn > wide ? tn : (few < wide ? (few > tn ? few : tn) : wide);
     kp.dense_T = static_cast<int>(a.dense_T);
     kp.dense_rows = static_cast<int>(a.dense_rows);
     kp.dense_num_kb = static_cast<int>((a.dense_K + kBlockK - 1) / kBlockK);
-    kp.dense_row_tiles = swiglu ? (kp.dense_rows / 2 + 127) / 128 : (kp.dense_rows + kTileN - 1) / kTileN;
+    kp.dense_row_tiles = swiglu ? (kp.dense_rows / 2 + 64 * ctas - 1) / (64 * ctas) : (kp.dense_rows + kTileN - 1) / kTileN;
     kp.dense_items = kp.dense_row_tiles * ((kp.dense_T + kp.dense_tn - 1) / kp.dense_tn);
     kp.dense_out = a.dense_out;
     if (!cached_tmap(&dw, a.dense_w, a.dense_rows, a.dense_K, a.dense_K, 64)) return "moe_gemm: dense weight tensor map rejected";
-    if (!cached_tmap(&dx, a.dense_x, a.dense_T, a.dense_K, a.dense_K, swiglu ? kp.dense_tn / 2 : kp.dense_tn)) return "moe_gemm: dense activation tensor map rejected";
+    if (!cached_tmap(&dx, a.dense_x, a.dense_T, a.dense_K, a.dense_K, kp.dense_tn / ctas)) return "moe_gemm: dense activation tensor map rejected";
   }
   const long long max_items = static_cast<long long>(a.max_tiles) * kp.n_row_tiles + kp.dense_items;
-  cudaError_t e = a.epi == kMoeEpiSwiglu ? launch<kMoeEpiSwiglu>(tw, tx, dw, dx, kp, max_items, a.stream, a.pdl)
-                                         : launch<kMoeEpiReturn>(tw, tx, dw, dx, kp, max_items, a.stream, a.pdl);
+  cudaError_t e = !swiglu ? launch<kMoeEpiReturn, false>(tw, tx, dw, dx, kp, max_items, a.stream, a.pdl)
+                  : pair  ? launch<kMoeEpiSwiglu, true>(tw, tx, dw, dx, kp, max_items, a.stream, a.pdl)
+                          : launch<kMoeEpiSwiglu, false>(tw, tx, dw, dx, kp, max_items, a.stream, a.pdl);
   return e == cudaSuccess ? nullptr : cudaGetErrorString(e);
 }
 
