@@ -388,8 +388,10 @@ __global__ void __launch_bounds__(kThreads, 2) paged_attn_fp4_kernel(const Paged
 // Returns cudaErrorNotSupported when the problem is outside this kernel (the caller takes the one of paged_attention_mma.cu).
 cudaError_t paged_attention_fp4_split(const PagedAttnParams& p, cudaStream_t stream, bool pdl) {
   const int G = p.n_q_heads / p.n_kv_heads;
-  // (a thread reads the sixteen scales of a row at once)
-  if (p.kv.format != kKvNvfp4 || p.head_dim != D || G > kRows || p.split_keys % kTileKeys ||
+  // A thread reads the sixteen scales of a row at once.  From splits of four tiles on: with one or two its start and end cost more than
+  // it gives (us, general kernel and this one: 6 heads over 1, splits of 128 keys, one sequence of 64 keys 6.0 and 6.5, 32 of 500 8.5 and
+  // 9.7, 32 of 1500 16.0 and 16.7; 24 over 4, one of 2048 9.1 and 9.3; splits of 256, one of 20000 30.7 -> 27.8, 8 of 4000 27.8 -> 24.6).
+  if (p.split_keys < 4 * kTileKeys || p.kv.format != kKvNvfp4 || p.head_dim != D || G > kRows || p.split_keys % kTileKeys ||
       reinterpret_cast<uintptr_t>(p.kv.k_scales) % 16)
     return cudaErrorNotSupported;
   static const cudaError_t attr =

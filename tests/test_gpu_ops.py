@@ -500,10 +500,10 @@ def test_prefill_attention_tile_edges(ops, status, name, fmt, group, hq, hkv, n,
 @pytest.mark.parametrize("P,window,tree", [(64, 0, False), (7, 0, True), (48, 100, False), (160, 300, False)])
 def test_nvfp4_decode_attention_of_aligned_scales(ops, hq, hkv, P, window, tree):
     """Row scales at a 16-byte boundary are read sixteen at once, by a kernel whose products and sums are those of the general
-    one, which takes scales at any address: the same bits, for any page size, released pages, windows, tree masks and lengths at
-    the edges of tiles and splits."""
+    one, which takes scales at any address (and splits of fewer than four tiles): the same bits, for any page size, released pages,
+    windows, tree masks and lengths at the edges of tiles and splits."""
     torch.manual_seed(P)
-    D, lens, split, ns = 256, [1, 63, 64, 65, 129, 700, 128, 511], 128, 6
+    D, lens, split, ns = 256, [1, 63, 64, 65, 257, 700, 256, 511], 256, 3
     B, pages = len(lens), (max(lens) + P - 1) // P
     table = torch.randperm(B * pages + 1)[: B * pages].int().view(B, pages).cuda()
     k, v, ks, vs = _planes(B * pages + 1, hkv, P, D, R.KV_NVFP4, 16)
