@@ -311,6 +311,37 @@ def test_gdn_step_of_many_states(ops, heads, pdl, ragged):
     assert not got[1][1].isnan().any() and not torch.equal(got[1][0], states)
 
 
+@pytest.mark.parametrize("heads", [(16, 48), (16, 32)])
+def test_gdn_step_of_many_states_quantises_its_rows(ops, status, heads):
+    """The streaming step's rows as the next product's nvfp4 operand: codes and scales of the general kernel (`commit` of ones), and
+    those of the quantiser over the step's output."""
+    torch.manual_seed(4)
+    (hk, hv), d = heads, 128
+    B = -(-13 * torch.cuda.get_device_properties(0).multi_processor_count // (2 * hv)) + 1
+    qk, vd = hk * d, hv * d
+    C = 2 * qk + vd
+    conv = torch.randn(B, C, device="cuda").to(torch.bfloat16)
+    proj = torch.randn(B, C + vd + 2 * hv, device="cuda").to(torch.bfloat16)
+    A_log, dt_bias = torch.rand(hv, device="cuda") * 2 - 1, torch.rand(hv, device="cuda") * 2 - 1.5
+    nw = (1 + 0.1 * torch.randn(d, device="cuda")).to(torch.bfloat16)
+    cu, slot = torch.arange(B + 1, device="cuda").int(), torch.randperm(B, device="cuda").int()
+    states = torch.randn(B, hv, d, d, device="cuda") * 0.2
+    size = int(ops.nvfp4_act_scale_bytes(B, vd))
+    got = []
+    for commit in (torch.ones(B, dtype=torch.uint8, device="cuda"), None):
+        out = torch.full((B, vd), float("nan"), dtype=torch.bfloat16, device="cuda")
+        codes, plane = torch.full((B, vd // 2), 255, dtype=torch.uint8, device="cuda"), torch.zeros(size, dtype=torch.uint8, device="cuda")
+        ops.gdn_recurrent(conv, 0, qk, 2 * qk, proj, C, C + vd, C + vd + hv, hk, hv, A_log, dt_bias, nw, 1e-6, cu, slot, states.clone(),
+                          True, out, True, None, commit, None, None, None, codes, plane, status.tensor)
+        got.append((out, codes, plane))
+    codes, plane = torch.empty_like(got[0][1]), torch.zeros_like(got[0][2])
+    ops.quant_act_nvfp4(got[0][0], codes, plane)
+    for a, b in zip(*got):
+        assert torch.equal(a, b)
+    assert torch.equal(got[1][1], codes) and torch.equal(got[1][2], plane)
+    status.check("streaming step")
+
+
 @pytest.mark.parametrize("T", [9, 200])
 def test_embed_rmsnorm(ops, T):
     torch.manual_seed(0)
