@@ -88,7 +88,7 @@ _ROUTES: Dict[Tuple[str, str], Tuple[str, Cap]] = {
     ("decode_attention", "fp8"): ("csrc/attention/paged_attention_tc.cu", Cap.TMA_TENSOR | Cap.TCGEN05_F8F6F4 | Cap.CVT_FP8),
     ("decode_attention", "bf16"): ("csrc/attention/paged_attention_mma.cu", Cap.MMA_SYNC_BF16 | Cap.PDL),
     ("decode_attention", "int8"): ("csrc/attention/paged_attention_mma.cu", Cap.MMA_SYNC_BF16 | Cap.PDL),
-    ("decode_attention", "nvfp4"): ("csrc/attention/paged_attention_fp4.cu", Cap.MMA_SYNC_BF16 | Cap.CVT_FP4 | Cap.CVT_FP8),
+    ("decode_attention", "nvfp4"): ("csrc/attention/paged_attention_fp4.cu, paged_attention_mma.cu", Cap.MMA_SYNC_BF16 | Cap.CVT_FP4 | Cap.CVT_FP8),
     ("decode_attention", "mixed"): ("csrc/attention/paged_attention_mma.cu", Cap.MMA_SYNC_BF16 | Cap.CVT_FP4 | Cap.CVT_FP8),
     ("prefill_attention", "*"): ("csrc/attention/paged_attention_prefill.cu", Cap.TCGEN05_F16 | Cap.CVT_FP8 | Cap.CVT_FP4 | Cap.PDL),
     ("gdn", "*"): ("csrc/gdn/gdn_recurrent.cu, gdn_chunked.cu", Cap.MMA_SYNC_BF16 | Cap.CLUSTER_DSMEM | Cap.PDL),

@@ -11,7 +11,7 @@
 // issue slots (6000 a tile of 64 keys, 50 %) and shared memory (1550 wavefronts a tile, 58 %); now 105, 3500 and 800, and the
 // latencies between two barriers with the sixteen warps that the registers admit.  Of these 40 us the conversion of a word of codes in one
 // statement gave 10, K past shared memory 10, one barrier per tile for four and the transposed products 15, the second product by
-// the V group alone, which waited for the other, 6.  32 sequences of 2600 keys 54 -> 42, one of 2048 keys 11.5 -> 10.2.
+// the V group alone, which waited for the other, 6.  32 sequences of 2600 keys 54 -> 42.
 // Warps 0..3: K, S and softmax of sixteen keys of a tile each; 4..7: V as fp16 into shared memory, page look-ups, O of 64 columns
 // each.  One barrier per tile: between two of them the probabilities of tile i, V of tile i, the scores of tile i + 1
 // and the product of P and V of tile i - 1 are made.

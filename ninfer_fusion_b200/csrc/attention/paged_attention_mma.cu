@@ -20,9 +20,9 @@
 // * groups of at most 8 query heads (kRows = 8) read only the eight rows of Q and P that exist;
 // * S is summed from two accumulators: one chain of sixteen dependent MMAs took longer than their operands.
 // 8 sequences of 26,000 keys, 24 heads in 4 groups: int8 220 -> 171 us at the same split, bf16 288 -> 243; one sequence of 2048
-// nvfp4 keys 19.5 -> 17.4.  nvfp4 pages and groups of up to eight heads are paged_attention_fp4.cu's.  (Its scheme, with every
-// format through shared memory: int8 158 -> 155 us, bf16 203 -> 224, whose conversions are few and whose raw rows fill the
-// registers; these stay here.)
+// nvfp4 keys 19.5 -> 17.4.  nvfp4 pages and groups of up to eight heads are paged_attention_fp4.cu's where splits have four tiles and
+// more.  (Its scheme, with every format through shared memory: int8 158 -> 155 us, bf16 203 -> 224, whose conversions are few and
+// whose raw rows fill the registers; these stay here.)
 // Splits cover absolute key ranges and tiles start at split boundaries, so the
 // reduction order for a query depends only on key positions.  Output partials
 // (m, l, un-normalised O) use the same layout as the SIMT kernel and are

@@ -37,9 +37,9 @@ constexpr int kWTileBytes = kTileN * 128;
 // grid of ~100 CTAs still keeps ~200 KB per SM in flight (the memory system needs ~30 MB in flight overall).
 template <int TN, bool DEEP = false>
 struct GemmCfg {
-  // TN = 256 (prefill): the main loop already runs at the tensor rate, so what matters is hiding the epilogue
-  // (9-24 us per tile against a 33 us main loop at K = 5120).  Two stages = 96 KB let two CTAs share an SM (and its
-  // 512 TMEM columns): one drains its accumulator while the other feeds the tensor core.  A grid that fits in one
+  // Plain epilogues above 32 tokens take the persistent kernel; TN = 128 and 256 serve the split, gathered and peer epilogues.
+  // TN = 256: the main loop runs at the tensor rate, so what matters is hiding the epilogue.  Two stages = 96 KB let two CTAs share
+  // an SM (and its 512 TMEM columns): one drains its accumulator while the other feeds the tensor core.  A grid that fits in one
   // wave keeps the four-stage pipeline (DEEP).
   static constexpr int kStages =
       DEEP ? (TN <= 32 ? 10 : (TN == 256 ? 4 : 8)) : (TN <= 32 ? 5 : (TN == 64 ? 4 : (TN == 128 ? 6 : 2)));
@@ -789,7 +789,10 @@ constexpr double pair_kblock_ns(int tn) {
   return tn >= 160 ? 264. + 1.18 * (tn - 160) : tn >= 128 ? 264. : 264. - 0.81 * (128 - tn);
 }
 constexpr double kPairStartNs = 1500.;    // cluster launch, its barriers and the farther commit
-constexpr double kPersistTailNs = 30.;   // per token of the last tile, whose epilogue nothing overlaps
+// Per token of the last tile, whose epilogue nothing overlaps.  (The epilogue alone takes 14 now.  That, or 20, is the better with
+// contractions up to K = 512, and for 12288 x 1024, 129 tokens, 10.0 us for 13.1; but 16480 x 5120, 1466 tokens, then takes wider
+// tiles in fewer rounds, 206 for 184, and 24576 x 4096, 1884 tokens, 296 for 274.)
+constexpr double kPersistTailNs = 30.;
 
 template <int EPI, bool PAIR>
 __global__ void __launch_bounds__(kPersistThreads, 1) gemm_persist_kernel(const __grid_constant__ CUtensorMap tmap_w,

@@ -13,9 +13,10 @@ namespace nfb {
 constexpr int kNvfp4SfTileBytes = 512;   // 128 rows x 4 scales
 
 // e2m1 code of v / s, to nearest, ties to even, for a bf16 v and an e4m3 s > 0.  The boundaries lie midway between the grid's
-// values; a boundary times s has six bits at most and v eight, so that v is on the boundary or 2^-9 of it away: comparing products
-// gives what comparing the quotient, rounded to fp32, gives, at a third of the instructions (quantiser, 2048 x 17408: 55 -> 33 us;
-// 256 x 5120: 6.9 -> 4.6).
+// values and have three significant bits at most, s has four, so that a boundary times s is exact and has seven; v has eight.  Two
+// different numbers of eight bits lie at least 2^-8 of the larger apart, far more than the rounding of a quotient to fp32: comparing
+// products gives what comparing that quotient gives, at a third of the instructions (quantiser, 2048 x 17408: 55 -> 33 us; 256 x 5120:
+// 6.9 -> 4.6).
 __device__ __forceinline__ uint32_t e2m1_code(float v, float s) {
   const float a = fabsf(v);
   // (as negations: a NaN takes the largest code)
