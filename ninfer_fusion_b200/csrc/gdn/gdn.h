@@ -74,6 +74,8 @@ struct GdnParams {
   uint8_t* q_sf = nullptr;
   int* status = nullptr;     // optional status word: where the streaming step reports a wait that ran out
 };
+// `pdl`: states, slots and sequence ranges are read before the kernel in front of this one is done, so that one must not write them
+// (seq_end passes wait for it first).
 const char* gdn_recurrent(const GdnParams& p, cudaStream_t stream, bool pdl);
 // Multi-token variant (token groups staged in shared memory); gdn_recurrent dispatches to it when T > n_seq.
 const char* gdn_prefill(const GdnParams& p, cudaStream_t stream, bool pdl);
